@@ -37,10 +37,11 @@ extern "C" {
 #define WB_ECANCELED -9   /* job was cancelled before it ran                 */
 #define WB_EIO -10        /* a file could not be written                    */
 
-/* Classify kernel shapes: one warp per group of up to 32 points of a grid
- * column (0-2) or one warp per point (3-7); warps per block / resident blocks
- * per SM (register cap): 0 = groups 4/5 (default), 1 = groups 8/3,
- * 2 = groups 8/2, 3 = 8/3, 4 = 4/6, 5 = 4/8, 6 = 8/4, 7 = 2/12. */
+/* Classify kernel shapes: one warp per group of up to 32 nearby points (0-2)
+ * or one warp per point (3-7); warps per block / resident blocks per SM
+ * (register cap): 0 = groups 4/6 (default), 1 = groups 4/5, 2 = groups 4/4,
+ * 3 = 8/3, 4 = 4/6, 5 = 4/8, 6 = 8/4, 7 = 2/12.  Calls that want decision
+ * margins run their own kernel whatever the shape. */
 #define WB_N_SHAPES 8
 
 typedef struct wb_ctx wb_ctx;

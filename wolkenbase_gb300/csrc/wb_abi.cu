@@ -32,7 +32,7 @@ int wb_fail(wb_ctx *c, int code, const std::string &msg)
 static bool coldBuffer(const wb_ctx *c, const DevBuf &b)
 {
   const DevBuf *cold[] = {&c->rec, &c->key0, &c->key1, &c->idx0, &c->idx1, &c->tmp32, &c->tmp32b,
-                          &c->gKey0, &c->gKey1, &c->gVal0, &c->gVal1, &c->tilePts, &c->survivorOf, &c->pointLeaf};
+                          &c->gVal0, &c->gVal1, &c->tilePts, &c->survivorOf, &c->pointLeaf};
   for (const DevBuf *x : cold)
     if (x == &b)
       return true;
@@ -125,7 +125,7 @@ void wb_release_buffers(wb_ctx *c)
                    &c->tileHuge, &c->hugePre, &c->scanTot, &c->tileFrm,
                    &c->tileH, &c->tileN, &c->tileNg, &c->label, &c->clsDev, &c->ambiguous, &c->deferred, &c->angleT,
                    &c->flowCache, &c->gKey0, &c->gKey1, &c->gVal0, &c->gVal1, &c->stray, &c->cellStart,
-                   &c->gpt, &c->cellRec, &c->superRec, &c->ptSetup, &c->groups, &c->groupCnt, &c->lasAngles,
+                   &c->gpt, &c->cellRec, &c->superRec, &c->ptSetup, &c->groups, &c->colGroups, &c->groupCnt, &c->lasAngles,
                    &c->marginBuf, &c->marginRec};
   for (DevBuf *b : all)
     wb_free_buf(c, *b);

@@ -599,6 +599,7 @@ int wb_build_impl(wb_ctx *c, const wb_cloud *cl)
   if (n == 0)
   {
     c->nd = c->n_leaves = c->n_nodes = 0;
+    c->grid = GridInfo{};   // no columns or groups of an earlier cloud
     c->stage = 1;
     return 0;
   }

@@ -9,26 +9,27 @@
  * function of the neighbour set alone: 1 (not ground) if it surrounds p, else 2.
  * The neighbour set is what OctStore::pointsIn returns for the hyperboloid.
  *
- * Two kernels walk the same neighbourhood.  The column-group kernel
- * (classifyGroup, the fast pass) gives one warp to up to 32 points of one
- * grid column and shares the walk between them; the one-point kernel
- * (classifyPoint) gives one warp to one point and serves the points a group
- * hands over, and the exact pass.  Both walk rings of grid columns outward
- * from the point, so directions from every side arrive early, and stop as soon
- * as the directions seen surround the point.  Per column they first check
- * whether the column's lowest point could be inside the hyperboloid at the
- * column's nearest distance.  Each candidate is tested in FP32 in a frame centred on p
- * (integer record differences times the scale); the few whose FP32 value lies
- * within 1e-5 of the boundary, and points outside the octree root cube (which
- * the reference treats through their leaf's cube), are tested exactly in
- * FP64 as the reference computes it.  Directions are FP32 arctangents
+ * The fast pass (wb_classify_group.cuh) gives one warp to a group of up to 32
+ * nearby points and decides nearly all of them with FP32 tests and the open
+ * arcs of each point's directions; the points of groups whose neighbourhood is
+ * very large go to a kernel with one warp per point.  What FP32 leaves in doubt
+ * (membership within 1e-5 of the boundary, points outside the octree root cube,
+ * which the reference treats through their leaf's cube) is tested exactly in
+ * FP64 as the reference computes it, and a point whose widest gap ends within
+ * the direction error of 144 degrees is re-run by the exact kernel with the
+ * reference's own integer atan2i (angle.cpp:117-155).
+ *
+ * The kernels of this file keep direction extremes in bins instead, which forms
+ * every largest gap: classifyPoint (one warp per point, 64 bins) for the exact
+ * re-run, and with classifyGroup (one warp per up to 32 points of a grid
+ * column, 8 bins of 45 degrees a lane) for the margins of wb_classify_ex.  They
+ * walk rings of grid columns outward from the point; per column they first
+ * check whether the column's lowest point could be inside the hyperboloid at
+ * the column's nearest distance.  Directions are FP32 arctangents
  * (wb_dir_units_f32, error below 1000 units) in the reference's integer angle
- * unit; bins (64 in the one-point kernel, 8 per lane in the group kernel) keep
- * their extremes, and the largest circular gap follows from them.  With the direction error bounded by kMargin units, a
- * gap estimate below 144 degrees - 2*kMargin proves "surrounded" and one
- * above 144 degrees + 2*kMargin proves the opposite;
- * anything between is re-run by the exact kernel with the reference's own
- * integer atan2i (angle.cpp:117-155) and exact bins.
+ * unit.  With the direction error bounded by kMargin units, a gap estimate below
+ * 144 degrees - 2*kMargin proves "surrounded" and one above 144 degrees +
+ * 2*kMargin proves the opposite.
  *
  * A point is classified with the hyperboloid size of its owner tile, the last
  * tile in flowsnake order whose cylinder contains it, because that tile's
@@ -39,6 +40,7 @@
 #include <cmath>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <string>
 #include <vector>
 #include "wb_internal.h"
@@ -51,12 +53,11 @@
  * tested, 4 candidates read, 5 candidates inside, 6 surround tests,
  * 7 columns scanned; SM clock cycles 8 near field, 9 far field, 10 final
  * gap, 11 whole point, 12 inside column scans, 13 inside surround tests.
- * Row 0 is the column-group kernel: 0 groups, 1 columns read, 2 candidates
- * kept, 3 kept x undecided lanes, 4 active lanes, 5 lanes handed over,
- * 6 cycles, 7 super-cell rings, 8 lanes ending ground; 9-11 cycles, count
- * and kept candidates of the groups that kept more than 1000; cycles 12 in
- * column reads, 13 forming the envelope again, 14 candidate tests, 15
- * surround tests. */
+ * Row 0 is the point-group kernel: 0 groups, 1 groups read, 2 octets tested,
+ * 3 groups taken from the list, 4 super-cells, 5 super-cell rings, 6 candidates
+ * tested, 7 those times the undecided lanes, 8 cycles in the candidate tests,
+ * 10 rounds of direction updates, 11 cycles, 12 lanes handed over, 15 lanes
+ * ending ground. */
 #ifdef WB_CLASSIFY_STATS
 __device__ unsigned long long gClassifyStats[3][16];
 extern "C" int wb_classify_stats(unsigned long long *out, int reset)
@@ -125,7 +126,12 @@ struct ClsArgs
   uint64_t ncell;
   const int4 *col;     /* two int4 per column: {x0, y0, x1, y1}, {zmin, begin, end, flags} */
   const int4 *gpt;     /* int4 {X, Y, Z, position | stray bit} per point, column order */
-  const uint2 *groups; /* column groups: {column, first point} */
+  const int4 *groups;     /* point groups, two int4 each (groupBoxKernel) */
+  const int2 *bxy, *bzw;  /* their points: {X, Y} and {Z, store position | stray bit} */
+  const unsigned long long *groupsTaken;   /* their number, above the low 36 bits */
+  const uint2 *colGroups; /* column groups {column, first point}, when margins are wanted */
+  float gky, gkz;         /* y record unit / x record unit; z record unit / (slope * x record unit) */
+  float gInv, gTiny;      /* 1 / (slope * x record unit); 1e-12 m^2 in that unit squared */
   int snx, sny;
   const int4 *super;   /* super-cell records, the column layout */
   double zmin;
@@ -1416,6 +1422,8 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
     }
   }
 }
+
+#include "wb_classify_group.cuh"
 }  // namespace
 
 /* Decoding is strictly increasing in every record integer when the step
@@ -1493,6 +1501,8 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
   a.sinT = tab + 511;
   a.cosT = tab + 1023;
   a.label = (uint8_t *)c->label.p;
+  if ((rc = wb_point_groups(c, &a.groupsTaken)))
+    return rc;
   a.gx0 = c->grid.x0;
   a.gy0 = c->grid.y0;
   a.cell = c->grid.cell;
@@ -1505,7 +1515,11 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
   a.ncell = c->grid.ncell;
   a.col = (const int4 *)c->cellRec.p;
   a.gpt = (const int4 *)c->gpt.p;
-  a.groups = (const uint2 *)c->groups.p;
+  a.groups = (const int4 *)c->groups.p;
+  a.bxy = (const int2 *)c->gKey0.p;
+  a.bzw = (const int2 *)c->gKey1.p;
+  a.colGroups = nullptr;
+  c->n_col_groups = 0;
   a.snx = c->grid.snx;
   a.sny = c->grid.sny;
   a.super = (const int4 *)c->superRec.p;
@@ -1519,6 +1533,11 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
   a.fsy = (float)(g.scale[1] * g.unit);
   a.fsz = (float)(g.scale[2] * g.unit);
   a.fs2 = (float)(p->max_slope * p->max_slope);
+  const double gunit = p->max_slope * (g.scale[0] * g.unit);
+  a.gky = (float)(g.scale[1] / g.scale[0]);
+  a.gkz = (float)(g.scale[2] * g.unit / gunit);
+  a.gInv = (float)(1.0 / gunit);
+  a.gTiny = (float)(1e-12 / gunit / gunit);
   a.setup = (PtSetup *)c->ptSetup.p;
   a.ambList = (uint32_t *)c->ambiguous.p;
   a.ambCount = (uint32_t *)((char *)c->small.p + 448);
@@ -1536,6 +1555,8 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
     if ((rc = wb_ensure(c, c->marginBuf, nd * 4 + 64)))
       return rc;
     a.margin = (float *)c->marginBuf.p;
+    if ((rc = wb_column_groups(c, &a.colGroups, &c->n_col_groups)))
+      return rc;
     if (onDevice)
       a.marginOut = c->marginDst;
     else
@@ -1602,13 +1623,14 @@ __global__ void batchSetup(const BatchHdr *__restrict__ h)
   }
 }
 
-/* MODE 0: every point of every job; 1: the points column groups deferred;
- * 2: the ambiguous points (exact pass). */
-template <int MODE, int W, int MINB>
+/* MODE 0: every point of every job; 1: the points the groups deferred; 2: the
+ * ambiguous points (exactly; in the precision mode again in FP32, by the bins'
+ * extremes).  ARCS: by open arcs, else by bins, which form every largest gap. */
+template <int MODE, bool ARCS, int W, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const BatchOut *o)
 {
-  constexpr bool EXACT = MODE == 2;
-  __shared__ uint32_t bmin[W][kBins], bmax[W][kBins];
+  __shared__ uint32_t bmin[W][ARCS ? 1 : kBins], bmax[W][ARCS ? 1 : kBins];
+  __shared__ PointShared psm[W];
   __shared__ ClsArgs sa[W];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = h->k;
@@ -1641,18 +1663,24 @@ __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const Ba
       }
       const ClsArgs &a = sa[w];
       uint64_t item = g - lo;
-      classifyPoint<EXACT>(a, MODE == 2 ? a.ambList[item] : (MODE == 1 ? a.deferList[item] : item), lane, bmin[w],
-                           bmax[w]);
+      const uint64_t j = MODE == 2 ? a.ambList[item] : (MODE == 1 ? a.deferList[item] : item);
+      if constexpr (ARCS)
+        classifyPointArcs(a, j, lane, psm[w]);
+      else if (MODE == 2 && !a.fp32Only)
+        classifyPoint<true>(a, j, lane, bmin[w], bmax[w]);
+      else
+        classifyPoint<false>(a, j, lane, bmin[w], bmax[w]);
     }
   }
 }
 
-/* The fast pass by column groups: warps take chunks of groups (of all jobs)
- * from a global counter. */
-template <int W, int MINB>
+/* The fast pass by point groups (ARCS) or, when decision margins are wanted,
+ * by column groups, which form every largest gap: warps take chunks of groups
+ * (of all jobs) from a global counter. */
+template <bool ARCS, int W, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB) batchGroups(BatchHdr *h, const BatchOut *o)
 {
-  __shared__ GroupSmem gsm[W];
+  __shared__ typename std::conditional<ARCS, GroupShared, GroupSmem>::type gsm[W];
   __shared__ ClsArgs sa[W];
   (void)o;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1684,9 +1712,37 @@ __global__ void __launch_bounds__(32 * W, MINB) batchGroups(BatchHdr *h, const B
           dst[i] = src[i];
         __syncwarp();
       }
-      classifyGroup(sa[w], sa[w].groups[g - lo], lane, gsm[w]);
+      if constexpr (ARCS)
+        classifyGroupArcs(sa[w], g - lo, lane, gsm[w]);
+      else
+        classifyGroup(sa[w], sa[w].colGroups[g - lo], lane, gsm[w]);
     }
   }
+}
+
+/* Where each job's point groups start in the batch, from the numbers the
+ * grouping left on the device (column groups are counted on the host). */
+__global__ void __launch_bounds__(WB_BATCH_MAX) batchGroupStarts(BatchHdr *h)
+{
+  __shared__ unsigned warpSum[WB_BATCH_MAX / 32];
+  const int t = threadIdx.x, lane = t & 31;
+  if (h->startGrp[h->k])
+    return;   // column groups
+  unsigned v = t < h->k ? (unsigned)(*h->jobs[t].groupsTaken >> 36) : 0u;
+  for (int o = 1; o < 32; o <<= 1)
+  {
+    const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o)
+      v += u;
+  }
+  if (lane == 31)
+    warpSum[t >> 5] = v;
+  __syncthreads();
+  uint64_t before = 0;
+  for (int w = 0; w < t >> 5; w++)
+    before += warpSum[w];
+  if (t < h->k)
+    h->startGrp[t + 1] = before + v;
 }
 
 /* Prefix of the jobs' deferred (which = 0) or ambiguous (which = 1) counts. */
@@ -1778,11 +1834,11 @@ struct WbBatch
   cudaStream_t capture = nullptr;
   BatchHdr *dIn = nullptr, *hIn = nullptr;
   BatchOut *dOut = nullptr, *hOut = nullptr;
-  int per[WB_N_SHAPES + 2] = {0};   /* resident blocks per SM of each classify kernel */
+  int per[WB_N_SHAPES + 4] = {0};   /* resident blocks per SM of each classify kernel */
   cudaGraphExec_t graphs[WB_N_SHAPES] = {nullptr};
 };
 
-const WbShape kWbShapes[WB_N_SHAPES] = {{8, 3}, {4, 5}, {8, 2}, {8, 3}, {4, 6}, {4, 8}, {8, 4}, {2, 12}};
+const WbShape kWbShapes[WB_N_SHAPES] = {{4, 6}, {4, 5}, {4, 4}, {8, 3}, {4, 6}, {4, 8}, {8, 4}, {2, 12}};
 
 namespace
 {
@@ -1791,7 +1847,8 @@ typedef void (*RingsFn)(BatchHdr *, const BatchOut *);
 /* Kernels of the fused classify: 0..WB_N_SHAPES-1 the fast pass of each
  * shape (one point per warp, or column groups), kDeferred the one-point pass
  * over the points column groups handed over, kExactPass the exact pass. */
-constexpr int kDeferred = WB_N_SHAPES, kExactPass = WB_N_SHAPES + 1;
+constexpr int kDeferred = WB_N_SHAPES, kExactPass = WB_N_SHAPES + 1, kMarginGroups = WB_N_SHAPES + 2,
+              kMarginDeferred = WB_N_SHAPES + 3;
 
 RingsFn ringsFn(int idx)
 {
@@ -1799,22 +1856,30 @@ RingsFn ringsFn(int idx)
   // thread); 3-7: one point per warp (about 85, 85, 64, 64 and 85)
   switch (idx)
   {
-  case 1: return batchGroups<4, 5>;
-  case 2: return batchGroups<8, 2>;
-  case 3: return batchRings<0, 8, 3>;
-  case 4: return batchRings<0, 4, 6>;
-  case 5: return batchRings<0, 4, 8>;
-  case 6: return batchRings<0, 8, 4>;
-  case 7: return batchRings<0, 2, 12>;
-  case kDeferred: return batchRings<1, 8, 3>;
-  case kExactPass: return batchRings<2, 4, 6>;
-  default: return batchGroups<8, 3>;
+  case 1: return batchGroups<true, 4, 5>;
+  case 2: return batchGroups<true, 4, 4>;
+  case 3: return batchRings<0, true, 8, 3>;
+  case 4: return batchRings<0, true, 4, 6>;
+  case 5: return batchRings<0, true, 4, 8>;
+  case 6: return batchRings<0, true, 8, 4>;
+  case 7: return batchRings<0, true, 2, 12>;
+  case kDeferred: return batchRings<1, true, 4, 8>;
+  case kExactPass: return batchRings<2, false, 4, 6>;
+  case kMarginDeferred: return batchRings<1, false, 8, 3>;
+  case kMarginGroups: return batchGroups<false, 8, 3>;
+  default: return batchGroups<true, 4, 6>;
   }
 }
 
 int ringsWarps(int idx)
 {
-  return idx == kExactPass ? 4 : (idx == kDeferred ? 8 : kWbShapes[idx].warps);
+  return idx == kExactPass || idx == kDeferred ? 4 : (idx == kMarginDeferred || idx == kMarginGroups ? 8 : kWbShapes[idx].warps);
+}
+
+/* The one-point pass that goes with a fast pass. */
+int deferredOf(int shape)
+{
+  return shape == kMarginGroups ? kMarginDeferred : kDeferred;
 }
 
 __global__ void batchAmbReset(const BatchHdr *__restrict__ h)
@@ -1846,17 +1911,18 @@ cudaError_t ringsGrid(WbBatch *b, int shape, unsigned *grid)
 /* The fused classify on stream s: upload of the job table, set-up, the
  * persistent fast pass, the deferred prefix and one-point pass, the ambiguous
  * prefix and exact pass, ground counts (per tile and per job), the
- * class-byte scatter and the read-back of the per-job totals (9 kernels).  With mark, stage events go on mark's stream. */
+ * class-byte scatter and the read-back of the per-job totals (10 kernels).  With mark, stage events go on mark's stream. */
 cudaError_t enqueueBatch(WbBatch *b, cudaStream_t s, int shape, const unsigned grids[3], wb_ctx *mark)
 {
   const unsigned grid = (unsigned)b->sm * 8;
   cudaError_t e = cudaMemcpyAsync(b->dIn, b->hIn, sizeof(BatchHdr), cudaMemcpyDefault, s);
   if (e != cudaSuccess)
     return e;
+  batchGroupStarts<<<1, WB_BATCH_MAX, 0, s>>>(b->dIn);
   batchSetup<<<grid, 256, 0, s>>>(b->dIn);
   ringsFn(shape)<<<grids[0], 32 * ringsWarps(shape), 0, s>>>(b->dIn, b->dOut);
   batchPrefix<<<1, 32, 0, s>>>(b->dIn, b->dOut, 0);
-  ringsFn(kDeferred)<<<grids[1], 32 * ringsWarps(kDeferred), 0, s>>>(b->dIn, b->dOut);
+  ringsFn(deferredOf(shape))<<<grids[1], 32 * ringsWarps(deferredOf(shape)), 0, s>>>(b->dIn, b->dOut);
   if (mark)
     wb_mark(mark, "classify");
   batchPrefix<<<1, 32, 0, s>>>(b->dIn, b->dOut, 1);
@@ -1877,7 +1943,7 @@ cudaError_t batchGrids(WbBatch *b, int shape, unsigned grids[3])
 {
   cudaError_t e = ringsGrid(b, shape, &grids[0]);
   if (e == cudaSuccess)
-    e = ringsGrid(b, kDeferred, &grids[1]);
+    e = ringsGrid(b, deferredOf(shape), &grids[1]);
   if (e == cudaSuccess)
     e = ringsGrid(b, kExactPass, &grids[2]);
   return e;
@@ -1904,9 +1970,8 @@ cudaError_t captureBatch(WbBatch *b, int shape, cudaGraphExec_t *exec)
   return e;
 }
 
-/* Fills the pinned job table from the staged contexts; with sample > 0 the
- * point ranges are cut after the first `sample` points. */
-int fillTable(WbBatch *b, wb_ctx *const *jobs, int k, int chunk, uint64_t sample, std::string &err)
+/* Fills the pinned job table from the staged contexts. */
+int fillTable(WbBatch *b, wb_ctx *const *jobs, int k, int chunk, std::string &err)
 {
   if (k < 1 || k > WB_BATCH_MAX)
   {
@@ -1927,16 +1992,10 @@ int fillTable(WbBatch *b, wb_ctx *const *jobs, int k, int chunk, uint64_t sample
       return WB_ESTATE;
     }
     memcpy(&h->jobs[q], c->clsArgs, sizeof(ClsArgs));
-    uint64_t nd = c->nd;
-    if (sample && h->startNd[q] + nd > sample)
-      nd = sample > h->startNd[q] ? sample - h->startNd[q] : 0;
-    h->startNd[q + 1] = h->startNd[q] + nd;
+    h->startNd[q + 1] = h->startNd[q] + c->nd;
     h->startN[q + 1] = h->startN[q] + c->n;
     h->startT[q + 1] = h->startT[q] + c->n_tiles;
-    uint64_t ng = c->grid.nGroups;
-    if (sample && c->nd)
-      ng = (uint64_t)((double)ng * (double)(h->startNd[q + 1] - h->startNd[q]) / (double)c->nd + 0.999);
-    h->startGrp[q + 1] = h->startGrp[q] + ng;
+    h->startGrp[q + 1] = h->startGrp[q] + c->n_col_groups;   // point groups: batchGroupStarts
   }
   return 0;
 }
@@ -2005,11 +2064,11 @@ int wb_classify_stage(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDevice)
   return 0;
 }
 
-int wb_batch_time(WbBatch *b, wb_ctx *const *jobs, int k, uint64_t sample, int shape, int chunk, cudaStream_t s,
+int wb_batch_time(WbBatch *b, wb_ctx *const *jobs, int k, int shape, int chunk, cudaStream_t s,
                   float *ms, std::string &err)
 {
   shape = clampShape(shape);
-  int rc = fillTable(b, jobs, k, chunk, sample, err);
+  int rc = fillTable(b, jobs, k, chunk, err);
   if (rc)
     return rc;
   WbDeviceGuard deviceGuard(b->device);
@@ -2024,11 +2083,12 @@ int wb_batch_time(WbBatch *b, wb_ctx *const *jobs, int k, uint64_t sample, int s
     e = cudaMemcpyAsync(b->dIn, b->hIn, sizeof(BatchHdr), cudaMemcpyDefault, s);
   if (e == cudaSuccess)
   {
+    batchGroupStarts<<<1, WB_BATCH_MAX, 0, s>>>(b->dIn);
     batchSetup<<<(unsigned)b->sm * 8, 256, 0, s>>>(b->dIn);
     cudaEventRecord(e0, s);
     ringsFn(shape)<<<grids[0], 32 * ringsWarps(shape), 0, s>>>(b->dIn, b->dOut);
     batchPrefix<<<1, 32, 0, s>>>(b->dIn, b->dOut, 0);
-    ringsFn(kDeferred)<<<grids[1], 32 * ringsWarps(kDeferred), 0, s>>>(b->dIn, b->dOut);
+    ringsFn(deferredOf(shape))<<<grids[1], 32 * ringsWarps(deferredOf(shape)), 0, s>>>(b->dIn, b->dOut);
     cudaEventRecord(e1, s);
     batchAmbReset<<<1, 256, 0, s>>>(b->dIn);
     e = cudaGetLastError();
@@ -2053,7 +2113,7 @@ int wb_batch_launch(WbBatch *b, wb_ctx *const *jobs, int k, cudaStream_t s, int 
                     uint64_t *launches, std::string &err)
 {
   shape = clampShape(shape);
-  int rc = fillTable(b, jobs, k, chunk, 0, err);
+  int rc = fillTable(b, jobs, k, chunk, err);
   if (rc)
     return rc;
   WbDeviceGuard deviceGuard(b->device);
@@ -2082,7 +2142,7 @@ int wb_batch_launch(WbBatch *b, wb_ctx *const *jobs, int k, cudaStream_t s, int 
     return WB_ECUDA;
   }
   if (launches)
-    *launches += 9;   /* kernel nodes of the graph */
+    *launches += 10;   /* kernel nodes of the graph */
   return 0;
 }
 
@@ -2091,7 +2151,8 @@ void wb_batch_collect(WbBatch *b, wb_ctx *const *jobs, int k)
   for (int q = 0; q < k; q++)
   {
     wb_ctx *c = jobs[q];
-    c->n_ambiguous = b->hOut->startAmb[q + 1] - b->hOut->startAmb[q];
+    // in the precision mode the list holds points run again in FP32
+    c->n_ambiguous = ((const ClsArgs *)c->clsArgs)->fp32Only ? 0 : b->hOut->startAmb[q + 1] - b->hOut->startAmb[q];
     c->n_ground = b->hOut->ground[q];
     c->clsFinal = ((const ClsArgs *)c->clsArgs)->cls;
     c->clsStaged = false;
@@ -2113,12 +2174,14 @@ int wb_classify_impl(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDevice)
     return wb_fail(c, rc, err);
   WbBatch *b = c->batch;
   int shape = clampShape(c->shape);
-  if ((rc = fillTable(b, &c, 1, c->chunk, 0, err)))
+  if (c->marginDst)
+    shape = kMarginGroups;
+  if ((rc = fillTable(b, &c, 1, c->chunk, err)))
     return wb_fail(c, rc, "wb_classify: " + err);
   unsigned grids[3];
   WB_CUDA(c, batchGrids(b, shape, grids));
   WB_CUDA(c, enqueueBatch(b, c->stream, shape, grids, c));
-  c->launches += 9;
+  c->launches += 10;
   ClsArgs *a = (ClsArgs *)c->clsArgs;
   if (!onDevice && c->n)
     WB_CUDA(c, cudaMemcpyAsync(cls, a->cls, c->n, cudaMemcpyDefault, c->stream));
@@ -2148,7 +2211,7 @@ int wb_autotune_jobs(WbBatch *b, const WbTuneJob *jobs, int k, cudaStream_t s, i
     for (int r = 0; r < 2; r++)
     {
       float ms = 0;
-      if (rc == 0 && (rc = wb_batch_time(b, ctxs.data(), k, 0, sh, ch, s, &ms, err)) == 0)
+      if (rc == 0 && (rc = wb_batch_time(b, ctxs.data(), k, sh, ch, s, &ms, err)) == 0)
         best = std::min(best, ms);
     }
     return best;

@@ -225,7 +225,7 @@ __global__ void cellFillKernel(uint64_t ncell, const uint32_t *__restrict__ star
   }
 }
 
-/* Column groups (the classify work items): a column of n points is
+/* Column groups (the work items of the margin pass): a column of n points is
  * ceil(n / 32) groups of consecutive points. */
 __global__ void groupCountKernel(uint64_t ncell, const int4 *__restrict__ rec, uint32_t *__restrict__ cnt)
 {
@@ -248,9 +248,178 @@ __global__ void groupFillKernel(uint64_t ncell, const int4 *__restrict__ rec, co
   }
 }
 
-/* Record-integer extent of the cloud: out[0..2] minima, out[3..5] maxima. */
+/* Position of cell (x, y) of an 8 x 8 block along a Hilbert curve. */
+__device__ __forceinline__ int hilbert8(int x, int y)
+{
+  int d = 0;
+#pragma unroll
+  for (int s = 4; s; s >>= 1)
+  {
+    const int rx = (x & s) != 0, ry = (y & s) != 0;
+    d += s * s * ((3 * rx) ^ ry);
+    if (!ry)
+    {
+      if (rx)
+      {
+        x = 7 - x;
+        y = 7 - y;
+      }
+      const int t = x;
+      x = y;
+      y = t;
+    }
+  }
+  return d;
+}
+
+/* The point groups of classify: the points of each super-cell in an order
+ * whose runs of 32 are compact (and whose runs of 8 are still more so), and the
+ * runs.  Points near their column's lowest (mostly ground) follow a Hilbert
+ * curve over an 8 x 8 division of the super-cell; points more than a column's
+ * width above it (roofs, walls, trees) come after them by height, so that they
+ * do not stretch the ground groups.  One warp per super-cell: a histogram of
+ * the points' buckets, its prefix, and a scatter; the warps take their places
+ * in the two lists from one counter (points in the low 36 bits, groups above).
+ * A super-cell's groups are consecutive: its record gets the first one and
+ * their number. */
+constexpr int kOrderWarps = 8, kOrderBuckets = 96;
+__global__ void __launch_bounds__(32 * kOrderWarps) groupOrderKernel(int nx, int ny, int snx, int sny, float colUnits,
+                                                                     const int4 *__restrict__ rec,
+                                                                     int4 *__restrict__ srec,
+                                                                     const int4 *__restrict__ gpt,
+                                                                     int2 *__restrict__ bxy, int2 *__restrict__ bzw,
+                                                                     int4 *__restrict__ groups,
+                                                                     unsigned long long *__restrict__ taken)
+{
+  __shared__ uint32_t hist[kOrderWarps][kOrderBuckets];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint64_t s = (uint64_t)blockIdx.x * kOrderWarps + w;
+  if (s >= (uint64_t)snx * sny)
+    return;
+  const int si = (int)(s % snx), sj = (int)(s / snx);
+  const int4 box = srec[2 * s];
+  if (box.x == INT32_MAX)
+    return;
+  uint32_t *h = hist[w];
+  for (int b = lane; b < kOrderBuckets; b += 32)
+    h[b] = 0;
+  __syncwarp();
+  const int i0 = si * WB_SUPER, ni = min(WB_SUPER, nx - i0);
+  const float fx = 8.f / ((float)((int64_t)box.z - box.x) + 1.f), fy = 8.f / ((float)((int64_t)box.w - box.y) + 1.f);
+  const float perCol = 1.f / colUnits;
+  // the super-cell's points, column row by column row: f(point, bucket)
+  auto forPoints = [&](auto f) {
+    for (int r = 0; r < WB_SUPER && sj * WB_SUPER + r < ny; r++)
+    {
+      const uint64_t c0 = (uint64_t)(sj * WB_SUPER + r) * nx + i0;
+      for (int q = 0; q < ni; q++)
+      {
+        const int4 r1 = rec[2 * (c0 + q) + 1];
+        for (uint32_t t = (uint32_t)r1.y + lane; t < (uint32_t)r1.z; t += 32)
+        {
+          const int4 p = gpt[t];
+          const float up = (float)((int64_t)p.z - r1.x) * perCol;   // column widths above the column's lowest point
+          int b;
+          if (up > 1.f)
+            b = 64 + (int)fminf(up - 1.f, 31.f);
+          else
+            b = hilbert8(min(7, (int)((float)((int64_t)p.x - box.x) * fx)), min(7, (int)((float)((int64_t)p.y - box.y) * fy)));
+          f(p, b);
+        }
+      }
+    }
+  };
+  forPoints([&](const int4 &, int b) { atomicAdd(&h[b], 1u); });
+  __syncwarp();
+  // exclusive prefix over the buckets, three per lane; points of the first 64
+  uint32_t c[3], sum = 0;
+  for (int q = 0; q < 3; q++)
+  {
+    c[q] = h[lane * 3 + q];
+    sum += c[q];
+  }
+  uint32_t inc = sum;
+  for (int o = 1; o < 32; o <<= 1)
+  {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o)
+      inc += v;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+  uint32_t run = inc - sum, low = 0;
+  __syncwarp();
+  for (int q = 0; q < 3; q++)
+  {
+    h[lane * 3 + q] = run;
+    if (lane * 3 + q < 64)
+      low += c[q];
+    run += c[q];
+  }
+  low = __reduce_add_sync(0xffffffffu, low);
+  const uint32_t gLow = (low + 31) / 32, gAll = gLow + (total - low + 31) / 32;
+  unsigned long long at = 0;
+  if (lane == 0)
+    at = atomicAdd(taken, ((unsigned long long)gAll << 36) | total);
+  at = __shfl_sync(0xffffffffu, at, 0);
+  const uint32_t base = (uint32_t)(at & ((1ull << 36) - 1)), g0 = (uint32_t)(at >> 36);
+  // first point, points and super-cell of each group; groupBoxKernel adds the bounds
+  for (uint32_t k = lane; k < gAll; k += 32)
+    groups[2 * (uint64_t)(g0 + k) + 1] =
+        k < gLow ? make_int4(0, (int)(base + 32 * k), (int)min(32u, low - 32 * k), 0)
+                 : make_int4(0, (int)(base + low + 32 * (k - gLow)), (int)min(32u, total - low - 32 * (k - gLow)), 0);
+  if (lane == 0)
+  {
+    srec[2 * s + 1].y = (int)g0;
+    srec[2 * s + 1].z = (int)gAll;
+  }
+  __syncwarp();
+  forPoints([&](const int4 &p, int b) {
+    const uint32_t at = base + atomicAdd(&h[b], 1u);
+    bxy[at] = make_int2(p.x, p.y);
+    bzw[at] = make_int2(p.z, p.w);
+  });
+}
+
+/* The groups' records: two int4 per group, {x0, y0, x1, y1} and {zmin, first,
+ * points, flags} (flags: holds a point beside or above the root cube, which
+ * the queries can take with its block without the hyperboloid holding the point
+ * itself); one warp per group. */
+__global__ void groupBoxKernel(GridArgs g, const unsigned long long *__restrict__ taken, const int2 *__restrict__ bxy,
+                               const int2 *__restrict__ bzw, int4 *__restrict__ groups)
+{
+  const int lane = threadIdx.x & 31;
+  const uint64_t n = *taken >> 36, warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t k = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += warps)
+  {
+    const int4 r1 = groups[2 * k + 1];
+    const bool ok = lane < r1.z;
+    int2 p = make_int2(0, 0), q = make_int2(0, 0);
+    if (ok)
+    {
+      p = bxy[(uint32_t)r1.y + lane];
+      q = bzw[(uint32_t)r1.y + lane];
+    }
+    const int x0 = __reduce_min_sync(0xffffffffu, ok ? p.x : INT32_MAX), x1 = __reduce_max_sync(0xffffffffu, ok ? p.x : INT32_MIN);
+    const int y0 = __reduce_min_sync(0xffffffffu, ok ? p.y : INT32_MAX), y1 = __reduce_max_sync(0xffffffffu, ok ? p.y : INT32_MIN);
+    const int z0 = __reduce_min_sync(0xffffffffu, ok ? q.x : INT32_MAX);
+    bool stray = ok && q.y < 0;
+    if (stray)
+    {
+      const double x = wb_decode(p.x, g.off[0], g.scale[0], g.unit), y = wb_decode(p.y, g.off[1], g.scale[1], g.unit),
+                   z = wb_decode(q.x, g.off[2], g.scale[2], g.unit);
+      stray = x < g.rootLo[0] || y < g.rootLo[1] || x >= g.rootHi[0] || y >= g.rootHi[1] || z >= g.rootHi[2];
+    }
+    stray = __any_sync(0xffffffffu, stray);
+    if (lane == 0)
+    {
+      groups[2 * k] = make_int4(x0, y0, x1, y1);
+      groups[2 * k + 1] = make_int4(z0, r1.y, r1.z, stray ? 1 : 0);
+    }
+  }
+}
+
 /* Records of each block of WB_SUPER x WB_SUPER columns (the column record
- * layout; begin/end unused). */
+ * layout; begin/end unused; flags: some column's flags). */
 __global__ void superKernel(int nx, int ny, int snx, int sny, const int4 *__restrict__ rec, int4 *__restrict__ srec)
 {
   uint64_t ns = (uint64_t)snx * sny;
@@ -258,6 +427,7 @@ __global__ void superKernel(int nx, int ny, int snx, int sny, const int4 *__rest
   {
     int si = (int)(s % snx), sj = (int)(s / snx);
     int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[2] = {INT32_MIN, INT32_MIN};
+    int flags = 0;
     for (int dj = 0; dj < WB_SUPER; dj++)
       for (int di = 0; di < WB_SUPER; di++)
       {
@@ -273,12 +443,29 @@ __global__ void superKernel(int nx, int ny, int snx, int sny, const int4 *__rest
         mx[0] = max(mx[0], r0.z);
         mx[1] = max(mx[1], r0.w);
         mn[2] = min(mn[2], r1.x);
+        flags |= r1.w;
       }
     srec[2 * s] = make_int4(mn[0], mn[1], mx[0], mx[1]);
-    srec[2 * s + 1] = make_int4(mn[2], 0, 0, 0);
+    srec[2 * s + 1] = make_int4(mn[2], 0, 0, flags);   // y, z: groupOrderKernel
   }
 }
 }  // namespace
+
+static GridArgs gridArgs(const wb_ctx *c)
+{
+  GridArgs a{};
+  const WbGeom &g = c->g;
+  a.nd = c->nd;
+  for (int k = 0; k < 3; k++)
+  {
+    a.off[k] = g.off[k];
+    a.scale[k] = g.scale[k];
+    a.rootLo[k] = g.root_lo[k];
+    a.rootHi[k] = g.root_lo[k] + g.root_side;
+  }
+  a.unit = g.unit;
+  return a;
+}
 
 int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
 {
@@ -305,16 +492,7 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
       (rc = wb_ensure(c, c->gpt, nd * 16 + 64)) || (rc = wb_ensure(c, c->cellRec, ncell * 32 + 64)) ||
       (rc = wb_ensure(c, c->colOf, nd * 8 + 64)))
     return rc;
-  GridArgs a;
-  a.nd = nd;
-  for (int k = 0; k < 3; k++)
-  {
-    a.off[k] = g.off[k];
-    a.scale[k] = g.scale[k];
-    a.rootLo[k] = g.root_lo[k];
-    a.rootHi[k] = g.root_lo[k] + g.root_side;
-  }
-  a.unit = g.unit;
+  GridArgs a = gridArgs(c);
   a.x0 = x0;
   a.y0 = y0;
   a.cell = cell;
@@ -363,29 +541,13 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
     return rc;
   { superKernel<<<(unsigned)std::min<uint64_t>((nsup + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
         nx, ny, snx, sny, (const int4 *)c->cellRec.p, (int4 *)c->superRec.p); ++c->launches; }
-  // column groups: counts, their prefix, the list
-  uint32_t *gTot = (uint32_t *)((char *)c->small.p + 640);
-  if ((rc = wb_ensure(c, c->groupCnt, (ncell + 1) * 8 + 64)))
-    return rc;
-  uint32_t *gcnt = (uint32_t *)c->groupCnt.p, *gfirst = gcnt + ncell + 1;
-  { groupCountKernel<<<(unsigned)std::min<uint64_t>((ncell + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-        ncell, (const int4 *)c->cellRec.p, gcnt); ++c->launches; }
-  if ((rc = wb_exclusive_scan_u32(c, gcnt, gfirst, ncell, gTot)))
-    return rc;
-  // at most nd / 32 + ncell groups
-  if ((rc = wb_ensure(c, c->groups, (nd / 32 + ncell + 1) * 8 + 64)))
-    return rc;
-  { groupFillKernel<<<(unsigned)std::min<uint64_t>((ncell + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-        ncell, (const int4 *)c->cellRec.p, gfirst, (uint2 *)c->groups.p); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
   unsigned long long ns = 0;
-  uint32_t ngroups = 0;
   int ext[6];
   WB_CUDA(c, cudaMemcpyAsync(&ns, dStray, 8, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaMemcpyAsync(ext, dExt, 24, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaMemcpyAsync(&ngroups, gTot, 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  c->grid.nGroups = ngroups;
+  c->grid.grouped = false;
   c->grid.nStray = ns;
   c->grid.zminInt = ext[2];
   for (int k = 0; k < 3; k++)
@@ -393,5 +555,67 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
     c->grid.imin[k] = ext[k];
     c->grid.imax[k] = ext[3 + k];
   }
+  return 0;
+}
+
+/* The column groups of the margin pass (groups of consecutive points of a
+ * column); synchronises. */
+int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count)
+{
+  const uint64_t ncell = c->grid.ncell, nd = c->nd;
+  uint32_t *gTot = (uint32_t *)((char *)c->small.p + 640);
+  int rc;
+  *groups = nullptr;
+  *count = 0;
+  if (!nd)
+    return 0;
+  if ((rc = wb_ensure(c, c->groupCnt, (ncell + 1) * 8 + 64)))
+    return rc;
+  uint32_t *gcnt = (uint32_t *)c->groupCnt.p, *gfirst = gcnt + ncell + 1;
+  const unsigned blocks = (unsigned)std::min<uint64_t>((ncell + 255) / 256, (uint64_t)c->sm_count * 16);
+  { groupCountKernel<<<blocks, 256, 0, c->stream>>>(ncell, (const int4 *)c->cellRec.p, gcnt); ++c->launches; }
+  if ((rc = wb_exclusive_scan_u32(c, gcnt, gfirst, ncell, gTot)))
+    return rc;
+  // at most nd / 32 + ncell groups
+  if ((rc = wb_ensure(c, c->colGroups, (nd / 32 + ncell + 1) * 8 + 64)))
+    return rc;
+  { groupFillKernel<<<blocks, 256, 0, c->stream>>>(ncell, (const int4 *)c->cellRec.p, gfirst, (uint2 *)c->colGroups.p); ++c->launches; }
+  WB_CUDA(c, cudaGetLastError());
+  uint32_t ngroups = 0;
+  WB_CUDA(c, cudaMemcpyAsync(&ngroups, gTot, 4, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  *groups = (const uint2 *)c->colGroups.p;
+  *count = ngroups;
+  return 0;
+}
+
+/* The point groups of the fast pass, formed once per grid when a classify
+ * first wants them (an octree or a scan alone does not).  Their number stays on
+ * the device: *taken, groups above the low 36 bits. */
+int wb_point_groups(wb_ctx *c, const unsigned long long **taken)
+{
+  unsigned long long *gTot = (unsigned long long *)((char *)c->small.p + 704);
+  *taken = gTot;
+  if (c->grid.grouped)
+    return 0;
+  const uint64_t nd = c->nd, nsup = (uint64_t)c->grid.snx * c->grid.sny;
+  int rc;
+  // at most 32 points each, two partly filled ones per super-cell
+  if ((rc = wb_ensure(c, c->groups, (nd / 32 + 2 * std::min<uint64_t>(nsup, nd) + 1) * 32 + 64)))
+    return rc;
+  WB_CUDA(c, cudaMemsetAsync(gTot, 0, 8, c->stream));
+  if (nd)
+  {
+    const WbGeom &g = c->g;
+    // the points in group order take the place of the grid sort's key buffers
+    { groupOrderKernel<<<(unsigned)((nsup + kOrderWarps - 1) / kOrderWarps), 32 * kOrderWarps, 0, c->stream>>>(
+          c->grid.nx, c->grid.ny, c->grid.snx, c->grid.sny, (float)(c->grid.cell / fabs(g.scale[2] * g.unit)),
+          (const int4 *)c->cellRec.p, (int4 *)c->superRec.p, (const int4 *)c->gpt.p, (int2 *)c->gKey0.p,
+          (int2 *)c->gKey1.p, (int4 *)c->groups.p, gTot); ++c->launches; }
+    { groupBoxKernel<<<(unsigned)std::min<uint64_t>((nd / 32 + 8) / 8, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
+          gridArgs(c), gTot, (const int2 *)c->gKey0.p, (const int2 *)c->gKey1.p, (int4 *)c->groups.p); ++c->launches; }
+    WB_CUDA(c, cudaGetLastError());
+  }
+  c->grid.grouped = true;
   return 0;
 }

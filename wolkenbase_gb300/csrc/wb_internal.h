@@ -38,7 +38,7 @@ struct GridInfo
   int32_t imin[3] = {0, 0, 0}, imax[3] = {0, 0, 0};   /* record-integer extent of the cloud */
   /* super-cells: blocks of WB_SUPER x WB_SUPER columns with their own bounds */
   int snx = 0, sny = 0;
-  uint64_t nGroups = 0;             /* column groups of up to 32 points */
+  bool grouped = false;             /* the point groups of this grid are formed */
 };
 #define WB_SUPER 3
 /* a warp tests a super-cell's columns with one lane each */
@@ -87,7 +87,8 @@ struct wb_ctx
      {x0, y0, x1, y1} and {zmin, begin, end, flags}, x0 == INT32_MAX for an
      empty column; superRec the same two int4 per super-cell */
   DevBuf gKey0, gKey1, gVal0, gVal1, stray, cellStart, gpt, cellRec, superRec, ptSetup;
-  DevBuf groups, groupCnt;          /* column groups: uint2 {column, first point} of up to 32 points */
+  DevBuf groups;                    /* point groups: two int4 each; their points are in gKey0 and gKey1 */
+  DevBuf colGroups, groupCnt;       /* column groups {column, first point}, formed when margins are wanted */
   GridInfo grid;
   /* fused fast-pass settings (wb_set_tuning; a server's autotuner picks them
      per batch): kernel shape, work chunk and points per grid column */
@@ -106,6 +107,7 @@ struct wb_ctx
   /* classify arguments formed by wb_classify_stage for a fused launch */
   alignas(16) unsigned char clsArgs[768];
   bool clsStaged = false;
+  uint64_t n_col_groups = 0;        /* column groups of the staged classify (margins) */
   uint8_t *clsHost = nullptr;       /* host destination of the class bytes, or NULL */
   const uint8_t *clsFinal = nullptr; /* device class bytes of the last classify (per record) */
   uint64_t n_ground = 0;
@@ -199,6 +201,8 @@ int wb_radix_sort_pairs(wb_ctx *c, uint64_t *&keys, uint32_t *&vals, uint64_t *k
 int wb_point_leaf_map(wb_ctx *c);   /* point -> leaf map into c->pointLeaf */
 int wb_build_impl(wb_ctx *c, const wb_cloud *cloud);
 int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1);
+int wb_point_groups(wb_ctx *c, const unsigned long long **taken);
+int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count);
 int wb_scan_impl(wb_ctx *c, const wb_params *p);
 int wb_classify_impl(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDevice);
 int wb_find_block_impl(wb_ctx *c, const double *xyz, uint64_t m, int64_t *leaf);
@@ -219,10 +223,10 @@ struct WbShape
   int warps, minBlocks;
 };
 extern const WbShape kWbShapes[WB_N_SHAPES];
-/* Times the fused fast pass alone over the first `sample` points of the
- * staged jobs (set-up included, untimed); the jobs' ambiguous lists are
- * cleared afterwards, so the batch can be launched normally. */
-int wb_batch_time(WbBatch *b, wb_ctx *const *jobs, int k, uint64_t sample, int shape, int chunk, cudaStream_t s,
+/* Times the fused fast pass and its one-point pass over the staged jobs
+ * (set-up included, untimed); the jobs' ambiguous lists are cleared
+ * afterwards, so the batch can be launched normally. */
+int wb_batch_time(WbBatch *b, wb_ctx *const *jobs, int k, int shape, int chunk, cudaStream_t s,
                   float *ms, std::string &err);
 struct WbTuneJob
 {
