@@ -31,8 +31,8 @@ int wb_fail(wb_ctx *c, int code, const std::string &msg)
  * them in host memory first, so that HBM holds what classify reads at random. */
 static bool coldBuffer(const wb_ctx *c, const DevBuf &b)
 {
-  const DevBuf *cold[] = {&c->rec, &c->key0, &c->key1, &c->idx0, &c->idx1, &c->tmp32, &c->tmp32b,
-                          &c->gVal0, &c->gVal1, &c->tilePts, &c->survivorOf, &c->pointLeaf};
+  const DevBuf *cold[] = {&c->rec, &c->key0, &c->key1, &c->idx0, &c->idx1,
+                          &c->gVal0, &c->gVal1, &c->tilePts, &c->pointLeaf};
   for (const DevBuf *x : cold)
     if (x == &b)
       return true;
@@ -117,10 +117,10 @@ void wb_mark(wb_ctx *c, const char *name)
 
 void wb_release_buffers(wb_ctx *c)
 {
-  DevBuf *all[] = {&c->rec, &c->key0, &c->key1, &c->idx0, &c->idx1, &c->tmp32, &c->tmp32b, &c->tmp8, &c->scanTmp,
-                   &c->small, &c->lev, &c->cpl, &c->pre, &c->suf, &c->leafId, &c->leafFirst, &c->leafCount,
-                   &c->leafLevel, &c->leafKey, &c->leafBox, &c->sidx, &c->sx, &c->sy, &c->sz, &c->xyzd, &c->colOf, &c->gridBounds, &c->pointLeaf,
-                   &c->storeOf, &c->survivorOf, &c->nodeChild, &c->nodeBox, &c->nodeStart, &c->nodeIdLevel,
+  DevBuf *all[] = {&c->rec, &c->key0, &c->key1, &c->idx0, &c->idx1, &c->tmp8, &c->scanTmp,
+                   &c->small, &c->pre, &c->suf, &c->leafId, &c->leafFirst, &c->leafCount,
+                   &c->leafLevel, &c->leafKey, &c->sidx, &c->sx, &c->sy, &c->sz, &c->xyzd, &c->colOf, &c->gridBounds, &c->pointLeaf,
+                   &c->storeOf,
                    &c->tileEx, &c->tileEy, &c->tileLookup, &c->tileStart, &c->tilePts, &c->owner, &c->tileRes,
                    &c->tileHuge, &c->hugePre, &c->scanTot, &c->tileFrm,
                    &c->tileH, &c->tileN, &c->tileNg, &c->label, &c->clsDev, &c->ambiguous, &c->deferred, &c->angleT,

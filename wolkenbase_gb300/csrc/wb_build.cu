@@ -16,9 +16,7 @@
  *   K4  common-prefix level of keys 537 apart; the leaf level of a point is
  *       1 + the largest such level over the 538-point windows that contain it
  *       (a node holds >537 points iff one window fits inside it)
- *   K5  leaf starts, leaf table, per-leaf order by input index, leaf boxes
- *   K6  explicit node hierarchy (8 children per internal node) with boxes,
- *       used by the cylinder and hyperboloid queries
+ *   K5  leaf starts, leaf table, per-leaf order by input index
  */
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -26,6 +24,7 @@
 #include <cmath>
 #include "wb_internal.h"
 #include "wb_device.cuh"
+#include "wb_lookback.cuh"
 
 namespace
 {
@@ -40,8 +39,9 @@ struct KeyArgs
   double lo[3], cell;
   /* Fixed-point form of the level-21 cell coordinate, per axis:
      t(X) = (C + (X - x0) * R) / 2^shift, with |X - x0| <= dmax.  A point
-     whose fraction lies more than eps from an integer takes floor(t); the
-     rest (and all of an axis with fixed = 0) take the exact FP64 path. */
+     whose fraction lies more than eps from an integer takes floor(t); for the
+     rest the decoded coordinate is compared with that one boundary.  All of an
+     axis with fixed = 0 take the general FP64 path. */
   int fixed[3], shift[3];
   long long x0[3], dmax[3], rfix[3], cfix[3], eps[3];
 };
@@ -67,7 +67,7 @@ __device__ __forceinline__ void loadXYZ(const uint8_t *rec, uint32_t stride, uin
   }
 }
 
-__global__ void keyKernel(KeyArgs a, uint64_t *__restrict__ keys, uint32_t *__restrict__ idx)
+__global__ void keyKernel(KeyArgs a, uint64_t *__restrict__ keys)
 {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x)
   {
@@ -78,24 +78,28 @@ __global__ void keyKernel(KeyArgs a, uint64_t *__restrict__ keys, uint32_t *__re
     for (int ax = 0; ax < 3; ax++)
     {
       const long long d = (long long)q[ax] - a.x0[ax];
-      bool done = false;
+      const long long kMax = (1 << WB_LEVELS) - 1;
       if (a.fixed[ax] && d >= -a.dmax[ax] && d <= a.dmax[ax])
       {
         const long long tf = d * a.rfix[ax] + a.cfix[ax];
-        const long long k0 = tf >> a.shift[ax];
+        long long k0 = tf >> a.shift[ax];
         const long long fr = tf - k0 * (1ll << a.shift[ax]);
-        if (fr > a.eps[ax] && fr < (1ll << a.shift[ax]) - a.eps[ax])
+        // within eps of cell boundary kb: the decoded coordinate decides (cell
+        // sides are dyadic, so with decimal coordinates one point in 125 lies
+        // on a boundary and most warps hold one: seven FP64 instructions here,
+        // where the general search took 40 and the FP64 pipe bounded the kernel)
+        const bool below = fr <= a.eps[ax], above = fr >= (1ll << a.shift[ax]) - a.eps[ax];
+        if (below || above)
         {
-          const long long kMax = (1 << WB_LEVELS) - 1;
-          k[ax] = (uint32_t)(k0 < 0 ? 0 : (k0 > kMax ? kMax : k0));
-          done = true;
+          const long long kb = k0 + above;
+          k0 = wb_decode(q[ax], a.off[ax], a.scale[ax], a.unit) >= a.lo[ax] + (double)(int)kb * a.cell ? kb : kb - 1;
         }
+        k[ax] = (uint32_t)(k0 < 0 ? 0 : (k0 > kMax ? kMax : k0));
       }
-      if (!done)
+      else
         k[ax] = wb_cell_index(wb_decode(q[ax], a.off[ax], a.scale[ax], a.unit), a.lo[ax], a.cell);
     }
     keys[i] = wb_morton(k[0], k[1], k[2]);
-    idx[i] = (uint32_t)i;
   }
 }
 
@@ -111,104 +115,297 @@ __device__ __forceinline__ bool sameDoubles(const KeyArgs &a, uint32_t i, uint32
   return true;
 }
 
-/* survivor[i] = 1 unless a later record in the same key run has the same xyz. */
-__global__ void survivorKernel(KeyArgs a, const uint64_t *__restrict__ keys, const uint32_t *__restrict__ idx,
-                               uint32_t *__restrict__ surv)
+/* The counters of a build, in the context's scratch block from
+ * WB_SMALL_LOOKBACK on. */
+struct BuildFlags
 {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x)
-  {
-    uint32_t s = 1;
-    uint64_t k = keys[i];
-    for (uint64_t j = i + 1; j < a.n && keys[j] == k; j++)
-      if (sameDoubles(a, idx[i], idx[j]))
+  int lookback;        /* a look-back gave up (kept by the primitives too)    */
+  uint32_t dups;       /* records a later identical point replaced            */
+  uint32_t longRuns;   /* runs of equal sorted bits too long for runKernel     */
+  uint32_t unsorted;   /* one of them was too long for longRunKernel as well   */
+  uint32_t leaves;
+  int tooDeep, maxLevel;
+};
+
+/* Whether sorted record i survives: no later record of its key has the same xyz. */
+__device__ __forceinline__ bool survives(const KeyArgs &a, const uint64_t *keys, const uint32_t *idx, uint64_t i)
+{
+  const uint64_t k = keys[i];
+  for (uint64_t j = i + 1; j < a.n && keys[j] == k; j++)
+    if (sameDoubles(a, idx[i], idx[j]))
+      return false;
+  return true;
+}
+
+__device__ __forceinline__ void countDups(uint32_t dups, BuildFlags *f)
+{
+  dups = __reduce_add_sync(0xffffffffu, dups);
+  if ((threadIdx.x & 31) == 0 && dups)
+    atomicAdd(&f->dups, dups);
+}
+
+/* The radix sort orders the keys' bits from `begin` up, enough of them to tell
+ * almost all points apart; this finishes the order and marks the survivors.
+ * One thread per run of equal sorted bits (its first record's): runs are one or
+ * two points long, and the run is in input order for equal keys, so a stable
+ * insertion sort of the rest of the key gives the full sort's order.  Longer
+ * runs are listed for longRunKernel.
+ * 145 us for 20M points (keys read, flags written); with it five radix passes do
+ * where eight did (50M points: sort 4.4 -> 2.3 ms). */
+constexpr int kRunMax = 32;
+__global__ void runKernel(KeyArgs a, int begin, uint64_t *keys, uint32_t *idx, uint8_t *__restrict__ surv,
+                          uint32_t *__restrict__ longRuns, BuildFlags *f)
+{
+  uint32_t dups = 0;
+  if (!f->lookback)
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x)
+    {
+      const uint64_t p = keys[i] >> begin;
+      if (i && (keys[i - 1] >> begin) == p)
+        continue;
+      int m = 1;
+      while (m <= kRunMax && i + m < a.n && (keys[i + m] >> begin) == p)
+        m++;
+      if (m > kRunMax)
       {
-        s = 0;
+        longRuns[atomicAdd(&f->longRuns, 1u)] = (uint32_t)i;
+        continue;
+      }
+      for (int q = 1; q < m; q++)
+      {
+        const uint64_t k = keys[i + q];
+        const uint32_t v = idx[i + q];
+        int b = q;
+        for (; b > 0 && keys[i + b - 1] > k; b--)
+        {
+          keys[i + b] = keys[i + b - 1];
+          idx[i + b] = idx[i + b - 1];
+        }
+        if (b != q)
+        {
+          keys[i + b] = k;
+          idx[i + b] = v;
+        }
+      }
+      for (int q = 0; q < m; q++)
+      {
+        // later records of the run only: another run may be on the move
+        bool s = true;
+        const uint64_t k = keys[i + q];
+        for (int u = q + 1; s && u < m && keys[i + u] == k; u++)
+          s = !sameDoubles(a, idx[i + q], idx[i + u]);
+        surv[i + q] = s;
+        dups += !s;
+      }
+    }
+  countDups(dups, f);
+}
+
+/* The listed runs, one block each: sorted by (key, input index) in shared
+ * memory up to kLongRunMax points (lines and stacks of points); a longer one
+ * raises `unsorted` and the caller sorts all bits. */
+constexpr int kLongRunMax = 2048;
+__global__ void __launch_bounds__(256) longRunKernel(KeyArgs a, int begin, uint64_t *keys, uint32_t *idx,
+                                                     uint8_t *__restrict__ surv, const uint32_t *__restrict__ longRuns,
+                                                     BuildFlags *f)
+{
+  __shared__ uint64_t k[kLongRunMax];
+  __shared__ uint32_t v[kLongRunMax];
+  __shared__ int len;
+  uint32_t dups = 0;
+  const uint32_t runs = f->longRuns;
+  for (uint32_t r = blockIdx.x; r < runs; r += gridDim.x)
+  {
+    const uint64_t i = longRuns[r], p = keys[i] >> begin;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      len = kLongRunMax + 1;
+    __syncthreads();
+    for (int q = threadIdx.x; q <= kLongRunMax; q += 256)
+      if (i + q >= a.n || (keys[i + q] >> begin) != p)
+      {
+        atomicMin(&len, q);
         break;
       }
-    surv[i] = s;
-  }
-}
-
-__global__ void compactKernel(uint64_t n, const uint64_t *__restrict__ keys, const uint32_t *__restrict__ idx,
-                              const uint32_t *__restrict__ surv, const uint32_t *__restrict__ rank,
-                              uint64_t *__restrict__ dkey, uint32_t *__restrict__ didx)
-{
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    if (surv[i])
+    __syncthreads();
+    const int m = len;
+    if (m > kLongRunMax)
     {
-      dkey[rank[i]] = keys[i];
-      didx[rank[i]] = idx[i];
+      if (threadIdx.x == 0)
+        f->unsorted = 1;
+      continue;
     }
+    int P = 64;
+    while (P < m)
+      P <<= 1;
+    for (int q = threadIdx.x; q < P; q += 256)
+    {
+      k[q] = q < m ? keys[i + q] : ~0ull;
+      v[q] = q < m ? idx[i + q] : ~0u;
+    }
+    __syncthreads();
+    for (int size = 2; size <= P; size <<= 1)
+      for (int j = size >> 1; j > 0; j >>= 1)
+      {
+        for (int q = threadIdx.x; q < P; q += 256)
+        {
+          const int u = q ^ j;
+          if (u > q)
+          {
+            const bool up = (q & size) == 0;
+            const uint64_t kx = k[q], ky = k[u];
+            const uint32_t vx = v[q], vy = v[u];
+            if ((kx > ky || (kx == ky && vx > vy)) == up)
+            {
+              k[q] = ky;
+              k[u] = kx;
+              v[q] = vy;
+              v[u] = vx;
+            }
+          }
+        }
+        __syncthreads();
+      }
+    for (int q = threadIdx.x; q < m; q += 256)
+    {
+      keys[i + q] = k[q];
+      idx[i + q] = v[q];
+      bool s = true;
+      for (int u = q + 1; s && u < m && k[u] == k[q]; u++)
+        s = !sameDoubles(a, v[q], v[u]);
+      surv[i + q] = s;
+      dups += !s;
+    }
+  }
+  countDups(dups, f);
 }
 
-/* cpl[s] = common levels of dkey[s] and dkey[s+537], s in [0, nd-538]. */
-__global__ void cplKernel(const uint64_t *__restrict__ dkey, uint64_t nw, uint8_t *__restrict__ cpl)
+/* The survivors of fully sorted keys. */
+__global__ void survivorKernel(KeyArgs a, const uint64_t *__restrict__ keys, const uint32_t *__restrict__ idx,
+                               uint8_t *__restrict__ surv, BuildFlags *f)
 {
-  for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nw; s += (uint64_t)gridDim.x * blockDim.x)
-    cpl[s] = (uint8_t)wb_common_levels(dkey[s], dkey[s + kWindow - 1]);
+  uint32_t dups = 0;
+  if (!f->lookback)
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x)
+    {
+      const bool s = survives(a, keys, idx, i);
+      surv[i] = s;
+      dups += !s;
+    }
+  countDups(dups, f);
 }
 
-/* Prefix and suffix maxima inside aligned segments of kWindow windows
- * (van Herk / Gil-Werman): one warp per segment. */
-__global__ void segMaxKernel(const uint8_t *__restrict__ cpl, uint64_t nw, uint8_t *__restrict__ pre,
+/* The survivors' keys and indices, closed up. */
+struct CompactScan
+{
+  const uint8_t *surv;
+  const uint64_t *keys;
+  const uint32_t *idx;
+  uint64_t *dkey;
+  uint32_t *didx;
+  __device__ uint32_t value(uint64_t i) const { return surv[i]; }
+  __device__ void put(uint64_t i, uint32_t before, uint32_t v) const
+  {
+    if (v)
+    {
+      dkey[before] = keys[i];
+      didx[before] = idx[i];
+    }
+  }
+};
+__global__ void __launch_bounds__(256) compactKernel(uint64_t n, CompactScan f, unsigned *counter,
+                                                     unsigned long long *status, int *err)
+{
+  lookbackScan(n, f, counter, status, nullptr, err);
+}
+
+/* Prefix and suffix maxima, inside aligned segments of kWindow windows, of
+ * the common levels of keys kWindow - 1 apart (van Herk / Gil-Werman): one warp
+ * per segment, the levels of its windows in registers between the two. */
+__global__ void segMaxKernel(const uint64_t *__restrict__ dkey, uint64_t nw, uint8_t *__restrict__ pre,
                              uint8_t *__restrict__ suf)
 {
-  uint64_t seg = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  uint64_t b = seg * kWindow;
+  constexpr int ROWS = (kWindow + 31) / 32;
+  const uint64_t seg = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint64_t b = seg * kWindow;
   if (b >= nw)
     return;
-  uint64_t e = b + kWindow < nw ? b + kWindow : nw;
-  int run = 0;
-  for (uint64_t s0 = b; s0 < e; s0 += 32)
+  const uint64_t e = b + kWindow < nw ? b + kWindow : nw;
+  int v[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; r++)
   {
-    uint64_t s = s0 + lane;
-    int v = s < e ? cpl[s] : 0;
+    const uint64_t s = b + 32 * r + lane;
+    v[r] = s < e ? wb_common_levels(dkey[s], dkey[s + kWindow - 1]) : 0;
+  }
+  int run = 0;
+#pragma unroll
+  for (int r = 0; r < ROWS; r++)
+  {
+    const uint64_t s = b + 32 * r + lane;
+    int x = v[r];
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1)
     {
-      int t = __shfl_up_sync(0xffffffffu, v, o);
+      const int t = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o)
-        v = max(v, t);
+        x = max(x, t);
     }
-    v = max(v, run);
+    x = max(x, run);
     if (s < e)
-      pre[s] = (uint8_t)v;
-    run = __shfl_sync(0xffffffffu, v, 31);
+      pre[s] = (uint8_t)x;
+    run = __shfl_sync(0xffffffffu, x, 31);
   }
   run = 0;
-  uint64_t len = e - b;
-  for (uint64_t r0 = 0; r0 < len; r0 += 32)
+#pragma unroll
+  for (int r = ROWS - 1; r >= 0; r--)
   {
-    uint64_t r = r0 + lane;   // distance from the end
-    uint64_t s = e - 1 - r;
-    int v = r < len ? cpl[s] : 0;
+    const uint64_t s = b + 32 * r + lane;
+    int x = v[r];
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1)
     {
-      int t = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o)
-        v = max(v, t);
+      const int t = __shfl_down_sync(0xffffffffu, x, o);
+      if (lane + o < 32)
+        x = max(x, t);
     }
-    v = max(v, run);
-    if (r < len)
-      suf[s] = (uint8_t)v;
-    run = __shfl_sync(0xffffffffu, v, 31);
+    x = max(x, run);
+    if (s < e)
+      suf[s] = (uint8_t)x;
+    run = __shfl_sync(0xffffffffu, x, 0);
   }
 }
 
-/* lev[i] = 1 + max cpl over windows [s, s+537] containing i. */
-__global__ void levelKernel(uint64_t nd, uint64_t nw, const uint8_t *__restrict__ pre, const uint8_t *__restrict__ suf,
-                            uint8_t *__restrict__ lev, int *__restrict__ err)
+__device__ __forceinline__ uint64_t prefixAt(uint64_t key, int level)
 {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (uint64_t)gridDim.x * blockDim.x)
+  return level <= 0 ? 0 : key >> (63 - 3 * level);
+}
+
+/* The leaves: point i's leaf level is 1 + the largest common level over the
+ * windows [s, s + 537] that contain it; a leaf starts where the level or the
+ * key's prefix at that level changes.  One pass forms the leaf of every point
+ * and the leaf table (up to cap entries: the caller makes room and runs it
+ * again when there are more). */
+struct LeafScan
+{
+  uint64_t nw, cap;
+  const uint64_t *dkey;
+  const uint8_t *pre, *suf;
+  uint32_t *leafId, *first;
+  uint8_t *leafLev;
+  uint64_t *leafKey;
+  BuildFlags *f;
+  __device__ int level(uint64_t i) const
   {
     int d = 0;
     if (nw > 0)
     {
-      uint64_t a = i >= (uint64_t)(kWindow - 1) ? i - (kWindow - 1) : 0;
-      uint64_t b = i < nw - 1 ? i : nw - 1;
+      const uint64_t a = i >= (uint64_t)(kWindow - 1) ? i - (kWindow - 1) : 0;
+      const uint64_t b = i < nw - 1 ? i : nw - 1;
       if (a <= b)
       {
-        uint64_t sa = a / kWindow, sb = b / kWindow;
+        const uint64_t sa = a / kWindow, sb = b / kWindow;
         if (sa != sb)
           d = max((int)suf[a], (int)pre[b]);
         else if (a == sa * kWindow)
@@ -219,81 +416,63 @@ __global__ void levelKernel(uint64_t nd, uint64_t nw, const uint8_t *__restrict_
     }
     if (d >= WB_LEVELS)
     {
-      atomicExch(err, 1);
+      f->tooDeep = 1;
       d = WB_LEVELS - 1;
     }
-    lev[i] = (uint8_t)(d + 1);
+    return d + 1;
   }
-}
-
-__device__ __forceinline__ uint64_t prefixAt(uint64_t key, int level)
-{
-  return level <= 0 ? 0 : key >> (63 - 3 * level);
-}
-
-__global__ void leafStartKernel(uint64_t nd, const uint64_t *__restrict__ dkey, const uint8_t *__restrict__ lev,
-                                uint32_t *__restrict__ start)
-{
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (uint64_t)gridDim.x * blockDim.x)
+  __device__ uint32_t value(uint64_t i) const
   {
-    uint32_t s = 1;
-    if (i > 0)
-    {
-      int l = lev[i];
-      s = (lev[i - 1] != l) || (prefixAt(dkey[i - 1], l) != prefixAt(dkey[i], l));
-    }
-    start[i] = s;
+    if (i == 0)
+      return 1;
+    const int l = level(i);
+    return level(i - 1) != l || prefixAt(dkey[i - 1], l) != prefixAt(dkey[i], l);
   }
-}
-
-__global__ void leafTableKernel(uint64_t nd, const uint64_t *__restrict__ dkey, const uint8_t *__restrict__ lev,
-                                const uint32_t *__restrict__ start, const uint32_t *__restrict__ ex,
-                                uint32_t *__restrict__ leafId, uint32_t *__restrict__ first,
-                                uint8_t *__restrict__ leafLev, uint64_t *__restrict__ leafKey)
-{
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (uint64_t)gridDim.x * blockDim.x)
+  __device__ void put(uint64_t i, uint32_t before, uint32_t v) const
   {
-    uint32_t l = ex[i] + start[i] - 1;
+    const uint32_t l = before + v - 1;
     leafId[i] = l;
-    if (start[i])
+    if (v && l < cap)
     {
-      int lv = lev[i];
+      const int lv = level(i);
       first[l] = (uint32_t)i;
       leafLev[l] = (uint8_t)lv;
-      uint64_t mask = (lv >= WB_LEVELS) ? ~0ULL : ~((1ULL << (63 - 3 * lv)) - 1);
+      const uint64_t mask = (lv >= WB_LEVELS) ? ~0ULL : ~((1ULL << (63 - 3 * lv)) - 1);
       leafKey[l] = dkey[i] & mask;
+      if (lv > f->maxLevel)
+        atomicMax(&f->maxLevel, lv);
     }
   }
-}
-
-__global__ void leafCountKernel(uint64_t L, uint64_t nd, const uint32_t *__restrict__ first, uint32_t *__restrict__ count)
+};
+__global__ void __launch_bounds__(256) leafKernel(uint64_t nd, LeafScan f, unsigned *counter, unsigned long long *status,
+                                                  int *err)
 {
-  for (uint64_t l = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; l < L; l += (uint64_t)gridDim.x * blockDim.x)
-    count[l] = (uint32_t)((l + 1 < L ? first[l + 1] : nd) - first[l]);
+  lookbackScan(nd, f, counter, status, &f.f->leaves, err);
 }
 
 /* One block per leaf: bitonic sort of the leaf's input indices (<= 537, padded
- * to a power of two, at most 1024), gather of X/Y/Z into store order, integer
- * bounding box, and each stored record's store slot and leaf.  Each thread is
+ * to a power of two, at most 1024), gather of X/Y/Z into store order, and each
+ * stored record's store slot.  Each thread is
  * one comparator of a stage (kLeafThreads comparators per pass).  A stage
  * whose partners lie at most 32 apart touches only its warp's own 64-element
  * window, so between two such stages a warp barrier is enough. */
 constexpr int kLeafThreads = 256;
 __global__ void __launch_bounds__(kLeafThreads) leafSortKernel(KeyArgs a, const uint32_t *__restrict__ first,
-                                                               const uint32_t *__restrict__ count,
+                                                               uint32_t *__restrict__ count,
                                                                const uint32_t *__restrict__ didx,
                                                                uint32_t *__restrict__ sidx, int32_t *__restrict__ sx,
                                                                int32_t *__restrict__ sy, int32_t *__restrict__ sz,
-                                                               int32_t *__restrict__ box, uint32_t *__restrict__ storeOf,
+                                                               uint32_t *__restrict__ storeOf,
                                                                uint64_t L,
                                                                double *__restrict__ xyzd, uint64_t nd)
 {
   __shared__ uint32_t v[1024];
-  __shared__ int32_t red[6][kLeafThreads / 32];
   const uint64_t l = blockIdx.x;
   if (l >= L)
     return;
-  const uint32_t f = first[l], cnt = count[l];
+  const uint32_t f = first[l], cnt = (uint32_t)((l + 1 < L ? first[l + 1] : nd) - f);
+  if (threadIdx.x == 0)
+    count[l] = cnt;
   int P = 64;
   while (P < (int)cnt)
     P <<= 1;
@@ -326,7 +505,6 @@ __global__ void __launch_bounds__(kLeafThreads) leafSortKernel(KeyArgs a, const 
         __syncthreads();
     }
   __syncthreads();
-  int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
   for (int t = threadIdx.x; t < (int)cnt; t += kLeafThreads)
   {
     const uint32_t id = v[t];
@@ -340,41 +518,12 @@ __global__ void __launch_bounds__(kLeafThreads) leafSortKernel(KeyArgs a, const 
     for (int ax = 0; ax < 3; ax++)
       xyzd[(uint64_t)ax * nd + f + t] = wb_decode(q[ax], a.off[ax], a.scale[ax], a.unit);
     storeOf[id] = f + t;
-#pragma unroll
-    for (int ax = 0; ax < 3; ax++)
-    {
-      mn[ax] = min(mn[ax], q[ax]);
-      mx[ax] = max(mx[ax], q[ax]);
-    }
-  }
-#pragma unroll
-  for (int ax = 0; ax < 3; ax++)
-    for (int o = 16; o; o >>= 1)
-    {
-      mn[ax] = min(mn[ax], __shfl_xor_sync(0xffffffffu, mn[ax], o));
-      mx[ax] = max(mx[ax], __shfl_xor_sync(0xffffffffu, mx[ax], o));
-    }
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0)
-    for (int ax = 0; ax < 3; ax++)
-    {
-      red[ax][w] = mn[ax];
-      red[3 + ax][w] = mx[ax];
-    }
-  __syncthreads();
-  if (threadIdx.x < 6)
-  {
-    const int ax = threadIdx.x;
-    int32_t r = ax < 3 ? INT32_MAX : INT32_MIN;
-    for (int q = 0; q < kLeafThreads / 32; q++)
-      r = ax < 3 ? min(r, red[ax][q]) : max(r, red[ax][q]);
-    box[(uint64_t)ax * L + l] = r;
   }
 }
 
 /* Records overwritten by a later duplicate point at the survivor's slot. */
 __global__ void dupMapKernel(KeyArgs a, const uint64_t *__restrict__ keys, const uint32_t *__restrict__ idx,
-                             const uint32_t *__restrict__ surv, uint32_t *__restrict__ storeOf)
+                             const uint8_t *__restrict__ surv, uint32_t *__restrict__ storeOf)
 {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (uint64_t)gridDim.x * blockDim.x)
     if (!surv[i])
@@ -393,76 +542,6 @@ __global__ void pointLeafKernel(uint64_t n, const uint32_t *__restrict__ storeOf
 {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     pointLeaf[i] = leafId[storeOf[i]];
-}
-
-/* ---- node hierarchy ---- */
-__global__ void nodeStartKernel(uint64_t L, int D, const uint8_t *__restrict__ leafLev,
-                                const uint64_t *__restrict__ leafKey, uint32_t *__restrict__ flag)
-{
-  uint64_t total = L * (uint64_t)D;
-  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x)
-  {
-    int d = (int)(t / L);
-    uint64_t l = t % L;
-    uint32_t f = 0;
-    if (leafLev[l] > d)
-      f = (l == 0) || (leafLev[l - 1] <= d) || (prefixAt(leafKey[l - 1], d) != prefixAt(leafKey[l], d));
-    flag[t] = f;
-  }
-}
-
-__device__ __forceinline__ int32_t nodeIdAt(const uint32_t *ex, const uint32_t *flag, uint64_t L, int d, uint64_t l)
-{
-  uint64_t t = (uint64_t)d * L + l;
-  return (int32_t)(ex[t] + flag[t]) - 1;
-}
-
-/* child encoding: >=0 internal node, -1 empty, <=-2 leaf (-2 - leaf). */
-__global__ void nodeLinkKernel(uint64_t L, int D, const uint8_t *__restrict__ leafLev,
-                               const uint64_t *__restrict__ leafKey, const uint32_t *__restrict__ flag,
-                               const uint32_t *__restrict__ ex, int32_t *__restrict__ child,
-                               const int32_t *__restrict__ leafBox, int32_t *__restrict__ nodeBox, uint64_t N)
-{
-  for (uint64_t l = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; l < L; l += (uint64_t)gridDim.x * blockDim.x)
-  {
-    int lv = leafLev[l];
-    uint64_t key = leafKey[l];
-    int32_t b[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++)
-      b[k] = leafBox[(uint64_t)k * L + l];
-    for (int d = 0; d < lv && d < D; d++)
-    {
-      int32_t nid = nodeIdAt(ex, flag, L, d, l);
-      int oct = (int)((key >> (60 - 3 * d)) & 7);
-      if (lv == d + 1)
-        child[(uint64_t)nid * 8 + oct] = -2 - (int32_t)l;
-      else if (flag[(uint64_t)(d + 1) * L + l])
-        child[(uint64_t)nid * 8 + oct] = nodeIdAt(ex, flag, L, d + 1, l);
-      for (int k = 0; k < 3; k++)
-      {
-        atomicMin(&nodeBox[(uint64_t)k * N + nid], b[k]);
-        atomicMax(&nodeBox[(uint64_t)(3 + k) * N + nid], b[3 + k]);
-      }
-    }
-  }
-}
-
-__global__ void fillI32(int32_t *p, uint64_t n, int32_t v)
-{
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    p[i] = v;
-}
-
-__global__ void maxLevelKernel(uint64_t L, const uint8_t *__restrict__ leafLev, int *__restrict__ out)
-{
-  int m = 0;
-  for (uint64_t l = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; l < L; l += (uint64_t)gridDim.x * blockDim.x)
-    m = max(m, (int)leafLev[l]);
-  for (int o = 16; o; o >>= 1)
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0)
-    atomicMax(out, m);
 }
 
 }  // namespace
@@ -598,133 +677,132 @@ int wb_build_impl(wb_ctx *c, const wb_cloud *cl)
   wb_mark(c, "upload");
   if (n == 0)
   {
-    c->nd = c->n_leaves = c->n_nodes = 0;
+    c->nd = c->n_leaves = 0;
     c->grid = GridInfo{};   // no columns or groups of an earlier cloud
     c->stage = 1;
     return 0;
   }
   if ((rc = wb_ensure(c, c->key0, n * 8)) || (rc = wb_ensure(c, c->key1, n * 8)) ||
       (rc = wb_ensure(c, c->idx0, n * 4)) || (rc = wb_ensure(c, c->idx1, n * 4)) ||
-      (rc = wb_ensure(c, c->tmp32, n * 4)) || (rc = wb_ensure(c, c->storeOf, n * 4)) ||
-      (rc = wb_ensure(c, c->survivorOf, n * 4)) ||
-      (rc = wb_ensure(c, c->small, 4096)))
+      (rc = wb_ensure(c, c->tmp8, n)) || (rc = wb_ensure(c, c->storeOf, n * 4)) || (rc = wb_small(c)))
     return rc;
-  uint64_t *keys = (uint64_t *)c->key0.p;
-  uint32_t *idx = (uint32_t *)c->idx0.p;
-  { keyKernel<<<gridFor(c, n), 256, 0, c->stream>>>(a, keys, idx); ++c->launches; }
+  BuildFlags *flags = (BuildFlags *)((char *)c->small.p + WB_SMALL_LOOKBACK), fl;
+  auto readFlags = [&]() -> int {
+    WB_CUDA(c, cudaMemcpyAsync(&fl, flags, sizeof fl, cudaMemcpyDefault, c->stream));
+    WB_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (fl.lookback)
+    {
+      WB_CUDA(c, cudaMemsetAsync(flags, 0, 4, c->stream));
+      return wb_fail(c, WB_ETIMEDOUT, "wb_octree_build: a look-back wait gave up");
+    }
+    return 0;
+  };
+  WB_CUDA(c, cudaMemsetAsync(&flags->dups, 0, sizeof(BuildFlags) - 4, c->stream));
+  uint64_t *keys = (uint64_t *)c->key0.p, *kAlt = (uint64_t *)c->key1.p;
+  uint32_t *idx = (uint32_t *)c->idx0.p, *iAlt = (uint32_t *)c->idx1.p;
+  uint8_t *surv = (uint8_t *)c->tmp8.p;
+  { keyKernel<<<gridFor(c, n), 256, 0, c->stream>>>(a, keys); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
   wb_mark(c, "decode_key");
-  uint64_t *kAlt = (uint64_t *)c->key1.p;
-  uint32_t *iAlt = (uint32_t *)c->idx1.p;
-  if ((rc = wb_radix_sort_pairs(c, keys, idx, kAlt, iAlt, n, 0, 63)))
+  auto swapIfMoved = [&]() {
+    kAlt = (keys == (uint64_t *)c->key0.p) ? (uint64_t *)c->key1.p : (uint64_t *)c->key0.p;
+    iAlt = (idx == (uint32_t *)c->idx0.p) ? (uint32_t *)c->idx1.p : (uint32_t *)c->idx0.p;
+  };
+  // The points lie on surfaces, so about log4(n) levels (three key bits each)
+  // and one more tell nearly all apart; the nearest whole number of passes.
+  const int passes = std::min(8, std::max(2, (int)((3 * (std::log2((double)n) / 2 + 1) + 4) / 8)));
+  const int begin = std::max(0, 63 - 8 * passes);
+  if ((rc = wb_radix_sort_pairs(c, keys, idx, kAlt, iAlt, n, begin, 63, ~0ull, true)))
     return rc;
-  kAlt = (keys == (uint64_t *)c->key0.p) ? (uint64_t *)c->key1.p : (uint64_t *)c->key0.p;
-  iAlt = (idx == (uint32_t *)c->idx0.p) ? (uint32_t *)c->idx1.p : (uint32_t *)c->idx0.p;
+  swapIfMoved();
   wb_mark(c, "sort");
-
-  uint32_t *surv = (uint32_t *)c->tmp32.p;
-  uint32_t *rank = (uint32_t *)c->survivorOf.p;   // scratch: survivor rank
-  int *dErr = (int *)c->small.p;
-  uint32_t *dTot = (uint32_t *)((char *)c->small.p + 64);
-  int *dMax = (int *)((char *)c->small.p + 128);
-  WB_CUDA(c, cudaMemsetAsync(c->small.p, 0, 256, c->stream));
-  { survivorKernel<<<gridFor(c, n), 256, 0, c->stream>>>(a, keys, idx, surv); ++c->launches; }
-  if ((rc = wb_exclusive_scan_u32(c, surv, rank, n, dTot)))
-    return rc;
-  uint32_t ndh = 0;
-  WB_CUDA(c, cudaMemcpyAsync(&ndh, dTot, 4, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  uint64_t nd = ndh;
-  c->nd = nd;
-  uint64_t *dkey = kAlt;
-  uint32_t *didx = iAlt;
-  { compactKernel<<<gridFor(c, n), 256, 0, c->stream>>>(n, keys, idx, surv, rank, dkey, didx); ++c->launches; }
-  wb_mark(c, "dedup");
-
-  uint64_t nw = nd >= (uint64_t)kWindow ? nd - kWindow + 1 : 0;
-  if ((rc = wb_ensure(c, c->cpl, nw + 64)) || (rc = wb_ensure(c, c->pre, nw + 64)) ||
-      (rc = wb_ensure(c, c->suf, nw + 64)) || (rc = wb_ensure(c, c->lev, nd + 64)) ||
-      (rc = wb_ensure(c, c->leafId, nd * 4 + 64)) || (rc = wb_ensure(c, c->tmp32b, nd * 4 * 2 + 64)))
-    return rc;
-  uint8_t *cpl = (uint8_t *)c->cpl.p, *pre = (uint8_t *)c->pre.p, *suf = (uint8_t *)c->suf.p;
-  uint8_t *lev = (uint8_t *)c->lev.p;
-  if (nw)
-  {
-    { cplKernel<<<gridFor(c, nw), 256, 0, c->stream>>>(dkey, nw, cpl); ++c->launches; }
-    uint64_t segs = (nw + kWindow - 1) / kWindow;
-    { segMaxKernel<<<(unsigned)((segs * 32 + 255) / 256), 256, 0, c->stream>>>(cpl, nw, pre, suf); ++c->launches; }
-  }
-  { levelKernel<<<gridFor(c, nd), 256, 0, c->stream>>>(nd, nw, pre, suf, lev, dErr); ++c->launches; }
-  uint32_t *start = (uint32_t *)c->tmp32b.p;
-  uint32_t *startEx = start + nd;
-  { leafStartKernel<<<gridFor(c, nd), 256, 0, c->stream>>>(nd, dkey, lev, start); ++c->launches; }
-  if ((rc = wb_exclusive_scan_u32(c, start, startEx, nd, dTot)))
-    return rc;
-  uint32_t Lh = 0;
-  int errh = 0;
-  WB_CUDA(c, cudaMemcpyAsync(&Lh, dTot, 4, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaMemcpyAsync(&errh, dErr, 4, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (errh)
-    return wb_fail(c, WB_EDEPTH, "wb_octree_build: more than 537 distinct points in a cell 21 levels below the root");
-  uint64_t L = Lh;
-  c->n_leaves = L;
-  if ((rc = wb_ensure(c, c->leafFirst, L * 4 + 64)) || (rc = wb_ensure(c, c->leafCount, L * 4 + 64)) ||
-      (rc = wb_ensure(c, c->leafLevel, L + 64)) || (rc = wb_ensure(c, c->leafKey, L * 8 + 64)) ||
-      (rc = wb_ensure(c, c->leafBox, L * 24 + 64)) || (rc = wb_ensure(c, c->sidx, nd * 4 + 64)) ||
-      (rc = wb_ensure(c, c->sx, nd * 4 + 64)) || (rc = wb_ensure(c, c->sy, nd * 4 + 64)) ||
-      (rc = wb_ensure(c, c->sz, nd * 4 + 64)) || (rc = wb_ensure(c, c->xyzd, nd * 24 + 64)))
-    return rc;
-  uint32_t *leafId = (uint32_t *)c->leafId.p, *first = (uint32_t *)c->leafFirst.p, *count = (uint32_t *)c->leafCount.p;
-  uint8_t *leafLev = (uint8_t *)c->leafLevel.p;
-  uint64_t *leafKey = (uint64_t *)c->leafKey.p;
-  { leafTableKernel<<<gridFor(c, nd), 256, 0, c->stream>>>(nd, dkey, lev, start, startEx, leafId, first, leafLev, leafKey); ++c->launches; }
-  { leafCountKernel<<<gridFor(c, L), 256, 0, c->stream>>>(L, nd, first, count); ++c->launches; }
-  wb_mark(c, "leaves");
-  int32_t *box = (int32_t *)c->leafBox.p;
-  uint32_t *storeOf = (uint32_t *)c->storeOf.p;
-  { leafSortKernel<<<(unsigned)L, kLeafThreads, 0, c->stream>>>(a, first, count, didx, (uint32_t *)c->sidx.p,
-                                                               (int32_t *)c->sx.p, (int32_t *)c->sy.p, (int32_t *)c->sz.p,
-                                                               box, storeOf, L,
-                                                               (double *)c->xyzd.p, nd); ++c->launches; }
+  // (the list of long runs takes the free half of the index buffers)
+  { runKernel<<<gridFor(c, n), 256, 0, c->stream>>>(a, begin, keys, idx, surv, iAlt, flags); ++c->launches; }
+  { longRunKernel<<<(unsigned)c->sm_count, 256, 0, c->stream>>>(a, begin, keys, idx, surv, iAlt, flags); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
-  wb_mark(c, "leaf_order");
-  // records a later identical point overwrote take their survivor's slot
+  if ((rc = readFlags()))
+    return rc;
+  if (fl.unsorted)
+  {
+    // the runs' partial order is stable, so sorting all bits gives the full order
+    WB_CUDA(c, cudaMemsetAsync(&flags->dups, 0, 4, c->stream));
+    if ((rc = wb_radix_sort_pairs(c, keys, idx, kAlt, iAlt, n, 0, 63)))
+      return rc;
+    swapIfMoved();
+    { survivorKernel<<<gridFor(c, n), 256, 0, c->stream>>>(a, keys, idx, surv, flags); ++c->launches; }
+    if ((rc = readFlags()))
+      return rc;
+  }
+  const uint64_t nd = n - fl.dups;
+  c->nd = nd;
+  uint64_t *dkey = keys;
+  uint32_t *didx = idx;
+  unsigned *counter;
+  unsigned long long *status;
   if (nd != n)
   {
-    { dupMapKernel<<<gridFor(c, n), 256, 0, c->stream>>>(a, keys, idx, surv, storeOf); ++c->launches; }
+    dkey = kAlt;
+    didx = iAlt;
+    const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
+    if ((rc = wb_lookback_words(c, tiles, &counter, &status)))
+      return rc;
+    { compactKernel<<<(unsigned)tiles, 256, 0, c->stream>>>(n, CompactScan{surv, keys, idx, dkey, didx}, counter, status,
+                                                            &flags->lookback); ++c->launches; }
   }
-  { maxLevelKernel<<<gridFor(c, L), 256, 0, c->stream>>>(L, leafLev, dMax); ++c->launches; }
-  int maxLev = 0;
-  WB_CUDA(c, cudaMemcpyAsync(&maxLev, dMax, 4, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  c->max_depth = (uint32_t)maxLev;
-  wb_mark(c, "point_map");
+  wb_mark(c, "dedup");
 
-  // node hierarchy over levels 0 .. maxLev-1
-  int D = maxLev;
-  uint64_t LD = L * (uint64_t)D;
-  if ((rc = wb_ensure(c, c->nodeStart, LD * 8 + 64)))
+  const uint64_t nw = nd >= (uint64_t)kWindow ? nd - kWindow + 1 : 0;
+  if ((rc = wb_ensure(c, c->pre, nw + 64)) || (rc = wb_ensure(c, c->suf, nw + 64)) ||
+      (rc = wb_ensure(c, c->leafId, nd * 4 + 64)))
     return rc;
-  uint32_t *flag = (uint32_t *)c->nodeStart.p;
-  uint32_t *flagEx = flag + LD;
-  { nodeStartKernel<<<gridFor(c, LD), 256, 0, c->stream>>>(L, D, leafLev, leafKey, flag); ++c->launches; }
-  if ((rc = wb_exclusive_scan_u32(c, flag, flagEx, LD, dTot)))
+  uint8_t *pre = (uint8_t *)c->pre.p, *suf = (uint8_t *)c->suf.p;
+  if (nw)
+  {
+    const uint64_t segs = (nw + kWindow - 1) / kWindow;
+    { segMaxKernel<<<(unsigned)((segs * 32 + 255) / 256), 256, 0, c->stream>>>(dkey, nw, pre, suf); ++c->launches; }
+  }
+  // room for the leaves a surface usually has (200 to 300 points each); more
+  // are counted, then made room for
+  uint64_t L = std::min<uint64_t>(nd, nd / 64 + 4096);
+  for (int tries = 0;; tries++)
+  {
+    if ((rc = wb_ensure(c, c->leafFirst, L * 4 + 64)) || (rc = wb_ensure(c, c->leafCount, L * 4 + 64)) ||
+        (rc = wb_ensure(c, c->leafLevel, L + 64)) || (rc = wb_ensure(c, c->leafKey, L * 8 + 64)))
+      return rc;
+    const uint64_t tiles = (nd + kScanTile - 1) / kScanTile;
+    if ((rc = wb_lookback_words(c, tiles, &counter, &status)))
+      return rc;
+    { leafKernel<<<(unsigned)tiles, 256, 0, c->stream>>>(
+          nd, LeafScan{nw, L, dkey, pre, suf, (uint32_t *)c->leafId.p, (uint32_t *)c->leafFirst.p,
+                       (uint8_t *)c->leafLevel.p, (uint64_t *)c->leafKey.p, flags}, counter, status,
+          &flags->lookback); ++c->launches; }
+    WB_CUDA(c, cudaGetLastError());
+    if ((rc = readFlags()))
+      return rc;
+    if (fl.tooDeep)
+      return wb_fail(c, WB_EDEPTH, "wb_octree_build: more than 537 distinct points in a cell 21 levels below the root");
+    const bool fits = fl.leaves <= L;
+    L = fl.leaves;
+    if (fits || tries)
+      break;
+  }
+  c->n_leaves = L;
+  c->max_depth = (uint32_t)fl.maxLevel;
+  if ((rc = wb_ensure(c, c->sidx, nd * 4 + 64)) || (rc = wb_ensure(c, c->sx, nd * 4 + 64)) ||
+      (rc = wb_ensure(c, c->sy, nd * 4 + 64)) || (rc = wb_ensure(c, c->sz, nd * 4 + 64)) ||
+      (rc = wb_ensure(c, c->xyzd, nd * 24 + 64)))
     return rc;
-  uint32_t Nh = 0;
-  WB_CUDA(c, cudaMemcpyAsync(&Nh, dTot, 4, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  uint64_t N = Nh;
-  c->n_nodes = N;
-  if ((rc = wb_ensure(c, c->nodeChild, N * 32 + 64)) || (rc = wb_ensure(c, c->nodeBox, N * 24 + 64)))
-    return rc;
-  int32_t *child = (int32_t *)c->nodeChild.p, *nbox = (int32_t *)c->nodeBox.p;
-  { fillI32<<<gridFor(c, N * 8), 256, 0, c->stream>>>(child, N * 8, -1); ++c->launches; }
-  { fillI32<<<gridFor(c, N * 3), 256, 0, c->stream>>>(nbox, N * 3, INT32_MAX); ++c->launches; }
-  { fillI32<<<gridFor(c, N * 3), 256, 0, c->stream>>>(nbox + N * 3, N * 3, INT32_MIN); ++c->launches; }
-  { nodeLinkKernel<<<gridFor(c, L), 256, 0, c->stream>>>(L, D, leafLev, leafKey, flag, flagEx, child, box, nbox, N); ++c->launches; }
+  wb_mark(c, "leaves");
+  uint32_t *storeOf = (uint32_t *)c->storeOf.p;
+  { leafSortKernel<<<(unsigned)L, kLeafThreads, 0, c->stream>>>(a, (const uint32_t *)c->leafFirst.p,
+                                                               (uint32_t *)c->leafCount.p, didx, (uint32_t *)c->sidx.p,
+                                                               (int32_t *)c->sx.p, (int32_t *)c->sy.p, (int32_t *)c->sz.p,
+                                                               storeOf, L, (double *)c->xyzd.p, nd); ++c->launches; }
+  // records a later identical point overwrote take their survivor's slot
+  if (nd != n)
+    { dupMapKernel<<<gridFor(c, n), 256, 0, c->stream>>>(a, keys, idx, surv, storeOf); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
-  wb_mark(c, "nodes");
+  wb_mark(c, "leaf_order");
   c->grid_bounds[0] = mn[0];
   c->grid_bounds[1] = mn[1];
   c->grid_bounds[2] = mx[0];

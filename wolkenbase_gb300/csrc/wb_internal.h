@@ -3,6 +3,7 @@
 #ifndef WB_INTERNAL_H
 #define WB_INTERNAL_H
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <string>
@@ -61,7 +62,7 @@ struct wb_ctx
 
   /* state */
   int stage = 0;                    /* 0 empty, 1 built, 2 scanned, 3 classified */
-  uint64_t n = 0, nd = 0, n_leaves = 0, n_nodes = 0, n_tiles = 0;
+  uint64_t n = 0, nd = 0, n_leaves = 0, n_tiles = 0;
   uint32_t max_depth = 0;
   uint64_t n_ambiguous = 0;         /* points the exact classify pass re-ran */
   WbGeom g{};
@@ -69,16 +70,15 @@ struct wb_ctx
   int precision = WB_PRECISION_EXACT;   /* wb_set_precision */
 
   /* named device buffers */
-  DevBuf rec, key0, key1, idx0, idx1, tmp32, tmp32b, tmp8, scanTmp, small;
-  DevBuf lev, cpl, pre, suf, leafId;
-  DevBuf leafFirst, leafCount, leafLevel, leafKey, leafBox;
-  DevBuf sidx, sx, sy, sz, pointLeaf, storeOf, survivorOf;
+  DevBuf rec, key0, key1, idx0, idx1, tmp8, scanTmp, small;
+  DevBuf pre, suf, leafId;
+  DevBuf leafFirst, leafCount, leafLevel, leafKey;
+  DevBuf sidx, sx, sy, sz, pointLeaf, storeOf;
   /* decoded coordinates of the stored points, three planes of nd doubles
      (x, y, z), each the reference's (offset + scale * X) * unit */
   DevBuf xyzd;
   DevBuf colOf;   /* column {i, j} of each stored point (unclamped, within +-1e9) */
   DevBuf gridBounds;   /* record-integer column boundaries and root-cube faces */
-  DevBuf nodeChild, nodeBox, nodeStart, nodeIdLevel;
   DevBuf tileEx, tileEy, tileLookup, tileStart, tilePts, owner, tileRes, tileH, tileN, tileNg, tileHuge, hugePre,
       scanTot, tileFrm;
   DevBuf label, clsDev, ambiguous, deferred, angleT;
@@ -194,8 +194,18 @@ void wb_flowsnake_order(int idx, std::vector<int32_t> &ex, std::vector<int32_t> 
 int wb_exclusive_scan_u32(wb_ctx *c, const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *total_dev);
 int wb_copy_in(wb_ctx *c, void *dst, const void *src, size_t bytes);   /* caller's host buffer -> device */
 bool wb_device_accessible(const void *p);   /* device, managed or device-mapped host memory */
+/* Stable sort by key bits [beginBit, endBit), at most 64 of them; digits with
+ * none of the bits of `varying` are skipped.  iota: the values are the keys'
+ * indices (vals need not be filled). */
 int wb_radix_sort_pairs(wb_ctx *c, uint64_t *&keys, uint32_t *&vals, uint64_t *keysAlt, uint32_t *valsAlt,
-                        uint64_t n, int beginBit, int endBit);
+                        uint64_t n, int beginBit, int endBit, uint64_t varying = ~0ull, bool iota = false);
+/* The context's scratch block of counters and flags, cleared when it is made.
+ * The word at WB_SMALL_LOOKBACK is set by a look-back that gave up; the words
+ * after it are the octree build's (wb_build.cu). */
+#define WB_SMALL_LOOKBACK 832
+int wb_small(wb_ctx *c);
+int *wb_lookback_err(wb_ctx *c);
+int wb_lookback_words(wb_ctx *c, uint64_t words, unsigned **counter, unsigned long long **status);
 
 /* stages */
 int wb_point_leaf_map(wb_ctx *c);   /* point -> leaf map into c->pointLeaf */

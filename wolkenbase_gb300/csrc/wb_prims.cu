@@ -1,233 +1,202 @@
 /* Device-wide primitives written for this library: exclusive scan of u32 and
- * a stable LSD radix sort of (u64 key, u32 value) pairs.
+ * a stable LSD radix sort of (u64 key, u32 value) pairs, both in one pass over
+ * the data per step (wb_lookback.cuh).
  *
- * Radix sort: 8-bit digits.  Per pass, one kernel counts digits per tile of
- * 4096 keys, the digit-major count table is scanned, and a second kernel
- * ranks each key inside its tile with warp __match_any_sync groups (stable:
- * a warp walks its 512 keys in order, 32 at a time) and scatters.  Passes
- * whose digit is constant over all keys are skipped.
+ * Radix sort: 8-bit digits.  One kernel counts all passes' digits in one read
+ * of the keys; then each pass is one kernel: a block takes the next tile, ranks
+ * its keys with warp __match_any_sync groups (stable: a warp walks its keys in
+ * order, 32 at a time), publishes the tile's digit counts, puts the tile in
+ * digit order in shared memory, looks back for its digits' places (one thread a
+ * digit) and writes each digit's run with consecutive threads.  A pass over 20M
+ * pairs takes 150-200 us (2.4-3.2 TB/s; issue 43-58%, ranking and look-back);
+ * counting, scanning and scattering in three to five kernels took 220.
  */
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "wb_internal.h"
+#include "wb_lookback.cuh"
 
 namespace
 {
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
-
-__device__ __forceinline__ uint32_t warpInclusive(uint32_t v)
+struct PlainScan
 {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1)
-  {
-    uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o)
-      v += t;
-  }
-  return v;
-}
+  const uint32_t *in;
+  uint32_t *out;
+  __device__ uint32_t value(uint64_t i) const { return in[i]; }
+  __device__ void put(uint64_t i, uint32_t before, uint32_t) const { out[i] = before; }
+};
 
-/* Block-wide exclusive scan of kScanTile values; writes block total. */
-__global__ void scanTiles(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, uint64_t n,
-                          uint32_t *__restrict__ blockSums)
+__global__ void __launch_bounds__(256) scanKernel(uint64_t n, PlainScan f, unsigned *counter, unsigned long long *status,
+                                                  uint32_t *total, int *err)
 {
-  __shared__ uint32_t warpSums[32];
-  uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-  uint32_t v[kScanItems];
-  uint32_t s = 0;
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++)
-  {
-    v[k] = (base + k < n) ? in[base + k] : 0;
-    s += v[k];
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t inc = warpInclusive(s);
-  if (lane == 31)
-    warpSums[warp] = inc;
-  __syncthreads();
-  if (warp == 0)
-  {
-    uint32_t w = warpSums[lane];
-    uint32_t wi = warpInclusive(w);
-    warpSums[lane] = wi - w;
-    if (lane == 31 && blockSums)
-      blockSums[blockIdx.x] = wi;
-  }
-  __syncthreads();
-  uint32_t run = inc - s + warpSums[warp];
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++)
-  {
-    if (base + k < n)
-      out[base + k] = run;
-    run += v[k];
-  }
-}
-
-__global__ void addOffsets(uint32_t *__restrict__ out, uint64_t n, const uint32_t *__restrict__ offs)
-{
-  uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-  uint32_t add = offs[blockIdx.x];
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++)
-    if (base + k < n)
-      out[base + k] += add;
-}
-
-__global__ void totalOf(const uint32_t *in, const uint32_t *ex, uint64_t n, uint32_t *total)
-{
-  *total = n ? ex[n - 1] + in[n - 1] : 0;
+  lookbackScan(n, f, counter, status, total, err);
 }
 
 /* ---------------- radix sort ---------------- */
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortPerLane = 8;
-constexpr int kSortTile = kSortThreads * kSortPerLane;   // 2048
+constexpr int kSortPasses = 8;
 
-__global__ void __launch_bounds__(kSortThreads) digitCounts(const uint64_t *__restrict__ keys, uint64_t n,
-                                                           int shift, uint32_t *__restrict__ counts,
-                                                           int numTiles)
+/* Digit counts of every pass (digits `begin + 8 p` of the keys). */
+__global__ void __launch_bounds__(kSortThreads) radixCounts(const uint64_t *__restrict__ keys, uint64_t n, int begin,
+                                                           int passes, uint32_t *__restrict__ hist)
 {
-  __shared__ uint32_t h[256];
-  for (int i = threadIdx.x; i < 256; i += kSortThreads)
+  __shared__ uint32_t h[kSortPasses * 256];
+  for (int i = threadIdx.x; i < passes * 256; i += kSortThreads)
     h[i] = 0;
   __syncthreads();
-  uint64_t base = (uint64_t)blockIdx.x * kSortTile;
-  for (int k = 0; k < kSortPerLane; k++)
+  for (uint64_t i = (uint64_t)blockIdx.x * kSortThreads + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kSortThreads)
   {
-    uint64_t i = base + (uint64_t)k * kSortThreads + threadIdx.x;
-    if (i < n)
-      atomicAdd(&h[(keys[i] >> shift) & 255], 1u);
+    const uint64_t k = keys[i] >> begin;
+    for (int p = 0; p < passes; p++)
+      atomicAdd(&h[p * 256 + ((k >> (8 * p)) & 255)], 1u);
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += kSortThreads)
-    counts[(uint64_t)d * numTiles + blockIdx.x] = h[d];
+  for (int i = threadIdx.x; i < passes * 256; i += kSortThreads)
+    if (h[i])
+      atomicAdd(&hist[i], h[i]);
 }
 
-/* One stable pass of an 8-bit digit over a tile of kSortTile pairs: warps rank
- * their keys per digit (match_any), the tile is put in digit order in shared
- * memory, and consecutive threads then write consecutive positions of each
- * digit's run, so the global writes coalesce. */
-__global__ void __launch_bounds__(kSortThreads) digitScatter(const uint64_t *__restrict__ keys,
-                                                            const uint32_t *__restrict__ vals, uint64_t n,
-                                                            int shift, const uint32_t *__restrict__ offsets,
-                                                            int numTiles, uint64_t *__restrict__ keysOut,
-                                                            uint32_t *__restrict__ valsOut)
+/* One stable pass of an 8-bit digit; vals NULL: a key's value is its index.
+ * Full tiles (all but the last) run without bounds checks.  The values are read
+ * after the keys are out, so that only the ranks are in registers during the
+ * look-back. */
+template <int ITEMS, typename Word>
+__global__ void __launch_bounds__(kSortThreads, ITEMS == 16 ? 3 : 4)
+    radixPass(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint64_t n, int shift,
+              const uint32_t *__restrict__ hist, unsigned *counter, Word *status, unsigned tag,
+              uint64_t *__restrict__ keysOut, uint32_t *__restrict__ valsOut, int *err)
 {
+  constexpr int TILE = ITEMS * kSortThreads;
   __shared__ uint32_t wcount[kSortWarps][256];
   __shared__ uint32_t localStart[256], globalStart[256];
-  __shared__ uint64_t skeys[kSortTile];
-  __shared__ uint32_t svals[kSortTile];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortThreads)
-    (&wcount[0][0])[i] = 0;
+  __shared__ uint64_t skeys[TILE];   // then the values
+  __shared__ uint32_t warpSums[kSortWarps];
+  __shared__ unsigned tileS;
+  __shared__ int failed;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d0 = threadIdx.x;
+  if (threadIdx.x == 0)
+  {
+    tileS = atomicAdd(counter, 1u);
+    failed = 0;
+  }
+#pragma unroll
+  for (int i = 0; i < kSortWarps; i++)
+    wcount[i][threadIdx.x] = 0;
   __syncthreads();
-  const uint64_t tbase = (uint64_t)blockIdx.x * kSortTile;
-  const uint32_t tileN = (uint32_t)(n - tbase < (uint64_t)kSortTile ? n - tbase : (uint64_t)kSortTile);
-  uint64_t wbase = tbase + (uint64_t)warp * (kSortPerLane * 32);
-  uint64_t k8[kSortPerLane];
-  uint32_t v8[kSortPerLane];
-  uint32_t rank[kSortPerLane];
+  const unsigned tile = tileS;
+  const uint64_t tbase = (uint64_t)tile * TILE;
+  const uint32_t tileN = (uint32_t)(n - tbase < (uint64_t)TILE ? n - tbase : (uint64_t)TILE);
+  const bool full = tileN == TILE;
+  const uint32_t at0 = (uint32_t)warp * (ITEMS * 32) + lane;   // the thread's first item
+  const uint64_t *kin = keys + tbase + at0;
+  uint64_t key[ITEMS];
+  uint32_t at[ITEMS];
   const unsigned lt = (1u << lane) - 1;
-#pragma unroll
-  for (int s = 0; s < kSortPerLane; s++)
+  uint32_t *wc = wcount[warp];
+  if (full)
   {
-    uint64_t i = wbase + (uint64_t)s * 32 + lane;
-    bool ok = i < n;
-    uint64_t key = ok ? keys[i] : 0;
-    k8[s] = key;
-    v8[s] = ok ? vals[i] : 0;
-    uint32_t d = ok ? (uint32_t)((key >> shift) & 255) : 256u;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    uint32_t pre = (d < 256) ? wcount[warp][d] : 0;
-    rank[s] = pre + __popc(peers & lt);
-    __syncwarp();
-    if (d < 256 && (peers & lt) == 0)
-      wcount[warp][d] = pre + __popc(peers);
-    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < ITEMS; s++)
+      key[s] = kin[32 * s];
+#pragma unroll
+    for (int s = 0; s < ITEMS; s++)
+    {
+      const uint32_t d = (uint32_t)(key[s] >> shift) & 255;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);   // a vote per bit took half as many instructions again
+      const uint32_t pre = wc[d];
+      at[s] = pre + __popc(peers & lt);
+      __syncwarp();
+      if ((peers & lt) == 0)
+        wc[d] = pre + __popc(peers);
+      __syncwarp();
+    }
   }
-  __syncthreads();
-  // per digit: exclusive prefix over warps, the tile's total, and where the
-  // digit's run starts in the tile and in the output
-  for (int d = threadIdx.x; d < 256; d += kSortThreads)
+  else
   {
-    uint32_t run = 0;
-    for (int w = 0; w < kSortWarps; w++)
-    {
-      uint32_t c = wcount[w][d];
-      wcount[w][d] = run;
-      run += c;
-    }
-    localStart[d] = run;   // the digit's count for now
-    globalStart[d] = offsets[(uint64_t)d * numTiles + blockIdx.x];
-  }
-  __syncthreads();
-  if (warp == 0)
-  {
-    // exclusive prefix of the 256 digit counts, 8 per lane
-    uint32_t c[8], sum = 0;
 #pragma unroll
-    for (int q = 0; q < 8; q++)
+    for (int s = 0; s < ITEMS; s++)
     {
-      c[q] = localStart[lane * 8 + q];
-      sum += c[q];
-    }
-    uint32_t inc = sum;
-    for (int o = 1; o < 32; o <<= 1)
-    {
-      uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o)
-        inc += v;
-    }
-    uint32_t run = inc - sum;
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-    {
-      localStart[lane * 8 + q] = run;
-      run += c[q];
+      const bool ok = at0 + 32 * s < tileN;
+      key[s] = ok ? kin[32 * s] : 0;
+      const uint32_t d = ok ? (uint32_t)(key[s] >> shift) & 255 : 256u;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t pre = ok ? wc[d & 255] : 0;
+      at[s] = pre + __popc(peers & lt);
+      __syncwarp();
+      if (ok && (peers & lt) == 0)
+        wc[d & 255] = pre + __popc(peers);
+      __syncwarp();
     }
   }
   __syncthreads();
+  // per digit (one thread each): exclusive prefix over the warps and the tile's count
+  uint32_t cnt = 0;
 #pragma unroll
-  for (int s = 0; s < kSortPerLane; s++)
+  for (int w = 0; w < kSortWarps; w++)
   {
-    uint64_t i = wbase + (uint64_t)s * 32 + lane;
-    if (i < n)
+    const uint32_t c = wcount[w][d0];
+    wcount[w][d0] = cnt;
+    cnt += c;
+  }
+  lookbackPut(status + (uint64_t)tile * 256 + d0, DigitWord<Word>::make(tag, tile == 0, cnt));
+  uint32_t total;
+  const uint32_t start = blockExclusive256(cnt, warpSums, total), bin = blockExclusive256(hist[d0], warpSums, total);
+#pragma unroll
+  for (int w = 0; w < kSortWarps; w++)
+    wcount[w][d0] += start;
+  localStart[d0] = start;
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < ITEMS; s++)
+    if (full || at0 + 32 * s < tileN)
     {
-      uint32_t d = (uint32_t)((k8[s] >> shift) & 255);
-      uint32_t lp = localStart[d] + wcount[warp][d] + rank[s];
-      skeys[lp] = k8[s];
-      svals[lp] = v8[s];
+      at[s] += wc[(uint32_t)(key[s] >> shift) & 255];
+      skeys[at[s]] = key[s];
+    }
+  Word before = 0;
+  if (tile && !lookbackColumn<Word, sizeof(Word) == 4 ? 32 : 16>(status + d0, 256, tag, (int64_t)tile, before, err))
+    failed = 1;
+  else if (tile)
+    lookbackPut(status + (uint64_t)tile * 256 + d0, DigitWord<Word>::make(tag, true, before + cnt));
+  globalStart[d0] = bin + (uint32_t)before - start;
+  __syncthreads();
+  if (failed)
+    return;
+  uint32_t pos[ITEMS];
+#pragma unroll
+  for (int s = 0; s < ITEMS; s++)
+  {
+    const uint32_t t = threadIdx.x + s * kSortThreads;
+    if (full || t < tileN)
+    {
+      const uint64_t k = skeys[t];
+      pos[s] = globalStart[(uint32_t)(k >> shift) & 255] + t;
+      if (pos[s] < n)
+        keysOut[pos[s]] = k;
     }
   }
+  uint32_t val[ITEMS];
+  const uint32_t *vin = vals + tbase + at0;
+#pragma unroll
+  for (int s = 0; s < ITEMS; s++)
+    val[s] = vals ? (full || at0 + 32 * s < tileN ? vin[32 * s] : 0u) : (uint32_t)tbase + at0 + 32 * s;
   __syncthreads();
-  for (uint32_t t = threadIdx.x; t < tileN; t += kSortThreads)
+  uint32_t *svals = (uint32_t *)skeys;
+#pragma unroll
+  for (int s = 0; s < ITEMS; s++)
+    if (full || at0 + 32 * s < tileN)
+      svals[at[s]] = val[s];
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < ITEMS; s++)
   {
-    uint64_t key = skeys[t];
-    uint32_t d = (uint32_t)((key >> shift) & 255);
-    uint32_t pos = globalStart[d] + (t - localStart[d]);
-    keysOut[pos] = key;
-    valsOut[pos] = svals[t];
+    const uint32_t t = threadIdx.x + s * kSortThreads;
+    if ((full || t < tileN) && pos[s] < n)
+      valsOut[pos[s]] = svals[t];
   }
 }
 
-/* Bits that differ between any key and keys[0]. */
-__global__ void keySpread(const uint64_t *__restrict__ keys, uint64_t n, unsigned long long *orBits)
-{
-  uint64_t first = keys[0];
-  uint64_t acc = 0;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    acc |= keys[i] ^ first;
-  for (int o = 16; o; o >>= 1)
-    acc |= __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0 && acc)
-    atomicOr(orBits, (unsigned long long)acc);
-}
 __global__ void pullKernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, uint64_t n16)
 {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += (uint64_t)gridDim.x * blockDim.x)
@@ -282,82 +251,92 @@ bool wb_device_accessible(const void *p)
          (at.type == cudaMemoryTypeHost && at.devicePointer == p);
 }
 
+int wb_small(wb_ctx *c)
+{
+  if (c->small.p)
+    return 0;
+  int rc = wb_ensure(c, c->small, 4096);
+  if (rc)
+    return rc;
+  WB_CUDA(c, cudaMemsetAsync(c->small.p, 0, 4096, c->stream));
+  return 0;
+}
+
+int *wb_lookback_err(wb_ctx *c)
+{
+  return (int *)((char *)c->small.p + WB_SMALL_LOOKBACK);
+}
+
+/* Counter and status words of a look-back sequence of `words` words, cleared. */
+int wb_lookback_words(wb_ctx *c, uint64_t words, unsigned **counter, unsigned long long **status)
+{
+  int rc = wb_small(c);
+  if (rc || (rc = wb_ensure(c, c->scanTmp, words * 8 + 64)))
+    return rc;
+  WB_CUDA(c, cudaMemsetAsync(c->scanTmp.p, 0, words * 8 + 64, c->stream));
+  *counter = (unsigned *)c->scanTmp.p;
+  *status = (unsigned long long *)((char *)c->scanTmp.p + 64);
+  return 0;
+}
+
 int wb_exclusive_scan_u32(wb_ctx *c, const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *total_dev)
 {
   if (n == 0)
     return 0;
-  uint64_t tiles = (n + kScanTile - 1) / kScanTile;
-  if (tiles == 1)
-  {
-    { scanTiles<<<1, kScanThreads, 0, c->stream>>>(in, out, n, nullptr); ++c->launches; }
-  }
-  else
-  {
-    // block sums live in a scratch region carved per recursion level
-    uint64_t need = 0;
-    for (uint64_t t = tiles; t > 1; t = (t + kScanTile - 1) / kScanTile)
-      need += 2 * t;
-    int rc = wb_ensure(c, c->scanTmp, (need + 64) * sizeof(uint32_t));
-    if (rc)
-      return rc;
-    uint32_t *sums = (uint32_t *)c->scanTmp.p;
-    uint32_t *sumsEx = sums + tiles;
-    { scanTiles<<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(in, out, n, sums); ++c->launches; }
-    // recurse on the block sums (their scratch follows)
-    DevBuf saved = c->scanTmp;
-    // shift scratch window for the nested call
-    c->scanTmp.p = (void *)(sumsEx + tiles);
-    c->scanTmp.cap = saved.cap - 2 * tiles * sizeof(uint32_t);
-    rc = wb_exclusive_scan_u32(c, sums, sumsEx, tiles, nullptr);
-    c->scanTmp = saved;
-    if (rc)
-      return rc;
-    { addOffsets<<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(out, n, sumsEx); ++c->launches; }
-  }
-  if (total_dev)
-    { totalOf<<<1, 1, 0, c->stream>>>(in, out, n, total_dev); ++c->launches; }
+  const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
+  unsigned *counter;
+  unsigned long long *status;
+  int rc = wb_lookback_words(c, tiles, &counter, &status);
+  if (rc)
+    return rc;
+  { scanKernel<<<(unsigned)tiles, 256, 0, c->stream>>>(n, PlainScan{in, out}, counter, status, total_dev,
+                                                       wb_lookback_err(c)); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
   return 0;
 }
 
 int wb_radix_sort_pairs(wb_ctx *c, uint64_t *&keys, uint32_t *&vals, uint64_t *keysAlt, uint32_t *valsAlt,
-                        uint64_t n, int beginBit, int endBit)
+                        uint64_t n, int beginBit, int endBit, uint64_t varying, bool iota)
 {
-  if (n <= 1)
+  if (n <= 1 && !iota)
     return 0;
-  int rc = wb_ensure(c, c->small, 4096);
-  if (rc)
+  const int passes = (endBit - beginBit + 7) / 8;
+  // keys a tile: enough tiles to fill the GPU, else large ones (fewer look-backs)
+  const int items = n >= (1ull << 21) ? 16 : (n >= (1ull << 19) ? 8 : 4);
+  const uint64_t tiles = (n + (uint64_t)items * kSortThreads - 1) / ((uint64_t)items * kSortThreads);
+  const size_t head = kSortPasses * 256 * 4 + 64;   // digit counts, tile counters
+  const bool small = n < (1ull << 26);
+  const size_t words = tiles * 256 * (small ? 4 : 8);
+  int rc = wb_small(c);
+  if (rc || (rc = wb_ensure(c, c->scanTmp, head + words + 64)))
     return rc;
-  unsigned long long *dOr = (unsigned long long *)c->small.p;
-  WB_CUDA(c, cudaMemsetAsync(dOr, 0, 8, c->stream));
-  { keySpread<<<c->sm_count * 4, 256, 0, c->stream>>>(keys, n, dOr); ++c->launches; }
-  unsigned long long spread = 0;
-  WB_CUDA(c, cudaMemcpyAsync(&spread, dOr, 8, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  int numTiles = (int)((n + kSortTile - 1) / kSortTile);
-  size_t cntBytes = (size_t)numTiles * 256 * sizeof(uint32_t);
-  rc = wb_ensure(c, c->tmp32b, 2 * cntBytes + 64);
-  if (rc)
-    return rc;
-  uint32_t *counts = (uint32_t *)c->tmp32b.p;
-  uint32_t *offs = counts + (size_t)numTiles * 256;
-  for (int shift = beginBit; shift < endBit; shift += 8)
+  uint32_t *hist = (uint32_t *)c->scanTmp.p;
+  unsigned *counter = (unsigned *)(hist + kSortPasses * 256);
+  void *status = (char *)c->scanTmp.p + head;
+  WB_CUDA(c, cudaMemsetAsync(c->scanTmp.p, 0, head + words, c->stream));
+  { radixCounts<<<(unsigned)std::min<uint64_t>((n + 2047) / 2048, (uint64_t)c->sm_count * 4), kSortThreads, 0,
+                  c->stream>>>(keys, n, beginBit, passes, hist); ++c->launches; }
+  int *err = wb_lookback_err(c);
+  const uint32_t *in = iota ? nullptr : vals;
+  for (int p = 0; p < passes; p++)
   {
-    uint64_t mask = (shift + 8 >= 64) ? (~0ULL << shift) : (((1ULL << 8) - 1) << shift);
-    if ((spread & mask) == 0)
-      continue;   // digit identical for all keys: pass would be the identity
-    { digitCounts<<<numTiles, kSortThreads, 0, c->stream>>>(keys, n, shift, counts, numTiles); ++c->launches; }
-    rc = wb_exclusive_scan_u32(c, counts, offs, (uint64_t)numTiles * 256, nullptr);
-    if (rc)
-      return rc;
-    { digitScatter<<<numTiles, kSortThreads, 0, c->stream>>>(keys, vals, n, shift, offs, numTiles, keysAlt, valsAlt); ++c->launches; }
-    WB_CUDA(c, cudaGetLastError());
-    uint64_t *tk = keys;
-    keys = keysAlt;
-    keysAlt = tk;
-    uint32_t *tv = vals;
-    vals = valsAlt;
-    valsAlt = tv;
+    const int shift = beginBit + 8 * p;
+    if (!((varying >> shift) & 255) && in)
+      continue;   // digit the same for all keys: the pass would be the identity
+    auto launch = [&](auto pass, auto *words) {
+      pass<<<(unsigned)tiles, kSortThreads, 0, c->stream>>>(keys, in, n, shift, hist + p * 256, counter + p, words,
+                                                            (unsigned)p + 1, keysAlt, valsAlt, err);
+      ++c->launches;
+    };
+    if (small)
+      launch(items == 16 ? radixPass<16, uint32_t> : (items == 8 ? radixPass<8, uint32_t> : radixPass<4, uint32_t>),
+             (uint32_t *)status);
+    else
+      launch(radixPass<16, unsigned long long>, (unsigned long long *)status);
+    std::swap(keys, keysAlt);
+    std::swap(vals, valsAlt);
+    in = vals;
   }
+  WB_CUDA(c, cudaGetLastError());
   return 0;
 }

@@ -1,9 +1,9 @@
 /* Tile stage on the GPU: cylinder gathers, scanCylinder and postscanCylinder.
  *
  * Tile cylinders (Flowsnake::cyl, flowsnake.cpp:263-271) are gathered by one
- * warp per tile walking the node hierarchy depth-first in child order 0..7,
- * which visits leaves in the order Octree::findBlocks lists blocks; inside a
- * leaf, points are taken in store order.  That is the order
+ * warp per tile from the grid columns they meet and put in store order: leaves
+ * depth-first, the order Octree::findBlocks lists blocks, and inside a leaf
+ * input order.  That is the order
  * OctStore::pointsIn returns (octree.cpp:1214-1242) when each block holds its
  * points in input order, so the per-tile sums below are formed in the same
  * sequence as the reference's and the plane fit, the untilt and the
@@ -30,8 +30,6 @@ struct TileArgs
   uint64_t T;
   double cx, cy, spacing, rad;
   double off[3], scale[3], unit;
-  const int32_t *child, *nodeBox, *leafBox;
-  uint64_t N, L;
   const uint32_t *leafFirst, *leafCount;
   const uint64_t *leafKey;
   const uint8_t *leafLev;
@@ -1345,11 +1343,6 @@ static TileArgs tileArgs(wb_ctx *c)
     a.scale[k] = g.scale[k];
   }
   a.unit = g.unit;
-  a.child = (const int32_t *)c->nodeChild.p;
-  a.nodeBox = (const int32_t *)c->nodeBox.p;
-  a.leafBox = (const int32_t *)c->leafBox.p;
-  a.N = c->n_nodes;
-  a.L = c->n_leaves;
   a.leafFirst = (const uint32_t *)c->leafFirst.p;
   a.leafCount = (const uint32_t *)c->leafCount.p;
   a.leafKey = (const uint64_t *)c->leafKey.p;
@@ -1407,7 +1400,9 @@ static int sortHugeTiles(wb_ctx *c, uint32_t nh, const uint32_t *tileStart)
   int bits = 1;
   while ((1ull << bits) < nh)
     bits++;
-  if ((rc = wb_radix_sort_pairs(c, keys, vals, (uint64_t *)c->key1.p, (uint32_t *)c->idx1.p, total, 0, 32 + bits)))
+  // the keys' store positions and tile ranks have no more bits than these
+  const uint64_t varying = (((1ull << bits) - 1) << 32) | ((1ull << (64 - __builtin_clzll(c->nd | 1))) - 1);
+  if ((rc = wb_radix_sort_pairs(c, keys, vals, (uint64_t *)c->key1.p, (uint32_t *)c->idx1.p, total, 0, 32 + bits, varying)))
     return rc;
   { hugeBackKernel<<<g, 256, 0, c->stream>>>(nh, (const uint32_t *)c->tileHuge.p, tileStart, (const uint64_t *)c->hugePre.p,
                                              keys, (uint32_t *)c->tilePts.p); ++c->launches; }
@@ -1481,7 +1476,7 @@ int wb_scan_impl(wb_ctx *c, const wb_params *p)
   uint64_t T = c->n_tiles, nd = c->nd;
   if ((rc = wb_ensure(c, c->tileN, T * 4 + 64)) || (rc = wb_ensure(c, c->tileStart, (T + 1) * 4 + 64)) ||
       (rc = wb_ensure(c, c->owner, nd * 4 + 64)) || (rc = wb_ensure(c, c->tileRes, T * sizeof(TileRes) + 64)) ||
-      (rc = wb_ensure(c, c->tileH, T * 8 + 64)) || (rc = wb_ensure(c, c->small, 4096)))
+      (rc = wb_ensure(c, c->tileH, T * 8 + 64)) || (rc = wb_small(c)))
     return rc;
   TileArgs a = tileArgs(c);
   GridDev gd;
