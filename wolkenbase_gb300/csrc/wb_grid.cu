@@ -99,56 +99,75 @@ __device__ __forceinline__ int columnOf(const long long *__restrict__ b, int n, 
 }
 
 __global__ void cellKernel(GridArgs g, const int32_t *__restrict__ sx, const int32_t *__restrict__ sy,
-                           const int32_t *__restrict__ sz, uint64_t *__restrict__ key, uint32_t *__restrict__ val,
+                           const int32_t *__restrict__ sz, uint32_t *__restrict__ count, uint32_t *__restrict__ rank,
                            uint8_t *__restrict__ stray, unsigned long long *__restrict__ nStray,
                            int *__restrict__ ext, const double *__restrict__ xyzd, int2 *__restrict__ colOf)
 {
   // record-integer extent of the points ({min x, y, z}, {max x, y, z})
   int mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < g.nd; j += (uint64_t)gridDim.x * blockDim.x)
+  // whole warps step together, for the counts' runs
+  const int lane = threadIdx.x & 31;
+  for (uint64_t j0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < g.nd; j0 += (uint64_t)gridDim.x * blockDim.x)
   {
-    const int q[3] = {sx[j], sy[j], sz[j]};
-    for (int a = 0; a < 3; a++)
+    const uint64_t j = j0 + lane;
+    uint32_t cell = 0xffffffffu;
+    if (j < g.nd)
     {
-      mn[a] = min(mn[a], q[a]);
-      mx[a] = max(mx[a], q[a]);
-    }
-    // the point's column as the classify set-up needs it (unclamped, within
-    // +-1e9), and clamped into the grid for the sort key; from the integer
-    // thresholds where they apply, else in FP64
-    int ci, cj;
-    bool sxy, s;
-    if (g.thr)
-    {
-      const long long *xb = g.bounds, *yb = g.bounds + g.nx + 1, *face = g.bounds + g.nx + g.ny + 2;
-      const long long X = q[0], Y = q[1], Z = q[2];
-      if (X >= xb[0] && X < xb[g.nx])
-        ci = columnOf(xb, g.nx, X, g.colPerUnit[0]);
+      const int q[3] = {sx[j], sy[j], sz[j]};
+      for (int a = 0; a < 3; a++)
+      {
+        mn[a] = min(mn[a], q[a]);
+        mx[a] = max(mx[a], q[a]);
+      }
+      // the point's column as the classify set-up needs it (unclamped, within
+      // +-1e9), and clamped into the grid for the sort key; from the integer
+      // thresholds where they apply, else in FP64
+      int ci, cj;
+      bool sxy, s;
+      if (g.thr)
+      {
+        const long long *xb = g.bounds, *yb = g.bounds + g.nx + 1, *face = g.bounds + g.nx + g.ny + 2;
+        const long long X = q[0], Y = q[1], Z = q[2];
+        if (X >= xb[0] && X < xb[g.nx])
+          ci = columnOf(xb, g.nx, X, g.colPerUnit[0]);
+        else
+          ci = (int)fmax(fmin(floor((xyzd[j] - g.x0) / g.cell), 1e9), -1e9);
+        if (Y >= yb[0] && Y < yb[g.ny])
+          cj = columnOf(yb, g.ny, Y, g.colPerUnit[1]);
+        else
+          cj = (int)fmax(fmin(floor((xyzd[g.nd + j] - g.y0) / g.cell), 1e9), -1e9);
+        sxy = X < face[0] || Y < face[1] || X >= face[3] || Y >= face[4];
+        s = sxy || Z < face[2] || Z >= face[5];
+      }
       else
-        ci = (int)fmax(fmin(floor((xyzd[j] - g.x0) / g.cell), 1e9), -1e9);
-      if (Y >= yb[0] && Y < yb[g.ny])
-        cj = columnOf(yb, g.ny, Y, g.colPerUnit[1]);
-      else
-        cj = (int)fmax(fmin(floor((xyzd[g.nd + j] - g.y0) / g.cell), 1e9), -1e9);
-      sxy = X < face[0] || Y < face[1] || X >= face[3] || Y >= face[4];
-      s = sxy || Z < face[2] || Z >= face[5];
+      {
+        const double x = xyzd[j], y = xyzd[g.nd + j], z = xyzd[2 * g.nd + j];
+        ci = (int)fmax(fmin(floor((x - g.x0) / g.cell), 1e9), -1e9);
+        cj = (int)fmax(fmin(floor((y - g.y0) / g.cell), 1e9), -1e9);
+        sxy = x < g.rootLo[0] || y < g.rootLo[1] || x >= g.rootHi[0] || y >= g.rootHi[1];
+        s = sxy || z < g.rootLo[2] || z >= g.rootHi[2];
+      }
+      colOf[j] = make_int2(ci, cj);
+      const int cx = min(max(ci, 0), g.nx - 1), cy = min(max(cj, 0), g.ny - 1);
+      cell = (uint32_t)cy * (uint32_t)g.nx + cx;
+      stray[j] = (uint8_t)((s ? 1 : 0) | (sxy ? 2 : 0));
+      if (s)
+        atomicAdd(nStray, 1ull);
     }
-    else
-    {
-      const double x = xyzd[j], y = xyzd[g.nd + j], z = xyzd[2 * g.nd + j];
-      ci = (int)fmax(fmin(floor((x - g.x0) / g.cell), 1e9), -1e9);
-      cj = (int)fmax(fmin(floor((y - g.y0) / g.cell), 1e9), -1e9);
-      sxy = x < g.rootLo[0] || y < g.rootLo[1] || x >= g.rootHi[0] || y >= g.rootHi[1];
-      s = sxy || z < g.rootLo[2] || z >= g.rootHi[2];
-    }
-    colOf[j] = make_int2(ci, cj);
-    const int cx = min(max(ci, 0), g.nx - 1), cy = min(max(cj, 0), g.ny - 1);
-    // column in the high 32 bits, height (order-preserving int32 -> uint32) below
-    key[j] = (((uint64_t)cy * g.nx + cx) << 32) | (uint32_t)(q[2] ^ (int32_t)0x80000000);
-    val[j] = (uint32_t)j;
-    stray[j] = (uint8_t)((s ? 1 : 0) | (sxy ? 2 : 0));
-    if (s)
-      atomicAdd(nStray, 1ull);
+    // the point's place among its column's points: the store order is local,
+    // so neighbouring lanes share columns and each run of them takes its
+    // places with one atomic
+    const uint32_t left = __shfl_up_sync(0xffffffffu, cell, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || cell != left);
+    const int head = 31 - __clz(heads & ((2u << lane) - 1));
+    const unsigned after = lane == 31 ? 0u : heads >> (lane + 1);
+    const int len = (after ? lane + __ffs(after) : 32) - head;
+    uint32_t base = 0;
+    if (lane == head && j < g.nd)
+      base = atomicAdd(&count[cell], (uint32_t)len);
+    base = __shfl_sync(0xffffffffu, base, head);
+    if (j < g.nd)
+      rank[j] = base + (uint32_t)(lane - head);
   }
   for (int a = 0; a < 3; a++)
     for (int o = 16; o; o >>= 1)
@@ -164,44 +183,47 @@ __global__ void cellKernel(GridArgs g, const int32_t *__restrict__ sx, const int
     }
 }
 
-__global__ void cellStartKernel(uint64_t nd, uint64_t ncell, const uint64_t *__restrict__ key,
-                                uint32_t *__restrict__ start)
+__device__ __forceinline__ uint32_t cellOf(int2 col, int nx, int ny)
 {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nd; i += (uint64_t)gridDim.x * blockDim.x)
-  {
-    uint64_t k = key[i] >> 32;
-    uint64_t prev = i ? key[i - 1] >> 32 : (uint64_t)-1;
-    if (i == 0)
-      for (uint64_t c = 0; c <= k; c++)
-        start[c] = 0;
-    else if (k != prev)
-      for (uint64_t c = prev + 1; c <= k; c++)
-        start[c] = (uint32_t)i;
-    if (i == nd - 1)
-      for (uint64_t c = k + 1; c <= ncell; c++)
-        start[c] = (uint32_t)nd;
-  }
+  return (uint32_t)min(max(col.y, 0), ny - 1) * (uint32_t)nx + (uint32_t)min(max(col.x, 0), nx - 1);
 }
 
-/* Gathers the points into column order as int4 {X, Y, Z, position} and
- * forms each column's record; one warp per column. */
-__global__ void cellFillKernel(uint64_t ncell, const uint32_t *__restrict__ start, const uint32_t *__restrict__ pos,
-                               const int32_t *__restrict__ sx, const int32_t *__restrict__ sy,
-                               const int32_t *__restrict__ sz, const uint8_t *__restrict__ stray,
-                               int4 *__restrict__ gpt, int4 *__restrict__ rec)
+/* Order of a column's points: by height, then store position. */
+__device__ __forceinline__ uint64_t heightKey(int32_t z, uint64_t j)
 {
-  uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (c >= ncell)
-    return;
-  uint32_t b = start[c], e = start[c + 1];
-  int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-  bool xyStray = false;
-  for (uint32_t i = b + lane; i < e; i += 32)
+  return ((uint64_t)(uint32_t)(z ^ (int32_t)0x80000000) << 32) | (uint32_t)j;
+}
+
+/* Puts every point's (height, store position) at its place in its column. */
+__global__ void cellScatterKernel(uint64_t nd, int nx, int ny, const int2 *__restrict__ colOf,
+                                  const uint32_t *__restrict__ rank, const uint32_t *__restrict__ start,
+                                  const int32_t *__restrict__ sz, uint64_t *__restrict__ slots)
+{
+  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += (uint64_t)gridDim.x * blockDim.x)
+    slots[start[cellOf(colOf[j], nx, ny)] + rank[j]] = heightKey(sz[j], j);
+}
+
+/* The same as sort keys, for the radix sort: the column above. */
+__global__ void cellKeyKernel(uint64_t nd, int nx, int ny, const int2 *__restrict__ colOf, const int32_t *__restrict__ sz,
+                              uint64_t *__restrict__ key)
+{
+  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += (uint64_t)gridDim.x * blockDim.x)
+    key[j] = ((uint64_t)cellOf(colOf[j], nx, ny) << 32) | (uint32_t)(sz[j] ^ (int32_t)0x80000000);
+}
+
+/* Gathers a column's points, in the order of `at(i)` (store positions), as
+ * int4 {X, Y, Z, position} and forms the column's record. */
+template <typename At>
+__device__ __forceinline__ void fillColumn(uint64_t c, uint32_t b, uint32_t e, int lane, int lanes, At at,
+                                           const int32_t *__restrict__ sx, const int32_t *__restrict__ sy,
+                                           const int32_t *__restrict__ sz, const uint8_t *__restrict__ stray,
+                                           int4 *__restrict__ gpt, int32_t mn[3], int32_t mx[3], bool &xyStray)
+{
+  for (uint32_t i = b + lane; i < e; i += lanes)
   {
-    uint32_t j = pos[i];
-    int32_t q[3] = {sx[j], sy[j], sz[j]};
-    uint8_t st = stray[j];
+    const uint32_t j = at(i);
+    const int32_t q[3] = {sx[j], sy[j], sz[j]};
+    const uint8_t st = stray[j];
     gpt[i] = make_int4(q[0], q[1], q[2], (int)(j | ((st & 1) ? 0x80000000u : 0u)));
     xyStray |= (st & 2) != 0;
     for (int a = 0; a < 3; a++)
@@ -210,19 +232,204 @@ __global__ void cellFillKernel(uint64_t ncell, const uint32_t *__restrict__ star
       mx[a] = max(mx[a], q[a]);
     }
   }
+}
+
+/* Warp-wide part of a column's record; lane 0 writes it. */
+__device__ __forceinline__ void writeColumn(uint64_t c, uint32_t b, uint32_t e, int lane, int32_t mn[3], int32_t mx[3],
+                                            bool xyStray, int4 *__restrict__ rec)
+{
   for (int a = 0; a < 3; a++)
-    for (int o = 16; o; o >>= 1)
-    {
-      mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-      mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
-    }
+  {
+    mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
+    mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
+  }
   // a column holding a point outside the root cube in x or y is read in full
-  unsigned any = __ballot_sync(0xffffffffu, xyStray);
+  const bool any = __any_sync(0xffffffffu, xyStray);
   if (lane == 0)
   {
     rec[2 * c] = make_int4(mn[0], mn[1], mx[0], mx[1]);
     rec[2 * c + 1] = make_int4(mn[2], (int)b, (int)e, any ? 1 : 0);
   }
+}
+
+/* Sorts and fills the columns, one warp each: up to 64 points in registers, two
+ * a lane, up to kColumnMax in shared memory; larger columns are listed for
+ * bigColumnKernel.  Replaces the radix sort of all points by (column, height)
+ * where columns are of ordinary size: five passes over 12-byte pairs. */
+constexpr int kColumnWarps = 4, kColumnMax = 512, kBigColumnMax = 4096;
+__global__ void __launch_bounds__(32 * kColumnWarps) columnKernel(uint64_t ncell, const uint32_t *__restrict__ start,
+                                                                  const uint64_t *__restrict__ slots,
+                                                                  const int32_t *__restrict__ sx,
+                                                                  const int32_t *__restrict__ sy,
+                                                                  const int32_t *__restrict__ sz,
+                                                                  const uint8_t *__restrict__ stray,
+                                                                  int4 *__restrict__ gpt, int4 *__restrict__ rec,
+                                                                  uint32_t *__restrict__ big, uint32_t *__restrict__ nBig)
+{
+  __shared__ uint64_t buf[kColumnWarps][kColumnMax];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint64_t c = (uint64_t)blockIdx.x * kColumnWarps + w;
+  if (c >= ncell)
+    return;
+  const uint32_t b = start[c], e = start[c + 1], n = e - b;
+  int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+  bool xyStray = false;
+  uint64_t *k = buf[w];
+  if (n > kColumnMax)
+  {
+    if (lane == 0)
+      big[atomicAdd(nBig, 1u)] = (uint32_t)c;
+    return;
+  }
+  if (n <= 64)
+  {
+    // bitonic over 64 keys, element lane + 32 r in register r
+    uint64_t v[2];
+    v[0] = (uint32_t)lane < n ? slots[b + lane] : ~0ull;
+    v[1] = (uint32_t)lane + 32 < n ? slots[b + 32 + lane] : ~0ull;
+    auto exchange = [&](uint64_t &x, int j, bool up) {
+      const uint64_t y = __shfl_xor_sync(0xffffffffu, x, j);
+      const bool low = !(lane & j);
+      x = ((x < y) == (low == up)) ? x : y;
+    };
+    if (n > 1)
+    {
+#pragma unroll
+      for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+        for (int j = size >> 1; j > 0; j >>= 1)
+        {
+          exchange(v[0], j, size == 32 || !(lane & size));
+          exchange(v[1], j, size == 32 ? false : !(lane & size));
+        }
+      if (n > 32)
+      {
+        const uint64_t lo = v[0] < v[1] ? v[0] : v[1], hi = v[0] < v[1] ? v[1] : v[0];
+        v[0] = lo;
+        v[1] = hi;
+#pragma unroll
+        for (int j = 16; j > 0; j >>= 1)
+        {
+          exchange(v[0], j, true);
+          exchange(v[1], j, true);
+        }
+      }
+    }
+    k[lane] = v[0];
+    k[lane + 32] = v[1];
+    __syncwarp();
+  }
+  else
+  {
+    int P = 128;
+    while (P < (int)n)
+      P <<= 1;
+    for (int q = lane; q < P; q += 32)
+      k[q] = q < (int)n ? slots[b + q] : ~0ull;
+    __syncwarp();
+    for (int size = 2; size <= P; size <<= 1)
+      for (int j = size >> 1; j > 0; j >>= 1)
+      {
+        for (int t = lane; t < P / 2; t += 32)
+        {
+          const int i = 2 * t - (t & (j - 1)), u = i + j;
+          const uint64_t x = k[i], y = k[u];
+          if ((x > y) == ((i & size) == 0))
+          {
+            k[i] = y;
+            k[u] = x;
+          }
+        }
+        __syncwarp();
+      }
+  }
+  fillColumn(c, b, e, lane, 32, [&](uint32_t i) { return (uint32_t)k[i - b]; }, sx, sy, sz, stray, gpt, mn, mx, xyStray);
+  writeColumn(c, b, e, lane, mn, mx, xyStray, rec);
+}
+
+/* The listed columns, one block each, up to kBigColumnMax points in shared
+ * memory; a larger one raises *unsorted and the caller sorts by radix passes. */
+__global__ void __launch_bounds__(512) bigColumnKernel(const uint32_t *__restrict__ big, const uint32_t *__restrict__ nBig,
+                                                       const uint32_t *__restrict__ start,
+                                                       const uint64_t *__restrict__ slots, const int32_t *__restrict__ sx,
+                                                       const int32_t *__restrict__ sy, const int32_t *__restrict__ sz,
+                                                       const uint8_t *__restrict__ stray, int4 *__restrict__ gpt,
+                                                       int4 *__restrict__ rec, uint32_t *__restrict__ unsorted)
+{
+  __shared__ uint64_t k[kBigColumnMax];
+  __shared__ int32_t ext[6];
+  __shared__ int flag;
+  const uint32_t nb = *nBig;
+  for (uint32_t r = blockIdx.x; r < nb; r += gridDim.x)
+  {
+    const uint32_t c = big[r], b = start[c], e = start[c + 1], n = e - b;
+    __syncthreads();
+    if (n > kBigColumnMax)
+    {
+      if (threadIdx.x == 0)
+        *unsorted = 1;
+      continue;
+    }
+    int P = 1024;
+    while (P < (int)n)
+      P <<= 1;
+    for (int q = threadIdx.x; q < P; q += 512)
+      k[q] = q < (int)n ? slots[b + q] : ~0ull;
+    if (threadIdx.x < 6)
+      ext[threadIdx.x] = threadIdx.x < 3 ? INT32_MAX : INT32_MIN;
+    if (threadIdx.x == 0)
+      flag = 0;
+    __syncthreads();
+    for (int size = 2; size <= P; size <<= 1)
+      for (int j = size >> 1; j > 0; j >>= 1)
+      {
+        for (int t = threadIdx.x; t < P / 2; t += 512)
+        {
+          const int i = 2 * t - (t & (j - 1)), u = i + j;
+          const uint64_t x = k[i], y = k[u];
+          if ((x > y) == ((i & size) == 0))
+          {
+            k[i] = y;
+            k[u] = x;
+          }
+        }
+        __syncthreads();
+      }
+    int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+    bool xyStray = false;
+    fillColumn(c, b, e, (int)threadIdx.x, 512, [&](uint32_t i) { return (uint32_t)k[i - b]; }, sx, sy, sz, stray, gpt, mn, mx,
+               xyStray);
+    for (int a = 0; a < 3; a++)
+    {
+      atomicMin(&ext[a], mn[a]);
+      atomicMax(&ext[3 + a], mx[a]);
+    }
+    if (xyStray)
+      flag = 1;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+      rec[2 * (uint64_t)c] = make_int4(ext[0], ext[1], ext[3], ext[4]);
+      rec[2 * (uint64_t)c + 1] = make_int4(ext[2], (int)b, (int)e, flag);
+    }
+  }
+}
+
+/* Fills columns whose points are already in order (pos), one warp each. */
+__global__ void cellFillKernel(uint64_t ncell, const uint32_t *__restrict__ start, const uint32_t *__restrict__ pos,
+                               const int32_t *__restrict__ sx, const int32_t *__restrict__ sy,
+                               const int32_t *__restrict__ sz, const uint8_t *__restrict__ stray,
+                               int4 *__restrict__ gpt, int4 *__restrict__ rec)
+{
+  const uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (c >= ncell)
+    return;
+  const uint32_t b = start[c], e = start[c + 1];
+  int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+  bool xyStray = false;
+  fillColumn(c, b, e, lane, 32, [&](uint32_t i) { return pos[i]; }, sx, sy, sz, stray, gpt, mn, mx, xyStray);
+  writeColumn(c, b, e, lane, mn, mx, xyStray, rec);
 }
 
 /* Column groups (the work items of the margin pass): a column of n points is
@@ -488,7 +695,7 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
   int rc;
   if ((rc = wb_ensure(c, c->gKey0, nd * 8 + 64)) || (rc = wb_ensure(c, c->gKey1, nd * 8 + 64)) ||
       (rc = wb_ensure(c, c->gVal0, nd * 4 + 64)) || (rc = wb_ensure(c, c->gVal1, nd * 4 + 64)) ||
-      (rc = wb_ensure(c, c->stray, nd + 64)) || (rc = wb_ensure(c, c->cellStart, (ncell + 1) * 4 + 64)) ||
+      (rc = wb_ensure(c, c->stray, nd + 64)) || (rc = wb_ensure(c, c->cellStart, (ncell + 1) * 8 + 64)) ||
       (rc = wb_ensure(c, c->gpt, nd * 16 + 64)) || (rc = wb_ensure(c, c->cellRec, ncell * 32 + 64)) ||
       (rc = wb_ensure(c, c->colOf, nd * 8 + 64)))
     return rc;
@@ -518,21 +725,49 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
   WB_CUDA(c, cudaMemsetAsync(dStray, 0, 8, c->stream));
   WB_CUDA(c, cudaMemcpyAsync(dExt, kExtInit, 24, cudaMemcpyDefault, c->stream));
   unsigned blocks = (unsigned)std::min<uint64_t>((nd + 255) / 256 + 1, (uint64_t)c->sm_count * 16);
-  uint64_t *key = (uint64_t *)c->gKey0.p;
-  uint32_t *val = (uint32_t *)c->gVal0.p;
-  { cellKernel<<<blocks, 256, 0, c->stream>>>(a, (const int32_t *)c->sx.p, (const int32_t *)c->sy.p,
-                                              (const int32_t *)c->sz.p, key, val, (uint8_t *)c->stray.p, dStray,
-                                              dExt, (const double *)c->xyzd.p, (int2 *)c->colOf.p); ++c->launches; }
-  int bits = 1;
-  while ((1ull << bits) < ncell)
-    bits++;
-  if ((rc = wb_radix_sort_pairs(c, key, val, (uint64_t *)c->gKey1.p, (uint32_t *)c->gVal1.p, nd, 0, 32 + bits)))
+  // a counting sort by column (counts, their prefix, the points' places), then
+  // each column by height
+  uint32_t *start = (uint32_t *)c->cellStart.p, *count = start + ncell + 1, *rank = (uint32_t *)c->gVal0.p;
+  uint32_t *dBig = (uint32_t *)((char *)c->small.p + 640);   // big columns, and whether one was too big
+  uint64_t *slots = (uint64_t *)c->gKey0.p;
+  const int32_t *sx = (const int32_t *)c->sx.p, *sy = (const int32_t *)c->sy.p, *sz = (const int32_t *)c->sz.p;
+  const uint8_t *stray = (const uint8_t *)c->stray.p;
+  const int2 *colOf = (const int2 *)c->colOf.p;
+  int4 *gpt = (int4 *)c->gpt.p, *cellRec = (int4 *)c->cellRec.p;
+  WB_CUDA(c, cudaMemsetAsync(count, 0, (ncell + 1) * 4, c->stream));
+  WB_CUDA(c, cudaMemsetAsync(dBig, 0, 8, c->stream));
+  { cellKernel<<<blocks, 256, 0, c->stream>>>(a, sx, sy, sz, count, rank, (uint8_t *)c->stray.p, dStray, dExt,
+                                              (const double *)c->xyzd.p, (int2 *)c->colOf.p); ++c->launches; }
+  if ((rc = wb_exclusive_scan_u32(c, count, start, ncell + 1, nullptr)))
     return rc;
-  uint32_t *start = (uint32_t *)c->cellStart.p;
-  { cellStartKernel<<<blocks, 256, 0, c->stream>>>(nd, ncell, key, start); ++c->launches; }
-  { cellFillKernel<<<(unsigned)((ncell * 32 + 255) / 256), 256, 0, c->stream>>>(
-        ncell, start, val, (const int32_t *)c->sx.p, (const int32_t *)c->sy.p, (const int32_t *)c->sz.p,
-        (const uint8_t *)c->stray.p, (int4 *)c->gpt.p, (int4 *)c->cellRec.p); ++c->launches; }
+  { cellScatterKernel<<<blocks, 256, 0, c->stream>>>(nd, nx, ny, colOf, rank, start, sz, slots); ++c->launches; }
+  { columnKernel<<<(unsigned)((ncell + kColumnWarps - 1) / kColumnWarps), 32 * kColumnWarps, 0, c->stream>>>(
+        ncell, start, slots, sx, sy, sz, stray, gpt, cellRec, count, dBig); ++c->launches; }
+  { bigColumnKernel<<<(unsigned)c->sm_count, 512, 0, c->stream>>>(count, dBig, start, slots, sx, sy, sz, stray, gpt, cellRec,
+                                                                  dBig + 1); ++c->launches; }
+  WB_CUDA(c, cudaGetLastError());
+  unsigned long long ns = 0;
+  int ext[6];
+  uint32_t bigs[2];
+  WB_CUDA(c, cudaMemcpyAsync(&ns, dStray, 8, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaMemcpyAsync(ext, dExt, 24, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaMemcpyAsync(bigs, dBig, 8, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (bigs[1])
+  {
+    // a column of more than kBigColumnMax points (an outlier far from the rest
+    // stretches the grid): all points by radix passes
+    uint64_t *key = (uint64_t *)c->gKey0.p;
+    uint32_t *val = (uint32_t *)c->gVal0.p;
+    int bits = 1;
+    while ((1ull << bits) < ncell)
+      bits++;
+    { cellKeyKernel<<<blocks, 256, 0, c->stream>>>(nd, nx, ny, colOf, sz, key); ++c->launches; }
+    if ((rc = wb_radix_sort_pairs(c, key, val, (uint64_t *)c->gKey1.p, (uint32_t *)c->gVal1.p, nd, 0, 32 + bits, ~0ull, true)))
+      return rc;
+    { cellFillKernel<<<(unsigned)((ncell * 32 + 255) / 256), 256, 0, c->stream>>>(ncell, start, val, sx, sy, sz, stray, gpt,
+                                                                                 cellRec); ++c->launches; }
+  }
   int snx = (nx + WB_SUPER - 1) / WB_SUPER, sny = (ny + WB_SUPER - 1) / WB_SUPER;
   c->grid.snx = snx;
   c->grid.sny = sny;
@@ -542,11 +777,6 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
   { superKernel<<<(unsigned)std::min<uint64_t>((nsup + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
         nx, ny, snx, sny, (const int4 *)c->cellRec.p, (int4 *)c->superRec.p); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
-  unsigned long long ns = 0;
-  int ext[6];
-  WB_CUDA(c, cudaMemcpyAsync(&ns, dStray, 8, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaMemcpyAsync(ext, dExt, 24, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
   c->grid.grouped = false;
   c->grid.nStray = ns;
   c->grid.zminInt = ext[2];
