@@ -176,13 +176,14 @@ class Classifier:
         or by height when sorted."""
         sh = self._shape(kind, v, r, s)
         n = C.c_uint64(0)
-        rc = self.L.wb_points_in(self.ctx, C.byref(sh), int(sorted), None, 0, C.byref(n))
-        if rc not in (0, _lib.WB_EINVAL) or (rc == _lib.WB_EINVAL and n.value == 0):
-            self._check(rc)
-        out = np.zeros(n.value, np.uint32)
-        self._check(self.L.wb_points_in(self.ctx, C.byref(sh), int(sorted), out.ctypes.data, out.shape[0],
-                                        C.byref(n)))
-        return out
+        # a neighbourhood usually fits the first buffer; a larger answer says its size
+        out = np.empty(4096, np.uint32)
+        rc = self.L.wb_points_in(self.ctx, C.byref(sh), int(sorted), out.ctypes.data, out.shape[0], C.byref(n))
+        if rc == _lib.WB_EINVAL and n.value > out.shape[0]:
+            out = np.empty(n.value, np.uint32)
+            rc = self.L.wb_points_in(self.ctx, C.byref(sh), int(sorted), out.ctypes.data, out.shape[0], C.byref(n))
+        self._check(rc)
+        return out[:n.value].copy()
 
     # -- tiles --
     def scan(self, params=None):

@@ -316,7 +316,7 @@ struct CompactScan
 __global__ void __launch_bounds__(256) compactKernel(uint64_t n, CompactScan f, unsigned *counter,
                                                      unsigned long long *status, int *err)
 {
-  lookbackScan(n, f, counter, status, nullptr, err);
+  lookbackScan<kScanItems>(n, f, counter, status, nullptr, err);
 }
 
 /* Prefix and suffix maxima, inside aligned segments of kWindow windows, of
@@ -447,7 +447,7 @@ struct LeafScan
 __global__ void __launch_bounds__(256) leafKernel(uint64_t nd, LeafScan f, unsigned *counter, unsigned long long *status,
                                                   int *err)
 {
-  lookbackScan(nd, f, counter, status, &f.f->leaves, err);
+  lookbackScan<kScanItems>(nd, f, counter, status, &f.f->leaves, err);
 }
 
 /* One block per leaf: bitonic sort of the leaf's input indices (<= 537, padded

@@ -98,7 +98,8 @@ struct wb_ctx
   double grid_bounds[4] = {0, 0, 0, 0};   /* x0, y0, x1, y1 the column grid spans */
   DevBuf flowCache;
   DevBuf lasAngles;                 /* scan-angle tables of the LAS decode and writer */
-  void *hostStage = nullptr;        /* pinned staging for per-block tables (grow-only) */
+  DevBuf queryBuf;                  /* leaves a shape query meets */
+  void *hostStage = nullptr;        /* pinned staging for per-block tables and query answers (grow-only) */
   size_t hostStageCap = 0;
   std::vector<int32_t> flowHostEx, flowHostEy;   /* cached flowsnake order for snake_idx */
   int flowIdxCached = -1;
@@ -204,6 +205,7 @@ int wb_radix_sort_pairs(wb_ctx *c, uint64_t *&keys, uint32_t *&vals, uint64_t *k
  * after it are the octree build's (wb_build.cu). */
 #define WB_SMALL_LOOKBACK 832
 int wb_small(wb_ctx *c);
+int wb_host_stage(wb_ctx *c, size_t bytes);   /* grows c->hostStage */
 int *wb_lookback_err(wb_ctx *c);
 int wb_lookback_words(wb_ctx *c, uint64_t words, unsigned **counter, unsigned long long **status);
 

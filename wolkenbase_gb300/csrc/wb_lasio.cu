@@ -1112,16 +1112,8 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
   // per (block, set) counts, first records and files go through one pinned
   // host buffer of the context (16 bytes per entry)
   const size_t stageBytes = L * S * 16 + 64;
-  if (c->hostStageCap < stageBytes)
-  {
-    WB_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (c->hostStage)
-      cudaFreeHost(c->hostStage);
-    c->hostStage = nullptr;
-    c->hostStageCap = 0;
-    WB_CUDA(c, cudaHostAlloc(&c->hostStage, stageBytes, cudaHostAllocDefault));
-    c->hostStageCap = stageBytes;
-  }
+  if ((rc = wb_host_stage(c, stageBytes)))
+    return rc;
   uint64_t *base = (uint64_t *)c->hostStage;
   uint32_t *cnt = (uint32_t *)(base + L * S), *fof = cnt + L * S;
   if (L)

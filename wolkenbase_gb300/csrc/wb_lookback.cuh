@@ -182,12 +182,12 @@ __device__ __forceinline__ uint32_t blockExclusive256(uint32_t v, uint32_t *warp
   return before + inc - v;
 }
 
-/* One-pass scan of 256-thread tiles of kScanItems items: flag(i) is item i's
+/* One-pass scan of 256-thread tiles of ITEMS items a thread: flag(i) is item i's
  * value, put(i, before, value) receives the sum before it.  The last tile
  * writes the total.  counter and status (one word per tile) are zero on
  * entry. */
 constexpr int kScanItems = 16, kScanTile = 256 * kScanItems;
-template <typename F>
+template <int ITEMS, typename F>
 __device__ __forceinline__ void lookbackScan(uint64_t n, F &f, unsigned *counter, unsigned long long *status,
                                              uint32_t *total, int *err)
 {
@@ -202,19 +202,19 @@ __device__ __forceinline__ void lookbackScan(uint64_t n, F &f, unsigned *counter
   }
   __syncthreads();
   const unsigned tile = tileS;
-  const uint64_t base = (uint64_t)tile * kScanTile;
+  const uint64_t base = (uint64_t)tile * (256 * ITEMS);
   // a warp's items lie together, a lane's 32 apart
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint64_t wbase = base + (uint64_t)w * (32 * kScanItems);
-  uint32_t v[kScanItems], ex[kScanItems], run = 0;
+  const uint64_t wbase = base + (uint64_t)w * (32 * ITEMS);
+  uint32_t v[ITEMS], ex[ITEMS], run = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++)
+  for (int k = 0; k < ITEMS; k++)
   {
     const uint64_t i = wbase + 32 * k + lane;
     v[k] = i < n ? f.value(i) : 0;
   }
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++)
+  for (int k = 0; k < ITEMS; k++)
   {
     uint32_t inc = v[k];
 #pragma unroll
@@ -250,7 +250,7 @@ __device__ __forceinline__ void lookbackScan(uint64_t n, F &f, unsigned *counter
         lookbackPut(status + tile, lookbackWord(1, true, b + sum));
       beforeS = b;
       failed = !ok;
-      if (ok && base + kScanTile >= n && total)
+      if (ok && base + 256 * ITEMS >= n && total)
         *total = (uint32_t)(b + sum);
     }
   }
@@ -259,7 +259,7 @@ __device__ __forceinline__ void lookbackScan(uint64_t n, F &f, unsigned *counter
     return;
   const uint32_t off = (uint32_t)beforeS + before;
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++)
+  for (int k = 0; k < ITEMS; k++)
   {
     const uint64_t i = wbase + 32 * k + lane;
     if (i < n)

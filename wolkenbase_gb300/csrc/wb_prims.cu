@@ -29,7 +29,7 @@ struct PlainScan
 __global__ void __launch_bounds__(256) scanKernel(uint64_t n, PlainScan f, unsigned *counter, unsigned long long *status,
                                                   uint32_t *total, int *err)
 {
-  lookbackScan(n, f, counter, status, total, err);
+  lookbackScan<kScanItems>(n, f, counter, status, total, err);
 }
 
 /* ---------------- radix sort ---------------- */
@@ -259,6 +259,20 @@ int wb_small(wb_ctx *c)
   if (rc)
     return rc;
   WB_CUDA(c, cudaMemsetAsync(c->small.p, 0, 4096, c->stream));
+  return 0;
+}
+
+int wb_host_stage(wb_ctx *c, size_t bytes)
+{
+  if (c->hostStageCap >= bytes)
+    return 0;
+  WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (c->hostStage)
+    cudaFreeHost(c->hostStage);
+  c->hostStage = nullptr;
+  c->hostStageCap = 0;
+  WB_CUDA(c, cudaHostAlloc(&c->hostStage, bytes, cudaHostAllocDefault));
+  c->hostStageCap = bytes;
   return 0;
 }
 

@@ -14,9 +14,16 @@
  * height (the reference's std::sort by z leaves ties in no particular order;
  * here ties keep the unsorted order).
  *
- * One warp per leaf: the cube tests on lane 0's doubles, the per-point tests
- * across the lanes with ballot compaction (store order kept), a scan of the
- * per-leaf counts, a second pass writing the record indices.
+ * One thread per leaf lists the leaves that meet the shape, in order, in one
+ * pass (a look-back scan).  A query that meets few leaves (up to kFewLeaves: a
+ * neighbourhood) is answered by one block, which tests the leaves' points, places
+ * them, sorts them when asked and writes them to pinned host memory, so the
+ * call is two kernels and one wait.  Larger ones count, scan, fill and
+ * radix-sort over the listed leaves.  Points are tested in FP32 relative to the
+ * shape, exactly in FP64 within 1e-5 of its surface: FP64 issues at 1/64 rate.
+ * A sorted hyperboloid query of 2M points: 388 us before (a warp per leaf, FP64
+ * throughout, eight allocations and waits), of which 80% was allocation,
+ * launches and waits.
  */
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -26,6 +33,7 @@
 #include <vector>
 #include "wb_internal.h"
 #include "wb_device.cuh"
+#include "wb_lookback.cuh"
 
 namespace
 {
@@ -44,10 +52,10 @@ struct QArgs
   const uint64_t *leafKey;
   const uint8_t *leafLev;
   const uint32_t *first, *count;
-  const int32_t *sx, *sy, *sz;
+  const double *xyzd;   /* decoded x, y, z planes of nd doubles */
+  uint64_t nd;
   const uint32_t *sidx;
   double rootLo[3], rootSide;
-  double off[3], scale[3], unit;
 };
 
 __device__ __forceinline__ bool shapeIn(const QShape &s, double x, double y, double z)
@@ -84,79 +92,281 @@ __device__ __forceinline__ bool shapeHolds(const QShape &s, double cx, double cy
   return all;
 }
 
-/* mode 0: meet[l] = whether leaf l meets the shape (findBlocks);
- * mode 1: cnt[l] = points of leaf l that pointsIn returns;
- * mode 2: those points' record indices written from out + off[l]. */
-template <int MODE>
-__global__ void leafQueryKernel(QArgs a, uint32_t *__restrict__ cnt, const uint32_t *__restrict__ off,
-                                uint32_t *__restrict__ out)
+/* The shape against leaf l's cube; cubes far from it are told by their centre
+ * alone, with half a side to spare. */
+__device__ __forceinline__ bool leafMeets(const QArgs &a, uint64_t l)
+{
+  double cx, cy, cz, side;
+  wb_leaf_cube(a.leafKey[l], a.leafLev[l], a.rootLo, a.rootSide, cx, cy, cz, side);
+  const double ax = fabs(a.s.cx - cx) - side, ay = fabs(a.s.cy - cy) - side;
+  if (a.s.kind == WB_SHAPE_CYLINDER)
+  {
+    if (ax > a.s.r || ay > a.s.r)
+      return false;
+  }
+  else if (a.s.slope > 0)
+  {
+    const double zd = a.s.cz - (cz - side / 2);
+    if (!(zd > 0) || ax * a.s.slope > zd || ay * a.s.slope > zd)
+      return false;
+  }
+  return shapeMeets(a.s, cx, cy, cz, side);
+}
+
+/* The listed leaves, in depth-first order. */
+struct MeetScan
+{
+  QArgs a;
+  uint32_t *list;
+  __device__ uint32_t value(uint64_t l) const { return leafMeets(a, l); }
+  __device__ void put(uint64_t l, uint32_t before, uint32_t v) const
+  {
+    if (v)
+      list[before] = (uint32_t)l;
+  }
+};
+__global__ void __launch_bounds__(256) meetKernel(MeetScan f, unsigned *counter, unsigned long long *status,
+                                                  uint32_t *total, int *err)
+{
+  lookbackScan<1>(f.a.L, f, counter, status, total, err);
+}
+
+/* shapeIn of stored point j. */
+__device__ __forceinline__ bool pointIn(const QArgs &a, uint64_t j)
+{
+  const double x = a.xyzd[j], y = a.xyzd[a.nd + j], z = a.xyzd[2 * a.nd + j];
+  const float dx = (float)(a.s.cx - x), dy = (float)(a.s.cy - y), d2 = dx * dx + dy * dy;
+  if (a.s.kind == WB_SHAPE_CYLINDER)
+  {
+    const float r = (float)a.s.r, r2 = r * r;
+    if (r2 > 1e-30f && r2 < 1e30f)
+    {
+      if (d2 < r2 * (1 - 1e-5f))
+        return true;
+      if (d2 > r2 * (1 + 1e-5f))
+        return false;
+    }
+  }
+  else if (a.s.slope > 0)
+  {
+    const float zd = (float)(a.s.cz - z), s = (float)a.s.slope, w = zd * zd, r2 = s * s * d2, p = (float)a.s.por2;
+    const float f = w - r2 - p, tol = 1e-5f * (w + r2 + p);
+    if (tol > 1e-30f && tol < 1e30f)
+    {
+      if (zd < 0 || f < -tol)
+        return false;
+      if (f > tol)
+        return true;
+    }
+  }
+  return shapeIn(a.s, x, y, z);
+}
+
+/* Order-preserving key of a height. */
+__device__ __forceinline__ uint64_t heightBits(double z)
+{
+  if (z == 0)
+    z = 0;   // -0 and +0 compare equal
+  uint64_t u;
+  memcpy(&u, &z, 8);
+  return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+}
+
+/* A warp tests leaf l's points, 32 a row (at most 17 rows): lane r keeps row
+ * r's hits; returns how many. */
+constexpr int kLeafRows = (WB_RECORDS + 31) / 32;
+__device__ __forceinline__ uint32_t leafRows(const QArgs &a, uint32_t l, unsigned &hits)
 {
   const int lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t l = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < a.L; l += warps)
+  double cx, cy, cz, side;
+  wb_leaf_cube(a.leafKey[l], a.leafLev[l], a.rootLo, a.rootSide, cx, cy, cz, side);
+  const bool whole = shapeHolds(a.s, cx, cy, cz, side);
+  const uint32_t f = a.first[l], n = a.count[l];
+  uint32_t taken = 0;
+  hits = 0;
+  for (int r = 0; 32u * r < n; r++)
   {
-    double cx, cy, cz, side;
-    wb_leaf_cube(a.leafKey[l], a.leafLev[l], a.rootLo, a.rootSide, cx, cy, cz, side);
-    const bool meets = shapeMeets(a.s, cx, cy, cz, side);
-    if (MODE == 0)
+    const uint32_t t = 32u * r + lane;
+    const bool in = t < n && (whole || pointIn(a, f + t));
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (lane == r)
+      hits = b;
+    taken += __popc(b);
+  }
+  return taken;
+}
+
+/* What the one-block answer leaves in pinned host memory. */
+constexpr int kFewLeaves = 128, kFewPoints = 8192, kFewSorted = 2048;
+struct QueryAnswer
+{
+  uint32_t leaves, points;
+  uint32_t complete;   /* rec holds the answer */
+  uint32_t failed;     /* the listing's look-back gave up */
+  uint32_t rec[kFewPoints];
+};
+
+/* One block answers a query of at most kFewLeaves leaves.  want: capacity of
+ * the caller (0: the count only). */
+__global__ void __launch_bounds__(1024) fewLeavesKernel(QArgs a, const uint32_t *__restrict__ list,
+                                                        const uint32_t *__restrict__ nList, uint64_t want, int sorted,
+                                                        const int *__restrict__ err, QueryAnswer *ans)
+{
+  __shared__ uint32_t cnt[kFewLeaves + 1];
+  __shared__ uint64_t key[kFewSorted];
+  __shared__ uint32_t ord[kFewSorted], rec[kFewSorted];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t n = *nList;
+  const bool failed = *err != 0;
+  if (threadIdx.x == 0)
+    ans->failed = failed;
+  if (failed || n > kFewLeaves)
+  {
+    if (threadIdx.x == 0)
+    {
+      ans->leaves = n;
+      ans->complete = 0;
+    }
+    return;
+  }
+  constexpr int ROUNDS = kFewLeaves / 32;
+  unsigned hits[ROUNDS];
+#pragma unroll
+  for (int q = 0; q < ROUNDS; q++)
+  {
+    const uint32_t i = q * 32 + w;
+    hits[q] = 0;
+    uint32_t taken = 0;
+    if (i < n)
+      taken = leafRows(a, list[i], hits[q]);
+    if (lane == 0)
+      cnt[i] = taken;
+  }
+  __syncthreads();
+  if (w == 0)
+  {
+    // exclusive prefix of the leaves' counts
+    uint32_t run = 0;
+    for (int q = 0; q < ROUNDS; q++)
+    {
+      const uint32_t v = cnt[q * 32 + lane];
+      uint32_t inc = v;
+      for (int o = 1; o < 32; o <<= 1)
+      {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o)
+          inc += u;
+      }
+      cnt[q * 32 + lane] = run + inc - v;
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0)
+      cnt[kFewLeaves] = run;
+  }
+  __syncthreads();
+  const uint32_t total = cnt[kFewLeaves];
+  const bool sort = sorted && total > 1, fits = total <= want && total <= (sort ? kFewSorted : kFewPoints);
+  if (threadIdx.x == 0)
+  {
+    ans->leaves = n;
+    ans->points = total;
+    ans->complete = fits || total > want;
+  }
+  if (!fits)
+    return;
+#pragma unroll
+  for (int q = 0; q < ROUNDS; q++)
+  {
+    const uint32_t i = q * 32 + w;
+    if (i >= n)
+      continue;
+    const uint32_t f = a.first[list[i]];
+    uint32_t at = cnt[i];
+    for (int r = 0; r < kLeafRows; r++)
+    {
+      const unsigned b = __shfl_sync(0xffffffffu, hits[q], r);
+      if ((b >> lane) & 1)
+      {
+        const uint32_t j = f + 32 * r + lane, p = at + __popc(b & ((1u << lane) - 1));
+        if (sort)
+        {
+          key[p] = heightBits(a.xyzd[2 * a.nd + j]);
+          ord[p] = p;
+          rec[p] = a.sidx[j];
+        }
+        else
+          ans->rec[p] = a.sidx[j];
+      }
+      at += __popc(b);
+    }
+  }
+  if (!sort)
+    return;
+  int P = 64;
+  while (P < (int)total)
+    P <<= 1;
+  for (int q = threadIdx.x + (int)total; q < P; q += 1024)
+  {
+    key[q] = ~0ull;
+    ord[q] = ~0u;
+  }
+  __syncthreads();
+  // by height, ties in the order found
+  for (int size = 2; size <= P; size <<= 1)
+    for (int j = size >> 1; j > 0; j >>= 1)
+    {
+      for (int t = threadIdx.x; t < P / 2; t += 1024)
+      {
+        const int i = 2 * t - (t & (j - 1)), u = i + j;
+        const uint64_t x = key[i], y = key[u];
+        const uint32_t ox = ord[i], oy = ord[u];
+        if ((x > y || (x == y && ox > oy)) == ((i & size) == 0))
+        {
+          key[i] = y;
+          key[u] = x;
+          ord[i] = oy;
+          ord[u] = ox;
+        }
+      }
+      __syncthreads();
+    }
+  for (uint32_t t = threadIdx.x; t < total; t += 1024)
+    ans->rec[t] = rec[ord[t]];
+}
+
+/* FILL false: cnt[i] = points of listed leaf i that pointsIn returns; true:
+ * their record indices (and, with keys, heights) written from off[i] on. */
+template <bool FILL>
+__global__ void listedKernel(QArgs a, const uint32_t *__restrict__ list, uint32_t n, uint32_t *__restrict__ cnt,
+                             const uint32_t *__restrict__ off, uint32_t *__restrict__ out, uint64_t *__restrict__ keys)
+{
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps)
+  {
+    unsigned hits;
+    const uint32_t taken = leafRows(a, list[i], hits);
+    if (!FILL)
     {
       if (lane == 0)
-        cnt[l] = meets ? 1u : 0u;
+        cnt[i] = taken;
       continue;
     }
-    const uint32_t f = a.first[l], n = a.count[l];
-    if (!meets)
+    const uint32_t f = a.first[list[i]];
+    uint32_t at = off[i];
+    for (int r = 0; r < kLeafRows; r++)
     {
-      if (MODE == 1 && lane == 0)
-        cnt[l] = 0;
-      continue;
-    }
-    const bool whole = shapeHolds(a.s, cx, cy, cz, side);
-    uint32_t taken = 0;
-    for (uint32_t t0 = 0; t0 < n; t0 += 32)
-    {
-      const uint32_t t = t0 + lane;
-      bool in = false;
-      if (t < n)
+      const unsigned b = __shfl_sync(0xffffffffu, hits, r);
+      if ((b >> lane) & 1)
       {
-        const uint32_t j = f + t;
-        in = whole || shapeIn(a.s, wb_decode(a.sx[j], a.off[0], a.scale[0], a.unit),
-                              wb_decode(a.sy[j], a.off[1], a.scale[1], a.unit),
-                              wb_decode(a.sz[j], a.off[2], a.scale[2], a.unit));
+        const uint32_t j = f + 32 * r + lane, p = at + __popc(b & ((1u << lane) - 1));
+        out[p] = a.sidx[j];
+        if (keys)
+          keys[p] = heightBits(a.xyzd[2 * a.nd + j]);
       }
-      const unsigned b = __ballot_sync(0xffffffffu, in);
-      if (MODE == 2 && in)
-        out[off[l] + taken + __popc(b & ((1u << lane) - 1))] = a.sidx[f + t];
-      taken += __popc(b);
+      at += __popc(b);
     }
-    if (MODE == 1 && lane == 0)
-      cnt[l] = taken;
   }
-}
-
-/* Order-preserving key of the height of record i (decoded), for the sort. */
-__global__ void heightKeyKernel(uint64_t m, const uint32_t *__restrict__ recIdx, const uint32_t *__restrict__ storeOf,
-                                const int32_t *__restrict__ sz, double off, double scale, double unit,
-                                uint64_t *__restrict__ key, uint32_t *__restrict__ val)
-{
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
-  {
-    double z = wb_decode(sz[storeOf[recIdx[i]]], off, scale, unit);
-    if (z == 0)
-      z = 0;   // -0 and +0 compare equal
-    uint64_t u;
-    memcpy(&u, &z, 8);
-    key[i] = (u >> 63) ? ~u : (u | 0x8000000000000000ull);
-    val[i] = recIdx[i];
-  }
-}
-
-__global__ void compactFlags(uint64_t L, const uint32_t *__restrict__ flag, const uint32_t *__restrict__ ex,
-                             int64_t *__restrict__ out)
-{
-  for (uint64_t l = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; l < L; l += (uint64_t)gridDim.x * blockDim.x)
-    if (flag[l])
-      out[ex[l]] = (int64_t)l;
 }
 
 int shapeArgs(wb_ctx *c, const wb_shape *sh, QArgs &a, const char *who)
@@ -192,24 +402,36 @@ int shapeArgs(wb_ctx *c, const wb_shape *sh, QArgs &a, const char *who)
   a.leafLev = (const uint8_t *)c->leafLevel.p;
   a.first = (const uint32_t *)c->leafFirst.p;
   a.count = (const uint32_t *)c->leafCount.p;
-  a.sx = (const int32_t *)c->sx.p;
-  a.sy = (const int32_t *)c->sy.p;
-  a.sz = (const int32_t *)c->sz.p;
+  a.xyzd = (const double *)c->xyzd.p;
+  a.nd = c->nd;
   a.sidx = (const uint32_t *)c->sidx.p;
   for (int k = 0; k < 3; k++)
-  {
     a.rootLo[k] = c->g.root_lo[k];
-    a.off[k] = c->g.off[k];
-    a.scale[k] = c->g.scale[k];
-  }
   a.rootSide = c->g.root_side;
-  a.unit = c->g.unit;
   return 0;
 }
 
-unsigned warpGrid(wb_ctx *c, uint64_t L)
+int lookbackFailed(wb_ctx *c, const char *who)
 {
-  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((L * 32 + 255) / 256, (uint64_t)c->sm_count * 32));
+  cudaMemsetAsync(wb_lookback_err(c), 0, 4, c->stream);
+  return wb_fail(c, WB_ETIMEDOUT, std::string(who) + ": a look-back wait gave up");
+}
+
+/* Lists the leaves that meet the shape: *list on the device, their number at
+ * *nList. */
+int listLeaves(wb_ctx *c, const QArgs &a, uint32_t **list, uint32_t **nList)
+{
+  const uint64_t tiles = (a.L + 255) / 256;   // a leaf a thread: FP64 cube tests, spread over the SMs
+  unsigned *counter;
+  unsigned long long *status;
+  int rc = wb_lookback_words(c, tiles, &counter, &status);
+  if (rc || (rc = wb_ensure(c, c->queryBuf, a.L * 4 + 64)))
+    return rc;
+  *nList = (uint32_t *)c->queryBuf.p;
+  *list = *nList + 16;
+  { meetKernel<<<(unsigned)tiles, 256, 0, c->stream>>>(MeetScan{a, *list}, counter, status, *nList, wb_lookback_err(c)); ++c->launches; }
+  WB_CUDA(c, cudaGetLastError());
+  return 0;
 }
 }  // namespace
 
@@ -227,28 +449,26 @@ extern "C" int wb_find_blocks(wb_ctx *c, const wb_shape *sh, int64_t *leaves, ui
   const uint64_t L = a.L;
   if (L == 0)
     return 0;
-  WbScratch flag(c), ex(c), outD(c);
-  if ((rc = wb_ensure(c, flag.b, L * 4 + 64)) || (rc = wb_ensure(c, ex.b, L * 4 + 64)) ||
-      (rc = wb_ensure(c, outD.b, L * 8 + 64)))
+  uint32_t *list, *nList, total = 0;
+  int err = 0;
+  if ((rc = listLeaves(c, a, &list, &nList)))
     return rc;
-  uint32_t *dTot = (uint32_t *)((uint8_t *)ex.b.p + L * 4);
-  { leafQueryKernel<0><<<warpGrid(c, L), 256, 0, c->stream>>>(a, (uint32_t *)flag.b.p, nullptr, nullptr); ++c->launches; }
-  if ((rc = wb_exclusive_scan_u32(c, (const uint32_t *)flag.b.p, (uint32_t *)ex.b.p, L, dTot)))
-    return rc;
-  uint32_t total = 0;
-  WB_CUDA(c, cudaMemcpyAsync(&total, dTot, 4, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaMemcpyAsync(&total, nList, 4, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaMemcpyAsync(&err, wb_lookback_err(c), 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (err)
+    return lookbackFailed(c, "wb_find_blocks");
   if (count)
     *count = total;
   if (total > capacity)
     return wb_fail(c, WB_EINVAL, "wb_find_blocks: " + std::to_string(total) + " blocks, capacity " +
                                      std::to_string(capacity));
-  { compactFlags<<<(unsigned)std::min<uint64_t>((L + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-        L, (const uint32_t *)flag.b.p, (const uint32_t *)ex.b.p, (int64_t *)outD.b.p); ++c->launches; }
-  WB_CUDA(c, cudaGetLastError());
-  if (total)
-    WB_CUDA(c, cudaMemcpyAsync(leaves, outD.b.p, (size_t)total * 8, cudaMemcpyDefault, c->stream));
+  if (!total)
+    return 0;
+  std::vector<uint32_t> l(total);
+  WB_CUDA(c, cudaMemcpyAsync(l.data(), list, (size_t)total * 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  std::copy(l.begin(), l.end(), leaves);
   return 0;
 }
 
@@ -267,12 +487,44 @@ extern "C" int wb_points_in(wb_ctx *c, const wb_shape *sh, int sorted, uint32_t 
   const uint64_t L = a.L;
   if (L == 0)
     return 0;
-  WbScratch cnt(c), ex(c);
-  if ((rc = wb_ensure(c, cnt.b, L * 4 + 64)) || (rc = wb_ensure(c, ex.b, L * 4 + 64)))
+  uint32_t *list, *nList;
+  if ((rc = listLeaves(c, a, &list, &nList)) || (rc = wb_host_stage(c, sizeof(QueryAnswer))))
     return rc;
-  uint32_t *dTot = (uint32_t *)((uint8_t *)ex.b.p + L * 4);
-  { leafQueryKernel<1><<<warpGrid(c, L), 256, 0, c->stream>>>(a, (uint32_t *)cnt.b.p, nullptr, nullptr); ++c->launches; }
-  if ((rc = wb_exclusive_scan_u32(c, (const uint32_t *)cnt.b.p, (uint32_t *)ex.b.p, L, dTot)))
+  QueryAnswer *ans = (QueryAnswer *)c->hostStage;
+  { fewLeavesKernel<<<1, 1024, 0, c->stream>>>(a, list, nList, capacity, sorted, wb_lookback_err(c), ans); ++c->launches; }
+  WB_CUDA(c, cudaGetLastError());
+  WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (ans->failed)
+    return lookbackFailed(c, "wb_points_in");
+  auto tooMany = [&](uint64_t total) {
+    return wb_fail(c, WB_EINVAL, "wb_points_in: " + std::to_string(total) + " points, capacity " +
+                                     std::to_string(capacity));
+  };
+  if (ans->complete)
+  {
+    const uint32_t total = ans->points;
+    if (count)
+      *count = total;
+    if (total > capacity)
+      return tooMany(total);
+    if (total && wb_device_accessible(records))
+    {
+      WB_CUDA(c, cudaMemcpyAsync(records, ans->rec, (size_t)total * 4, cudaMemcpyDefault, c->stream));
+      WB_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
+    else if (total)
+      memcpy(records, ans->rec, (size_t)total * 4);
+    return 0;
+  }
+  // many leaves or points: counts, their prefix, the points, a radix sort
+  const uint32_t n = ans->leaves;
+  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n * 32 + 255) / 256, (uint64_t)c->sm_count * 32));
+  WbScratch cnt(c), ex(c);
+  if ((rc = wb_ensure(c, cnt.b, (uint64_t)n * 4 + 64)) || (rc = wb_ensure(c, ex.b, (uint64_t)n * 4 + 64)))
+    return rc;
+  uint32_t *dTot = (uint32_t *)((uint8_t *)ex.b.p + (uint64_t)n * 4);
+  { listedKernel<false><<<grid, 256, 0, c->stream>>>(a, list, n, (uint32_t *)cnt.b.p, nullptr, nullptr, nullptr); ++c->launches; }
+  if ((rc = wb_exclusive_scan_u32(c, (const uint32_t *)cnt.b.p, (uint32_t *)ex.b.p, n, dTot)))
     return rc;
   uint32_t total = 0;
   WB_CUDA(c, cudaMemcpyAsync(&total, dTot, 4, cudaMemcpyDefault, c->stream));
@@ -280,35 +532,23 @@ extern "C" int wb_points_in(wb_ctx *c, const wb_shape *sh, int sorted, uint32_t 
   if (count)
     *count = total;
   if (total > capacity)
-    return wb_fail(c, WB_EINVAL, "wb_points_in: " + std::to_string(total) + " points, capacity " +
-                                     std::to_string(capacity));
+    return tooMany(total);
   if (total == 0)
     return 0;
-  WbScratch outD(c);
+  WbScratch outD(c), k0(c), k1(c), v1(c);
+  const bool sort = sorted && total > 1;
   if ((rc = wb_ensure(c, outD.b, (uint64_t)total * 4 + 64)))
     return rc;
-  { leafQueryKernel<2><<<warpGrid(c, L), 256, 0, c->stream>>>(a, nullptr, (const uint32_t *)ex.b.p,
-                                                             (uint32_t *)outD.b.p); ++c->launches; }
+  if (sort && ((rc = wb_ensure(c, k0.b, (uint64_t)total * 8 + 64)) || (rc = wb_ensure(c, k1.b, (uint64_t)total * 8 + 64)) ||
+               (rc = wb_ensure(c, v1.b, (uint64_t)total * 4 + 64))))
+    return rc;
+  uint32_t *vals = (uint32_t *)outD.b.p;
+  uint64_t *keys = (uint64_t *)k0.b.p;
+  { listedKernel<true><<<grid, 256, 0, c->stream>>>(a, list, n, nullptr, (const uint32_t *)ex.b.p, vals, sort ? keys : nullptr); ++c->launches; }
+  if (sort && (rc = wb_radix_sort_pairs(c, keys, vals, (uint64_t *)k1.b.p, (uint32_t *)v1.b.p, total, 0, 64)))
+    return rc;
   WB_CUDA(c, cudaGetLastError());
-  const uint32_t *res = (const uint32_t *)outD.b.p;
-  WbScratch k0(c), k1(c), v1(c);
-  if (sorted && total > 1)
-  {
-    if ((rc = wb_ensure(c, k0.b, (uint64_t)total * 8 + 64)) || (rc = wb_ensure(c, k1.b, (uint64_t)total * 8 + 64)) ||
-        (rc = wb_ensure(c, v1.b, (uint64_t)total * 4 + 64)))
-      return rc;
-    // the values are the record indices themselves; sort them by height in place of outD
-    uint32_t *v0 = (uint32_t *)outD.b.p;
-    { heightKeyKernel<<<(unsigned)std::min<uint64_t>((total + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0,
-                        c->stream>>>(total, v0, (const uint32_t *)c->storeOf.p, a.sz, a.off[2], a.scale[2], a.unit,
-                                     (uint64_t *)k0.b.p, v0); ++c->launches; }
-    uint64_t *keys = (uint64_t *)k0.b.p;
-    uint32_t *vals = v0;
-    if ((rc = wb_radix_sort_pairs(c, keys, vals, (uint64_t *)k1.b.p, (uint32_t *)v1.b.p, total, 0, 64)))
-      return rc;
-    res = vals;
-  }
-  WB_CUDA(c, cudaMemcpyAsync(records, res, (size_t)total * 4, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaMemcpyAsync(records, vals, (size_t)total * 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
   return 0;
 }
