@@ -97,6 +97,7 @@ struct Decode
 {
   double off[3], scale[3], unit;
 };
+  bool scaled;   /* unit is not 1 (tested on the host: a comparison is an FP64 instruction too) */
 
 __device__ __forceinline__ uint32_t rd16(const uint8_t *s, int o)
 {
@@ -273,6 +274,19 @@ __device__ __forceinline__ void parseRecord(const uint8_t *s, int f, const Layou
     p.angle = __ldg(at.bin16 + p.angleRaw);
     p.src = (uint16_t)rd16(s, 20);
   }
+/* (double)X from its bits: the exponent and the shifted magnitude.  FP64
+ * instructions issue at 1/64 rate here, the conversion among them; the decode
+ * is bound by them (12 a record, 82% of the pipe, with the conversions and the
+ * unit's comparison; six with neither). */
+__device__ __forceinline__ double intToDouble(int32_t X)
+{
+  const uint32_t m = X < 0 ? 0u - (uint32_t)X : (uint32_t)X;
+  const int lead = __clz(m);                    // 32 for zero
+  const uint32_t t = lead < 31 ? m << (lead + 1) : 0u;   // the magnitude below its leading one, at the top
+  const uint32_t hi = ((uint32_t)X & 0x80000000u) | ((uint32_t)(1023 + 31 - lead) << 20) | (t >> 12);
+  return m ? __hiloint2double((int)hi, (int)(t << 20)) : 0.0;
+}
+
   p.gps = L.gps >= 0 ? __longlong_as_double((long long)rd64(s, L.gps)) : 0.0;
   if (L.rgb >= 0)
   {
@@ -288,8 +302,8 @@ __device__ __forceinline__ void parseRecord(const uint8_t *s, int f, const Layou
 /* The location readPoint computes (las.cpp:808): (offset + scale*X) * unit. */
 __device__ __forceinline__ double decodeAxis(const Decode &d, int32_t X, int k)
 {
-  const double v = d.off[k] + d.scale[k] * (double)X;
-  return d.unit != 1 ? v * d.unit : v;   // x * 1 == x
+  const double v = d.off[k] + d.scale[k] * intToDouble(X);
+  return d.scaled ? v * d.unit : v;   // x * 1 == x
 }
 
 struct Encode
@@ -381,7 +395,7 @@ constexpr int kStageStride = 80;
 __global__ void __launch_bounds__(kBlock) decodeKernel(const DecodeArgs a)
 {
   __shared__ __align__(16) uint8_t stage[kBlock / 32][32 * kStageStride];
-  __shared__ uint32_t slots[kBlock * kSlotWords];
+  static_assert(kStageStride >= 4 * kSlotWords, "a slot fits a staged record's room");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Layout L = layoutOf(a.fmt);
   const bool staged = a.vec16 && a.stride <= (uint32_t)kStageStride;
@@ -407,7 +421,7 @@ __global__ void __launch_bounds__(kBlock) decodeKernel(const DecodeArgs a)
     }
     else
     {
-      uint8_t *slot = (uint8_t *)(slots + threadIdx.x * kSlotWords);
+      uint8_t *slot = (uint8_t *)((uint32_t *)stage[warp] + lane * kSlotWords);
       if (i < a.n)
         loadRecord(slot, a.rec + i * a.stride, L.len, a.words);
       s = slot;
@@ -1046,6 +1060,7 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
       }
     }
   }
+  a.d.scaled = cloud->unit != 1;
   if ((rc = angleTables(c, a.t)))
     return rc;
   for (int k = 0; k < 3; k++)
@@ -1153,6 +1168,7 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
         heap.pop();
       }
       else
+  a.d.scaled = cloud->unit != 1;
         for (int i = 1; i < nf; i++)
           if (fileCount[f0 + i] < fileCount[f])
             f = f0 + i;
