@@ -36,6 +36,7 @@
 #include <functional>
 #include <queue>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include "wb_internal.h"
 
@@ -96,8 +97,8 @@ struct LasPt
 struct Decode
 {
   double off[3], scale[3], unit;
-};
   bool scaled;   /* unit is not 1 (tested on the host: a comparison is an FP64 instruction too) */
+};
 
 __device__ __forceinline__ uint32_t rd16(const uint8_t *s, int o)
 {
@@ -223,19 +224,6 @@ __device__ __forceinline__ void loadRecord(uint8_t *slot, const uint8_t *src, in
       slot[k] = __ldg(src + k);
 }
 
-__device__ __forceinline__ void storeRecord(uint8_t *dst, const uint8_t *slot, int len, int width)
-{
-  if (width == 4)
-    for (int k = 0; k < len >> 2; k++)
-      ((uint32_t *)dst)[k] = ((const uint32_t *)slot)[k];
-  else if (width == 2)
-    for (int k = 0; k < len >> 1; k++)
-      ((uint16_t *)dst)[k] = ((const uint16_t *)slot)[k];
-  else
-    for (int k = 0; k < len; k++)
-      dst[k] = slot[k];
-}
-
 /* LasHeader::readPoint (las.cpp:735-820) from a record in shared memory. */
 __device__ __forceinline__ void parseRecord(const uint8_t *s, int f, const Layout &L, const Decode &d,
                                             const AngleTabs &at, LasPt &p)
@@ -274,6 +262,18 @@ __device__ __forceinline__ void parseRecord(const uint8_t *s, int f, const Layou
     p.angle = __ldg(at.bin16 + p.angleRaw);
     p.src = (uint16_t)rd16(s, 20);
   }
+  p.gps = L.gps >= 0 ? __longlong_as_double((long long)rd64(s, L.gps)) : 0.0;
+  if (L.rgb >= 0)
+  {
+    p.r = (uint16_t)rd16(s, L.rgb);
+    p.g = (uint16_t)rd16(s, L.rgb + 2);
+    p.b = (uint16_t)rd16(s, L.rgb + 4);
+  }
+  else
+    p.r = p.g = p.b = 0;
+  p.nir = L.nir >= 0 ? (uint16_t)rd16(s, L.nir) : 0;
+}
+
 /* (double)X from its bits: the exponent and the shifted magnitude.  FP64
  * instructions issue at 1/64 rate here, the conversion among them; the decode
  * is bound by them (12 a record, 82% of the pipe, with the conversions and the
@@ -285,18 +285,6 @@ __device__ __forceinline__ double intToDouble(int32_t X)
   const uint32_t t = lead < 31 ? m << (lead + 1) : 0u;   // the magnitude below its leading one, at the top
   const uint32_t hi = ((uint32_t)X & 0x80000000u) | ((uint32_t)(1023 + 31 - lead) << 20) | (t >> 12);
   return m ? __hiloint2double((int)hi, (int)(t << 20)) : 0.0;
-}
-
-  p.gps = L.gps >= 0 ? __longlong_as_double((long long)rd64(s, L.gps)) : 0.0;
-  if (L.rgb >= 0)
-  {
-    p.r = (uint16_t)rd16(s, L.rgb);
-    p.g = (uint16_t)rd16(s, L.rgb + 2);
-    p.b = (uint16_t)rd16(s, L.rgb + 4);
-  }
-  else
-    p.r = p.g = p.b = 0;
-  p.nir = L.nir >= 0 ? (uint16_t)rd16(s, L.nir) : 0;
 }
 
 /* The location readPoint computes (las.cpp:808): (offset + scale*X) * unit. */
@@ -459,20 +447,22 @@ __global__ void __launch_bounds__(kBlock) decodeKernel(const DecodeArgs a)
 
 /* Header figures of one output file while it is written (las.cpp:832-845,
  * 900-902): extreme record integers (decoding is monotone in them) and the
- * point counts, [0] all and [r] of return number r. */
-struct FileStat
+ * point counts, [0] all and [r] of return number r.  One more entry than there
+ * are files counts the blocks taken. */
+template <class Word>
+struct StatOf
 {
   int32_t mn[3], mx[3];
-  unsigned long long cnt[16];
+  Word cnt[16];
 };
+typedef StatOf<unsigned long long> FileStat;
 
 struct WriteArgs
 {
   const uint8_t *rec;
+  uint64_t n;
   uint32_t stride;
   int inFmt, outFmt;
-  bool inWords;
-  int outWidth;                  /* widest store the output records allow: 4, 2 or 1 */
   Decode d;
   Encode e;
   AngleTabs t;
@@ -482,13 +472,15 @@ struct WriteArgs
   const uint8_t *cls;            /* class byte per stored point, in store order */
   uint32_t nSets;
   uint16_t setOf[256];           /* class byte -> set of files */
-  unsigned long long *base;      /* per (block, set): next output record */
+  const unsigned long long *base;   /* per (block, set): its first record in its file */
   const uint32_t *fileOf;        /* per (block, set): the file chosen */
+  const unsigned long long *fileFirst;   /* per file: its first output record */
   uint32_t nFiles;
   FileStat *stats;
 };
 
-/* Stored points per (block, set): one warp per block. */
+/* Stored points per (block, set): one warp per block.  With at most 32 sets
+ * (a set per class: nearly always) lane s keeps set s's count. */
 __global__ void __launch_bounds__(kBlock) setCountKernel(const WriteArgs a, uint32_t *__restrict__ counts)
 {
   const int lane = threadIdx.x & 31;
@@ -496,30 +488,101 @@ __global__ void __launch_bounds__(kBlock) setCountKernel(const WriteArgs a, uint
   for (uint64_t leaf = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); leaf < a.nLeaves; leaf += warps)
   {
     const uint32_t first = a.leafFirst[leaf], cnt = a.leafCount[leaf];
+    uint32_t mine = 0;
+    for (uint32_t q = 32 + lane; q < a.nSets; q += 32)
+      counts[leaf * a.nSets + q] = 0;
+    __syncwarp();
     for (uint32_t c0 = 0; c0 < cnt; c0 += 32)
     {
       const bool valid = c0 + lane < cnt;
-      const unsigned act = __ballot_sync(0xffffffffu, valid);
-      if (valid)
+      const uint32_t s = valid ? a.setOf[a.cls[first + c0 + lane]] : 0xffffffffu;
+      unsigned left = __ballot_sync(0xffffffffu, valid);
+      while (left)
       {
-        const uint32_t s = a.setOf[a.cls[first + c0 + lane]];
-        const unsigned gm = __match_any_sync(act, s);
-        if (lane == __ffs(gm) - 1)
-          counts[leaf * a.nSets + s] += __popc(gm);
+        const uint32_t t = __shfl_sync(0xffffffffu, s, __ffs(left) - 1);
+        const unsigned m = __ballot_sync(0xffffffffu, s == t);
+        left &= ~m;
+        if (t < 32 && lane == (int)t)
+          mine += __popc(m);
+        if (t >= 32 && lane == 0)
+          counts[leaf * a.nSets + t] += __popc(m);
       }
-      __syncwarp();
     }
+    if (lane < (int)a.nSets)
+      counts[leaf * a.nSets + lane] = mine;
   }
 }
 
+/* Copies len bytes of record idx to a word-aligned slot, in aligned words
+ * whatever the record's alignment (the first and last record of the buffer byte
+ * by byte, so that no word reaches outside it). */
+__device__ __forceinline__ void loadAnyRecord(uint32_t *slot, const uint8_t *rec, uint64_t n, uint64_t idx, uint32_t stride,
+                                              int len)
+{
+  const uint8_t *src = rec + idx * stride;
+  if (idx == 0 || idx + 1 == n)
+  {
+    for (int k = 0; k < len; k++)
+      ((uint8_t *)slot)[k] = __ldg(src + k);
+    return;
+  }
+  const unsigned sh = 8 * (unsigned)((uintptr_t)src & 3);
+  const uint32_t *w = (const uint32_t *)((uintptr_t)src & ~(uintptr_t)3);
+  const int words = (len + 3) >> 2;
+  const bool spill = ((uintptr_t)src & 3) + len > 4u * words;   // the last slot word takes from one word more
+  uint32_t lo = __ldg(w);
+#pragma unroll 4
+  for (int k = 1; k < words; k++)
+  {
+    const uint32_t hi = __ldg(w + k);
+    slot[k - 1] = __funnelshift_r(lo, hi, sh);
+    lo = hi;
+  }
+  slot[words - 1] = __funnelshift_r(lo, spill ? __ldg(w + words) : 0u, sh);
+}
+
+/* Copies bytes from shared memory to any address in aligned words, a warp
+ * together (src: byte offset into the word-aligned buf). */
+__device__ __forceinline__ void copyOut(uint8_t *dst, const uint32_t *buf, uint32_t src, uint32_t bytes, int lane)
+{
+  const uint32_t head = min(bytes, (uint32_t)(-(intptr_t)dst & 3)), words = (bytes - head) >> 2;
+  const uint8_t *b = (const uint8_t *)buf;
+  if (lane < (int)head)
+    dst[lane] = b[src + lane];
+  const uint32_t s0 = src + head, sh = 8 * (s0 & 3);
+  uint32_t *d = (uint32_t *)(dst + head);
+  const uint32_t *w = buf + (s0 >> 2);
+  for (uint32_t k = lane; k < words; k += 32)
+    d[k] = sh ? __funnelshift_r(w[k], w[k + 1], sh) : w[k];
+  const uint32_t done = head + 4 * words;
+  if (lane < (int)(bytes - done))
+    dst[done + lane] = b[src + done + lane];
+}
+
+/* One warp per block: its stored points' records are gathered 32 at a time,
+ * re-encoded and packed in shared memory, each set's together, and each set's
+ * run is copied to its file's place in aligned words.  Records of 30 bytes
+ * loaded byte by byte and stored halfword by halfword, each lane its own, took
+ * 0.76 ms for 6M records; so it was 0.41 ms, a sixth of the time spent waiting
+ * at the end for the warp with the largest block.  Warps that take the blocks
+ * as they get free: 0.31 ms, bound by the latency of the random record reads
+ * (starting a row's reads a row ahead with cp.async gained nothing: it needs
+ * the shared memory of a quarter of the warps). */
+/* Shared words of a warp: 32 input slots, 32 packed output records and a word to read past them. */
+constexpr int kWarpWords = 2 * 32 * kSlotWords + 1;
 template <bool SHARED_STATS>
-__global__ void __launch_bounds__(kBlock) writeKernel(const WriteArgs a)
+__global__ void __launch_bounds__(kBlock, 4) writeKernel(const WriteArgs a)
 {
   extern __shared__ uint4 dyn[];
-  uint32_t *inSlots = (uint32_t *)dyn;
-  uint32_t *outSlots = inSlots + kBlock * kSlotWords;
-  FileStat *sst = (FileStat *)(outSlots + kBlock * kSlotWords);
-  FileStat *st = SHARED_STATS ? sst : a.stats;
+  uint32_t *inSlots = (uint32_t *)dyn + (threadIdx.x >> 5) * kWarpWords, *packed = inSlots + 32 * kSlotWords;
+  // a block's own counters have 32 bits (a shared 64-bit add is a loop)
+  typedef typename std::conditional<SHARED_STATS, StatOf<uint32_t>, FileStat>::type Stat;
+  StatOf<uint32_t> *sst = (StatOf<uint32_t> *)((uint32_t *)dyn + (kBlock / 32) * kWarpWords);
+  Stat *st;
+  if constexpr (SHARED_STATS)
+    st = sst;
+  else
+    st = a.stats;
   if (SHARED_STATS)
   {
     for (uint32_t f = threadIdx.x; f < a.nFiles; f += blockDim.x)
@@ -534,65 +597,121 @@ __global__ void __launch_bounds__(kBlock) writeKernel(const WriteArgs a)
     }
     __syncthreads();
   }
-  uint8_t *si = (uint8_t *)(inSlots + threadIdx.x * kSlotWords);
-  uint8_t *so = (uint8_t *)(outSlots + threadIdx.x * kSlotWords);
   const Layout Li = layoutOf(a.inFmt), Lo = layoutOf(a.outFmt);
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1;
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  for (uint64_t leaf = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); leaf < a.nLeaves; leaf += warps)
+  uint32_t *slot = inSlots + lane * kSlotWords;
+  for (;;)
   {
+    // the next block not taken yet: they differ by two orders of magnitude in points
+    unsigned long long leaf = 0;
+    if (lane == 0)
+      leaf = atomicAdd(&a.stats[a.nFiles].cnt[0], 1ull);
+    leaf = __shfl_sync(0xffffffffu, leaf, 0);
+    if (leaf >= a.nLeaves)
+      break;
     const uint32_t first = a.leafFirst[leaf], cnt = a.leafCount[leaf];
+    // lane s: where set s's next point of the block goes, and its file (sets
+    // from 32 on are looked up and counted as they are met)
+    uint32_t myFile = 0;
+    unsigned long long next = 0;
+    if (lane < (int)a.nSets)
+    {
+      myFile = a.fileOf[leaf * a.nSets + lane];
+      next = myFile < a.nFiles ? a.fileFirst[myFile] + a.base[leaf * a.nSets + lane] : 0;
+    }
+    uint32_t idx = 0, cl = 0, idxNext = 0, clNext = 0;
+    if (lane < (int)cnt)
+    {
+      idxNext = a.sidx[first + lane];
+      clNext = a.cls[first + lane];
+    }
     for (uint32_t c0 = 0; c0 < cnt; c0 += 32)
     {
       const bool valid = c0 + lane < cnt;
-      const unsigned act = __ballot_sync(0xffffffffu, valid);
+      LasPt p{};
+      int32_t q[3] = {0, 0, 0};
+      uint32_t s = 0xffffffffu;
+      // the next row's indices while this one's records are on their way
+      idx = idxNext;
+      cl = clNext;
+      if (c0 + 32 + lane < cnt)
+      {
+        idxNext = a.sidx[first + c0 + 32 + lane];
+        clNext = a.cls[first + c0 + 32 + lane];
+      }
       if (valid)
       {
-        const uint32_t idx = a.sidx[first + c0 + lane];
-        const uint8_t cl = a.cls[first + c0 + lane];
-        const uint32_t s = a.setOf[cl];
-        loadRecord(si, a.rec + (uint64_t)idx * a.stride, Li.len, a.inWords);
-        LasPt p;
-        parseRecord(si, a.inFmt, Li, a.d, a.t, p);
-        p.cls = cl;
-        int32_t q[3];
+        s = a.setOf[cl];
+        loadAnyRecord(slot, a.rec, a.n, idx, a.stride, Li.len);
+        parseRecord((const uint8_t *)slot, a.inFmt, Li, a.d, a.t, p);
+        p.cls = (uint16_t)cl;
         for (int k = 0; k < 3; k++)
           q[k] = a.e.shift[k] ? (int32_t)(uint32_t)(unsigned long long)((long long)p.X[k] + a.e.by[k])
                               : quantise(decodeAxis(a.d, p.X[k], k), a.e, k);
-        encodeRecord(so, a.outFmt, Lo, p, q, a.inFmt >= 6, a.t);
-        // the block's points of one set go to one file, in store order
-        const unsigned gm = __match_any_sync(act, s);
-        const int leader = __ffs(gm) - 1;
-        unsigned long long b = 0;
-        uint32_t file = 0;
-        if (lane == leader)
+      }
+      // the block's points of one set go to one file, in store order
+      unsigned left = __ballot_sync(0xffffffffu, valid);
+      uint32_t at = 0;   // records packed so far
+      while (left)
+      {
+        const uint32_t t = __shfl_sync(0xffffffffu, s, __ffs(left) - 1);
+        const unsigned m = __ballot_sync(0xffffffffu, s == t);
+        left &= ~m;
+        const uint32_t k = __popc(m);
+        uint32_t file;
+        unsigned long long pos;
+        if (t < 32)
         {
-          b = atomicAdd(&a.base[leaf * a.nSets + s], (unsigned long long)__popc(gm));
-          file = a.fileOf[leaf * a.nSets + s];
+          file = __shfl_sync(0xffffffffu, myFile, t);
+          pos = __shfl_sync(0xffffffffu, next, t);
+          if (lane == (int)t)
+            next += k;
         }
-        b = __shfl_sync(act, b, leader);
-        file = __shfl_sync(act, file, leader);
-        storeRecord(a.out + (b + __popc(gm & lt)) * (uint64_t)Lo.len, so, Lo.len, a.outWidth);
+        else
+        {
+          // points of set t in the block's earlier rows
+          uint32_t before = 0;
+          for (uint32_t r = lane; r < c0; r += 32)
+            before += a.setOf[a.cls[first + r]] == t;
+          before = __reduce_add_sync(0xffffffffu, before);
+          file = a.fileOf[leaf * a.nSets + t];
+          pos = a.fileFirst[file] + a.base[leaf * a.nSets + t] + before;
+        }
+        const bool mine = (m >> lane) & 1;
+        if (mine)
+          encodeRecord((uint8_t *)packed + (at + __popc(m & lt)) * Lo.len, a.outFmt, Lo, p, q, a.inFmt >= 6, a.t);
+        __syncwarp();
+        copyOut(a.out + pos * (uint64_t)Lo.len, packed, at * Lo.len, k * Lo.len, lane);
+        at += k;
         int32_t mn[3], mx[3];
-        for (int k = 0; k < 3; k++)
+        for (int d = 0; d < 3; d++)
         {
-          mn[k] = __reduce_min_sync(gm, q[k]);
-          mx[k] = __reduce_max_sync(gm, q[k]);
-        }
-        if (lane == leader)
-        {
-          for (int k = 0; k < 3; k++)
-          {
-            atomicMin(&st[file].mn[k], mn[k]);
-            atomicMax(&st[file].mx[k], mx[k]);
-          }
-          atomicAdd(&st[file].cnt[0], (unsigned long long)__popc(gm));
+          mn[d] = __reduce_min_sync(0xffffffffu, mine ? q[d] : INT32_MAX);
+          mx[d] = __reduce_max_sync(0xffffffffu, mine ? q[d] : INT32_MIN);
         }
         // nPoints[returnNum] for return numbers 1-15 (las.cpp:900-901)
-        const unsigned rm = __match_any_sync(act, (s << 4) | (p.ret & 15));
-        if (p.ret > 0 && p.ret < 16 && lane == __ffs(rm) - 1)
-          atomicAdd(&st[file].cnt[p.ret], (unsigned long long)__popc(rm));
+        const uint32_t ret = mine ? p.ret & 15 : 0xffu;
+        unsigned rleft = m;
+        uint32_t perRet = 0;   // lane r: points of return number r
+        while (rleft)
+        {
+          const uint32_t r = __shfl_sync(0xffffffffu, ret, __ffs(rleft) - 1);
+          const unsigned rm = __ballot_sync(0xffffffffu, ret == r);
+          rleft &= ~rm;
+          if (lane == (int)r)
+            perRet = __popc(rm);
+        }
+        if (lane == 0)
+          perRet = k;
+        Stat &f = st[file];
+        if (lane < 16 && perRet)
+          atomicAdd(&f.cnt[lane], (decltype(f.cnt[0] + 0))perRet);
+        if (lane < 3)
+        {
+          atomicMin(&f.mn[lane], lane == 0 ? mn[0] : (lane == 1 ? mn[1] : mn[2]));
+          atomicMax(&f.mx[lane], lane == 0 ? mx[0] : (lane == 1 ? mx[1] : mx[2]));
+        }
       }
       __syncwarp();
     }
@@ -611,7 +730,7 @@ __global__ void __launch_bounds__(kBlock) writeKernel(const WriteArgs a)
       }
       for (int k = 0; k < 16; k++)
         if (sst[f].cnt[k])
-          atomicAdd(&a.stats[f].cnt[k], sst[f].cnt[k]);
+          atomicAdd(&a.stats[f].cnt[k], (unsigned long long)sst[f].cnt[k]);
     }
   }
 }
@@ -630,25 +749,40 @@ __global__ void statInit(FileStat *st, uint32_t n)
   }
 }
 
-/* The class byte of every stored point in store order: from the last
- * classify's store-order labels where a tile decided the point (sequential
- * reads), else from the per-record class bytes (recCls). */
-__global__ void storeClassKernel(uint64_t nd, const uint32_t *__restrict__ sidx, const int32_t *__restrict__ owner,
-                                 const uint8_t *__restrict__ label, const uint8_t *__restrict__ recCls,
-                                 uint8_t *__restrict__ out)
-{
-  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += (uint64_t)gridDim.x * blockDim.x)
-    out[j] = (owner && owner[j] >= 0) ? label[j] : recCls[sidx[j]];
-}
-
-__global__ void storedTotals(uint64_t nd, const uint8_t *__restrict__ cls, unsigned long long *__restrict__ totals)
+/* The class byte of every stored point in store order, and how many have each:
+ * from the last classify's store-order labels where a tile decided the point
+ * (sequential reads), else from the per-record class bytes (recCls). */
+__global__ void __launch_bounds__(kBlock) storeClassKernel(uint64_t nd, const uint32_t *__restrict__ sidx,
+                                                           const int32_t *__restrict__ owner,
+                                                           const uint8_t *__restrict__ label,
+                                                           const uint8_t *__restrict__ recCls, uint8_t *__restrict__ out,
+                                                           unsigned long long *__restrict__ totals)
 {
   __shared__ unsigned int h[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x)
     h[i] = 0;
   __syncthreads();
-  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += (uint64_t)gridDim.x * blockDim.x)
-    atomicAdd(&h[cls[j]], 1u);
+  const int lane = threadIdx.x & 31;
+  for (uint64_t j0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < nd; j0 += (uint64_t)gridDim.x * blockDim.x)
+  {
+    const uint64_t j = j0 + lane;
+    uint32_t c = 0x100;
+    if (j < nd)
+    {
+      c = (owner && owner[j] >= 0) ? label[j] : recCls[sidx[j]];
+      out[j] = (uint8_t)c;
+    }
+    // a warp's points have one to three classes
+    unsigned left = __ballot_sync(0xffffffffu, j < nd);
+    while (left)
+    {
+      const uint32_t t = __shfl_sync(0xffffffffu, c, __ffs(left) - 1);
+      const unsigned m = __ballot_sync(0xffffffffu, c == t);
+      left &= ~m;
+      if (lane == 0)
+        atomicAdd(&h[t], (unsigned)__popc(m));
+    }
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < 256; i += blockDim.x)
     if (h[i])
@@ -926,6 +1060,7 @@ int wb_las_decode(wb_ctx *c, const wb_cloud *cloud, int fmt, const wb_las_points
     a.d.scale[k] = cloud->scale[k];
   }
   a.d.unit = cloud->unit;
+  a.d.scaled = cloud->unit != 1;
   WbScratch rin(c), fields(c);
   const bool host = !cloud->device_resident;
   a.rec = (const uint8_t *)cloud->records;
@@ -1021,7 +1156,7 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
   const uint64_t n = c->n, nd = c->nd, L = c->n_leaves;
   const Layout Li = layoutOf(in_format), Lo = layoutOf(opt->point_format);
   int rc;
-  WbScratch rin(c), cin(c), cstore(c), dout(c), tot(c), counts(c), bases(c), fileOf(c), stats(c);
+  WbScratch rin(c), cin(c), dout(c);
 
   WriteArgs a;
   a.stride = cloud->stride;
@@ -1033,6 +1168,7 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
     a.d.scale[k] = cloud->scale[k];
   }
   a.d.unit = cloud->unit;
+  a.d.scaled = cloud->unit != 1;
   // one scale and offset for every file: setScale gets the same box each time
   for (int k = 0; k < 3; k++)
     setScale(opt->min_cor[k], opt->max_cor[k], opt->scale[k], opt->unit, a.e.scale[k], a.e.off[k]);
@@ -1060,7 +1196,6 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
       }
     }
   }
-  a.d.scaled = cloud->unit != 1;
   if ((rc = angleTables(c, a.t)))
     return rc;
   for (int k = 0; k < 3; k++)
@@ -1078,7 +1213,7 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
   }
   else
     a.rec = nullptr;
-  a.inWords = ((uintptr_t)a.rec % 4 == 0) && (a.stride % 4 == 0);
+  a.n = n;
   const uint8_t *recCls;
   if (!cls)
     recCls = c->clsFinal;
@@ -1092,26 +1227,25 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
     recCls = (const uint8_t *)cin.b.p;
   }
   a.sidx = (const uint32_t *)c->sidx.p;
-  // class bytes in store order, read sequentially by every pass below
-  if ((rc = wb_ensure(c, cstore.b, nd + 16)))
+  // The build's scratch buffers serve here: class bytes in store order (read
+  // sequentially by every pass below) where the survivors were marked, the
+  // tables in a sort buffer.
+  if ((rc = wb_ensure(c, c->tmp8, nd + 16)) || (rc = wb_ensure(c, c->key0, 256 * 8)))
     return rc;
+  uint8_t *cstore = (uint8_t *)c->tmp8.p;
+  unsigned long long *tot = (unsigned long long *)c->key0.p;
+  // class totals of the stored points (OctStore::countClasses)
+  WB_CUDA(c, cudaMemsetAsync(tot, 0, 256 * 8, c->stream));
   if (nd)
     { storeClassKernel<<<gridOf(c, nd), kBlock, 0, c->stream>>>(
           nd, a.sidx, (!cls && c->stage >= 3) ? (const int32_t *)c->owner.p : nullptr, (const uint8_t *)c->label.p, recCls,
-          (uint8_t *)cstore.b.p); ++c->launches; }
-  a.cls = (const uint8_t *)cstore.b.p;
+          cstore, tot); ++c->launches; }
+  a.cls = cstore;
   a.leafFirst = (const uint32_t *)c->leafFirst.p;
   a.leafCount = (const uint32_t *)c->leafCount.p;
   a.nLeaves = L;
-
-  // class totals of the stored points (OctStore::countClasses)
-  if ((rc = wb_ensure(c, tot.b, 256 * 8)))
-    return rc;
-  WB_CUDA(c, cudaMemsetAsync(tot.b.p, 0, 256 * 8, c->stream));
-  if (nd)
-    { storedTotals<<<gridOf(c, nd), kBlock, 0, c->stream>>>(nd, a.cls, (unsigned long long *)tot.b.p); ++c->launches; }
   uint64_t T[256];
-  WB_CUDA(c, cudaMemcpyAsync(T, tot.b.p, sizeof T, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaMemcpyAsync(T, tot, sizeof T, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
 
   Plan P = planFiles(T, opt);
@@ -1123,67 +1257,93 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
   memcpy(a.setOf, P.setOf, sizeof a.setOf);
   a.nFiles = (uint32_t)P.nFiles;
 
-  // stored points per (block, set)
-  // per (block, set) counts, first records and files go through one pinned
-  // host buffer of the context (16 bytes per entry)
-  const size_t stageBytes = L * S * 16 + 64;
-  if ((rc = wb_host_stage(c, stageBytes)))
+  // stored points per (block, set): counts, first records and files go through
+  // one pinned host buffer of the context (16 bytes per entry)
+  const uint64_t entries = L * S;
+  if ((rc = wb_host_stage(c, entries * 16 + 64)))
     return rc;
   uint64_t *base = (uint64_t *)c->hostStage;
-  uint32_t *cnt = (uint32_t *)(base + L * S), *fof = cnt + L * S;
+  uint32_t *cnt = (uint32_t *)(base + entries), *fof = cnt + entries;
+  const size_t statBytes = sizeof(FileStat) * (P.nFiles + 1), firstBytes = 8 * ((size_t)P.nFiles + 1);
+  if ((rc = wb_ensure(c, c->key0, entries * 16 + statBytes + firstBytes + 64)))
+    return rc;
+  // device tables: first records and files (as in the host buffer), counts, file figures
+  uint64_t *dBase = (uint64_t *)c->key0.p;
+  uint32_t *dCnt = (uint32_t *)(dBase + entries), *dFof = dCnt + entries;
+  unsigned long long *dFirst = (unsigned long long *)(dFof + entries);
+  a.stats = (FileStat *)(dFirst + P.nFiles + 1);
+  a.base = (const unsigned long long *)dBase;
+  a.fileOf = dFof;
+  a.fileFirst = dFirst;
+  { statInit<<<gridOf(c, P.nFiles + 1), kBlock, 0, c->stream>>>(a.stats, (uint32_t)P.nFiles + 1); ++c->launches; }
   if (L)
   {
-    if ((rc = wb_ensure(c, counts.b, L * S * 4)))
-      return rc;
-    WB_CUDA(c, cudaMemsetAsync(counts.b.p, 0, L * S * 4, c->stream));
-    { setCountKernel<<<gridOf(c, L * 32, 8), kBlock, 0, c->stream>>>(a, (uint32_t *)counts.b.p); ++c->launches; }
-    WB_CUDA(c, cudaMemcpyAsync(cnt, counts.b.p, L * S * 4, cudaMemcpyDefault, c->stream));
+    { setCountKernel<<<gridOf(c, L * 32, 8), kBlock, 0, c->stream>>>(a, dCnt); ++c->launches; }
+    WB_CUDA(c, cudaMemcpyAsync(cnt, dCnt, entries * 4, cudaMemcpyDefault, c->stream));
     WB_CUDA(c, cudaStreamSynchronize(c->stream));
   }
-  memset(base, 0, L * S * 8);
-  memset(fof, 0, L * S * 4);
 
   // writeFiles: at each block, each set's points go to its file holding the
-  // fewest points, the first of them on a tie (cloudoutput.cpp:196-209)
-  std::vector<uint64_t> fileCount(P.nFiles, 0);
+  // fewest points, the first of them on a tie (cloudoutput.cpp:196-209).
+  // Entries without points are left as they are; nothing reads them.
+  // A set of few files keeps points and file in one word, so that the least word
+  // is the answer and no branch depends on it; the sets are walked side by side,
+  // so that their chains of choices overlap.
+  constexpr int kFewFiles = 16;
+  std::vector<uint64_t> fileCount(P.nFiles, 0), word((size_t)S * kFewFiles, ~0ull);
+  std::vector<uint32_t> few;
+  for (uint32_t s = 0; s < S; s++)
+  {
+    if (T[P.setClass[s]] && !P.setFiles[s])
+      return wb_fail(c, WB_ESTATE, "wb_las_write_output: points of a class without a file");
+    if (P.setFiles[s] && P.setFiles[s] <= kFewFiles)
+      few.push_back(s);
+    for (int i = 0; i < P.setFiles[s] && i < kFewFiles; i++)
+      word[(size_t)s * kFewFiles + i] = (uint64_t)i;
+  }
+  for (uint64_t leaf = 0; leaf < L; leaf++)
+    for (uint32_t s : few)
+    {
+      const uint64_t e = leaf * S + s;
+      const uint32_t k = cnt[e];
+      if (!k)
+        continue;
+      uint64_t *w = &word[(size_t)s * kFewFiles], least = w[0];
+      for (int i = 1; i < P.setFiles[s]; i++)
+        least = w[i] < least ? w[i] : least;
+      const int i = (int)(least % kFewFiles);
+      base[e] = least / kFewFiles;
+      fof[e] = (uint32_t)(P.setFile0[s] + i);
+      w[i] += (uint64_t)k * kFewFiles;
+    }
+  for (uint32_t s : few)
+    for (int i = 0; i < P.setFiles[s]; i++)
+      fileCount[P.setFile0[s] + i] = word[(size_t)s * kFewFiles + i] / kFewFiles;
   typedef std::pair<uint64_t, int> Entry;
   for (uint32_t s = 0; s < S; s++)
   {
     const int f0 = P.setFile0[s], nf = P.setFiles[s];
+    if (nf <= kFewFiles)
+      continue;
     std::priority_queue<Entry, std::vector<Entry>, std::greater<Entry>> heap;
-    if (nf > 16)
-      for (int i = 0; i < nf; i++)
-        heap.push(Entry(0, f0 + i));
+    for (int i = 0; i < nf; i++)
+      heap.push(Entry(0, f0 + i));
     for (uint64_t leaf = 0; leaf < L; leaf++)
     {
       const uint32_t k = cnt[leaf * S + s];
       if (!k)
         continue;
-      if (!nf)
-        return wb_fail(c, WB_ESTATE, "wb_las_write_output: points of a class without a file");
-      int f = f0;
-      if (nf > 16)
-      {
-        f = heap.top().second;
-        heap.pop();
-      }
-      else
-  a.d.scaled = cloud->unit != 1;
-        for (int i = 1; i < nf; i++)
-          if (fileCount[f0 + i] < fileCount[f])
-            f = f0 + i;
+      const int f = heap.top().second;
+      heap.pop();
       base[leaf * S + s] = fileCount[f];
       fof[leaf * S + s] = (uint32_t)f;
       fileCount[f] += k;
-      if (nf > 16)
-        heap.push(Entry(fileCount[f], f));
+      heap.push(Entry(fileCount[f], f));
     }
   }
   std::vector<uint64_t> fileFirst(P.nFiles + 1, 0);
   for (int f = 0; f < P.nFiles; f++)
     fileFirst[f + 1] = fileFirst[f] + fileCount[f];
-  for (uint64_t i = 0; i < L * S; i++)
-    base[i] += fileFirst[fof[i]];
 
   uint8_t *dst = (uint8_t *)out;
   const uint64_t outBytes = nd * (uint64_t)Lo.len;
@@ -1194,20 +1354,12 @@ int wb_las_write_output(wb_ctx *c, const wb_cloud *cloud, int in_format, const u
     dst = (uint8_t *)dout.b.p;
   }
   a.out = dst;
-  a.outWidth = ((uintptr_t)dst % 4 == 0 && Lo.len % 4 == 0) ? 4 : (((uintptr_t)dst % 2 == 0 && Lo.len % 2 == 0) ? 2 : 1);
-  if ((rc = wb_ensure(c, stats.b, sizeof(FileStat) * (P.nFiles + 1))))
-    return rc;
-  a.stats = (FileStat *)stats.b.p;
-  { statInit<<<gridOf(c, P.nFiles + 1), kBlock, 0, c->stream>>>(a.stats, (uint32_t)P.nFiles); ++c->launches; }
   if (L && nd)
   {
-    if ((rc = wb_ensure(c, bases.b, L * S * 8)) || (rc = wb_ensure(c, fileOf.b, L * S * 4)))
-      return rc;
-    WB_CUDA(c, cudaMemcpyAsync(bases.b.p, base, L * S * 8, cudaMemcpyDefault, c->stream));
-    WB_CUDA(c, cudaMemcpyAsync(fileOf.b.p, fof, L * S * 4, cudaMemcpyDefault, c->stream));
-    a.base = (unsigned long long *)bases.b.p;
-    a.fileOf = (const uint32_t *)fileOf.b.p;
-    const size_t slots = 2 * (size_t)kBlock * kSlotWords * 4;
+    WB_CUDA(c, cudaMemcpyAsync(dBase, base, entries * 8, cudaMemcpyDefault, c->stream));
+    WB_CUDA(c, cudaMemcpyAsync(dFof, fof, entries * 4, cudaMemcpyDefault, c->stream));
+    WB_CUDA(c, cudaMemcpyAsync(dFirst, fileFirst.data(), firstBytes, cudaMemcpyDefault, c->stream));
+    const size_t slots = (size_t)(kBlock / 32) * kWarpWords * 4;
     if (P.nFiles <= kSharedFiles)
     {
       const size_t smem = slots + sizeof(FileStat) * kSharedFiles;
