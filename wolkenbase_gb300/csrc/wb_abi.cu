@@ -463,24 +463,7 @@ int wb_tiles(wb_ctx *c, wb_tile *out, uint64_t capacity, uint64_t *count)
     return 0;
   if (capacity < T)
     return wb_fail(c, WB_EINVAL, "wb_tiles: capacity below the tile count");
-  std::vector<TileRes> r(T);
-  WB_CUDA(c, cudaMemcpyAsync(r.data(), c->tileRes.p, T * sizeof(TileRes), cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  for (uint64_t k = 0; k < T; k++)
-  {
-    wb_tile &t = out[k];
-    t.ex = c->flowHostEx[k];
-    t.ey = c->flowHostEy[k];
-    t.n_points = r[k].nPoints;
-    t.n_ground = r[k].nGround;
-    t.tree_flags = r[k].treeFlags;
-    t.pad = 0;
-    t.density = r[k].density;
-    t.h_scan = r[k].hScan;
-    t.hyperboloid_size = r[k].h;
-    t.height = r[k].height;
-  }
-  return 0;
+  return wb_read_tiles(c, out);
 }
 
 int wb_classify(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDevice)
@@ -556,14 +539,7 @@ int wb_tile_planes(wb_ctx *c, double *abc, uint64_t capacity)
   if (capacity < T)
     return wb_fail(c, WB_EINVAL, "wb_tile_planes: capacity below the tile count");
   WbDeviceGuard deviceGuard(c->device);
-  std::vector<TileRes> r(T);
-  if (T)
-    WB_CUDA(c, cudaMemcpyAsync(r.data(), c->tileRes.p, T * sizeof(TileRes), cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  for (uint64_t k = 0; k < T; k++)
-    for (int i = 0; i < 3; i++)
-      abc[3 * k + i] = r[k].plane[i];
-  return 0;
+  return wb_read_planes(c, abc);
 }
 
 int wb_get_tuning(wb_ctx *c, wb_tuning *t)

@@ -216,6 +216,8 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1);
 int wb_point_groups(wb_ctx *c, const unsigned long long **taken);
 int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count);
 int wb_scan_impl(wb_ctx *c, const wb_params *p);
+int wb_read_tiles(wb_ctx *c, wb_tile *out);      /* n_tiles entries each, host memory */
+int wb_read_planes(wb_ctx *c, double *abc);
 int wb_classify_impl(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDevice);
 int wb_find_block_impl(wb_ctx *c, const double *xyz, uint64_t m, int64_t *leaf);
 
