@@ -128,7 +128,8 @@ struct ClsArgs
   const int4 *gpt;     /* int4 {X, Y, Z, position | stray bit} per point, column order */
   const int4 *groups;     /* point groups, two int4 each (groupBoxKernel) */
   const int2 *bxy, *bzw;  /* their points: {X, Y} and {Z, store position | stray bit} */
-  const unsigned long long *groupsTaken;   /* their number, above the low 36 bits */
+  const unsigned long long *groupsTaken;   /* their number, above the low 36 bits; then the high ones, in the lower half */
+  uint64_t maxGroups;                      /* the order to take them in begins after as many records */
   const uint2 *colGroups; /* column groups {column, first point}, when margins are wanted */
   float gky, gkz;         /* y record unit / x record unit; z record unit / (slope * x record unit) */
   float gInv, gTiny;      /* 1 / (slope * x record unit); 1e-12 m^2 in that unit squared */
@@ -1501,7 +1502,7 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
   a.sinT = tab + 511;
   a.cosT = tab + 1023;
   a.label = (uint8_t *)c->label.p;
-  if ((rc = wb_point_groups(c, &a.groupsTaken)))
+  if ((rc = wb_point_groups(c, &a.groupsTaken, &a.maxGroups)))
     return rc;
   a.gx0 = c->grid.x0;
   a.gy0 = c->grid.y0;
@@ -1713,7 +1714,11 @@ __global__ void __launch_bounds__(32 * W, MINB) batchGroups(BatchHdr *h, const B
         __syncwarp();
       }
       if constexpr (ARCS)
-        classifyGroupArcs(sa[w], g - lo, lane, gsm[w]);
+        {
+        const uint64_t i = g - lo, high = (uint32_t)sa[w].groupsTaken[1];
+        const uint32_t *order = (const uint32_t *)(sa[w].groups + 2 * sa[w].maxGroups);
+        classifyGroupArcs(sa[w], order[i < high ? i : sa[w].maxGroups - 1 - (i - high)], lane, gsm[w]);
+      }
       else
         classifyGroup(sa[w], sa[w].colGroups[g - lo], lane, gsm[w]);
     }

@@ -488,14 +488,22 @@ __device__ __forceinline__ int hilbert8(int x, int y)
  * the points' buckets, its prefix, and a scatter; the warps take their places
  * in the two lists from one counter (points in the low 36 bits, groups above).
  * A super-cell's groups are consecutive: its record gets the first one and
- * their number. */
+ * their number.
+ *
+ * The order in which classify takes the groups, after the records: those of
+ * points high above their column from the front, the others from the back
+ * (taken[1] counts both, the high ones in its lower half).  A group under
+ * trees reads up to 20 times the groups an average one does, and the last
+ * groups to start hold a few warps while the rest of the GPU idles.  With the
+ * high ones first the fast pass takes 1.41 ms instead of 1.61 for 1M points and
+ * 6.16 instead of 6.63 for 5M; for 50M it is the same. */
 constexpr int kOrderWarps = 8, kOrderBuckets = 96;
 __global__ void __launch_bounds__(32 * kOrderWarps) groupOrderKernel(int nx, int ny, int snx, int sny, float colUnits,
                                                                      const int4 *__restrict__ rec,
                                                                      int4 *__restrict__ srec,
                                                                      const int4 *__restrict__ gpt,
                                                                      int2 *__restrict__ bxy, int2 *__restrict__ bzw,
-                                                                     int4 *__restrict__ groups,
+                                                                     int4 *__restrict__ groups, uint64_t maxGroups,
                                                                      unsigned long long *__restrict__ taken)
 {
   __shared__ uint32_t hist[kOrderWarps][kOrderBuckets];
@@ -564,16 +572,24 @@ __global__ void __launch_bounds__(32 * kOrderWarps) groupOrderKernel(int nx, int
   }
   low = __reduce_add_sync(0xffffffffu, low);
   const uint32_t gLow = (low + 31) / 32, gAll = gLow + (total - low + 31) / 32;
-  unsigned long long at = 0;
+  unsigned long long at = 0, turn = 0;
   if (lane == 0)
+  {
     at = atomicAdd(taken, ((unsigned long long)gAll << 36) | total);
+    turn = atomicAdd(taken + 1, ((unsigned long long)gLow << 32) | (gAll - gLow));
+  }
   at = __shfl_sync(0xffffffffu, at, 0);
+  turn = __shfl_sync(0xffffffffu, turn, 0);
+  uint32_t *order = (uint32_t *)(groups + 2 * maxGroups);
   const uint32_t base = (uint32_t)(at & ((1ull << 36) - 1)), g0 = (uint32_t)(at >> 36);
   // first point, points and super-cell of each group; groupBoxKernel adds the bounds
   for (uint32_t k = lane; k < gAll; k += 32)
+  {
+    order[k < gLow ? maxGroups - 1 - ((turn >> 32) + k) : (uint32_t)turn + (k - gLow)] = g0 + k;
     groups[2 * (uint64_t)(g0 + k) + 1] =
         k < gLow ? make_int4(0, (int)(base + 32 * k), (int)min(32u, low - 32 * k), 0)
                  : make_int4(0, (int)(base + low + 32 * (k - gLow)), (int)min(32u, total - low - 32 * (k - gLow)), 0);
+  }
   if (lane == 0)
   {
     srec[2 * s + 1].y = (int)g0;
@@ -822,18 +838,20 @@ int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count)
 /* The point groups of the fast pass, formed once per grid when a classify
  * first wants them (an octree or a scan alone does not).  Their number stays on
  * the device: *taken, groups above the low 36 bits. */
-int wb_point_groups(wb_ctx *c, const unsigned long long **taken)
+int wb_point_groups(wb_ctx *c, const unsigned long long **taken, uint64_t *maxGroups)
 {
   unsigned long long *gTot = (unsigned long long *)((char *)c->small.p + 704);
+  const uint64_t nd = c->nd, nsup = (uint64_t)c->grid.snx * c->grid.sny;
+  // at most 32 points each, two partly filled ones per super-cell
+  const uint64_t most = nd / 32 + 2 * std::min<uint64_t>(nsup, nd) + 1;
   *taken = gTot;
+  *maxGroups = most;
   if (c->grid.grouped)
     return 0;
-  const uint64_t nd = c->nd, nsup = (uint64_t)c->grid.snx * c->grid.sny;
   int rc;
-  // at most 32 points each, two partly filled ones per super-cell
-  if ((rc = wb_ensure(c, c->groups, (nd / 32 + 2 * std::min<uint64_t>(nsup, nd) + 1) * 32 + 64)))
+  if ((rc = wb_ensure(c, c->groups, most * 36 + 64)))
     return rc;
-  WB_CUDA(c, cudaMemsetAsync(gTot, 0, 8, c->stream));
+  WB_CUDA(c, cudaMemsetAsync(gTot, 0, 16, c->stream));
   if (nd)
   {
     const WbGeom &g = c->g;
@@ -841,7 +859,7 @@ int wb_point_groups(wb_ctx *c, const unsigned long long **taken)
     { groupOrderKernel<<<(unsigned)((nsup + kOrderWarps - 1) / kOrderWarps), 32 * kOrderWarps, 0, c->stream>>>(
           c->grid.nx, c->grid.ny, c->grid.snx, c->grid.sny, (float)(c->grid.cell / fabs(g.scale[2] * g.unit)),
           (const int4 *)c->cellRec.p, (int4 *)c->superRec.p, (const int4 *)c->gpt.p, (int2 *)c->gKey0.p,
-          (int2 *)c->gKey1.p, (int4 *)c->groups.p, gTot); ++c->launches; }
+          (int2 *)c->gKey1.p, (int4 *)c->groups.p, most, gTot); ++c->launches; }
     { groupBoxKernel<<<(unsigned)std::min<uint64_t>((nd / 32 + 8) / 8, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
           gridArgs(c), gTot, (const int2 *)c->gKey0.p, (const int2 *)c->gKey1.p, (int4 *)c->groups.p); ++c->launches; }
     WB_CUDA(c, cudaGetLastError());

@@ -213,7 +213,7 @@ int wb_lookback_words(wb_ctx *c, uint64_t words, unsigned **counter, unsigned lo
 int wb_point_leaf_map(wb_ctx *c);   /* point -> leaf map into c->pointLeaf */
 int wb_build_impl(wb_ctx *c, const wb_cloud *cloud);
 int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1);
-int wb_point_groups(wb_ctx *c, const unsigned long long **taken);
+int wb_point_groups(wb_ctx *c, const unsigned long long **taken, uint64_t *maxGroups);
 int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count);
 int wb_scan_impl(wb_ctx *c, const wb_params *p);
 int wb_read_tiles(wb_ctx *c, wb_tile *out);      /* n_tiles entries each, host memory */
