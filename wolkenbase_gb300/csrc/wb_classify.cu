@@ -369,17 +369,16 @@ __device__ __forceinline__ void setupPoint(const ClsArgs &a, uint64_t j)
   double hs = a.tiles[k].h;
   const double pz = a.xyzd[2 * a.nd + j];
   double por = hs * (a.slope * a.slope);
-  double por2 = por * por;
   double cz = (pz - a.thickness) + por;
   PtSetup s;
   s.czp = (float)(cz - pz);
-  s.por2f = (float)por2;
-  // horizontal reach of the hyperboloid at the lowest point of the cloud
-  double zdMax = cz - a.zmin;
-  // The ring counts only bound the search (columns beyond the reach hold no
-  // member), so they are formed in FP32 with a 1e-5 margin, far above the
-  // 1e-7 rounding of the FP32 root and products.
-  const float r2f = (float)((zdMax * zdMax - por2) * a.invSlope2);
+  s.por2f = (float)(por * por);
+  // Horizontal reach of the hyperboloid at the lowest point of the cloud.  The
+  // ring counts only bound the search (columns beyond the reach hold no
+  // member), so they are formed in FP32, both squares rounded apart by more
+  // than their error (the FP64 pipe bounds this kernel), with a 1e-5 margin.
+  const float zdMax = (float)(cz - a.zmin);
+  const float r2f = (zdMax * zdMax * (1 + 4e-7f) - s.por2f * (1 - 4e-7f)) * (float)a.invSlope2;
   const float reach = r2f > 0 ? sqrtf(r2f) * (1 + 1e-5f) + 1e-5f : 0.f;
   const int2 col = a.colOf[j];
   s.ci = col.x;
@@ -1786,6 +1785,8 @@ __global__ void batchGroundCount(const BatchHdr *__restrict__ h, BatchOut *__res
   // whole warps step together, so the ground points of a warp are counted
   // with one atomic per tile and one per job
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  int qRun = 0;                 // lane 0: the job counted last and its ground points not added yet
+  unsigned long long run = 0;   // (an atomic per warp and row on a job's one counter took 1.1 ms for 50M points)
   for (uint64_t w0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < total; w0 += stride)
   {
     const uint64_t g = w0 + lane;
@@ -1806,11 +1807,25 @@ __global__ void batchGroundCount(const BatchHdr *__restrict__ h, BatchOut *__res
       const unsigned sameT = __match_any_sync(m, ((unsigned long long)q << 32) | (uint32_t)t);
       if (lane == __ffs(sameT) - 1)
         atomicAdd(&((TileRes *)h->jobs[q].tiles)[t].nGround, __popc(sameT));
-      const unsigned sameQ = __match_any_sync(m, q);
-      if (lane == __ffs(sameQ) - 1)
-        atomicAdd(&o->ground[q], (unsigned long long)__popc(sameQ));
+    }
+    unsigned left = m;
+    while (left)   // one round, but where a row spans jobs
+    {
+      const int q0 = __shfl_sync(0xffffffffu, q, __ffs(left) - 1);
+      const unsigned sameQ = __ballot_sync(0xffffffffu, gnd && q == q0);
+      left &= ~sameQ;
+      if (lane == 0 && q0 != qRun)
+      {
+        if (run)
+          atomicAdd(&o->ground[qRun], run);
+        qRun = q0;
+        run = 0;
+      }
+      run += __popc(sameQ);
     }
   }
+  if (lane == 0 && run)
+    atomicAdd(&o->ground[qRun], run);
 }
 
 __global__ void batchScatter(const BatchHdr *__restrict__ h)

@@ -39,6 +39,7 @@
 #include <type_traits>
 #include <vector>
 #include "wb_internal.h"
+#include "wb_device.cuh"
 
 namespace
 {
@@ -274,23 +275,10 @@ __device__ __forceinline__ void parseRecord(const uint8_t *s, int f, const Layou
   p.nir = L.nir >= 0 ? (uint16_t)rd16(s, L.nir) : 0;
 }
 
-/* (double)X from its bits: the exponent and the shifted magnitude.  FP64
- * instructions issue at 1/64 rate here, the conversion among them; the decode
- * is bound by them (12 a record, 82% of the pipe, with the conversions and the
- * unit's comparison; six with neither). */
-__device__ __forceinline__ double intToDouble(int32_t X)
-{
-  const uint32_t m = X < 0 ? 0u - (uint32_t)X : (uint32_t)X;
-  const int lead = __clz(m);                    // 32 for zero
-  const uint32_t t = lead < 31 ? m << (lead + 1) : 0u;   // the magnitude below its leading one, at the top
-  const uint32_t hi = ((uint32_t)X & 0x80000000u) | ((uint32_t)(1023 + 31 - lead) << 20) | (t >> 12);
-  return m ? __hiloint2double((int)hi, (int)(t << 20)) : 0.0;
-}
-
 /* The location readPoint computes (las.cpp:808): (offset + scale*X) * unit. */
 __device__ __forceinline__ double decodeAxis(const Decode &d, int32_t X, int k)
 {
-  const double v = d.off[k] + d.scale[k] * intToDouble(X);
+  const double v = d.off[k] + d.scale[k] * wb_double(X);
   return d.scaled ? v * d.unit : v;   // x * 1 == x
 }
 
