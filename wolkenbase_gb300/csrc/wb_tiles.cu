@@ -436,54 +436,31 @@ struct ScanArgs
   TileArgs t;
   const uint32_t *tileStart, *tileN, *tilePts;   /* tile k: tilePts[tileStart[k] ...], tileN[k] points */
   double minH;
+  double rin;   /* the inner circle of the sector histogram, rad / sqrt(7) */
 };
 
 constexpr int kQ = 8;   // summed quantities: xx, yx, yy, x, y, xz, yz, z
 constexpr int kScanCache = 224;   // tile points whose coordinates stay in shared memory
 constexpr int kScanWarps = 6;     // tiles (one warp each) per block of the exact scan's sums and shape passes
 
-__device__ __forceinline__ void counterMergeGroup(double *part, uint64_t i, double g)
+__device__ __forceinline__ void counterMergeRow(double *part, uint64_t i, double g)
 {
-  uint64_t carry = i ^ (i + 8);
-  if (carry == 8)
-    part[3] = g;
+  uint64_t carry = i ^ (i + 32);
+  if (carry == 32)
+    part[5] = g;
   else
   {
-    part[3] += g;
-    int lvl = 4;
+    part[5] += g;
+    int lvl = 6;
     for (; carry >> (lvl + 1); lvl++)
       part[lvl] += part[lvl - 1];
     part[lvl] = part[lvl - 1];
   }
 }
 
-__device__ __forceinline__ void counterMergeOne(double *part, uint64_t i, double v)
-{
-  uint64_t carry = i ^ (i + 1);
-  if (carry == 1)
-    part[0] = v;
-  else
-  {
-    part[0] += v;
-    int lvl = 1;
-    for (; carry >> (lvl + 1); lvl++)
-      part[lvl] += part[lvl - 1];
-    part[lvl] = part[lvl - 1];
-  }
-}
-
-/* Partial sums of the binary counter: 24 levels cover tiles of up to 2^26
+/* Partial sums of the binary counter: 27 levels cover tiles of fewer than 2^27
  * points. */
-constexpr int kLevels = 24;
-
-__device__ double pairwiseFinish(const double *part, uint64_t n)
-{
-  double s = 0;
-  for (int i = 0; i < kLevels; i++)
-    if ((n >> i) & 1)
-      s += part[i];
-  return s;
-}
+constexpr int kLevels = 27;
 
 /* 3x3 Gauss-Jordan with the reference's ratio pivoting (matrix.cpp:262-422). */
 __device__ double pw3(double a, double b, double c)
@@ -592,6 +569,16 @@ __device__ void rowOp3(double m[3][3], double b[3], int row0, int row1, int piv)
   }
 }
 
+/* A double cut to FP32 (relative error below 1.2e-7) without the conversion, an
+ * FP64 instruction; 0 below and infinity above the range. */
+__device__ __forceinline__ float wb_floatOf(double v)
+{
+  const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+  const int e = (int)((hi >> 20) & 0x7ff) - 896;
+  const uint32_t m = e <= 0 ? 0u : (e >= 255 ? 0x7f800000u : ((uint32_t)e << 23) | (((hi << 3) | (lo >> 29)) & 0x7fffffu));
+  return __uint_as_float((hi & 0x80000000u) | m);
+}
+
 /* The histogram sector of a bottom point (scan.cpp:93-101): 0 inside the
  * inner circle hypot(x, y) < rin, else 1 + (rint(atan2(y, x) * 3 / pi) mod 6).
  * FP32 decides wherever it is at least 1e-5 (relative) away from the circle
@@ -599,7 +586,7 @@ __device__ void rowOp3(double m[3][3], double b[3], int row0, int row1, int piv)
  * evaluated in FP64 exactly as the reference writes it. */
 __device__ __forceinline__ int sectorOf(double x, double y, double rin)
 {
-  const float xf = (float)x, yf = (float)y, rf = (float)rin;
+  const float xf = wb_floatOf(x), yf = wb_floatOf(y), rf = wb_floatOf(rin);
   const float r2 = xf * xf + yf * yf, rin2 = rf * rf;
   bool inner;
   if (r2 < rin2 * (1 - 1e-5f))
@@ -628,7 +615,15 @@ __device__ __forceinline__ int sectorOf(double x, double y, double rin)
  * per tile (lanes over points), everything done once per tile (centre, the
  * reference's 3x3 Gauss-Jordan, the slope clamp, density and height) one
  * thread per tile.  A tile's intermediate values live in one ScanWork slot;
- * its centre comes from the frame the gather's bound pass stored. */
+ * its centre comes from the frame the gather's bound pass stored.
+ *
+ * An SM takes an FP64 instruction of a warp every 16 cycles, so their number is
+ * the time.  Sums: 16 a row of 32 points and one per binary digit of the count
+ * (22 a row and up to 16 a tile when the eights and the last points were merged
+ * one after another by eight lanes).  Shape: 6 a row and 2 a tile (9 a row and
+ * some 48 a tile with heights compared in FP64 and a division for the inner
+ * circle).  3M points on 117,649 tiles: sums 172 us (266), shape 126 us (298);
+ * 50M points: the stage takes 4.3 ms (6.5). */
 union ScanWork
 {
   double sums[kQ];   // scanSums -> scanSolve: the eight normal-equation sums
@@ -643,12 +638,12 @@ union ScanWork
 /* Pass 1: the eight sums of the normal equations that linearLeastSquares
  * forms from the tile's points (scan.cpp:60-68, matrix.cpp:194, 211) in the
  * reference's pairwise order (pairwisesum's binary counter over the points in
- * store order). */
+ * store order): the counter's lower five levels are a fixed tree over a row of
+ * 32 points, formed by all lanes, the others are merged row by row. */
 __global__ void __launch_bounds__(32 * kScanWarps) scanSums(ScanArgs s, const TileFrame *__restrict__ frames,
                                                              ScanWork *__restrict__ work)
 {
   __shared__ double part[kScanWarps][kQ][kLevels];
-  __shared__ double tail[kScanWarps][kQ][8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const TileArgs &a = s.t;
   const uint64_t k = (uint64_t)blockIdx.x * kScanWarps + w;
@@ -658,14 +653,17 @@ __global__ void __launch_bounds__(32 * kScanWarps) scanSums(ScanArgs s, const Ti
   if (M == 0)
     return;
   const double cx = frames[k].cx, cy = frames[k].cy;
-  const uint64_t G = M / 8;   // complete groups of eight
+  const bool l0 = lane & 1, l1 = (lane >> 1) & 1, l2 = (lane >> 2) & 1;
+  const int uq = 4 * l0 + 2 * l1 + l2;
+  uint32_t jNext = (uint32_t)lane < M ? s.tilePts[b0 + lane] : 0;
   for (uint32_t c0 = 0; c0 < M; c0 += 32)
   {
-    uint32_t i = c0 + lane;
+    const uint32_t i = c0 + lane, j = jNext;
+    if (i + 32 < M)
+      jNext = s.tilePts[b0 + i + 32];
     double q[kQ];
     if (i < M)
     {
-      uint32_t j = s.tilePts[b0 + i];
       double x = a.xyzd[j] - cx, y = a.xyzd[a.nd + j] - cy, z = a.xyzd[2 * a.nd + j] - 0.0;
       q[0] = x * x;
       q[1] = y * x;
@@ -679,13 +677,10 @@ __global__ void __launch_bounds__(32 * kScanWarps) scanSums(ScanArgs s, const Ti
     else
       for (int u = 0; u < kQ; u++)
         q[u] = 0;
-    uint64_t grp = i / 8;
-    // fixed tree inside each group of eight, ((a0+a1)+(a2+a3))+((a4+a5)+(a6+a7)),
-    // for the eight quantities of the chunk's four groups: 224 additions in
-    // seven FP64 instructions.  At each level a lane and its partner split
-    // the quantities they both hold, so every lane's addition is a useful
-    // one (addition commutes exactly; only the grouping is fixed).
-    const bool l0 = lane & 1, l1 = (lane >> 1) & 1, l2 = (lane >> 2) & 1;
+    // the row's fixed tree of additions for the eight quantities.  Over the
+    // first three levels a lane and its partner split the quantities they both
+    // hold, so every lane's addition is a useful one (addition commutes
+    // exactly; only the grouping is fixed).
     double s1[4], s2[2], g;
 #pragma unroll
     for (int r = 0; r < 4; r++)   // pairs: quantity 4*l0 + r
@@ -699,31 +694,47 @@ __global__ void __launch_bounds__(32 * kScanWarps) scanSums(ScanArgs s, const Ti
       const double give = l1 ? s1[t] : s1[2 + t];
       s2[t] = (l1 ? s1[2 + t] : s1[t]) + __shfl_xor_sync(0xffffffffu, give, 2);
     }
-    {                             // groups: quantity 4*l0 + 2*l1 + l2
+    {                             // eights: quantity uq
       const double give = l2 ? s2[0] : s2[1];
       g = (l2 ? s2[1] : s2[0]) + __shfl_xor_sync(0xffffffffu, give, 4);
     }
-    // lanes 0-7 merge their quantity for the up-to-4 complete groups of the
-    // chunk, in group order (lane l + 8 gq holds group gq of the same quantity)
-    const int uq = 4 * l0 + 2 * l1 + l2;
-    for (int gq = 0; gq < 4; gq++)
+    const double h = g + __shfl_xor_sync(0xffffffffu, g, 8);   // sixteens
+    const uint32_t m = M - c0;
+    if (m >= 32)
     {
-      const uint64_t gi = (uint64_t)c0 / 8 + gq;
-      const double gv = __shfl_sync(0xffffffffu, g, (lane & 7) + 8 * gq);
-      if (gi < G && lane < 8)
-        counterMergeGroup(part[w][uq], gi * 8, gv);
+      const double row = h + __shfl_xor_sync(0xffffffffu, h, 16);
+      if (lane < 8)
+        counterMergeRow(part[w][uq], c0, row);
     }
-    // stash the trailing incomplete group's values
-    if (i < M && grp == G)
-      for (int u = 0; u < kQ; u++)
-        tail[w][u][i - G * 8] = q[u];
-    __syncwarp();
+    else
+    {
+      // the last points: the counter's lower levels hold the blocks of sixteen,
+      // eight, four, two and one of m's binary digits, which lie in that order
+      if ((m & 16) && lane < 8)
+        part[w][uq][4] = h;
+      if ((m & 8) && lane >> 3 == (int)(m >> 4) * 2)
+        part[w][uq][3] = g;
+      if ((m & 4) && lane >> 2 == (int)(m >> 3) * 2)
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+          part[w][4 * l0 + 2 * l1 + t][2] = s2[t];
+      if ((m & 2) && lane >> 1 == (int)(m >> 2) * 2)
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          part[w][4 * l0 + r][1] = s1[r];
+      if ((m & 1) && lane == (int)(m >> 1) * 2)
+#pragma unroll
+        for (int u = 0; u < kQ; u++)
+          part[w][u][0] = q[u];
+    }
   }
+  __syncwarp();
   if (lane < kQ)
   {
-    for (uint64_t i = G * 8; i < M; i++)
-      counterMergeOne(part[w][lane], i, tail[w][lane][i - G * 8]);
-    work[k].sums[lane] = pairwiseFinish(part[w][lane], M);
+    double sum = 0;
+    for (uint32_t left = M; left; left &= left - 1)
+      sum += part[w][lane][__ffs(left) - 1];
+    work[k].sums[lane] = sum;
   }
 }
 
@@ -770,18 +781,48 @@ __global__ void scanSolve(uint64_t T, const uint32_t *__restrict__ tileN, ScanWo
   }
 }
 
+/* Doubles as signed integers in the same order, -0 as +0, and back: a
+ * comparison of these costs no FP64 instruction.  NaN is above everything. */
+__device__ __forceinline__ long long orderOf(double v)
+{
+  long long b = __double_as_longlong(v);
+  if ((b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll)
+    return 0x7fffffffffffffffll;
+  if (b == (long long)0x8000000000000000ull)
+    b = 0;
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double fromOrder(long long k)
+{
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+
+/* The least of the lanes' 64-bit integers. */
+__device__ __forceinline__ long long warpMin(long long k)
+{
+  const int hi = __reduce_min_sync(0xffffffffu, (int)(k >> 32));
+  const uint32_t lo = __reduce_min_sync(0xffffffffu, (int)(k >> 32) == hi ? (uint32_t)k : 0xffffffffu);
+  return ((long long)hi << 32) | lo;
+}
+
 /* Passes 2-4 of scanCylinder (scan.cpp:74-102): untilt by the clamped
  * slope, bottom (first minimum), bottom2 (minimum before it), top and the
- * sector histogram of the bottom points.  Each lane keeps its own minimum (with its first index), maximum
- * and bottom2 over its points and the warp combines them once per tile:
- * the first minimum is the least (height, index) pair whatever the order,
- * and fmin / fmax give the same value in any order (they order -0 below +0). */
+ * sector histogram of the bottom points.  Heights are compared as integers
+ * (the conversions, comparisons and minima in FP64 were three quarters of the
+ * FP64 instructions, which bound the pass).  Each lane keeps its own minimum
+ * (with its first index), maximum and bottom2 over its points and the warp
+ * combines them once per tile: the first minimum is the least (height, index)
+ * pair whatever the order.  The sign of a zero height is lost; it tells in none
+ * of the results. */
 __global__ void __launch_bounds__(32 * kScanWarps) scanShape(ScanArgs s, const TileFrame *__restrict__ frames,
                                                               ScanWork *__restrict__ work)
 {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr long long kInf = 0x7ff0000000000000ll;   // orderOf(infinity)
   // tile-local coordinates and untilted heights of tiles up to kScanCache
   // points, computed once
-  __shared__ double cxy[kScanWarps][4][kScanCache];
+  __shared__ double cxy[kScanWarps][2][kScanCache];
+  __shared__ long long cz[kScanWarps][kScanCache];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const TileArgs &a = s.t;
   const uint64_t k = (uint64_t)blockIdx.x * kScanWarps + w;
@@ -792,83 +833,68 @@ __global__ void __launch_bounds__(32 * kScanWarps) scanShape(ScanArgs s, const T
     return;
   const double cx = frames[k].cx, cy = frames[k].cy;
   const bool cached = M <= kScanCache;
-  if (cached)
-  {
-    for (uint32_t i = lane; i < M; i += 32)
-    {
-      uint32_t j = s.tilePts[b0 + i];
-      cxy[w][0][i] = a.xyzd[j] - cx;
-      cxy[w][1][i] = a.xyzd[a.nd + j] - cy;
-      cxy[w][2][i] = a.xyzd[2 * a.nd + j] - 0.0;
-    }
-    __syncwarp();
-  }
-  // coordinates of tile point i: from the cache, or decoded again
-  auto coords = [&](uint32_t i, double &x, double &y, double &z) {
+  const double sx = work[k].s.sx, sy = work[k].s.sy;
+  // coordinates and untilted height of the point at store position j
+  auto decode = [&](uint32_t j, double &x, double &y) -> long long {
+    x = __ldg(a.xyzd + j) - cx;
+    y = __ldg(a.xyzd + a.nd + j) - cy;
+    const double z = __ldg(a.xyzd + 2 * a.nd + j) - 0.0;
+    return orderOf(z - (sy * y + sx * x));
+  };
+  // the same of tile point i, once the first pass has stored it
+  auto coords = [&](uint32_t i, double &x, double &y) {
     if (cached)
     {
       x = cxy[w][0][i];
       y = cxy[w][1][i];
-      z = cxy[w][2][i];
     }
     else
-    {
-      uint32_t j = s.tilePts[b0 + i];
-      x = a.xyzd[j] - cx;
-      y = a.xyzd[a.nd + j] - cy;
-      z = a.xyzd[2 * a.nd + j] - 0.0;
-    }
+      decode(s.tilePts[b0 + i], x, y);
   };
-  const double sx = work[k].s.sx, sy = work[k].s.sy;
-  // untilted height of tile point i (cached tiles: from the cache once pass 2 stored it)
-  auto untilted = [&](uint32_t i) -> double {
+  auto untilted = [&](uint32_t i) -> long long {
     if (cached)
-      return cxy[w][3][i];
-    double x, y, z;
-    coords(i, x, y, z);
-    return z - (sy * y + sx * x);
+      return cz[w][i];
+    double x, y;
+    return decode(s.tilePts[b0 + i], x, y);
   };
   // untilt: bottom (first minimum), top
-  double mv = INFINITY, top = -INFINITY;
+  long long mv = kInf, mt = ~kInf;   // ~kInf: orderOf(-infinity)
   uint32_t mi = 0xffffffffu;
+  uint32_t jNext = (uint32_t)lane < M ? s.tilePts[b0 + lane] : 0;
   for (uint32_t i = lane; i < M; i += 32)
   {
-    double x, y, z;
-    coords(i, x, y, z);
-    const double uz = z - (sy * y + sx * x);
+    const uint32_t j = jNext;
+    if (i + 32 < M)
+      jNext = s.tilePts[b0 + i + 32];
+    double x, y;
+    const long long uz = decode(j, x, y);
     if (cached)
-      cxy[w][3][i] = uz;
+    {
+      cxy[w][0][i] = x;
+      cxy[w][1][i] = y;
+      cz[w][i] = uz;
+    }
     if (uz < mv)
     {
       mv = uz;
       mi = i;
     }
-    top = fmax(top, uz);
+    if (uz > mt && uz <= kInf)
+      mt = uz;
   }
-  for (int o = 16; o; o >>= 1)
-  {
-    const double ov = __shfl_xor_sync(0xffffffffu, mv, o);
-    const uint32_t oi = __shfl_xor_sync(0xffffffffu, mi, o);
-    if (ov < mv || (ov == mv && oi < mi))
-    {
-      mv = ov;
-      mi = oi;
-    }
-    top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
-  }
-  const double bottom = mv < INFINITY ? mv : INFINITY;
-  const uint32_t argmin = mv < INFINITY ? mi : 0xffffffffu;
+  const long long bottom = warpMin(mv), top = ~warpMin(~mt);
+  const uint32_t argmin = __reduce_min_sync(kAll, mv == bottom ? mi : 0xffffffffu);
   __syncwarp();
   // bottom2: the lowest untilted height before the first minimum
-  double bottom2 = INFINITY;
+  long long bottom2 = kInf;
   for (uint32_t i = lane; i < M && i < argmin; i += 32)
-    bottom2 = fmin(bottom2, untilted(i));
-  for (int o = 16; o; o >>= 1)
-    bottom2 = fmin(bottom2, __shfl_xor_sync(0xffffffffu, bottom2, o));
-  if (isinf(bottom2))
+    bottom2 = min(bottom2, untilted(i));
+  bottom2 = warpMin(bottom2);
+  if (bottom2 == kInf || bottom2 == ~kInf)
     bottom2 = bottom;
   // sector histogram of the points within 2 rad of bottom2
-  const double zcut = bottom2 + 2 * a.rad, rin = a.rad / 2.6457513110645905905016;
+  const double zlim = fromOrder(bottom2) + 2 * a.rad;
+  const long long zcut = isnan(zlim) ? (long long)0x8000000000000000ull : orderOf(zlim);
   uint32_t nBottom = 0;
   int histo[7] = {0, 0, 0, 0, 0, 0, 0};
   for (uint32_t c0 = 0; c0 < M; c0 += 32)
@@ -877,19 +903,19 @@ __global__ void __launch_bounds__(32 * kScanWarps) scanShape(ScanArgs s, const T
     int sector = -1;
     if (i < M && untilted(i) < zcut)
     {
-      double x, y, z;
-      coords(i, x, y, z);
-      sector = sectorOf(x, y, rin);
+      double x, y;
+      coords(i, x, y);
+      sector = sectorOf(x, y, s.rin);
     }
     for (int sct = 0; sct < 7; sct++)
-      histo[sct] += __popc(__ballot_sync(0xffffffffu, sector == sct));
-    nBottom += __popc(__ballot_sync(0xffffffffu, sector >= 0));
+      histo[sct] += __popc(__ballot_sync(kAll, sector == sct));
+    nBottom += __popc(__ballot_sync(kAll, sector >= 0));
   }
   if (lane == 0)
   {
     ScanWork &o = work[k];
-    o.s.top = top;
-    o.s.bottom = bottom;
+    o.s.top = fromOrder(top);
+    o.s.bottom = fromOrder(bottom);
     for (int i = 0; i < 7; i++)
       o.s.histo[i] = (uint32_t)histo[i];
     o.s.nBottom = nBottom;
@@ -1195,7 +1221,7 @@ __global__ void __launch_bounds__(32 * kScanWarps) scan32Shape(ScanArgs s, const
     bottom2 = fminf(bottom2, __shfl_xor_sync(0xffffffffu, bottom2, o));
   if (isinf(bottom2))
     bottom2 = bottom;
-  const float lim = __fadd_rn(bottom2, (float)(2 * a.rad)), inner = (float)(a.rad / 2.6457513110645905905016);
+  const float lim = __fadd_rn(bottom2, (float)(2 * a.rad)), inner = (float)s.rin;
   uint32_t nBottom = 0;
   int histo[7] = {0, 0, 0, 0, 0, 0, 0};
   for (uint32_t c0 = 0; c0 < M; c0 += 32)
@@ -1576,6 +1602,7 @@ int wb_scan_impl(wb_ctx *c, const wb_params *p)
   s.tileN = tileN;
   s.tilePts = (const uint32_t *)c->tilePts.p;
   s.minH = p->min_hyp_size;
+  s.rin = a.rad / 2.6457513110645905905016;
   TileRes *res = (TileRes *)c->tileRes.p;
   // one work slot per tile (64 B, 80 B in the precision mode); the centres
   // come from the tile frames
@@ -1658,6 +1685,7 @@ int wb_tile_residuals(wb_ctx *c, const double *abc_ref, double *max_diff, double
   s.tileN = (const uint32_t *)c->tileN.p;
   s.tilePts = (const uint32_t *)c->tilePts.p;
   s.minH = c->params.min_hyp_size;
+  s.rin = 0;
   double *md = (double *)out.b.p, *mr = md + T;
   { residualKernel<<<(unsigned)std::min<uint64_t>((T * 32 + 255) / 256, (uint64_t)c->sm_count * 32), 256, 0,
                      c->stream>>>(s, (const TileRes *)c->tileRes.p, (const double *)ref.b.p, md, mr); ++c->launches; }
