@@ -21,6 +21,7 @@
 #include <cmath>
 #include "wb_internal.h"
 #include "wb_device.cuh"
+#include "wb_warpsort.cuh"
 
 namespace
 {
@@ -261,9 +262,9 @@ __device__ __forceinline__ void writeColumn(uint64_t c, uint32_t b, uint32_t e, 
   }
 }
 
-/* Sorts and fills the columns, one warp each: up to 64 points in registers, two
- * a lane, up to kColumnMax in shared memory; larger columns are listed for
- * bigColumnKernel.  Replaces the radix sort of all points by (column, height)
+/* Sorts and fills the columns, one warp each: up to 256 points in registers, up
+ * to kColumnMax in shared memory (8M points: 155 us; 196 with those from 65 points
+ * on in shared memory); larger columns are listed for bigColumnKernel.  Replaces the radix sort of all points by (column, height)
  * where columns are of ordinary size: five passes over 12-byte pairs. */
 constexpr int kColumnWarps = 4, kColumnMax = 512, kBigColumnMax = 4096;
 __global__ void __launch_bounds__(32 * kColumnWarps) columnKernel(uint64_t ncell, const uint32_t *__restrict__ start,
@@ -291,46 +292,14 @@ __global__ void __launch_bounds__(32 * kColumnWarps) columnKernel(uint64_t ncell
     return;
   }
   if (n <= 64)
-  {
-    // bitonic over 64 keys, element lane + 32 r in register r
-    uint64_t v[2];
-    v[0] = (uint32_t)lane < n ? slots[b + lane] : ~0ull;
-    v[1] = (uint32_t)lane + 32 < n ? slots[b + 32 + lane] : ~0ull;
-    auto exchange = [&](uint64_t &x, int j, bool up) {
-      const uint64_t y = __shfl_xor_sync(0xffffffffu, x, j);
-      const bool low = !(lane & j);
-      x = ((x < y) == (low == up)) ? x : y;
-    };
-    if (n > 1)
-    {
-#pragma unroll
-      for (int size = 2; size <= 32; size <<= 1)
-#pragma unroll
-        for (int j = size >> 1; j > 0; j >>= 1)
-        {
-          exchange(v[0], j, size == 32 || !(lane & size));
-          exchange(v[1], j, size == 32 ? false : !(lane & size));
-        }
-      if (n > 32)
-      {
-        const uint64_t lo = v[0] < v[1] ? v[0] : v[1], hi = v[0] < v[1] ? v[1] : v[0];
-        v[0] = lo;
-        v[1] = hi;
-#pragma unroll
-        for (int j = 16; j > 0; j >>= 1)
-        {
-          exchange(v[0], j, true);
-          exchange(v[1], j, true);
-        }
-      }
-    }
-    k[lane] = v[0];
-    k[lane + 32] = v[1];
-    __syncwarp();
-  }
+    wb_warp_sort_to<2>(slots + b, k, n, lane);
+  else if (n <= 128)
+    wb_warp_sort_to<4>(slots + b, k, n, lane);
+  else if (n <= 256)
+    wb_warp_sort_to<8>(slots + b, k, n, lane);
   else
   {
-    int P = 128;
+    int P = 512;
     while (P < (int)n)
       P <<= 1;
     for (int q = lane; q < P; q += 32)

@@ -1,4 +1,4 @@
-/* A bitonic sort of 32 * E unsigned integers by one warp, in registers.
+/* A bitonic sort of 32 * E unsigned integers (32 or 64 bits) by one warp, in registers.
  *
  * Lane l holds the elements l * E to l * E + E - 1.  The network's first step
  * of each phase compares element i with its mirror image i ^ (k - 1), so every
@@ -13,8 +13,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
-template <int E>
-__device__ __forceinline__ void wb_warp_sort(uint32_t (&v)[E], int lane)
+template <int E, class T>
+__device__ __forceinline__ void wb_warp_sort(T (&v)[E], int lane)
 {
   constexpr unsigned kAll = 0xffffffffu;
 #pragma unroll
@@ -26,7 +26,7 @@ __device__ __forceinline__ void wb_warp_sort(uint32_t (&v)[E], int lane)
       for (int e = 0; e < E; e++)
         if ((e ^ (k - 1)) > e)
         {
-          const uint32_t x = v[e], y = v[e ^ (k - 1)];
+          const T x = v[e], y = v[e ^ (k - 1)];
           v[e] = min(x, y);
           v[e ^ (k - 1)] = max(x, y);
         }
@@ -37,10 +37,10 @@ __device__ __forceinline__ void wb_warp_sort(uint32_t (&v)[E], int lane)
 #pragma unroll
       for (int e = 0; e < (E + 1) / 2; e++)
       {
-        const uint32_t x = __shfl_xor_sync(kAll, v[E - 1 - e], k / E - 1);
+        const T x = __shfl_xor_sync(kAll, v[E - 1 - e], k / E - 1);
         if (E > 1)
         {
-          const uint32_t y = __shfl_xor_sync(kAll, v[e], k / E - 1);
+          const T y = __shfl_xor_sync(kAll, v[e], k / E - 1);
           v[E - 1 - e] = lower ? min(v[E - 1 - e], y) : max(v[E - 1 - e], y);
         }
         v[e] = lower ? min(v[e], x) : max(v[e], x);
@@ -55,7 +55,7 @@ __device__ __forceinline__ void wb_warp_sort(uint32_t (&v)[E], int lane)
 #pragma unroll
         for (int e = 0; e < E; e++)
         {
-          const uint32_t x = __shfl_xor_sync(kAll, v[e], j / E);
+          const T x = __shfl_xor_sync(kAll, v[e], j / E);
           v[e] = lower ? min(v[e], x) : max(v[e], x);
         }
       }
@@ -65,7 +65,7 @@ __device__ __forceinline__ void wb_warp_sort(uint32_t (&v)[E], int lane)
         for (int e = 0; e < E; e++)
           if ((e ^ j) > e)
           {
-            const uint32_t x = v[e], y = v[e ^ j];
+            const T x = v[e], y = v[e ^ j];
             v[e] = min(x, y);
             v[e ^ j] = max(x, y);
           }
@@ -74,31 +74,30 @@ __device__ __forceinline__ void wb_warp_sort(uint32_t (&v)[E], int lane)
   }
 }
 
-/* Sorts b[0, n) in shared memory (n <= 32 * E) through registers; up to three
- * entries after them are written too. */
-template <int E>
-__device__ __forceinline__ void wb_warp_sort_shared(uint32_t *b, uint32_t n, int lane)
+/* Sorts n <= 32 * E values through registers, from src to dst (the same array or
+ * another, 16-byte aligned); up to three entries after them are written too. */
+template <int E, class T>
+__device__ __forceinline__ void wb_warp_sort_to(const T *src, T *dst, uint32_t n, int lane)
 {
-  uint32_t v[E];
+  T v[E];
 #pragma unroll
   for (int e = 0; e < E; e++)
-    v[e] = e * 32 + lane < (int)n ? b[e * 32 + lane] : 0xffffffffu;
+    v[e] = e * 32 + lane < (int)n ? src[e * 32 + lane] : ~(T)0;
   __syncwarp();
   wb_warp_sort<E>(v, lane);
-  // b is 16-byte aligned
-  if constexpr (E % 4 == 0)
+  if constexpr (sizeof(T) == 4 && E % 4 == 0)
   {
 #pragma unroll
     for (int e = 0; e < E; e += 4)
       if (lane * E + e < (int)n)
-        ((uint4 *)b)[(lane * E + e) / 4] = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        ((uint4 *)dst)[(lane * E + e) / 4] = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
   }
   else
   {
 #pragma unroll
     for (int e = 0; e < E; e++)
       if (lane * E + e < (int)n)
-        b[lane * E + e] = v[e];
+        dst[lane * E + e] = v[e];
   }
   __syncwarp();
 }
@@ -107,16 +106,16 @@ __device__ __forceinline__ void wb_warp_sort_shared(uint32_t *b, uint32_t n, int
 __device__ __forceinline__ void wb_warp_sort_1024(uint32_t *b, uint32_t n, int lane)
 {
   if (n <= 32)
-    wb_warp_sort_shared<1>(b, n, lane);
+    wb_warp_sort_to<1>(b, b, n, lane);
   else if (n <= 64)
-    wb_warp_sort_shared<2>(b, n, lane);
+    wb_warp_sort_to<2>(b, b, n, lane);
   else if (n <= 128)
-    wb_warp_sort_shared<4>(b, n, lane);
+    wb_warp_sort_to<4>(b, b, n, lane);
   else if (n <= 256)
-    wb_warp_sort_shared<8>(b, n, lane);
+    wb_warp_sort_to<8>(b, b, n, lane);
   else if (n <= 512)
-    wb_warp_sort_shared<16>(b, n, lane);
+    wb_warp_sort_to<16>(b, b, n, lane);
   else
-    wb_warp_sort_shared<32>(b, n, lane);
+    wb_warp_sort_to<32>(b, b, n, lane);
 }
 #endif
