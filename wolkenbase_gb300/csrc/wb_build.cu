@@ -304,13 +304,13 @@ struct CompactScan
   const uint32_t *idx;
   uint64_t *dkey;
   uint32_t *didx;
-  __device__ uint32_t value(uint64_t i) const { return surv[i]; }
+  __device__ uint32_t value(uint64_t i, bool ok) const { return ok ? __ldg(surv + i) : 0; }
   __device__ void put(uint64_t i, uint32_t before, uint32_t v) const
   {
     if (v)
     {
-      dkey[before] = keys[i];
-      didx[before] = idx[i];
+      dkey[before] = __ldg(keys + i);   // (read past the stores of the items before)
+      didx[before] = __ldg(idx + i);
     }
   }
 };
@@ -403,17 +403,18 @@ struct LeafScan
     int d = 0;
     if (nw > 0)
     {
-      const uint64_t a = i >= (uint64_t)(kWindow - 1) ? i - (kWindow - 1) : 0;
-      const uint64_t b = i < nw - 1 ? i : nw - 1;
+      const uint32_t at = (uint32_t)i, last = (uint32_t)nw - 1;
+      const uint32_t a = at >= (uint32_t)(kWindow - 1) ? at - (kWindow - 1) : 0;
+      const uint32_t b = min(at, last);
       if (a <= b)
       {
-        const uint64_t sa = a / kWindow, sb = b / kWindow;
+        const uint32_t sa = a / kWindow, sb = b / kWindow;
         if (sa != sb)
-          d = max((int)suf[a], (int)pre[b]);
+          d = max((int)__ldg(suf + a), (int)__ldg(pre + b));
         else if (a == sa * kWindow)
-          d = pre[b];
+          d = __ldg(pre + b);
         else
-          d = suf[a];
+          d = __ldg(suf + a);
       }
     }
     if (d >= WB_LEVELS)
@@ -423,12 +424,20 @@ struct LeafScan
     }
     return d + 1;
   }
-  __device__ uint32_t value(uint64_t i) const
+  /* Of a warp's 32 consecutive points, together: each has its neighbour's level
+   * and key from the lane before. */
+  __device__ uint32_t value(uint64_t i, bool ok) const
   {
-    if (i == 0)
-      return 1;
-    const int l = level(i);
-    return level(i - 1) != l || prefixAt(dkey[i - 1], l) != prefixAt(dkey[i], l);
+    const int l = ok ? level(i) : 0;
+    const uint64_t key = ok ? __ldg(dkey + i) : 0;
+    int lb = __shfl_up_sync(0xffffffffu, l, 1);
+    uint64_t kb = __shfl_up_sync(0xffffffffu, key, 1);
+    if ((threadIdx.x & 31) == 0 && ok && i)
+    {
+      lb = level(i - 1);
+      kb = __ldg(dkey + i - 1);
+    }
+    return ok && (i == 0 || lb != l || prefixAt(kb, l) != prefixAt(key, l));
   }
   __device__ void put(uint64_t i, uint32_t before, uint32_t v) const
   {

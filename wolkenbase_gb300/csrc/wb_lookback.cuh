@@ -182,8 +182,9 @@ __device__ __forceinline__ uint32_t blockExclusive256(uint32_t v, uint32_t *warp
   return before + inc - v;
 }
 
-/* One-pass scan of 256-thread tiles of ITEMS items a thread: flag(i) is item i's
- * value, put(i, before, value) receives the sum before it.  The last tile
+/* One-pass scan of 256-thread tiles of ITEMS items a thread: value(i, i < n) is
+ * item i's value (0 past the end), asked of a warp's 32 consecutive items
+ * together; put(i, before, value) receives the sum before it.  The last tile
  * writes the total.  counter and status (one word per tile) are zero on
  * entry. */
 constexpr int kScanItems = 16, kScanTile = 256 * kScanItems;
@@ -211,7 +212,7 @@ __device__ __forceinline__ void lookbackScan(uint64_t n, F &f, unsigned *counter
   for (int k = 0; k < ITEMS; k++)
   {
     const uint64_t i = wbase + 32 * k + lane;
-    v[k] = i < n ? f.value(i) : 0;
+    v[k] = f.value(i, i < n);
   }
 #pragma unroll
   for (int k = 0; k < ITEMS; k++)

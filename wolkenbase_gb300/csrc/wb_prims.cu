@@ -22,7 +22,7 @@ struct PlainScan
 {
   const uint32_t *in;
   uint32_t *out;
-  __device__ uint32_t value(uint64_t i) const { return in[i]; }
+  __device__ uint32_t value(uint64_t i, bool ok) const { return ok ? in[i] : 0; }
   __device__ void put(uint64_t i, uint32_t before, uint32_t) const { out[i] = before; }
 };
 

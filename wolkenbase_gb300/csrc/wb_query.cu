@@ -118,7 +118,7 @@ struct MeetScan
 {
   QArgs a;
   uint32_t *list;
-  __device__ uint32_t value(uint64_t l) const { return leafMeets(a, l); }
+  __device__ uint32_t value(uint64_t l, bool ok) const { return ok && leafMeets(a, l); }
   __device__ void put(uint64_t l, uint32_t before, uint32_t v) const
   {
     if (v)
