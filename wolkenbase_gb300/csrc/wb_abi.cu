@@ -14,6 +14,23 @@
 
 static thread_local std::string gOpenError;
 
+/* Centre and side of every leaf's cube (34,095 leaves: 0.3 ms when the host
+ * walked the keys). */
+__global__ void cubeKernel(uint64_t L, const uint64_t *__restrict__ key, const uint8_t *__restrict__ lev, double x0,
+                           double y0, double z0, double rootSide, double *__restrict__ cs)
+{
+  const uint64_t l = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= L)
+    return;
+  const double lo[3] = {x0, y0, z0};
+  double x, y, z, side;
+  wb_leaf_cube(key[l], lev[l], lo, rootSide, x, y, z, side);
+  cs[4 * l + 0] = x;
+  cs[4 * l + 1] = y;
+  cs[4 * l + 2] = z;
+  cs[4 * l + 3] = side;
+}
+
 int wb_fail(wb_ctx *c, int code, const std::string &msg)
 {
   if (c)
@@ -364,34 +381,23 @@ int wb_octree_leaves(wb_ctx *c, double *cs, uint32_t *first, uint32_t *count)
   uint64_t L = c->n_leaves;
   if (L == 0)
     return 0;
-  std::vector<uint64_t> key(L);
-  std::vector<uint8_t> lev(L);
-  WB_CUDA(c, cudaMemcpyAsync(key.data(), c->leafKey.p, L * 8, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaMemcpyAsync(lev.data(), c->leafLevel.p, L, cudaMemcpyDefault, c->stream));
+  if (cs)
+  {
+    // laid out on the device in a buffer of the build's
+    int rc = wb_ensure(c, c->key0, L * 32);
+    if (rc)
+      return rc;
+    { cubeKernel<<<(unsigned)((L + 255) / 256), 256, 0, c->stream>>>(
+          L, (const uint64_t *)c->leafKey.p, (const uint8_t *)c->leafLevel.p, c->g.root_lo[0], c->g.root_lo[1],
+          c->g.root_lo[2], c->g.root_side, (double *)c->key0.p); ++c->launches; }
+    WB_CUDA(c, cudaGetLastError());
+    WB_CUDA(c, cudaMemcpyAsync(cs, c->key0.p, L * 32, cudaMemcpyDefault, c->stream));
+  }
   if (first)
     WB_CUDA(c, cudaMemcpyAsync(first, c->leafFirst.p, L * 4, cudaMemcpyDefault, c->stream));
   if (count)
     WB_CUDA(c, cudaMemcpyAsync(count, c->leafCount.p, L * 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (cs)
-    for (uint64_t l = 0; l < L; l++)
-    {
-      // Octree::cube: centre = parent centre +- side/4 per level, computed exactly
-      int lv = lev[l];
-      uint32_t ix = 0, iy = 0, iz = 0;
-      for (int d = 1; d <= lv; d++)
-      {
-        int oct = (int)((key[l] >> (63 - 3 * d)) & 7);
-        ix = (ix << 1) | (oct & 1);
-        iy = (iy << 1) | ((oct >> 1) & 1);
-        iz = (iz << 1) | ((oct >> 2) & 1);
-      }
-      double side = ldexp(c->g.root_side, -lv);
-      cs[4 * l + 0] = c->g.root_lo[0] + ((double)ix + 0.5) * side;
-      cs[4 * l + 1] = c->g.root_lo[1] + ((double)iy + 0.5) * side;
-      cs[4 * l + 2] = c->g.root_lo[2] + ((double)iz + 0.5) * side;
-      cs[4 * l + 3] = side;
-    }
   return 0;
 }
 
