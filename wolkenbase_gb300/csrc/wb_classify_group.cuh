@@ -414,14 +414,27 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       {
         WB_STAT(gst[10], 1);
         const int kk = max(k + __ffs(hits) - 1, 0);
-        const float ex = sm.cx[kk] - mx, ey = (sm.cy[kk] - my) * ky, zd = __fmaf_rn(mz + sm.cz[kk], kz, czp);
+        const float ex = sm.cx[kk] - mx, ey = (sm.cy[kk] - my) * ky;
+        // the arc may have shrunk since the candidate was found in it, and a lane
+        // with two arcs found all candidates inside
+        bool in = side * fminf(__fmaf_rn(ax, ey, -(ay * ex)), __fmaf_rn(ex, by, -(ey * bx))) > (two ? 0.f : arcMin);
+        if (two & !in)
+        {
+          const float2 p2 = sm.arc2a[lane], q2 = sm.arc2b[lane];
+          const float c0 = p2.x * ey - p2.y * ex, c1 = ex * q2.y - ey * q2.x;
+          in = p2.x * q2.y - p2.y * q2.x < 0.f ? (c0 > 0.f) | (c1 > 0.f) : (c0 > 0.f) & (c1 > 0.f);
+        }
+        in = in & (hits != 0) & !done;
+        hits &= hits - 1;
+        if (!__any_sync(kAll, in))
+          continue;
+        const float zd = __fmaf_rn(mz + sm.cz[kk], kz, czp);
         const float rr = __fmaf_rn(ex, ex, ey * ey);
-        bool in = (hits != 0) & !done & (rr > 0.f);
+        in = in & (rr > 0.f);
         const bool sure = zd * zd > kOut * (rr + por2 + a.gTiny);
         if (in & !sure)
           pend |= 1u << kk;
         in = in & sure;
-        hits &= hits - 1;
         const bool any = in & slow;
         if (__any_sync(kAll, any))
           addAny(any, ex, ey, rr);
@@ -429,8 +442,6 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
         if (__any_sync(kAll, in))
         {
           const float il = rsqrtf(rr), ux = ex * il, uy = ey * il;
-          // the arc may have shrunk since the candidate was found in it
-          in = in & (side * fminf(__fmaf_rn(ax, uy, -(ay * ux)), __fmaf_rn(ux, by, -(uy * bx))) > 0.f);
           if (in)
           {
             float2 l, q;
