@@ -55,3 +55,22 @@ def test_capacity(built):
         assert rc == want and n.value == full.size
         assert np.array_equal(out[:full.size], full) if rc == 0 else np.all(out == 7)
         assert np.all(out[full.size:] == 7)
+
+
+def test_heights_order_the_same_through_a_negative_scale(built):
+    # record integers order the heights of the one cloud, the heights themselves
+    # those of the other; the points are the same
+    import wolkenbase_gb300 as wb
+    from wolkenbase_gb300 import synth
+    clf, cloud = built
+    flipped = synth.Cloud(np.ascontiguousarray(cloud.xyz * np.array([1, 1, -1], np.int32)),
+                          (cloud.scale[0], cloud.scale[1], -cloud.scale[2]), cloud.offset, cloud.unit, cloud.minc,
+                          cloud.maxc)
+    assert np.array_equal(flipped.decoded(), cloud.decoded())
+    other = wb.Classifier(0)
+    other.build(flipped)
+    c = cloud.decoded()[cloud.n // 3]
+    for r in (0.3, 2.6, 40.0):
+        want = clf.points_in(1, (c[0], c[1]), r, sorted=True)
+        assert np.array_equal(other.points_in(1, (c[0], c[1]), r, sorted=True), want)
+    other.close()

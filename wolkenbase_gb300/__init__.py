@@ -76,6 +76,7 @@ class Classifier:
 
     def __init__(self, device=0, hbm_budget=0):
         self.L = _lib.load()
+        self._found = None   # where queries answer first
         self.ctx = self.L.wb_open(device, hbm_budget)
         if not self.ctx:
             raise WolkenbaseError(_lib.WB_ECUDA, self.L.wb_last_error(None).decode())
@@ -177,7 +178,9 @@ class Classifier:
         sh = self._shape(kind, v, r, s)
         n = C.c_uint64(0)
         # a neighbourhood usually fits the first buffer; a larger answer says its size
-        out = np.empty(4096, np.uint32)
+        if self._found is None:
+            self._found = np.empty(65536, np.uint32)
+        out = self._found
         rc = self.L.wb_points_in(self.ctx, C.byref(sh), int(sorted), out.ctypes.data, out.shape[0], C.byref(n))
         if rc == _lib.WB_EINVAL and n.value > out.shape[0]:
             out = np.empty(n.value, np.uint32)

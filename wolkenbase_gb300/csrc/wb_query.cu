@@ -27,6 +27,7 @@
  */
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <string>
@@ -335,10 +336,12 @@ __global__ void __launch_bounds__(1024) fewLeavesKernel(QArgs a, const uint32_t 
 }
 
 /* FILL false: cnt[i] = points of listed leaf i that pointsIn returns; true:
- * their record indices (and, with keys, heights) written from off[i] on. */
+ * their record indices (and, with keys, heights: record integers where sz gives
+ * them) written from off[i] on. */
 template <bool FILL>
 __global__ void listedKernel(QArgs a, const uint32_t *__restrict__ list, uint32_t n, uint32_t *__restrict__ cnt,
-                             const uint32_t *__restrict__ off, uint32_t *__restrict__ out, uint64_t *__restrict__ keys)
+                             const uint32_t *__restrict__ off, uint32_t *__restrict__ out, uint64_t *__restrict__ keys,
+                             const int32_t *__restrict__ sz)
 {
   const int lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -362,7 +365,7 @@ __global__ void listedKernel(QArgs a, const uint32_t *__restrict__ list, uint32_
         const uint32_t j = f + 32 * r + lane, p = at + __popc(b & ((1u << lane) - 1));
         out[p] = a.sidx[j];
         if (keys)
-          keys[p] = heightBits(a.xyzd[2 * a.nd + j]);
+          keys[p] = sz ? (uint64_t)((uint32_t)sz[j] ^ 0x80000000u) : heightBits(a.xyzd[2 * a.nd + j]);
       }
       at += __popc(b);
     }
@@ -418,14 +421,14 @@ int lookbackFailed(wb_ctx *c, const char *who)
 }
 
 /* Lists the leaves that meet the shape: *list on the device, their number at
- * *nList. */
+ * *nList; behind the list, room for two more words a leaf and one. */
 int listLeaves(wb_ctx *c, const QArgs &a, uint32_t **list, uint32_t **nList)
 {
   const uint64_t tiles = (a.L + 255) / 256;   // a leaf a thread: FP64 cube tests, spread over the SMs
   unsigned *counter;
   unsigned long long *status;
   int rc = wb_lookback_words(c, tiles, &counter, &status);
-  if (rc || (rc = wb_ensure(c, c->queryBuf, a.L * 4 + 64)))
+  if (rc || (rc = wb_ensure(c, c->queryBuf, a.L * 12 + 128)))
     return rc;
   *nList = (uint32_t *)c->queryBuf.p;
   *list = *nList + 16;
@@ -519,12 +522,9 @@ extern "C" int wb_points_in(wb_ctx *c, const wb_shape *sh, int sorted, uint32_t 
   // many leaves or points: counts, their prefix, the points, a radix sort
   const uint32_t n = ans->leaves;
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n * 32 + 255) / 256, (uint64_t)c->sm_count * 32));
-  WbScratch cnt(c), ex(c);
-  if ((rc = wb_ensure(c, cnt.b, (uint64_t)n * 4 + 64)) || (rc = wb_ensure(c, ex.b, (uint64_t)n * 4 + 64)))
-    return rc;
-  uint32_t *dTot = (uint32_t *)((uint8_t *)ex.b.p + (uint64_t)n * 4);
-  { listedKernel<false><<<grid, 256, 0, c->stream>>>(a, list, n, (uint32_t *)cnt.b.p, nullptr, nullptr, nullptr); ++c->launches; }
-  if ((rc = wb_exclusive_scan_u32(c, (const uint32_t *)cnt.b.p, (uint32_t *)ex.b.p, n, dTot)))
+  uint32_t *cnt = list + L, *ex = cnt + L, *dTot = ex + L;
+  { listedKernel<false><<<grid, 256, 0, c->stream>>>(a, list, n, cnt, nullptr, nullptr, nullptr, nullptr); ++c->launches; }
+  if ((rc = wb_exclusive_scan_u32(c, cnt, ex, n, dTot)))
     return rc;
   uint32_t total = 0;
   WB_CUDA(c, cudaMemcpyAsync(&total, dTot, 4, cudaMemcpyDefault, c->stream));
@@ -535,17 +535,28 @@ extern "C" int wb_points_in(wb_ctx *c, const wb_shape *sh, int sorted, uint32_t 
     return tooMany(total);
   if (total == 0)
     return 0;
-  WbScratch outD(c), k0(c), k1(c), v1(c);
+  // the build's sort buffers serve again (an allocation costs as much as a pass)
   const bool sort = sorted && total > 1;
-  if ((rc = wb_ensure(c, outD.b, (uint64_t)total * 4 + 64)))
+  if ((rc = wb_ensure(c, c->idx0, (uint64_t)total * 4)) || (rc = wb_ensure(c, c->idx1, (uint64_t)total * 4)) ||
+      (sort && ((rc = wb_ensure(c, c->key0, (uint64_t)total * 8)) || (rc = wb_ensure(c, c->key1, (uint64_t)total * 8)))))
     return rc;
-  if (sort && ((rc = wb_ensure(c, k0.b, (uint64_t)total * 8 + 64)) || (rc = wb_ensure(c, k1.b, (uint64_t)total * 8 + 64)) ||
-               (rc = wb_ensure(c, v1.b, (uint64_t)total * 4 + 64))))
-    return rc;
-  uint32_t *vals = (uint32_t *)outD.b.p;
-  uint64_t *keys = (uint64_t *)k0.b.p;
-  { listedKernel<true><<<grid, 256, 0, c->stream>>>(a, list, n, nullptr, (const uint32_t *)ex.b.p, vals, sort ? keys : nullptr); ++c->launches; }
-  if (sort && (rc = wb_radix_sort_pairs(c, keys, vals, (uint64_t *)k1.b.p, (uint32_t *)v1.b.p, total, 0, 64)))
+  uint32_t *vals = (uint32_t *)c->idx0.p;
+  uint64_t *keys = (uint64_t *)c->key0.p;
+  // where the decode increases with the record integer in steps FP64 resolves,
+  // that integer orders as the height does, in as many bits as the cloud's vary
+  const double step = c->g.scale[2] * c->g.unit;
+  const double mag = std::max(std::fabs((c->g.off[2] + c->g.scale[2] * c->grid.imin[2]) * c->g.unit),
+                              std::fabs((c->g.off[2] + c->g.scale[2] * c->grid.imax[2]) * c->g.unit)) +
+                     std::fabs(c->g.off[2] * c->g.unit) + step;
+  const bool ints = step > 0 && step >= 4 * std::ldexp(mag, -52);
+  int bits = 64;
+  if (ints)
+    for (bits = 0; bits < 32 && (((uint32_t)c->grid.imin[2] ^ (uint32_t)c->grid.imax[2]) >> bits);)
+      bits++;
+  { listedKernel<true><<<grid, 256, 0, c->stream>>>(a, list, n, nullptr, ex, vals, sort ? keys : nullptr,
+                                                   ints ? (const int32_t *)c->sz.p : nullptr); ++c->launches; }
+  if (sort && bits &&
+      (rc = wb_radix_sort_pairs(c, keys, vals, (uint64_t *)c->key1.p, (uint32_t *)c->idx1.p, total, 0, bits)))
     return rc;
   WB_CUDA(c, cudaGetLastError());
   WB_CUDA(c, cudaMemcpyAsync(records, vals, (size_t)total * 4, cudaMemcpyDefault, c->stream));
