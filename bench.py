@@ -701,12 +701,11 @@ def main():
                              "peak_Ginst_s": peak_inst / 1e9, "frac": ach_inst / peak_inst,
                              "ncu_issue_active": tr.get("issue_active_pct", 0) / 100,
                              "ncu_warps_active": tr.get("warps_active_pct", 0) / 100,
-                             "note": "warp instructions per point of the column-group fast pass (ncu, one launch "
+                             "note": "warp instructions per point of the point-group fast pass (ncu, one launch "
                                      "on 4M points) x points / the classify stage's time; peak = 4 issue slots "
                                      "per SM per cycle at the sampled SM clock"}
     # the octree build proper (sizeFit + put of every point); the column grid is this path's own index
-    build_ms = sum(v for k, v in stage_ms.items() if k in ("decode_key", "sort", "dedup", "leaves", "leaf_order",
-                                                         "point_map", "nodes"))
+    build_ms = sum(v for k, v in stage_ms.items() if k in ("decode_key", "sort", "dedup", "leaves", "leaf_order"))
     cpu = parity = None
     if gpu_res is not None:
         cpu, parity = oracle_baseline(cloud, os.cpu_count() or 1, args.cpu_tile_frac, args.seed + 7, gpu_res)

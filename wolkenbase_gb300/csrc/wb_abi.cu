@@ -383,15 +383,21 @@ int wb_octree_leaves(wb_ctx *c, double *cs, uint32_t *first, uint32_t *count)
     return 0;
   if (cs)
   {
-    // laid out on the device in a buffer of the build's
-    int rc = wb_ensure(c, c->key0, L * 32);
-    if (rc)
+    // laid out on the device in a sort buffer of the build's, as many at a time
+    // as it holds (nearly always all)
+    int rc;
+    if (c->key0.cap < 65536 && (rc = wb_ensure(c, c->key0, std::min<uint64_t>(L * 32, 65536))))
       return rc;
-    { cubeKernel<<<(unsigned)((L + 255) / 256), 256, 0, c->stream>>>(
-          L, (const uint64_t *)c->leafKey.p, (const uint8_t *)c->leafLevel.p, c->g.root_lo[0], c->g.root_lo[1],
-          c->g.root_lo[2], c->g.root_side, (double *)c->key0.p); ++c->launches; }
-    WB_CUDA(c, cudaGetLastError());
-    WB_CUDA(c, cudaMemcpyAsync(cs, c->key0.p, L * 32, cudaMemcpyDefault, c->stream));
+    const uint64_t most = c->key0.cap / 32;
+    for (uint64_t l = 0; l < L; l += most)
+    {
+      const uint64_t n = std::min(most, L - l);
+      { cubeKernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
+            n, (const uint64_t *)c->leafKey.p + l, (const uint8_t *)c->leafLevel.p + l, c->g.root_lo[0],
+            c->g.root_lo[1], c->g.root_lo[2], c->g.root_side, (double *)c->key0.p); ++c->launches; }
+      WB_CUDA(c, cudaGetLastError());
+      WB_CUDA(c, cudaMemcpyAsync(cs + 4 * l, c->key0.p, n * 32, cudaMemcpyDefault, c->stream));
+    }
   }
   if (first)
     WB_CUDA(c, cudaMemcpyAsync(first, c->leafFirst.p, L * 4, cudaMemcpyDefault, c->stream));

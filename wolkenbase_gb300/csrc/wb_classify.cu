@@ -143,7 +143,7 @@ struct ClsArgs
   /* ambiguous points for the exact pass */
   uint32_t *ambList;
   uint32_t *ambCount;
-  /* points a column group handed to the one-point kernel */
+  /* points a group handed to the one-point kernel */
   uint32_t *deferList;
   uint32_t *deferCount;
   const uint32_t *work;   /* exact pass: store positions to classify */
@@ -1587,7 +1587,7 @@ struct BatchHdr
   int k, chunk;
   unsigned long long next[3];   /* work counters: fast pass, deferred points, exact pass */
   uint64_t startNd[WB_BATCH_MAX + 1], startN[WB_BATCH_MAX + 1], startT[WB_BATCH_MAX + 1];
-  uint64_t startGrp[WB_BATCH_MAX + 1];   /* column groups (the column-group fast pass) */
+  uint64_t startGrp[WB_BATCH_MAX + 1];   /* groups of the fast pass */
   ClsArgs jobs[WB_BATCH_MAX];
 };
 struct BatchOut
@@ -1865,14 +1865,14 @@ namespace
 typedef void (*RingsFn)(BatchHdr *, const BatchOut *);
 
 /* Kernels of the fused classify: 0..WB_N_SHAPES-1 the fast pass of each
- * shape (one point per warp, or column groups), kDeferred the one-point pass
- * over the points column groups handed over, kExactPass the exact pass. */
+ * shape (one point per warp, or point groups), kDeferred the one-point pass
+ * over the points groups handed over, kExactPass the exact pass. */
 constexpr int kDeferred = WB_N_SHAPES, kExactPass = WB_N_SHAPES + 1, kMarginGroups = WB_N_SHAPES + 2,
               kMarginDeferred = WB_N_SHAPES + 3;
 
 RingsFn ringsFn(int idx)
 {
-  // kWbShapes 0-2: column groups (register caps of about 85, 102 and 128 a
+  // kWbShapes 0-2: point groups (register caps of about 85, 102 and 128 a
   // thread); 3-7: one point per warp (about 85, 85, 64, 64 and 85)
   switch (idx)
   {
@@ -2256,7 +2256,7 @@ int wb_autotune_jobs(WbBatch *b, const WbTuneJob *jobs, int k, cudaStream_t s, i
   };
   const int ch0 = *chunk > 0 ? *chunk : 1;
   static const double kDensity[] = {32, 48, 64, 96};
-  static const int kProbe[] = {0, 3};   // a column-group shape and a one-point shape
+  static const int kProbe[] = {0, 3};   // a group shape and a one-point shape
   float best = 1e30f;
   int bestShape = clampShape(*shape), bestChunk = ch0;
   double bestGp = *gridPoints > 0 ? *gridPoints : 64;

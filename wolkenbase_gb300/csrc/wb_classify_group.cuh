@@ -34,12 +34,12 @@
  * Bound: instruction issue (80% of the slots at 24 warps per SM, DRAM idle; 50M
  * points at 100 per square metre: 30,500 warp instructions a group, of which
  * 42% test candidates and update arcs, 20% octet boxes, 11% group boxes, 10%
- * staging, 15% listing).  The classify stage takes 51.6 ms there; 104 ms before
+ * staging, 15% listing).  The classify stage takes 50.3 ms there; 104 ms before
  * with groups of one column's points by height, 8 direction bins a lane (FP32
  * arctangents) and envelope tests only.  On the way: arcs instead of bins 85,
  * the lane's own reach per column, four candidates a step and updates by the
  * lanes that need them 58, compact groups as the index with octet boxes 54,
- * packed FP32 52 ms. */
+ * packed FP32 52, candidates held against the arcs before the update 50 ms. */
 
 constexpr float kRayPad = 1e-6f;
 /* cos(144 degrees -+ kArcBand) */

@@ -1639,24 +1639,30 @@ int wb_scan_impl(wb_ctx *c, const wb_params *p)
 }
 
 /* The last scan's tile records, or planes, in the caller's host array, laid out
- * on the device in a buffer of the build's. */
+ * on the device in a sort buffer of the build's, as many at a time as it holds
+ * (all of them, unless most tiles are empty). */
 static int readBack(wb_ctx *c, void *host, bool planes)
 {
-  const uint64_t T = c->n_tiles, bytes = T * (planes ? 3 * sizeof(double) : sizeof(wb_tile));
+  const uint64_t T = c->n_tiles, size = planes ? 3 * sizeof(double) : sizeof(wb_tile);
   int rc;
   if (!T)
     return 0;
-  if ((rc = wb_ensure(c, c->key0, bytes)))
+  if (c->key0.cap < 65536 && (rc = wb_ensure(c, c->key0, std::min<uint64_t>(T * size, 65536))))
     return rc;
-  const TileRes *res = (const TileRes *)c->tileRes.p;
-  if (planes)
-    { packPlanes<<<(unsigned)((3 * T + 255) / 256), 256, 0, c->stream>>>(T, res, (double *)c->key0.p); ++c->launches; }
-  else
-    { packTiles<<<(unsigned)((T + 255) / 256), 256, 0, c->stream>>>(T, res, (const int32_t *)c->tileEx.p,
-                                                                  (const int32_t *)c->tileEy.p, (wb_tile *)c->key0.p);
-      ++c->launches; }
-  WB_CUDA(c, cudaGetLastError());
-  WB_CUDA(c, cudaMemcpyAsync(host, c->key0.p, bytes, cudaMemcpyDefault, c->stream));
+  const uint64_t most = c->key0.cap / size;
+  for (uint64_t k = 0; k < T; k += most)
+  {
+    const uint64_t n = std::min(most, T - k);
+    const TileRes *res = (const TileRes *)c->tileRes.p + k;
+    if (planes)
+      { packPlanes<<<(unsigned)((3 * n + 255) / 256), 256, 0, c->stream>>>(n, res, (double *)c->key0.p); ++c->launches; }
+    else
+      { packTiles<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, res, (const int32_t *)c->tileEx.p + k,
+                                                                    (const int32_t *)c->tileEy.p + k, (wb_tile *)c->key0.p);
+        ++c->launches; }
+    WB_CUDA(c, cudaGetLastError());
+    WB_CUDA(c, cudaMemcpyAsync((char *)host + k * size, c->key0.p, n * size, cudaMemcpyDefault, c->stream));
+  }
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
   return 0;
 }
