@@ -87,13 +87,13 @@ __global__ void keyKernel(KeyArgs a, uint64_t *__restrict__ keys)
         const long long fr = tf - k0 * (1ll << a.shift[ax]);
         // within eps of cell boundary kb: the decoded coordinate decides (cell
         // sides are dyadic, so with decimal coordinates one point in 125 lies
-        // on a boundary and most warps hold one: seven FP64 instructions here,
+        // on a boundary and most warps hold one: six FP64 instructions here,
         // where the general search took 40 and the FP64 pipe bounded the kernel)
         const bool below = fr <= a.eps[ax], above = fr >= (1ll << a.shift[ax]) - a.eps[ax];
         if (below || above)
         {
           const long long kb = k0 + above;
-          k0 = wb_decode(q[ax], a.off[ax], a.scale[ax], a.unit) >= a.lo[ax] + (double)(int)kb * a.cell ? kb : kb - 1;
+          k0 = wb_decode(q[ax], a.off[ax], a.scale[ax], a.unit) >= a.lo[ax] + wb_double((int)kb) * a.cell ? kb : kb - 1;
         }
         k[ax] = (uint32_t)(k0 < 0 ? 0 : (k0 > kMax ? kMax : k0));
       }

@@ -99,7 +99,7 @@ __global__ void gridBoundsKernel(GridArgs g, long long *__restrict__ bounds)
  * [b[0], b[n]); a guess from the mean column width, then the thresholds. */
 __device__ __forceinline__ int columnOf(const long long *__restrict__ b, int n, long long X, float perUnit)
 {
-  int k = (int)((float)(X - b[0]) * perUnit);
+  int k = (int)((float)(uint32_t)(X - b[0]) * perUnit);   // (a 64-bit conversion is an FP64 instruction)
   k = min(max(k, 0), n - 1);
   while (k > 0 && X < b[k])
     k--;
@@ -117,13 +117,25 @@ __global__ void cellKernel(GridArgs g, const int32_t *__restrict__ sx, const int
   int mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
   // whole warps step together, for the counts' runs
   const int lane = threadIdx.x & 31;
-  for (uint64_t j0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < g.nd; j0 += (uint64_t)gridDim.x * blockDim.x)
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  int next[3] = {0, 0, 0};   // the next point, read while this one is placed
+  auto read = [&](uint64_t j) {
+    if (j < g.nd)
+    {
+      next[0] = __ldg(sx + j);
+      next[1] = __ldg(sy + j);
+      next[2] = __ldg(sz + j);
+    }
+  };
+  read((uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
+  for (uint64_t j0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < g.nd; j0 += step)
   {
     const uint64_t j = j0 + lane;
+    const int q[3] = {next[0], next[1], next[2]};
+    read(j + step);
     uint32_t cell = 0xffffffffu;
     if (j < g.nd)
     {
-      const int q[3] = {sx[j], sy[j], sz[j]};
       for (int a = 0; a < 3; a++)
       {
         mn[a] = min(mn[a], q[a]);
