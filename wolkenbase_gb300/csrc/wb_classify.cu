@@ -388,9 +388,11 @@ __device__ __forceinline__ void setupPoint(const ClsArgs &a, uint64_t j)
   a.setup[j] = s;
 }
 
-/* Classifies store position j with one warp; bminW/bmaxW are the warp's
- * 64-bin direction extremes in shared memory. */
-template <bool EXACT>
+/* Classifies store position j with one warp, or with the WARPS warps of a block;
+ * bminW/bmaxW are its 64-bin direction extremes in shared memory.  The warps of a
+ * block take the columns of a walk's step in turn; they decide on the same bins
+ * between two barriers, so all take the same way. */
+template <bool EXACT, int WARPS = 1>
 __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int lane, uint32_t *bminW,
                                               uint32_t *bmaxW)
 {
@@ -422,7 +424,11 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
     bminW[b] = 0xffffffffu;
     bmaxW[b] = 0;
   }
-  __syncwarp();
+  if (WARPS > 1)
+    __syncthreads();
+  else
+    __syncwarp();
+  const int turn = WARPS > 1 ? threadIdx.x >> 5 : 0;
   const int ci = ps.ci, cj = ps.cj, kmax = ps.kmax;
   HypExact hx;
   if (EXACT)
@@ -647,6 +653,11 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
     }
   };
   auto decide = [&]() {
+    if (WARPS > 1)
+    {
+      occLo = __ballot_sync(0xffffffffu, bminW[lane] != 0xffffffffu);
+      occHi = __ballot_sync(0xffffffffu, bminW[lane + 32] != 0xffffffffu);
+    }
 #ifdef WB_CLASSIFY_STATS
     const long long td = clock64();
 #endif
@@ -684,6 +695,20 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
         }
       }
       unsigned mask = __ballot_sync(0xffffffffu, ok);
+      if (WARPS > 1)
+      {
+        bool got = false;
+        for (int n = 0; mask; n++, mask &= mask - 1)
+        {
+          const int src = __ffs(mask) - 1;
+          const uint64_t cc = __shfl_sync(0xffffffffu, c, src);
+          if (n % WARPS == turn && arcWants(cb, src))
+            got |= column(cc);
+        }
+        if (__syncthreads_or(got))
+          decide();
+        __syncthreads();
+      }
       while (mask && !surrounded)
       {
         int src = __ffs(mask) - 1;
@@ -755,16 +780,20 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
         unsigned cm = __ballot_sync(0xffffffffu, cok);
         WB_STAT(stat[3], S * S);
         bool gotAny = false;
-        while (cm)
+        for (int n = 0; cm; n++)
         {
           int cs = __ffs(cm) - 1;
           cm &= cm - 1;
           const uint64_t cc = __shfl_sync(0xffffffffu, c, cs);
-          if (arcWants(cb, cs))
+          if ((WARPS == 1 || n % WARPS == turn) && arcWants(cb, cs))
             gotAny |= column(cc);
         }
+        if (WARPS > 1)
+          gotAny = __syncthreads_or(gotAny);
         if (gotAny)
           decide();
+        if (WARPS > 1)
+          __syncthreads();
       }
     }
   }
@@ -1623,9 +1652,8 @@ __global__ void batchSetup(const BatchHdr *__restrict__ h)
   }
 }
 
-/* MODE 0: every point of every job; 1: the points the groups deferred; 2: the
- * ambiguous points (exactly; in the precision mode again in FP32, by the bins'
- * extremes).  ARCS: by open arcs, else by bins, which form every largest gap. */
+/* MODE 0: every point of every job; 1: the points the groups deferred.  ARCS: by
+ * open arcs, else by bins, which form every largest gap. */
 template <int MODE, bool ARCS, int W, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const BatchOut *o)
 {
@@ -1634,7 +1662,7 @@ __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const Ba
   __shared__ ClsArgs sa[W];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = h->k;
-  const uint64_t *start = MODE == 2 ? o->startAmb : (MODE == 1 ? o->startDef : h->startNd);
+  const uint64_t *start = MODE == 1 ? o->startDef : h->startNd;
   const uint64_t total = start[k];
   const unsigned chunk = MODE == 0 ? (unsigned)h->chunk : 1u;
   uint64_t lo = 1, hi = 0;
@@ -1663,14 +1691,55 @@ __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const Ba
       }
       const ClsArgs &a = sa[w];
       uint64_t item = g - lo;
-      const uint64_t j = MODE == 2 ? a.ambList[item] : (MODE == 1 ? a.deferList[item] : item);
+      const uint64_t j = MODE == 1 ? a.deferList[item] : item;
       if constexpr (ARCS)
         classifyPointArcs(a, j, lane, psm[w]);
-      else if (MODE == 2 && !a.fp32Only)
-        classifyPoint<true>(a, j, lane, bmin[w], bmax[w]);
       else
         classifyPoint<false>(a, j, lane, bmin[w], bmax[w]);
     }
+  }
+}
+
+/* The ambiguous points (exactly; in the precision mode again in FP32, by the bins'
+ * extremes), a block each: they are a dozen of a cloud of millions, so the pass
+ * takes as long as the heaviest one's walk, mostly chains of FP64 directions.
+ * Eight warps that share its columns: 0.33 ms for 5M points and 0.40 for 50M (one
+ * warp a point: 0.55 and 0.95; four: 0.33 and 0.50). */
+template <int W>
+__global__ void __launch_bounds__(32 * W) batchExact(BatchHdr *h, const BatchOut *o)
+{
+  __shared__ uint32_t bmin[kBins], bmax[kBins];
+  __shared__ ClsArgs a;
+  __shared__ unsigned long long itemS;
+  const int lane = threadIdx.x & 31;
+  const int k = h->k;
+  const uint64_t *start = o->startAmb;
+  const uint64_t total = start[k];
+  uint64_t lo = 1, hi = 0;
+  for (;;)
+  {
+    __syncthreads();   // the point before is done with
+    if (threadIdx.x == 0)
+      itemS = atomicAdd(&h->next[2], 1ull);
+    __syncthreads();
+    const uint64_t g = itemS;
+    if (g >= total)
+      break;
+    if (g < lo || g >= hi)
+    {
+      const int q = batchJob(start, k, g);
+      lo = start[q];
+      hi = start[q + 1];
+      const uint32_t *src = (const uint32_t *)&h->jobs[q];
+      for (int i = threadIdx.x; i < (int)(sizeof(ClsArgs) / 4); i += 32 * W)
+        ((uint32_t *)&a)[i] = src[i];
+      __syncthreads();
+    }
+    const uint64_t j = a.ambList[g - lo];
+    if (a.fp32Only)
+      classifyPoint<false, W>(a, j, lane, bmin, bmax);
+    else
+      classifyPoint<true, W>(a, j, lane, bmin, bmax);
   }
 }
 
@@ -1884,7 +1953,7 @@ RingsFn ringsFn(int idx)
   case 6: return batchRings<0, true, 8, 4>;
   case 7: return batchRings<0, true, 2, 12>;
   case kDeferred: return batchRings<1, true, 4, 8>;
-  case kExactPass: return batchRings<2, false, 4, 6>;
+  case kExactPass: return batchExact<8>;
   case kMarginDeferred: return batchRings<1, false, 8, 3>;
   case kMarginGroups: return batchGroups<false, 8, 3>;
   default: return batchGroups<true, 4, 6>;
@@ -1893,7 +1962,7 @@ RingsFn ringsFn(int idx)
 
 int ringsWarps(int idx)
 {
-  return idx == kExactPass || idx == kDeferred ? 4 : (idx == kMarginDeferred || idx == kMarginGroups ? 8 : kWbShapes[idx].warps);
+  return idx == kDeferred ? 4 : (idx == kExactPass || idx == kMarginDeferred || idx == kMarginGroups ? 8 : kWbShapes[idx].warps);
 }
 
 /* The one-point pass that goes with a fast pass. */
