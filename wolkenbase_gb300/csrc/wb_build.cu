@@ -41,8 +41,9 @@ struct KeyArgs
   /* Fixed-point form of the level-21 cell coordinate, per axis:
      t(X) = (C + (X - x0) * R) / 2^shift, with |X - x0| <= dmax.  A point
      whose fraction lies more than eps from an integer takes floor(t); for the
-     rest the decoded coordinate is compared with that one boundary.  All of an
-     axis with fixed = 0 take the general FP64 path. */
+     rest the decoded coordinate is compared with that one boundary (eps is
+     below half of 2^shift).  All of an axis with fixed = 0 take the general
+     FP64 path. */
   int fixed[3], shift[3];
   long long x0[3], dmax[3], rfix[3], cfix[3], eps[3];
 };
@@ -587,6 +588,11 @@ static void keyFixedPoint(const WbGeom &g, double mn, double mx, int k, KeyArgs 
   // decode error: two roundings of |x| (<= |x0d| + dmax*u) and the subtraction of lo
   const double mag = fabs(x0d) + (double)dmax * u + fabs(g.root_lo[k]);
   const double errCells = (double)dmax / one + 1.0 / one + 8 * ldexp(mag, -52) / g.cell + ldexp(B, -50);
+  // eps below half a cell, so that a point can be in doubt about one boundary
+  // only, the one keyKernel compares it with: a cloud whose coordinates round
+  // to more than that (a root cube of centimetres at 1e9) is searched in FP64
+  if (!(16 * errCells < 0.5 - 32 / one))
+    return;
   a.fixed[k] = 1;
   a.shift[k] = shift;
   a.x0[k] = X0;
