@@ -1,0 +1,59 @@
+"""Clouds whose header box is smaller than their points, against the oracle: the
+tiles' counts and hyperboloid sizes.  Clumps of points
+lie beside, above and below the octree's root cube; the reference takes such a
+point with its block, whose cube lies at the root cube's face, so a
+point counts that the query's shape itself does not hold."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(seed, kinds):
+    r = np.random.default_rng(seed)
+    side = [7.8, 3.9, 15.5][seed % 3]   # the root cube is a little larger
+    u = lambda n, lo, hi: r.uniform(lo, hi, n)
+    ground = np.stack([u(1500, 0, side), u(1500, 0, side), 0.1 * side + u(1500, -0.05, 0.05)], 1)
+    high = np.stack([u(400, 0, side), u(400, 0, side), u(400, 0.2, 1.0) * side], 1)
+    edge = np.stack([side - u(150, 0, 0.1) * side, u(150, 0, side), u(150, 0.3, 1.0) * side], 1)
+    parts = [ground, high, edge, edge[:, [1, 0, 2]]]
+    for k in kinds:
+        m = int(r.integers(600, 2500))
+        a, b = u(1, 0, 0.8)[0] * side, u(1, 0, 0.5)[0] * side
+        # lower case: from the root cube's face on, upper case: farther than any query's reach
+        far = side * (1 + 10.0 ** (u(m, -2, 0.7) if k.islower() else u(m, 1.0, 1.5)))
+        p, q = a + u(m, 0, 0.2) * side, b + u(m, 0, 0.2) * side
+        parts.append({"x": np.stack([far, p, q], 1), "y": np.stack([p, far, q], 1), "w": np.stack([side - far, p, q], 1),
+                      "c": np.stack([far, far[::-1], q], 1), "a": np.stack([p, a + (q - b), far], 1),
+                      "b": np.stack([p, q, -far], 1)}[k.lower()])
+    d = np.concatenate(parts)
+    return d[r.permutation(len(d))], side
+
+
+def _cloud(seed, kinds, sign=(1, 1, 1), head=1.0):
+    """head: the part of the points' box that the header gives."""
+    from wolkenbase_gb300 import synth
+    d, side = _points(seed, kinds)
+    scale = tuple(0.001 * s for s in sign)
+    xyz = np.rint(d / np.array(scale)).astype(np.int32)
+    return synth.Cloud(np.ascontiguousarray(xyz), scale, (0.0, 0.0, 0.0), 1.0, (0.0,) * 3, (head * side,) * 3)
+
+
+CLOUDS = {f"{kinds or 'none'}_{seed}_{head}": (seed, kinds, head)
+          for kinds, seeds, head in (("x", (0, 1), 1.0), ("y", (2,), 1.0), ("w", (3,), 1.0), ("c", (4,), 1.0), ("a", (5, 6), 1.0),
+                                     ("b", (7,), 1.0), ("xywcab", (8, 9, 10), 1.0), ("", (0, 1, 2), 0.6), ("xa", (3, 4), 0.6),
+                                     ("X", (0, 1, 2, 3), 1.0), ("W", (4,), 1.0), ("XYW", (5, 6, 7), 1.0), ("A", (8,), 1.0), ("XA", (9, 10), 0.6))
+          for seed in seeds}
+
+
+@pytest.mark.parametrize("name", sorted(CLOUDS))
+def test_tiles(classifier, oracle_mod, name):
+    import wolkenbase_gb300 as wb
+    seed, kinds, head = CLOUDS[name]
+    cloud = _cloud(seed, kinds, head=head)
+    o = oracle_mod.run(cloud, canonical_order=True, threads=8, phases=2)
+    classifier.build(cloud)
+    classifier.scan(wb.Params())
+    t = classifier.tiles()
+    assert np.array_equal(t["n_points"], o["tiles"]["n_points"])
+    assert np.array_equal(t["hyperboloid_size"], o["tiles"]["h_final"])

@@ -162,11 +162,15 @@ __device__ __forceinline__ bool cellMeetsCyl(const TileArgs &a, const int4 &box,
 /* The same column test in the tile's FP32 frame, with the radius widened by
  * 2e-4 (relative) and 1e-4 (absolute, squared units): a superset of the FP64
  * test (the frame's rounding is about 1e-7 relative), so no column with a
- * member is skipped; an extra column only costs its points' tests.  The
- * bound and both fills use this one test, so a tile never gathers more
- * points than its bound counted. */
-__device__ __forceinline__ bool cellMeets(const TileArgs &a, const TileFrame &f, const int4 &box)
+ * member is skipped; an extra column only costs its points' tests.  A column
+ * with a point outside the root cube (flags) is always read: the cylinder can
+ * hold that point's block without reaching the point.  The bound and both fills
+ * use this one test, so a tile never gathers more points than its bound
+ * counted. */
+__device__ __forceinline__ bool cellMeets(const TileArgs &a, const TileFrame &f, const int4 &box, int flags)
 {
+  if (flags)
+    return true;
   if (!a.fast)
     return cellMeetsCyl(a, box, f.cx, f.cy);
   const float ax = ((float)(box.x - f.qx0) - f.fx) * f.sx, bx = ((float)(box.z - f.qx0) - f.fx) * f.sx;
@@ -230,7 +234,7 @@ __global__ void gridBound(TileArgs a, GridDev gd, uint32_t *__restrict__ bound, 
       {
         uint64_t c = (uint64_t)j * gd.nx + i;
         int4 box = gd.cell2[2 * c], r1 = gd.cell2[2 * c + 1];
-        if (r1.y != r1.z && cellMeets(a, f, box))
+        if (r1.y != r1.z && cellMeets(a, f, box, r1.w))
           room += (uint32_t)(r1.z - r1.y);
       }
     bound[k] = room;
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) gridFillWarp(TileArgs a, Grid
       const int4 box = gd.cell2[2 * c], r1 = gd.cell2[2 * c + 1];
       cb = (uint32_t)r1.y;
       ce = (uint32_t)r1.z;
-      meets = cb != ce && cellMeets(a, f, box);
+      meets = cb != ce && cellMeets(a, f, box, r1.w);
     }
     unsigned left = __ballot_sync(0xffffffffu, meets);
     const unsigned apart = __ballot_sync(0xffffffffu, cb != ce && !meets);
@@ -372,7 +376,7 @@ __global__ void __launch_bounds__(kFillThreads) gridFill(TileArgs a, GridDev gd,
       uint64_t c = (uint64_t)(f.j0 + q / nc) * gd.nx + f.i0 + q % nc;
       int4 box = gd.cell2[2 * c], r1 = gd.cell2[2 * c + 1];
       uint32_t b = (uint32_t)r1.y, e = (uint32_t)r1.z;
-      if (b == e || !cellMeets(a, f, box))
+      if (b == e || !cellMeets(a, f, box, r1.w))
         continue;
       for (uint32_t t = b + (threadIdx.x & 31); t < e; t += 32)
       {
