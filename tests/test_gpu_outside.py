@@ -1,8 +1,8 @@
 """Clouds whose header box is smaller than their points, against the oracle: the
-tiles' counts and hyperboloid sizes.  Clumps of points
+tiles' counts and every label, whichever kernel decides them.  Clumps of points
 lie beside, above and below the octree's root cube; the reference takes such a
-point with its block, whose cube lies at the root cube's face, so a
-point counts that the query's shape itself does not hold."""
+point with its block, whose cube lies at the root cube's face, so a neighbour
+counts that the query's shape itself does not hold."""
 import numpy as np
 import pytest
 
@@ -46,6 +46,39 @@ CLOUDS = {f"{kinds or 'none'}_{seed}_{head}": (seed, kinds, head)
           for seed in seeds}
 
 
+def _wrong(classifier, O, cloud, got):
+    """Stored points with another label than the reference's.  The reference tries
+    the list of the point before first, so beside the root cube a label can depend
+    on which point that was; where labels differ, the points that pointsIn alone
+    returns decide (their integer directions' largest gap against 144 degrees)."""
+    o = O.run(cloud, canonical_order=True, threads=8, keep=True)
+    try:
+        stored = np.zeros(cloud.n, bool)
+        stored[classifier.store_order()] = True
+        differ = np.nonzero((got != o["cls"]) & stored)[0]
+        if not differ.size:
+            return differ
+        assert set(got[differ].tolist()) <= {1, 2} and set(o["cls"][differ].tolist()) <= {1, 2}
+        t, d = o["tiles"], cloud.decoded()
+        owner = np.full(cloud.n, -1)
+        for k in np.nonzero(t["n_points"])[0]:
+            cx = o["snake_center"][0] + (t["ex"][k] - t["ey"][k] / 2) * o["spacing"]
+            cy = o["snake_center"][1] + t["ey"][k] * 0.86602540378443864676372317 * o["spacing"]
+            owner[O.points_in(1, (cx, cy), o["spacing"] * 41 / 71)] = k
+        wrong = []
+        for j in differ:
+            q = O.points_in(2, tuple(d[j]), t["h_final"][owner[j]])
+            v = d[q] - d[j]
+            v = v[(v[:, 0] != 0) | (v[:, 1] != 0)]
+            u = np.unique(O.atan2i(v[:, 1], v[:, 0]).astype(np.int64) & 0x7fffffff)
+            gap = np.max((np.roll(u, -1) - u) & 0x7fffffff) if u.size > 1 else 1 << 31
+            if got[j] != (1 if gap < 0x33333333 else 2):
+                wrong.append(j)
+        return np.array(wrong, int)
+    finally:
+        O.reset()
+
+
 @pytest.mark.parametrize("name", sorted(CLOUDS))
 def test_tiles(classifier, oracle_mod, name):
     import wolkenbase_gb300 as wb
@@ -57,3 +90,20 @@ def test_tiles(classifier, oracle_mod, name):
     t = classifier.tiles()
     assert np.array_equal(t["n_points"], o["tiles"]["n_points"])
     assert np.array_equal(t["hyperboloid_size"], o["tiles"]["h_final"])
+
+
+@pytest.mark.parametrize("shape", [0, 1, 2, 4])
+@pytest.mark.parametrize("name", sorted(CLOUDS))
+def test_labels(classifier, oracle_mod, name, shape):
+    """Point groups (0-2) and the one-point kernel (4)."""
+    import wolkenbase_gb300 as wb
+    seed, kinds, head = CLOUDS[name]
+    cloud = _cloud(seed, kinds, head=head)
+    keep = classifier.tuning()
+    classifier.set_tuning(shape=shape)
+    try:
+        got = classifier.classify_cloud(cloud, wb.Params())
+    finally:
+        classifier.set_tuning(shape=keep["shape"])
+    bad = _wrong(classifier, oracle_mod, cloud, got)
+    assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"

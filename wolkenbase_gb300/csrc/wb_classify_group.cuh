@@ -337,9 +337,12 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
   };
   envelope();
   // can a box {x0, y0, x1, y1} with lowest point zmin hold a member of any lane?
-  auto envMeets = [&](const int4 &b, int32_t zmin) -> bool {
+  // (always, when it holds a point beside or above the root cube: flags)
+  auto envMeets = [&](const int4 &b, int32_t zmin, int flags) -> bool {
     if (b.x == INT32_MAX)
       return false;
+    if (flags)
+      return true;
     const float dx = (float)max(0, max(b.x - gx1, gx0 - b.z)), dy = (float)max(0, max(b.y - gy1, gy0 - b.w)) * ky;
     const float zd = apex - (float)(zmin - gz0) * kz;
     const float r2 = __fmaf_rn(dx, dx, dy * dy);
@@ -626,7 +629,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
         r = a.groups[2 * (uint64_t)(gNext + lane) + 1];
       }
       gNext += 32;
-      list = __ballot_sync(kAll, envMeets(b, r.x));
+      list = __ballot_sync(kAll, envMeets(b, r.x, r.w));
       __syncwarp();
       sm.nbox[lane] = boxOfInts(b);
       sm.nrec[lane] = make_int4(__float_as_int((float)(r.x - gz0)), r.y, r.z, r.w);
@@ -669,7 +672,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
         r = a.super[2 * sc + 1];
       }
     }
-    supers = __ballot_sync(kAll, envMeets(b, r.x));
+    supers = __ballot_sync(kAll, envMeets(b, r.x, r.w));
     __syncwarp();
     sm.sbox[lane] = boxOfInts(b);
     sm.srec[lane] = make_int4(__float_as_int((float)(r.x - gz0)), r.y, r.z, r.w);

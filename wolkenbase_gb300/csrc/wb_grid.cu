@@ -145,7 +145,7 @@ __global__ void cellKernel(GridArgs g, const int32_t *__restrict__ sx, const int
       // +-1e9), and clamped into the grid for the sort key; from the integer
       // thresholds where they apply, else in FP64
       int ci, cj;
-      bool sxy, s;
+      bool beside, s;   // beside or above the root cube; outside it at all
       if (g.thr)
       {
         const long long *xb = g.bounds, *yb = g.bounds + g.nx + 1, *face = g.bounds + g.nx + g.ny + 2;
@@ -158,21 +158,21 @@ __global__ void cellKernel(GridArgs g, const int32_t *__restrict__ sx, const int
           cj = columnOf(yb, g.ny, Y, g.colPerUnit[1]);
         else
           cj = (int)fmax(fmin(floor((xyzd[g.nd + j] - g.y0) / g.cell), 1e9), -1e9);
-        sxy = X < face[0] || Y < face[1] || X >= face[3] || Y >= face[4];
-        s = sxy || Z < face[2] || Z >= face[5];
+        beside = X < face[0] || Y < face[1] || X >= face[3] || Y >= face[4] || Z >= face[5];
+        s = beside || Z < face[2];
       }
       else
       {
         const double x = xyzd[j], y = xyzd[g.nd + j], z = xyzd[2 * g.nd + j];
         ci = (int)fmax(fmin(floor((x - g.x0) / g.cell), 1e9), -1e9);
         cj = (int)fmax(fmin(floor((y - g.y0) / g.cell), 1e9), -1e9);
-        sxy = x < g.rootLo[0] || y < g.rootLo[1] || x >= g.rootHi[0] || y >= g.rootHi[1];
-        s = sxy || z < g.rootLo[2] || z >= g.rootHi[2];
+        beside = x < g.rootLo[0] || y < g.rootLo[1] || x >= g.rootHi[0] || y >= g.rootHi[1] || z >= g.rootHi[2];
+        s = beside || z < g.rootLo[2];
       }
       colOf[j] = make_int2(ci, cj);
       const int cx = min(max(ci, 0), g.nx - 1), cy = min(max(cj, 0), g.ny - 1);
       cell = (uint32_t)cy * (uint32_t)g.nx + cx;
-      stray[j] = (uint8_t)((s ? 1 : 0) | (sxy ? 2 : 0));
+      stray[j] = (uint8_t)((s ? 1 : 0) | (beside ? 2 : 0));
       if (s)
         atomicAdd(nStray, 1ull);
     }
@@ -239,7 +239,7 @@ template <typename At>
 __device__ __forceinline__ void fillColumn(uint64_t c, uint32_t b, uint32_t e, int lane, int lanes, At at,
                                            const int32_t *__restrict__ sx, const int32_t *__restrict__ sy,
                                            const int32_t *__restrict__ sz, const uint8_t *__restrict__ stray,
-                                           int4 *__restrict__ gpt, int32_t mn[3], int32_t mx[3], bool &xyStray)
+                                           int4 *__restrict__ gpt, int32_t mn[3], int32_t mx[3], bool &beside)
 {
   for (uint32_t i = b + lane; i < e; i += lanes)
   {
@@ -247,7 +247,7 @@ __device__ __forceinline__ void fillColumn(uint64_t c, uint32_t b, uint32_t e, i
     const int32_t q[3] = {sx[j], sy[j], sz[j]};
     const uint8_t st = stray[j];
     gpt[i] = make_int4(q[0], q[1], q[2], (int)(j | ((st & 1) ? 0x80000000u : 0u)));
-    xyStray |= (st & 2) != 0;
+    beside |= (st & 2) != 0;
     for (int a = 0; a < 3; a++)
     {
       mn[a] = min(mn[a], q[a]);
@@ -258,15 +258,16 @@ __device__ __forceinline__ void fillColumn(uint64_t c, uint32_t b, uint32_t e, i
 
 /* Warp-wide part of a column's record; lane 0 writes it. */
 __device__ __forceinline__ void writeColumn(uint64_t c, uint32_t b, uint32_t e, int lane, int32_t mn[3], int32_t mx[3],
-                                            bool xyStray, int4 *__restrict__ rec)
+                                            bool beside, int4 *__restrict__ rec)
 {
   for (int a = 0; a < 3; a++)
   {
     mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
     mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
   }
-  // a column holding a point outside the root cube in x or y is read in full
-  const bool any = __any_sync(0xffffffffu, xyStray);
+  // a column holding a point beside or above the root cube is read in full: a
+  // shape can hold that point's block without holding the point
+  const bool any = __any_sync(0xffffffffu, beside);
   if (lane == 0)
   {
     rec[2 * c] = make_int4(mn[0], mn[1], mx[0], mx[1]);
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(32 * kColumnWarps) columnKernel(uint64_t ncell
     return;
   const uint32_t b = start[c], e = start[c + 1], n = e - b;
   int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-  bool xyStray = false;
+  bool beside = false;
   uint64_t *k = buf[w];
   if (n > kColumnMax)
   {
@@ -333,8 +334,8 @@ __global__ void __launch_bounds__(32 * kColumnWarps) columnKernel(uint64_t ncell
         __syncwarp();
       }
   }
-  fillColumn(c, b, e, lane, 32, [&](uint32_t i) { return (uint32_t)k[i - b]; }, sx, sy, sz, stray, gpt, mn, mx, xyStray);
-  writeColumn(c, b, e, lane, mn, mx, xyStray, rec);
+  fillColumn(c, b, e, lane, 32, [&](uint32_t i) { return (uint32_t)k[i - b]; }, sx, sy, sz, stray, gpt, mn, mx, beside);
+  writeColumn(c, b, e, lane, mn, mx, beside, rec);
 }
 
 /* The listed columns, one block each, up to kBigColumnMax points in shared
@@ -386,15 +387,15 @@ __global__ void __launch_bounds__(512) bigColumnKernel(const uint32_t *__restric
         __syncthreads();
       }
     int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-    bool xyStray = false;
+    bool beside = false;
     fillColumn(c, b, e, (int)threadIdx.x, 512, [&](uint32_t i) { return (uint32_t)k[i - b]; }, sx, sy, sz, stray, gpt, mn, mx,
-               xyStray);
+               beside);
     for (int a = 0; a < 3; a++)
     {
       atomicMin(&ext[a], mn[a]);
       atomicMax(&ext[3 + a], mx[a]);
     }
-    if (xyStray)
+    if (beside)
       flag = 1;
     __syncthreads();
     if (threadIdx.x == 0)
@@ -417,9 +418,9 @@ __global__ void cellFillKernel(uint64_t ncell, const uint32_t *__restrict__ star
     return;
   const uint32_t b = start[c], e = start[c + 1];
   int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-  bool xyStray = false;
-  fillColumn(c, b, e, lane, 32, [&](uint32_t i) { return pos[i]; }, sx, sy, sz, stray, gpt, mn, mx, xyStray);
-  writeColumn(c, b, e, lane, mn, mx, xyStray, rec);
+  bool beside = false;
+  fillColumn(c, b, e, lane, 32, [&](uint32_t i) { return pos[i]; }, sx, sy, sz, stray, gpt, mn, mx, beside);
+  writeColumn(c, b, e, lane, mn, mx, beside, rec);
 }
 
 /* Column groups (the work items of the margin pass): a column of n points is
