@@ -107,3 +107,16 @@ def test_labels(classifier, oracle_mod, name, shape):
         classifier.set_tuning(shape=keep["shape"])
     bad = _wrong(classifier, oracle_mod, cloud, got)
     assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"
+
+
+@pytest.mark.parametrize("name", sorted(CLOUDS))
+def test_labels_with_margins(classifier, oracle_mod, name):
+    """The column groups and bins."""
+    import wolkenbase_gb300 as wb
+    seed, kinds, head = CLOUDS[name]
+    cloud = _cloud(seed, kinds, head=head)
+    classifier.build(cloud)
+    classifier.scan(wb.Params())
+    got, _ = classifier.classify_margins(wb.Params())
+    bad = _wrong(classifier, oracle_mod, cloud, got)
+    assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"

@@ -224,13 +224,18 @@ __device__ __noinline__ bool memberExact(const ClsArgs &a, const HypExact &h, ui
   return all || in;
 }
 
-/* Can any point of a box (integer bounds, 6 planes of N entries) be inside?
- * FP32 with generous slack.  Record differences are exact in 32 bits: the
- * host checks that the cloud's integer extent fits. */
-__device__ __forceinline__ bool boxMeets(const Hyp &h, const int4 &b, int32_t zmin)
+/* Can any point of a box (b: bounds; r1: lowest z and flags, the column
+ * layout) be inside?  FP32 with generous slack.  Record differences are exact
+ * in 32 bits: the host checks that the cloud's integer extent fits.  A box
+ * holding a point beside or above the root cube (flags) always can: that
+ * point's block decides. */
+__device__ __forceinline__ bool boxMeets(const Hyp &h, const int4 &b, const int4 &r1)
 {
   if (b.x == INT32_MAX)
     return false;   // empty block
+  if (r1.w)
+    return true;
+  const int32_t zmin = r1.x;
   // the bound takes the box's low record integers as its low coordinates:
   // only for a decode that increases with the record integer
   if (!(h.sx > 0.f && h.sy > 0.f && h.sz > 0.f))
@@ -477,7 +482,7 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
   // Points of a column are sorted by height.  None above pz + (czp -
   // sqrt(por^2 + s^2 d^2)) / sz, d the column's nearest distance, can be
   // inside: colZlim gives that bound (with slack) in record units relative to
-  // the point.  Columns holding points outside the root cube in x or y get no
+  // the point.  Columns holding points beside or above the root cube get no
   // bound (their blocks' cubes decide for them).
   auto colZlim = [&](const int4 &box, const int4 &r1) -> int32_t {
     if (!fp32Member || r1.w || !(h.sz > 0))
@@ -691,7 +696,7 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
         {
           c = (uint64_t)jj * a.nx + i;
           cb = a.col[2 * c];
-          ok = boxMeets(h, cb, a.col[2 * c + 1].x);
+          ok = boxMeets(h, cb, a.col[2 * c + 1]);
         }
       }
       unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -750,7 +755,7 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
         {
           const uint64_t sc = (uint64_t)SJ * a.snx + SI;
           sb = a.super[2 * sc];
-          ok = boxMeets(h, sb, a.super[2 * sc + 1].x);
+          ok = boxMeets(h, sb, a.super[2 * sc + 1]);
         }
       }
       unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -774,7 +779,7 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
           {
             c = (uint64_t)jj * a.nx + i;
             cb = a.col[2 * c];
-            cok = boxMeets(h, cb, a.col[2 * c + 1].x);
+            cok = boxMeets(h, cb, a.col[2 * c + 1]);
           }
         }
         unsigned cm = __ballot_sync(0xffffffffu, cok);
@@ -1032,15 +1037,17 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
 #ifdef WB_CLASSIFY_STATS
     bool farField = false;   // lane tests beyond the near field (instrumented builds)
 #endif
-    // envelope test of a box {x0, y0, x1, y1} with lowest point zmin
-    auto envMeets = [&](const int4 &b, int32_t zmin) -> bool {
+    // envelope test of a box {x0, y0, x1, y1} (r1: lowest z and flags, as in boxMeets)
+    auto envMeets = [&](const int4 &b, const int4 &r1) -> bool {
       if (b.x == INT32_MAX)
         return false;
+      if (r1.w)
+        return true;
       const int4 cb0 = sm.cbox;
       const float apex = sm.apex, por2min = sm.por2min;
       float dx = (float)max(0, max(b.x - cb0.z, cb0.x - b.z)) * sx;
       float dy = (float)max(0, max(b.y - cb0.w, cb0.y - b.w)) * sy;
-      float zd = apex - (float)(zmin - oz) * sz;
+      float zd = apex - (float)(r1.x - oz) * sz;
       float r2 = s2 * (dx * dx + dy * dy);
       float mag = zd * zd + r2 + por2min;
       if (zd < -1e-4f * (fabsf(zd) + 1e-3f))
@@ -1048,8 +1055,8 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
       return zd * zd - r2 - por2min >= -(1e-4f * mag + 1e-9f);
     };
     // height (record units above oz) above which no point of a column can be
-    // inside any lane's hyperboloid; columns holding points outside the root
-    // cube in x or y get no bound
+    // inside any lane's hyperboloid; columns holding points beside or above
+    // the root cube get no bound
     auto envZlim = [&](const int4 &b, const int4 &r1) -> int32_t {
       if (r1.w || !(sz > 0))
         return INT32_MAX;
@@ -1317,7 +1324,7 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
         {
           c = (uint64_t)jj * a.nx + i;
           cb = a.col[2 * c];
-          ok = envMeets(cb, a.col[2 * c + 1].x);
+          ok = envMeets(cb, a.col[2 * c + 1]);
         }
       }
       unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -1361,7 +1368,7 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
           {
             const uint64_t sc = (uint64_t)SJ * a.snx + SI;
             sb = a.super[2 * sc];
-            ok = envMeets(sb, a.super[2 * sc + 1].x);
+            ok = envMeets(sb, a.super[2 * sc + 1]);
           }
         }
         unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -1387,7 +1394,7 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
             {
               c = (uint64_t)jj * a.nx + i;
               cb = a.col[2 * c];
-              cok = envMeets(cb, a.col[2 * c + 1].x);
+              cok = envMeets(cb, a.col[2 * c + 1]);
             }
           }
           unsigned cm = __ballot_sync(0xffffffffu, cok);
