@@ -120,3 +120,15 @@ def test_labels_with_margins(classifier, oracle_mod, name):
     got, _ = classifier.classify_margins(wb.Params())
     bad = _wrong(classifier, oracle_mod, cloud, got)
     assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"
+
+
+@pytest.mark.parametrize("sign", [(-1, 1, 1), (1, 1, -1)])
+@pytest.mark.parametrize("name", sorted(CLOUDS))
+def test_labels_of_the_exact_pass(classifier, oracle_mod, name, sign):
+    """A scale below zero: the exact pass decides every point."""
+    import wolkenbase_gb300 as wb
+    seed, kinds, head = CLOUDS[name]
+    cloud = _cloud(seed, kinds, sign, head)
+    got = classifier.classify_cloud(cloud, wb.Params())
+    bad = _wrong(classifier, oracle_mod, cloud, got)
+    assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"

@@ -135,7 +135,7 @@ struct ClsArgs
   float gInv, gTiny;      /* 1 / (slope * x record unit); 1e-12 m^2 in that unit squared */
   int snx, sny;
   const int4 *super;   /* super-cell records, the column layout */
-  double zmin;
+  double zmin;     /* lowest height a member can have */
   int exactInts;   /* decode strictly increasing and 32-bit record differences exact */
   int fp32Only;    /* precision mode: FP32 decisions stand, no exact re-run */
   float fsx, fsy, fsz, fs2;   /* metres per record unit and slope^2, FP32 */
@@ -378,7 +378,7 @@ __device__ __forceinline__ void setupPoint(const ClsArgs &a, uint64_t j)
   PtSetup s;
   s.czp = (float)(cz - pz);
   s.por2f = (float)(por * por);
-  // Horizontal reach of the hyperboloid at the lowest point of the cloud.  The
+  // Horizontal reach of the hyperboloid at the lowest height a member can have.  The
   // ring counts only bound the search (columns beyond the reach hold no
   // member), so they are formed in FP32, both squares rounded apart by more
   // than their error (the FP64 pipe bounds this kernel), with a 1e-5 margin.
@@ -1559,7 +1559,13 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
   a.snx = c->grid.snx;
   a.sny = c->grid.sny;
   a.super = (const int4 *)c->superRec.p;
-  a.zmin = (g.off[2] + g.scale[2] * (double)c->grid.zminInt) * g.unit;
+  // the lowest height a member can have, for the reach: the lowest point's (the
+  // highest record integer's where the z scale is negative), or that of the root
+  // cube's top where a block there decides for points above it
+  a.zmin = std::min((g.off[2] + g.scale[2] * (double)c->grid.imin[2]) * g.unit,
+                    (g.off[2] + g.scale[2] * (double)c->grid.imax[2]) * g.unit);
+  if (c->grid.nStray)
+    a.zmin = std::min(a.zmin, g.root_lo[2] + g.root_side);
   bool fits32 = true;
   for (int k = 0; k < 3; k++)
     fits32 = fits32 && (int64_t)c->grid.imax[k] - (int64_t)c->grid.imin[k] < ((int64_t)1 << 30);

@@ -819,7 +819,6 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
   WB_CUDA(c, cudaGetLastError());
   c->grid.grouped = false;
   c->grid.nStray = ns;
-  c->grid.zminInt = ext[2];
   for (int k = 0; k < 3; k++)
   {
     c->grid.imin[k] = ext[k];
