@@ -132,3 +132,25 @@ def test_labels_of_the_exact_pass(classifier, oracle_mod, name, sign):
     got = classifier.classify_cloud(cloud, wb.Params())
     bad = _wrong(classifier, oracle_mod, cloud, got)
     assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"
+
+
+def _rough(seed, sign, head, n, side):
+    from wolkenbase_gb300 import synth
+    r = np.random.default_rng(seed)
+    d = np.stack([r.uniform(0, side, n), r.uniform(0, side, n), r.uniform(0, 0.1 * side, n)], 1)
+    scale = tuple(0.001 * s for s in sign)
+    lo = 0.5 * (side - head)
+    return synth.Cloud(np.rint(d / np.array(scale)).astype(np.int32), scale, (0.0, 0.0, 0.0), 1.0, (lo, lo, 0.0),
+                       (side - lo, side - lo, 0.1 * side))
+
+
+@pytest.mark.parametrize("sign", [(-1, 1, 1), (1, 1, -1)])
+@pytest.mark.parametrize("n", [2000, 60000])
+def test_exact_pass_beside_the_grid(classifier, oracle_mod, n, sign):
+    """Points up to fourteen columns beside the header's box and inside the root
+    cube; their nearest neighbours are in the grid's edge columns."""
+    import wolkenbase_gb300 as wb
+    cloud = _rough(3, sign, 2.05, n, 4.0)
+    got = classifier.classify_cloud(cloud, wb.Params())
+    bad = _wrong(classifier, oracle_mod, cloud, got)
+    assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"

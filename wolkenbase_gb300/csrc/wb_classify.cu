@@ -434,7 +434,9 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
   else
     __syncwarp();
   const int turn = WARPS > 1 ? threadIdx.x >> 5 : 0;
-  const int ci = ps.ci, cj = ps.cj, kmax = ps.kmax;
+  // A point beside the grid is at home in the nearest column of the grid, as the
+  // points it is compared with are: between two of them this shortens distances only.
+  const int ci = min(max(ps.ci, 0), a.nx - 1), cj = min(max(ps.cj, 0), a.ny - 1), kmax = ps.kmax;
   HypExact hx;
   if (EXACT)
     hx = exactHyp(a, (uint32_t)j);
@@ -676,8 +678,6 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
   const int kNear = 1;
   for (int ring = 0; ring <= kNear && ring <= kmax && !surrounded; ring++)
   {
-    if (ci + ring < 0 || ci - ring >= a.nx || cj + ring < 0 || cj - ring >= a.ny)
-      continue;
     int ncells = ring == 0 ? 1 : 8 * ring;
     int stride = ring == 0 ? 1 : 4 * ring - 1;
     WB_STAT(stat[1], ncells);
@@ -731,12 +731,10 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
   // Far field: rings of super-cells (WB_SUPER x WB_SUPER columns) pruned as a
   // block; columns already visited in the near field are skipped.
   const int S = WB_SUPER;
-  int si = ci >= 0 ? ci / S : -((-ci + S - 1) / S), sj = cj >= 0 ? cj / S : -((-cj + S - 1) / S);
+  const int si = ci / S, sj = cj / S;
   const int smax = ps.smax;
   for (int sr = 0; sr <= smax && !surrounded && kmax > kNear; sr++)
   {
-    if (si + sr < 0 || si - sr >= a.snx || sj + sr < 0 || sj - sr >= a.sny)
-      continue;
     int nsc = sr == 0 ? 1 : 8 * sr;
     WB_STAT(stat[2], nsc);
     for (int m0 = 0; m0 < nsc && !surrounded; m0 += 32)
