@@ -154,3 +154,21 @@ def test_exact_pass_beside_the_grid(classifier, oracle_mod, n, sign):
     got = classifier.classify_cloud(cloud, wb.Params())
     bad = _wrong(classifier, oracle_mod, cloud, got)
     assert bad.size == 0, f"{bad.size} of {cloud.n} labels differ, e.g. {bad[:8].tolist()}"
+
+
+@pytest.mark.parametrize("kernel", ["groups", "points", "bins", "exact"])
+def test_reach_of_many_grid_widths(classifier, oracle_mod, kernel):
+    """A slope of 1e-4: half a metre of height reaches six kilometres, the grid six metres."""
+    import wolkenbase_gb300 as wb
+    cloud = _rough(4, (-1, 1, 1) if kernel == "exact" else (1, 1, 1), 6.0, 1500, 6.0)
+    p = dict(max_slope=1e-4)
+    o = oracle_mod.run(cloud, canonical_order=True, threads=8, **p)
+    keep = classifier.tuning()
+    classifier.set_tuning(shape=4 if kernel == "points" else 0)
+    try:
+        classifier.build(cloud)
+        classifier.scan(wb.Params(**p))
+        got = classifier.classify_margins(wb.Params(**p))[0] if kernel == "bins" else classifier.classify(wb.Params(**p))
+    finally:
+        classifier.set_tuning(shape=keep["shape"])
+    assert np.array_equal(got, o["cls"])

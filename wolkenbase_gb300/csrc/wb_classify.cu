@@ -735,6 +735,9 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
   const int smax = ps.smax;
   for (int sr = 0; sr <= smax && !surrounded && kmax > kNear; sr++)
   {
+    // no ring beyond the grid, however far the reach
+    if (si - sr < 0 && si + sr >= a.snx && sj - sr < 0 && sj + sr >= a.sny)
+      break;
     int nsc = sr == 0 ? 1 : 8 * sr;
     WB_STAT(stat[2], nsc);
     for (int m0 = 0; m0 < nsc && !surrounded; m0 += 32)
@@ -1347,8 +1350,8 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
     const int si = ci0 / S, sj = cj0 / S;
     for (int sr = 0; sr <= sm.smaxG && sm.kmaxG > kNearG && !allDone(); sr++)
     {
-      if (si + sr < 0 || si - sr >= a.snx || sj + sr < 0 || sj - sr >= a.sny)
-        continue;
+      if (si - sr < 0 && si + sr >= a.snx && sj - sr < 0 && sj + sr >= a.sny)
+        break;   // no ring beyond the grid, however far the reach
       const int nsc = sr == 0 ? 1 : 8 * sr;
       for (int m0 = 0; m0 < nsc && !allDone(); m0 += 32)
       {
