@@ -695,12 +695,7 @@ int wb_build_impl(wb_ctx *c, const wb_cloud *cl)
   auto readFlags = [&]() -> int {
     WB_CUDA(c, cudaMemcpyAsync(&fl, flags, sizeof fl, cudaMemcpyDefault, c->stream));
     WB_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (fl.lookback)
-    {
-      WB_CUDA(c, cudaMemsetAsync(flags, 0, 4, c->stream));
-      return wb_fail(c, WB_ETIMEDOUT, "wb_octree_build: a look-back wait gave up");
-    }
-    return 0;
+    return fl.lookback ? wb_lookback_failed(c, "wb_octree_build") : 0;
   };
   WB_CUDA(c, cudaMemsetAsync(&flags->dups, 0, sizeof(BuildFlags) - 4, c->stream));
   uint64_t *keys = (uint64_t *)c->key0.p, *kAlt = (uint64_t *)c->key1.p;

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cmath>
+#include <cstring>
 #include "wb_internal.h"
 #include "wb_device.cuh"
 #include "wb_warpsort.cuh"
@@ -219,8 +220,10 @@ __device__ __forceinline__ uint64_t heightKey(int32_t z, uint64_t j)
 /* Puts every point's (height, store position) at its place in its column. */
 __global__ void cellScatterKernel(uint64_t nd, int nx, int ny, const int2 *__restrict__ colOf,
                                   const uint32_t *__restrict__ rank, const uint32_t *__restrict__ start,
-                                  const int32_t *__restrict__ sz, uint64_t *__restrict__ slots)
+                                  const int32_t *__restrict__ sz, uint64_t *__restrict__ slots, const int *__restrict__ err)
 {
+  if (*err)
+    return;   // start was not written
   for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += (uint64_t)gridDim.x * blockDim.x)
     slots[start[cellOf(colOf[j], nx, ny)] + rank[j]] = heightKey(sz[j], j);
 }
@@ -287,12 +290,13 @@ __global__ void __launch_bounds__(32 * kColumnWarps) columnKernel(uint64_t ncell
                                                                   const int32_t *__restrict__ sz,
                                                                   const uint8_t *__restrict__ stray,
                                                                   int4 *__restrict__ gpt, int4 *__restrict__ rec,
-                                                                  uint32_t *__restrict__ big, uint32_t *__restrict__ nBig)
+                                                                  uint32_t *__restrict__ big, uint32_t *__restrict__ nBig,
+                                                                  const int *__restrict__ err)
 {
   __shared__ uint64_t buf[kColumnWarps][kColumnMax];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint64_t c = (uint64_t)blockIdx.x * kColumnWarps + w;
-  if (c >= ncell)
+  if (c >= ncell || *err)   // err: start was not written, nothing is listed for bigColumnKernel
     return;
   const uint32_t b = start[c], e = start[c + 1], n = e - b;
   int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
@@ -410,11 +414,11 @@ __global__ void __launch_bounds__(512) bigColumnKernel(const uint32_t *__restric
 __global__ void cellFillKernel(uint64_t ncell, const uint32_t *__restrict__ start, const uint32_t *__restrict__ pos,
                                const int32_t *__restrict__ sx, const int32_t *__restrict__ sy,
                                const int32_t *__restrict__ sz, const uint8_t *__restrict__ stray,
-                               int4 *__restrict__ gpt, int4 *__restrict__ rec)
+                               int4 *__restrict__ gpt, int4 *__restrict__ rec, const int *__restrict__ err)
 {
   const uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (c >= ncell)
+  if (c >= ncell || *err)   // err: pos was not written
     return;
   const uint32_t b = start[c], e = start[c + 1];
   int32_t mn[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, mx[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
@@ -435,8 +439,10 @@ __global__ void groupCountKernel(uint64_t ncell, const int4 *__restrict__ rec, u
 }
 
 __global__ void groupFillKernel(uint64_t ncell, const int4 *__restrict__ rec, const uint32_t *__restrict__ first,
-                                uint2 *__restrict__ groups)
+                                uint2 *__restrict__ groups, const int *__restrict__ err)
 {
+  if (*err)
+    return;   // first was not written
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += (uint64_t)gridDim.x * blockDim.x)
   {
     int4 r1 = rec[2 * c + 1];
@@ -774,25 +780,31 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
   const uint8_t *stray = (const uint8_t *)c->stray.p;
   const int2 *colOf = (const int2 *)c->colOf.p;
   int4 *gpt = (int4 *)c->gpt.p, *cellRec = (int4 *)c->cellRec.p;
+  const int *err = wb_lookback_err(c);
   WB_CUDA(c, cudaMemsetAsync(count, 0, (ncell + 1) * 4, c->stream));
   WB_CUDA(c, cudaMemsetAsync(dBig, 0, 8, c->stream));
   { cellKernel<<<blocks, 256, 0, c->stream>>>(a, sx, sy, sz, count, rank, (uint8_t *)c->stray.p, dStray, dExt,
                                               (const double *)c->xyzd.p, (int2 *)c->colOf.p); ++c->launches; }
   if ((rc = wb_exclusive_scan_u32(c, count, start, ncell + 1, nullptr)))
     return rc;
-  { cellScatterKernel<<<blocks, 256, 0, c->stream>>>(nd, nx, ny, colOf, rank, start, sz, slots); ++c->launches; }
+  { cellScatterKernel<<<blocks, 256, 0, c->stream>>>(nd, nx, ny, colOf, rank, start, sz, slots, err); ++c->launches; }
   { columnKernel<<<(unsigned)((ncell + kColumnWarps - 1) / kColumnWarps), 32 * kColumnWarps, 0, c->stream>>>(
-        ncell, start, slots, sx, sy, sz, stray, gpt, cellRec, count, dBig); ++c->launches; }
+        ncell, start, slots, sx, sy, sz, stray, gpt, cellRec, count, dBig, err); ++c->launches; }
   { bigColumnKernel<<<(unsigned)c->sm_count, 512, 0, c->stream>>>(count, dBig, start, slots, sx, sy, sz, stray, gpt, cellRec,
                                                                   dBig + 1); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
-  unsigned long long ns = 0;
-  int ext[6];
-  uint32_t bigs[2];
-  WB_CUDA(c, cudaMemcpyAsync(&ns, dStray, 8, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaMemcpyAsync(ext, dExt, 24, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaMemcpyAsync(bigs, dBig, 8, cudaMemcpyDefault, c->stream));
+  unsigned char back[WB_SMALL_LOOKBACK + 4];   // the scratch block's words, in one copy
+  WB_CUDA(c, cudaMemcpyAsync(back, c->small.p, sizeof back, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  unsigned long long ns;
+  int ext[6], gaveUp;
+  uint32_t bigs[2];
+  memcpy(&ns, back + 256, 8);
+  memcpy(ext, back + 512, 24);
+  memcpy(bigs, back + 640, 8);
+  memcpy(&gaveUp, back + WB_SMALL_LOOKBACK, 4);
+  if (gaveUp)
+    return wb_lookback_failed(c, "column grid");
   if (bigs[1])
   {
     // a column of more than kBigColumnMax points (an outlier far from the rest
@@ -806,7 +818,11 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
     if ((rc = wb_radix_sort_pairs(c, key, val, (uint64_t *)c->gKey1.p, (uint32_t *)c->gVal1.p, nd, 0, 32 + bits, ~0ull, true)))
       return rc;
     { cellFillKernel<<<(unsigned)((ncell * 32 + 255) / 256), 256, 0, c->stream>>>(ncell, start, val, sx, sy, sz, stray, gpt,
-                                                                                 cellRec); ++c->launches; }
+                                                                                 cellRec, err); ++c->launches; }
+    WB_CUDA(c, cudaMemcpyAsync(&gaveUp, err, 4, cudaMemcpyDefault, c->stream));
+    WB_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (gaveUp)
+      return wb_lookback_failed(c, "column grid");
   }
   int snx = (nx + WB_SUPER - 1) / WB_SUPER, sny = (ny + WB_SUPER - 1) / WB_SUPER;
   c->grid.snx = snx;
@@ -848,11 +864,16 @@ int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count)
   // at most nd / 32 + ncell groups
   if ((rc = wb_ensure(c, c->colGroups, (nd / 32 + ncell + 1) * 8 + 64)))
     return rc;
-  { groupFillKernel<<<blocks, 256, 0, c->stream>>>(ncell, (const int4 *)c->cellRec.p, gfirst, (uint2 *)c->colGroups.p); ++c->launches; }
+  { groupFillKernel<<<blocks, 256, 0, c->stream>>>(ncell, (const int4 *)c->cellRec.p, gfirst, (uint2 *)c->colGroups.p,
+                                                    wb_lookback_err(c)); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
   uint32_t ngroups = 0;
+  int gaveUp = 0;
   WB_CUDA(c, cudaMemcpyAsync(&ngroups, gTot, 4, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaMemcpyAsync(&gaveUp, wb_lookback_err(c), 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (gaveUp)
+    return wb_lookback_failed(c, "wb_classify");
   *groups = (const uint2 *)c->colGroups.p;
   *count = ngroups;
   return 0;

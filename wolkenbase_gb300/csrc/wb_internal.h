@@ -206,6 +206,7 @@ int wb_radix_sort_pairs(wb_ctx *c, uint64_t *&keys, uint32_t *&vals, uint64_t *k
 int wb_small(wb_ctx *c);
 int wb_host_stage(wb_ctx *c, size_t bytes);   /* grows c->hostStage */
 int *wb_lookback_err(wb_ctx *c);
+int wb_lookback_failed(wb_ctx *c, const char *who);   /* clears the word; WB_ETIMEDOUT */
 int wb_lookback_words(wb_ctx *c, uint64_t words, unsigned **counter, unsigned long long **status);
 
 /* stages */

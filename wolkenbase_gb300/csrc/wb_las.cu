@@ -99,8 +99,10 @@ __global__ void classKeysKernel(const uint8_t *__restrict__ rec, uint64_t n, uin
  * of the widest size the stride and both bases allow. */
 template <typename Word>
 __global__ void gatherRecordsKernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, uint64_t n,
-                                    uint32_t stride, const uint32_t *__restrict__ perm)
+                                    uint32_t stride, const uint32_t *__restrict__ perm, const int *__restrict__ err)
 {
+  if (*err)
+    return;   // perm was not written
   const uint32_t words = stride / (uint32_t)sizeof(Word);
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
   {
@@ -148,8 +150,10 @@ __global__ void __launch_bounds__(kPartThreads) partCount(const uint8_t *__restr
 __global__ void __launch_bounds__(kPartThreads) partScatter(const uint8_t *__restrict__ rec, uint64_t n,
                                                             uint32_t stride, int format, uint32_t numTiles,
                                                             const uint32_t *__restrict__ offs,
-                                                            uint8_t *__restrict__ out)
+                                                            uint8_t *__restrict__ out, const int *__restrict__ err)
 {
+  if (*err)
+    return;   // offs was not written
   constexpr int W = kPartThreads / 32;
   __shared__ uint32_t wcount[W][256];
   __shared__ uint32_t localStart[256], globalStart[256];
@@ -396,17 +400,22 @@ int wb_las_split_by_class(wb_ctx *c, const void *records, uint64_t n, uint32_t s
     if ((rc = wb_exclusive_scan_u32(c, (const uint32_t *)cnt.b.p, (uint32_t *)off.b.p, numTiles * 256, nullptr)))
       return rc;
     { partScatter<<<(unsigned)numTiles, kPartThreads, 0, c->stream>>>(din, n, stride, point_format, (uint32_t)numTiles,
-                                                                     (const uint32_t *)off.b.p, dout); ++c->launches; }
+                                                                     (const uint32_t *)off.b.p, dout, wb_lookback_err(c)); ++c->launches; }
     uint64_t h[256];
+    int gaveUp = 0;
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(h, hist.b.p, sizeof h, cudaMemcpyDefault, c->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(&gaveUp, wb_lookback_err(c), 4, cudaMemcpyDefault, c->stream);
     if (e == cudaSuccess && !on_device)
       e = cudaMemcpyAsync(out, dout, n * stride, cudaMemcpyDefault, c->stream);
     if (e == cudaSuccess)
       e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess)
       return wb_fail(c, WB_ECUDA, std::string("wb_las_split_by_class: ") + cudaGetErrorString(e));
+    if (gaveUp)
+      return wb_lookback_failed(c, "wb_las_split_by_class");
     for (int k = 0; k < 256; k++)
       offsets[k + 1] = offsets[k] + h[k];
     return 0;
@@ -422,24 +431,30 @@ int wb_las_split_by_class(wb_ctx *c, const void *records, uint64_t n, uint32_t s
   // one stable pass of the 8-bit digit: records keep their order within a class
   if ((rc = wb_radix_sort_pairs(c, keys, idx, (uint64_t *)c->key1.p, (uint32_t *)c->idx1.p, n, 0, 8)))
     return rc;
+  const int *err = wb_lookback_err(c);
   if (stride % 16 == 0 && ((uintptr_t)din % 16 == 0) && ((uintptr_t)dout % 16 == 0))
-    { gatherRecordsKernel<uint4><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx); ++c->launches; }
+    { gatherRecordsKernel<uint4><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx, err); ++c->launches; }
   else if (stride % 8 == 0 && ((uintptr_t)din % 8 == 0) && ((uintptr_t)dout % 8 == 0))
-    { gatherRecordsKernel<uint2><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx); ++c->launches; }
+    { gatherRecordsKernel<uint2><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx, err); ++c->launches; }
   else if (stride % 4 == 0 && ((uintptr_t)din % 4 == 0) && ((uintptr_t)dout % 4 == 0))
-    { gatherRecordsKernel<uint32_t><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx); ++c->launches; }
+    { gatherRecordsKernel<uint32_t><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx, err); ++c->launches; }
   else
-    { gatherRecordsKernel<uint8_t><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx); ++c->launches; }
+    { gatherRecordsKernel<uint8_t><<<gridOf(c, n), 256, 0, c->stream>>>(din, dout, n, stride, idx, err); ++c->launches; }
   uint64_t h[256];
+  int gaveUp = 0;
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(h, hist.b.p, sizeof h, cudaMemcpyDefault, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&gaveUp, err, 4, cudaMemcpyDefault, c->stream);
   if (e == cudaSuccess && !on_device)
     e = cudaMemcpyAsync(out, dout, n * stride, cudaMemcpyDefault, c->stream);
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess)
     return wb_fail(c, WB_ECUDA, std::string("wb_las_split_by_class: ") + cudaGetErrorString(e));
+  if (gaveUp)
+    return wb_lookback_failed(c, "wb_las_split_by_class");
   for (int k = 0; k < 256; k++)
     offsets[k + 1] = offsets[k] + h[k];
   return 0;

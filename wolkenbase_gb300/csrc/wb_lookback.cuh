@@ -3,9 +3,12 @@
  *
  * Blocks take their tile numbers from a counter, so the tiles before a running
  * one are running or finished, and each publishes its own sum before it waits
- * for anyone.  A wait is bounded all the same: after kLookbackSpins polls the
- * block sets *err and gives up (its caller returns without writing, and the
- * host answers WB_ETIMEDOUT at its next look at *err).
+ * for anyone.  A wait is bounded all the same: after kLookbackSpins polls, or
+ * when another block gave up, the block sets *err and gives up: its caller
+ * returns without writing.  What it would have written then holds whatever was
+ * there before, so every kernel that takes an address from it returns when *err
+ * is set, and the host reads *err with the stage's own read-back, clears it and
+ * answers WB_ETIMEDOUT.
  *
  * A status word holds a tag (which pass of a kernel sequence it belongs to, 0
  * never), whether the value is the tile's own sum or includes everything
@@ -16,7 +19,10 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
-constexpr int kLookbackSpins = 1 << 20;
+#ifndef WB_LOOKBACK_SPINS
+#define WB_LOOKBACK_SPINS (1 << 20)   /* about a second */
+#endif
+constexpr int kLookbackSpins = WB_LOOKBACK_SPINS;
 constexpr int kLookbackValueBits = 48;   /* tag 15 bits, inclusive 1 bit, value 48 bits */
 
 __device__ __forceinline__ unsigned long long lookbackWord(unsigned tag, bool inclusive, unsigned long long v)
@@ -34,6 +40,13 @@ __device__ __forceinline__ unsigned long long lookbackGet(const unsigned long lo
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
+}
+
+/* Whether poll number `spins` of a wait is its last: the limit, or another
+ * block's error, looked at every 64 polls so that later blocks need not wait. */
+__device__ __forceinline__ bool lookbackGivesUp(int spins, const int *err)
+{
+  return spins > kLookbackSpins || (spins % 64 == 0 && *(const volatile int *)err);
 }
 
 /* Status words of the radix passes, one per digit and tile: 32 bits while the
@@ -98,7 +111,7 @@ __device__ __forceinline__ bool lookbackColumn(const Word *status, uint64_t stri
     if (end)
       return true;
     t -= step;
-    if (t >= 0 && step < WINDOW && ++spins > kLookbackSpins)
+    if (t >= 0 && step < WINDOW && lookbackGivesUp(++spins, err))
     {
       *err = 1;
       return false;
@@ -143,7 +156,7 @@ __device__ __forceinline__ bool lookbackWarp(const unsigned long long *status, u
     if (end)
       return true;
     t -= n;
-    if (n < 32 && ++spins > kLookbackSpins)
+    if (n < 32 && __any_sync(0xffffffffu, lookbackGivesUp(++spins, err)))
     {
       if (lane == 0)
         *err = 1;

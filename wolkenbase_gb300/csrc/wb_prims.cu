@@ -281,6 +281,13 @@ int *wb_lookback_err(wb_ctx *c)
   return (int *)((char *)c->small.p + WB_SMALL_LOOKBACK);
 }
 
+/* The answer of a call whose look-back gave up; the next call starts afresh. */
+int wb_lookback_failed(wb_ctx *c, const char *who)
+{
+  cudaMemsetAsync(wb_lookback_err(c), 0, 4, c->stream);
+  return wb_fail(c, WB_ETIMEDOUT, std::string(who) + ": a look-back wait gave up");
+}
+
 /* Counter and status words of a look-back sequence of `words` words, cleared. */
 int wb_lookback_words(wb_ctx *c, uint64_t words, unsigned **counter, unsigned long long **status)
 {

@@ -414,12 +414,6 @@ int shapeArgs(wb_ctx *c, const wb_shape *sh, QArgs &a, const char *who)
   return 0;
 }
 
-int lookbackFailed(wb_ctx *c, const char *who)
-{
-  cudaMemsetAsync(wb_lookback_err(c), 0, 4, c->stream);
-  return wb_fail(c, WB_ETIMEDOUT, std::string(who) + ": a look-back wait gave up");
-}
-
 /* Lists the leaves that meet the shape: *list on the device, their number at
  * *nList; behind the list, room for two more words a leaf and one. */
 int listLeaves(wb_ctx *c, const QArgs &a, uint32_t **list, uint32_t **nList)
@@ -460,7 +454,7 @@ extern "C" int wb_find_blocks(wb_ctx *c, const wb_shape *sh, int64_t *leaves, ui
   WB_CUDA(c, cudaMemcpyAsync(&err, wb_lookback_err(c), 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
   if (err)
-    return lookbackFailed(c, "wb_find_blocks");
+    return wb_lookback_failed(c, "wb_find_blocks");
   if (count)
     *count = total;
   if (total > capacity)
@@ -498,7 +492,7 @@ extern "C" int wb_points_in(wb_ctx *c, const wb_shape *sh, int sorted, uint32_t 
   WB_CUDA(c, cudaGetLastError());
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
   if (ans->failed)
-    return lookbackFailed(c, "wb_points_in");
+    return wb_lookback_failed(c, "wb_points_in");
   auto tooMany = [&](uint64_t total) {
     return wb_fail(c, WB_EINVAL, "wb_points_in: " + std::to_string(total) + " points, capacity " +
                                      std::to_string(capacity));
@@ -527,8 +521,15 @@ extern "C" int wb_points_in(wb_ctx *c, const wb_shape *sh, int sorted, uint32_t 
   if ((rc = wb_exclusive_scan_u32(c, cnt, ex, n, dTot)))
     return rc;
   uint32_t total = 0;
+  int err = 0;
+  auto failed = [&]() -> int {
+    WB_CUDA(c, cudaMemcpyAsync(&err, wb_lookback_err(c), 4, cudaMemcpyDefault, c->stream));
+    WB_CUDA(c, cudaStreamSynchronize(c->stream));
+    return err ? wb_lookback_failed(c, "wb_points_in") : 0;
+  };
   WB_CUDA(c, cudaMemcpyAsync(&total, dTot, 4, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  if ((rc = failed()))
+    return rc;
   if (count)
     *count = total;
   if (total > capacity)
@@ -560,6 +561,5 @@ extern "C" int wb_points_in(wb_ctx *c, const wb_shape *sh, int sorted, uint32_t 
     return rc;
   WB_CUDA(c, cudaGetLastError());
   WB_CUDA(c, cudaMemcpyAsync(records, vals, (size_t)total * 4, cudaMemcpyDefault, c->stream));
-  WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  return 0;
+  return failed();
 }

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cmath>
+#include <cstring>
 #include "wb_internal.h"
 #include "wb_device.cuh"
 #include "wb_warpsort.cuh"
@@ -208,8 +209,10 @@ __global__ void hugeKeysKernel(uint32_t nh, const uint32_t *__restrict__ hugeLis
 
 __global__ void hugeBackKernel(uint32_t nh, const uint32_t *__restrict__ hugeList, const uint32_t *__restrict__ tileStart,
                                const uint64_t *__restrict__ pre, const uint64_t *__restrict__ keys,
-                               uint32_t *__restrict__ tilePts)
+                               uint32_t *__restrict__ tilePts, const int *__restrict__ err)
 {
+  if (*err)
+    return;   // keys were not written
   const uint64_t total = pre[nh];
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x)
   {
@@ -257,13 +260,14 @@ __global__ void __launch_bounds__(32 * kTileWarps) gridFillWarp(TileArgs a, Grid
                                                                 uint32_t *__restrict__ tileN,
                                                                 uint32_t *__restrict__ tilePts, int32_t *__restrict__ owner,
                                                                 uint32_t *__restrict__ bigList, uint32_t *__restrict__ bigCount,
-                                                                const TileFrame *__restrict__ frames)
+                                                                const TileFrame *__restrict__ frames,
+                                                                const int *__restrict__ err)
 {
   __shared__ __align__(16) uint32_t buf[kTileWarps][kWarpFill];
   static_assert(kWarpFill == 1024, "the size wb_warp_sort_1024 sorts");
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint64_t k = (uint64_t)blockIdx.x * kTileWarps + w;
-  if (k >= a.T)
+  if (k >= a.T || *err)   // err: tileStart was not written, nothing is listed for gridFill
     return;
   const uint32_t base = tileStart[k];
   if (tileStart[k + 1] == base)
@@ -1462,9 +1466,12 @@ static int sortHugeTiles(wb_ctx *c, uint32_t nh, const uint32_t *tileStart)
   if ((rc = wb_radix_sort_pairs(c, keys, vals, (uint64_t *)c->key1.p, (uint32_t *)c->idx1.p, total, 0, 32 + bits, varying)))
     return rc;
   { hugeBackKernel<<<g, 256, 0, c->stream>>>(nh, (const uint32_t *)c->tileHuge.p, tileStart, (const uint64_t *)c->hugePre.p,
-                                             keys, (uint32_t *)c->tilePts.p); ++c->launches; }
+                                             keys, (uint32_t *)c->tilePts.p, wb_lookback_err(c)); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
-  return 0;
+  int gaveUp = 0;
+  WB_CUDA(c, cudaMemcpyAsync(&gaveUp, wb_lookback_err(c), 4, cudaMemcpyDefault, c->stream));
+  WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  return gaveUp ? wb_lookback_failed(c, "wb_scan_tiles") : 0;
 }
 
 /* Per tile, over its points (x, y from the tile centre, z as decoded): the
@@ -1585,18 +1592,25 @@ int wb_scan_impl(wb_ctx *c, const wb_params *p)
   // huge-tile count and big-tile count (bytes 384..395 of the scratch block)
   WB_CUDA(c, cudaMemsetAsync(dOvf, 0, 16, c->stream));
   { gridFillWarp<<<blocks, 32 * kTileWarps, 0, c->stream>>>(a, gd, tileStart, tileN, (uint32_t *)c->tilePts.p, owner,
-                                                           (uint32_t *)c->tileNg.p, dBig, frames); ++c->launches; }
+                                                           (uint32_t *)c->tileNg.p, dBig, frames, wb_lookback_err(c)); ++c->launches; }
   if ((rc = wb_ensure(c, c->tileHuge, T * 4 + 64)))
     return rc;
   { gridFill<<<(unsigned)c->sm_count, kFillThreads, 0, c->stream>>>(a, gd, tileStart, tileN, (uint32_t *)c->tilePts.p,
                                                                    owner, dOvf, (const uint32_t *)c->tileNg.p, dBig,
                                                                    (uint32_t *)c->tileHuge.p, frames); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
-  int nHuge = 0;
-  WB_CUDA(c, cudaMemcpyAsync(&nHuge, dOvf, 4, cudaMemcpyDefault, c->stream));
+  unsigned char back[WB_SMALL_LOOKBACK + 4];   // the scratch block's words, in one copy
+  WB_CUDA(c, cudaMemcpyAsync(back, c->small.p, sizeof back, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (nHuge && (rc = sortHugeTiles(c, (uint32_t)nHuge, tileStart)))
+  int nHuge, gaveUp;
+  memcpy(&nHuge, back + 384, 4);
+  memcpy(&gaveUp, back + WB_SMALL_LOOKBACK, 4);
+  rc = gaveUp ? wb_lookback_failed(c, "wb_scan_tiles") : (nHuge ? sortHugeTiles(c, (uint32_t)nHuge, tileStart) : 0);
+  if (rc)
+  {
+    c->stage = 1;   // the octree stands, an earlier scan's tiles do not
     return rc;
+  }
   wb_mark(c, "tile_gather");
   ScanArgs s;
   s.t = a;
