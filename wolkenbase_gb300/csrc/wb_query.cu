@@ -465,7 +465,14 @@ extern "C" int wb_find_blocks(wb_ctx *c, const wb_shape *sh, int64_t *leaves, ui
   std::vector<uint32_t> l(total);
   WB_CUDA(c, cudaMemcpyAsync(l.data(), list, (size_t)total * 4, cudaMemcpyDefault, c->stream));
   WB_CUDA(c, cudaStreamSynchronize(c->stream));
-  std::copy(l.begin(), l.end(), leaves);
+  if (wb_device_accessible(leaves))
+  {
+    const std::vector<int64_t> wide(l.begin(), l.end());
+    WB_CUDA(c, cudaMemcpyAsync(leaves, wide.data(), (size_t)total * 8, cudaMemcpyDefault, c->stream));
+    WB_CUDA(c, cudaStreamSynchronize(c->stream));
+  }
+  else
+    std::copy(l.begin(), l.end(), leaves);
   return 0;
 }
 
