@@ -1715,21 +1715,63 @@ __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const Ba
 }
 
 /* The ambiguous points (exactly; in the precision mode again in FP32, by the bins'
- * extremes), a block each: they are a dozen of a cloud of millions, so the pass
- * takes as long as the heaviest one's walk, mostly chains of FP64 directions.
- * Eight warps that share its columns: 0.33 ms for 5M points and 0.40 for 50M (one
- * warp a point: 0.55 and 0.95; four: 0.33 and 0.50). */
+ * extremes).  Mostly they are a dozen of a cloud of millions, and the pass takes as
+ * long as the heaviest one's walk, mostly chains of FP64 directions: a block of W
+ * warps each, which share its columns.  W = 8: 0.33 ms for 5M points and 0.40 for
+ * 50M (one warp a point: 0.55 and 0.95; four: 0.33 and 0.50).
+ * A cloud that FP32 cannot tell apart at all (a negative scale, a step below
+ * four ulps) lists every point.  From kExactRounds points a resident block on
+ * (3648 on 152 SMs) the barriers and the shared walk's later stop cost more than
+ * the sharing gives, and each warp takes points of its own: with blocks 1.03 ms
+ * for 2000 points, 3.35 for 4000, 28.1 for 16,000, 7.54 s for a million; with warps
+ * 1.20, 3.42, 27.1 and 7.04. */
+constexpr int kExactRounds = 12;
 template <int W>
 __global__ void __launch_bounds__(32 * W) batchExact(BatchHdr *h, const BatchOut *o)
 {
-  __shared__ uint32_t bmin[kBins], bmax[kBins];
-  __shared__ ClsArgs a;
+  __shared__ uint32_t bmin[W][kBins], bmax[W][kBins];
+  __shared__ ClsArgs sa[W];
   __shared__ unsigned long long itemS;
   const int lane = threadIdx.x & 31;
   const int k = h->k;
   const uint64_t *start = o->startAmb;
   const uint64_t total = start[k];
   uint64_t lo = 1, hi = 0;
+  // copies the job's arguments when item g is the first of another job's
+  auto jobOf = [&](uint64_t g, ClsArgs &a, int t, int threads) -> bool {
+    if (g >= lo && g < hi)
+      return false;
+    const int q = batchJob(start, k, g);
+    lo = start[q];
+    hi = start[q + 1];
+    const uint32_t *src = (const uint32_t *)&h->jobs[q];
+    for (int i = t; i < (int)(sizeof(ClsArgs) / 4); i += threads)
+      ((uint32_t *)&a)[i] = src[i];
+    return true;
+  };
+  if (total > (uint64_t)kExactRounds * gridDim.x)
+  {
+    const int w = threadIdx.x >> 5;
+    const ClsArgs &a = sa[w];
+    for (;;)
+    {
+      unsigned long long g = 0;
+      if (lane == 0)
+        g = atomicAdd(&h->next[2], 1ull);
+      g = __shfl_sync(0xffffffffu, g, 0);
+      if (g >= total)
+        break;
+      __syncwarp();   // the point before is done with
+      if (jobOf(g, sa[w], lane, 32))
+        __syncwarp();
+      const uint64_t j = a.ambList[g - lo];
+      if (a.fp32Only)
+        classifyPoint<false>(a, j, lane, bmin[w], bmax[w]);
+      else
+        classifyPoint<true>(a, j, lane, bmin[w], bmax[w]);
+    }
+    return;
+  }
   for (;;)
   {
     __syncthreads();   // the point before is done with
@@ -1739,21 +1781,14 @@ __global__ void __launch_bounds__(32 * W) batchExact(BatchHdr *h, const BatchOut
     const uint64_t g = itemS;
     if (g >= total)
       break;
-    if (g < lo || g >= hi)
-    {
-      const int q = batchJob(start, k, g);
-      lo = start[q];
-      hi = start[q + 1];
-      const uint32_t *src = (const uint32_t *)&h->jobs[q];
-      for (int i = threadIdx.x; i < (int)(sizeof(ClsArgs) / 4); i += 32 * W)
-        ((uint32_t *)&a)[i] = src[i];
+    if (jobOf(g, sa[0], threadIdx.x, 32 * W))
       __syncthreads();
-    }
+    const ClsArgs &a = sa[0];
     const uint64_t j = a.ambList[g - lo];
     if (a.fp32Only)
-      classifyPoint<false, W>(a, j, lane, bmin, bmax);
+      classifyPoint<false, W>(a, j, lane, bmin[0], bmax[0]);
     else
-      classifyPoint<true, W>(a, j, lane, bmin, bmax);
+      classifyPoint<true, W>(a, j, lane, bmin[0], bmax[0]);
   }
 }
 
