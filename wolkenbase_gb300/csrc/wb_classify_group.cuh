@@ -325,12 +325,15 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
   if (done)
     mz = -INFINITY;
 
-  // the envelope of the lanes still undecided; the apex is raised by more than
-  // its rounding
+  // the envelope of the lanes still undecided.  The apex, and a box's height below
+  // it, are rounded eight times in all by 6e-8 of |czp| (the centre, the two
+  // factors, their products and sums) and four times by 6e-8 of the lane's height in
+  // the group: the apex is raised by 6e-7 of both, so that the envelope holds every
+  // lane's hyperboloid however far its centre lies from it (|czp| / por below 1e5)
   float apex, pK;
   int smaxG;
   auto envelope = [&]() {
-    apex = orderedFloat(__reduce_max_sync(kAll, orderedInt(done ? -INFINITY : __fmaf_rn(mz, kz, czp) + 2.5e-7f * __fmaf_rn(mz, kz, fabsf(czp)))));
+    apex = orderedFloat(__reduce_max_sync(kAll, orderedInt(done ? -INFINITY : __fmaf_rn(mz, kz, czp) + 6e-7f * __fmaf_rn(mz, kz, fabsf(czp)))));
     // members have zd^2 - r2 >= por^2; 1.0004 zd^2 - r2 >= pK allows for rounding
     pK = __int_as_float(__reduce_min_sync(kAll, done ? 0x7f800000 : __float_as_int(por2))) * 0.9998f - a.gTiny;
     smaxG = __reduce_max_sync(kAll, done ? 0 : smaxL);
