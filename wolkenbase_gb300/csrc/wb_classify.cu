@@ -224,6 +224,14 @@ __device__ __noinline__ bool memberExact(const ClsArgs &a, const HypExact &h, ui
   return all || in;
 }
 
+/* How far zd = dz + czp may be off in FP32, a height difference and a centre
+ * offset rounded three times each by 6e-8 of their size: it tells where both are
+ * large and zd is small, with a thickness far above the polar radius. */
+__device__ __forceinline__ float zdError(float dz, float czp)
+{
+  return 4e-7f * (fabsf(dz) + fabsf(czp));
+}
+
 /* Can any point of a box (b: bounds; r1: lowest z and flags, the column
  * layout) be inside?  FP32 with generous slack.  Record differences are exact
  * in 32 bits: the host checks that the cloud's integer extent fits.  A box
@@ -242,7 +250,8 @@ __device__ __forceinline__ bool boxMeets(const Hyp &h, const int4 &b, const int4
     return true;
   float xl = (float)(b.x - h.qx) * h.sx, xh = (float)(b.z - h.qx) * h.sx;
   float yl = (float)(b.y - h.qy) * h.sy, yh = (float)(b.w - h.qy) * h.sy;
-  float zd = (float)(h.qz - zmin) * h.sz + h.czp;
+  const float dz = (float)(h.qz - zmin) * h.sz;
+  float zd = dz + h.czp + zdError(dz, h.czp);
   float dx = xl > 0 ? xl : (xh < 0 ? -xh : 0.f);
   float dy = yl > 0 ? yl : (yh < 0 ? -yh : 0.f);
   float r2 = h.s2 * (dx * dx + dy * dy);
@@ -517,7 +526,8 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
           float zd = dzm + h.czp;
           float r2 = h.s2 * (dx * dx + dy * dy);
           float f = zd * zd - r2 - h.por2f;
-          float tol = 1e-5f * (zd * zd + r2 + h.por2f) + 1e-12f;
+          const float ez = zdError(dzm, h.czp);
+          float tol = 1e-5f * (zd * zd + r2 + h.por2f) + ez * (2 * fabsf(zd) + ez) + 1e-12f;
           float ztol = 1e-5f * (fabsf(dzm) + fabsf(h.czp)) + 1e-12f;
           if (zd > ztol && f > tol)
             in = true;
@@ -1011,7 +1021,8 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
     const float czp = ps.czp, por2 = ps.por2f;
     // the envelope's values live in shared memory (one copy per warp)
     auto envelope = [&]() {
-      float ap = !done ? (float)(me.z - oz) * sz + czp : -INFINITY;
+      const float dz = (float)(me.z - oz) * sz;
+      float ap = !done ? dz + czp + zdError(dz, czp) : -INFINITY;
       float pm = !done ? por2 : INFINITY;
       int km = !done ? sm.kmax[lane] : 0;
       int sg = !done ? sm.smax[lane] : 0;
@@ -1048,7 +1059,8 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
       const float apex = sm.apex, por2min = sm.por2min;
       float dx = (float)max(0, max(b.x - cb0.z, cb0.x - b.z)) * sx;
       float dy = (float)max(0, max(b.y - cb0.w, cb0.y - b.w)) * sy;
-      float zd = apex - (float)(r1.x - oz) * sz;
+      const float dz = (float)(r1.x - oz) * sz;
+      float zd = apex - dz + zdError(dz, 0.f);
       float r2 = s2 * (dx * dx + dy * dy);
       float mag = zd * zd + r2 + por2min;
       if (zd < -1e-4f * (fabsf(zd) + 1e-3f))
@@ -1143,7 +1155,8 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
         const float zd = dzm + czp;
         const float r2 = s2 * __fmaf_rn(dx, dx, dy * dy);
         const float f = __fmaf_rn(zd, zd, -r2) - por2;
-        const float tol = __fmaf_rn(1e-5f, __fmaf_rn(zd, zd, r2) + por2, 1e-12f);
+        const float ez = zdError(dzm, czp);
+        const float tol = __fmaf_rn(1e-5f, __fmaf_rn(zd, zd, r2) + por2, __fmaf_rn(ez, __fmaf_rn(2.f, fabsf(zd), ez), 1e-12f));
         const float ztol = __fmaf_rn(1e-5f, fabsf(dzm) + fabsf(czp), 1e-12f);
         const bool sureIn = zd > ztol && f > tol, sureOut = zd < -ztol || f < -tol;
         int m = sureIn ? 1 : 0;
@@ -1177,7 +1190,8 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
             const float apex = sm.apex, por2min = sm.por2min;
             float ex = (float)max(0, max(q.x - cb0.z, cb0.x - q.x)) * sx;
             float ey = (float)max(0, max(q.y - cb0.w, cb0.y - q.y)) * sy;
-            float zd = apex - (float)(q.z - oz) * sz;
+            const float dz = (float)(q.z - oz) * sz;
+            float zd = apex - dz + zdError(dz, 0.f);
             float r2 = s2 * (ex * ex + ey * ey);
             float mag = zd * zd + r2 + por2min;
             keep = zd >= -1e-4f * (fabsf(zd) + 1e-3f) && zd * zd - r2 - por2min >= -(1e-4f * mag + 1e-9f);
