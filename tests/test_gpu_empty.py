@@ -1,5 +1,6 @@
 """A cloud without records between two runs of another: it reports nothing, and
-leaves nothing of itself or of the first to the second."""
+leaves nothing of itself or of the first to the second.  So does one that is a
+context's first."""
 import numpy as np
 import pytest
 
@@ -30,3 +31,19 @@ def test_empty_cloud_between(cuda_lib_path, shape):
         assert np.array_equal(clf.tiles(), tiles)
     finally:
         clf.close()
+
+
+def test_empty_cloud_first(cuda_lib_path):
+    import wolkenbase_gb300 as wb
+    from wolkenbase_gb300 import synth
+    cloud = synth.density_tile(6000, 91)
+    empty = synth.Cloud(np.zeros((0, 3), np.int32), cloud.scale, cloud.offset, 1.0, cloud.minc, cloud.maxc)
+    clf, other = wb.Classifier(0), wb.Classifier(0)
+    try:
+        assert clf.classify_cloud(empty).size == 0
+        assert clf.tiles().size > 0 and not clf.tiles()["n_points"].any()
+        assert np.array_equal(clf.classify_cloud(cloud), other.classify_cloud(cloud))
+        assert np.array_equal(clf.tiles(), other.tiles())
+    finally:
+        clf.close()
+        other.close()

@@ -112,10 +112,11 @@ __device__ TileFrame tileFrame(const TileArgs &a, const GridDev &gd, uint64_t k)
   f.r2lo = r2 * (1 - 2e-5f);
   f.r2hi = r2 * (1 + 2e-5f);
   double r = a.rad * (1 + 1e-9) + 1e-9;
+  // (a cloud without points has no columns: nx = ny = 0, and the ranges are 0 to -1)
   f.i0 = max(0, min(gd.nx - 1, (int)floor((f.cx - r - gd.x0) / gd.cell)));
-  f.i1 = max(0, min(gd.nx - 1, (int)floor((f.cx + r - gd.x0) / gd.cell)));
+  f.i1 = min(gd.nx - 1, max(0, (int)floor((f.cx + r - gd.x0) / gd.cell)));
   f.j0 = max(0, min(gd.ny - 1, (int)floor((f.cy - r - gd.y0) / gd.cell)));
-  f.j1 = max(0, min(gd.ny - 1, (int)floor((f.cy + r - gd.y0) / gd.cell)));
+  f.j1 = min(gd.ny - 1, max(0, (int)floor((f.cy + r - gd.y0) / gd.cell)));
   return f;
 }
 
