@@ -2415,7 +2415,6 @@ int wb_autotune_jobs(WbBatch *b, const WbTuneJob *jobs, int k, cudaStream_t s, i
     }
   }
   regrid(bestGp);
-  const int probeChunk = bestChunk;
   for (int sh = 0; sh < WB_N_SHAPES; sh++)
   {
     if (sh == kProbe[0] || sh == kProbe[1])
@@ -2428,7 +2427,6 @@ int wb_autotune_jobs(WbBatch *b, const WbTuneJob *jobs, int k, cudaStream_t s, i
       bestChunk = sh < 3 ? 1 : 4;
     }
   }
-  (void)probeChunk;
   static const int kChunk[] = {1, 2, 4, 16};
   const int c0 = bestChunk;
   for (int ch : kChunk)
