@@ -1552,7 +1552,10 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
   a.sinT = tab + 511;
   a.cosT = tab + 1023;
   a.label = (uint8_t *)c->label.p;
-  if ((rc = wb_point_groups(c, &a.groupsTaken, &a.maxGroups)))
+  a.groupsTaken = nullptr;
+  a.maxGroups = 0;
+  // (calls that want margins run over column groups)
+  if ((!c->marginDst || !nd) && (rc = wb_point_groups(c, &a.groupsTaken, &a.maxGroups)))
     return rc;
   a.gx0 = c->grid.x0;
   a.gy0 = c->grid.y0;

@@ -833,7 +833,8 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
   { superKernel<<<(unsigned)std::min<uint64_t>((nsup + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
         nx, ny, snx, sny, (const int4 *)c->cellRec.p, (int4 *)c->superRec.p); ++c->launches; }
   WB_CUDA(c, cudaGetLastError());
-  c->grid.grouped = false;
+  c->grid.grouped = c->grid.colGrouped = false;
+  c->grid.nColGroups = 0;
   c->grid.nStray = ns;
   for (int k = 0; k < 3; k++)
   {
@@ -844,15 +845,16 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
 }
 
 /* The column groups of the margin pass (groups of consecutive points of a
- * column); synchronises. */
+ * column), formed once per grid when a classify first wants margins;
+ * synchronises then. */
 int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count)
 {
   const uint64_t ncell = c->grid.ncell, nd = c->nd;
   uint32_t *gTot = (uint32_t *)((char *)c->small.p + 640);
   int rc;
-  *groups = nullptr;
-  *count = 0;
-  if (!nd)
+  *groups = (const uint2 *)c->colGroups.p;
+  *count = c->grid.nColGroups;
+  if (c->grid.colGrouped || !nd)
     return 0;
   if ((rc = wb_ensure(c, c->groupCnt, (ncell + 1) * 8 + 64)))
     return rc;
@@ -875,7 +877,8 @@ int wb_column_groups(wb_ctx *c, const uint2 **groups, uint64_t *count)
   if (gaveUp)
     return wb_lookback_failed(c, "wb_classify");
   *groups = (const uint2 *)c->colGroups.p;
-  *count = ngroups;
+  *count = c->grid.nColGroups = ngroups;
+  c->grid.colGrouped = true;
   return 0;
 }
 

@@ -39,6 +39,8 @@ struct GridInfo
   /* super-cells: blocks of WB_SUPER x WB_SUPER columns with their own bounds */
   int snx = 0, sny = 0;
   bool grouped = false;             /* the point groups of this grid are formed */
+  bool colGrouped = false;          /* and the column groups */
+  uint64_t nColGroups = 0;
 };
 #define WB_SUPER 3
 /* a warp tests a super-cell's columns with one lane each */
