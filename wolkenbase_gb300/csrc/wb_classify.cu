@@ -135,6 +135,8 @@ struct ClsArgs
   float gInv, gTiny;      /* 1 / (slope * x record unit); 1e-12 m^2 in that unit squared */
   int snx, sny;
   const int4 *super;   /* super-cell records, the column layout */
+  const int4 *strayCol, *straySuper, *strayGrp;   /* where flags say so: the outside points' blocks (wb_ctx) */
+  double unitOff[3], perStep[3];   /* off * unit, 1 / (scale * unit) */
   double zmin;     /* lowest height a member can have */
   int exactInts;   /* decode strictly increasing and 32-bit record differences exact */
   int fp32Only;    /* precision mode: FP32 decisions stand, no exact re-run */
@@ -232,18 +234,13 @@ __device__ __forceinline__ float zdError(float dz, float czp)
   return 4e-7f * (fabsf(dz) + fabsf(czp));
 }
 
-/* Can any point of a box (b: bounds; r1: lowest z and flags, the column
- * layout) be inside?  FP32 with generous slack.  Record differences are exact
- * in 32 bits: the host checks that the cloud's integer extent fits.  A box
- * holding a point beside or above the root cube (flags) always can: that
- * point's block decides. */
-__device__ __forceinline__ bool boxMeets(const Hyp &h, const int4 &b, const int4 &r1)
+/* Can any point of a box (integer bounds, lowest z) be inside?  FP32 with
+ * generous slack.  Record differences are exact in 32 bits: the host checks that
+ * the cloud's integer extent fits. */
+__device__ __forceinline__ bool boxReached(const Hyp &h, const int4 &b, int32_t zmin)
 {
   if (b.x == INT32_MAX)
     return false;   // empty block
-  if (r1.w)
-    return true;
-  const int32_t zmin = r1.x;
   // the bound takes the box's low record integers as its low coordinates:
   // only for a decode that increases with the record integer
   if (!(h.sx > 0.f && h.sy > 0.f && h.sz > 0.f))
@@ -259,6 +256,15 @@ __device__ __forceinline__ bool boxMeets(const Hyp &h, const int4 &b, const int4
   if (zd < -1e-4f * (fabsf(zd) + 1e-3f))
     return false;
   return zd * zd - r2 - h.por2f >= -(1e-4f * mag + 1e-9f);
+}
+
+/* The same of a column or super-cell (bounds, record with lowest z and flags),
+ * also by the blocks of its points beside or above the root cube (flags, sr): such
+ * a point is a member when its whole block is inside, the top of its cube
+ * included, wherever the point is. */
+__device__ __forceinline__ bool boxMeets(const Hyp &h, const int4 &b, const int4 &r1, const int4 *sr)
+{
+  return boxReached(h, b, r1.x) || (r1.w && boxReached(h, sr[0], sr[1].x));
 }
 
 /* Column offset of ring cell m (0 <= m < 8k) at Chebyshev distance k. */
@@ -506,6 +512,9 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
     float dz = (h.czp - need + 1e-4f * (fabsf(h.czp) + need) + 1e-6f) / h.sz + 2.f;
     return dz > 2.1e9f ? INT32_MAX : (dz < -2.1e9f ? INT32_MIN : (int32_t)floorf(dz));
   };
+  // Whether the hyperboloid may reach the blocks of the outside points of the
+  // column being read, and may hold them as a whole (where the box tests apply).
+  bool blockMeets = true, blockHolds = false;
   // Whether candidate pt lies inside the hyperboloid, and its direction u.
   auto testPoint = [&](const int4 &pt, uint32_t &u) -> bool {
     bool in = false;
@@ -518,9 +527,6 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
       if (dxi != 0 || dyi != 0)
       {
         float dx = (float)dxi * h.sx, dy = (float)dyi * h.sy;
-        if (gp & kStray)
-          in = memberExact(a, exactHyp(a, h.j), gp, qx, qy, qz);
-        else
         {
           float dzm = (float)(h.qz - qz) * h.sz;
           float zd = dzm + h.czp;
@@ -529,7 +535,10 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
           const float ez = zdError(dzm, h.czp);
           float tol = 1e-5f * (zd * zd + r2 + h.por2f) + ez * (2 * fabsf(zd) + ez) + 1e-12f;
           float ztol = 1e-5f * (fabsf(dzm) + fabsf(h.czp)) + 1e-12f;
-          if (zd > ztol && f > tol)
+          if (gp & kStray)
+            // by its block: the exact test, where that may hold
+            in = blockMeets && (blockHolds || !(zd < -ztol || f < -tol)) && memberExact(a, exactHyp(a, h.j), gp, qx, qy, qz);
+          else if (zd > ztol && f > tol)
             in = true;
           else if (zd < -ztol || f < -tol)
             in = false;
@@ -606,6 +615,13 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
     const int4 box = a.col[2 * cc], r1 = a.col[2 * cc + 1];
     const uint32_t e = (uint32_t)r1.z;
     const int32_t zlim = colZlim(box, r1);
+    blockMeets = true;
+    blockHolds = false;
+    if (r1.w)
+    {
+      blockMeets = boxReached(h, a.strayCol[2 * cc], a.strayCol[2 * cc + 1].y);
+      blockHolds = boxReached(h, a.strayCol[2 * cc], a.strayCol[2 * cc + 1].x);
+    }
     for (uint32_t t0 = (uint32_t)r1.y; t0 < e; t0 += 32)
     {
       uint32_t t = t0 + lane;
@@ -706,7 +722,7 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
         {
           c = (uint64_t)jj * a.nx + i;
           cb = a.col[2 * c];
-          ok = boxMeets(h, cb, a.col[2 * c + 1]);
+          ok = boxMeets(h, cb, a.col[2 * c + 1], a.strayCol + 2 * c);
         }
       }
       unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -766,7 +782,7 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
         {
           const uint64_t sc = (uint64_t)SJ * a.snx + SI;
           sb = a.super[2 * sc];
-          ok = boxMeets(h, sb, a.super[2 * sc + 1]);
+          ok = boxMeets(h, sb, a.super[2 * sc + 1], a.straySuper + 2 * sc);
         }
       }
       unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -790,7 +806,7 @@ __device__ __forceinline__ void classifyPoint(const ClsArgs &a, uint64_t j, int 
           {
             c = (uint64_t)jj * a.nx + i;
             cb = a.col[2 * c];
-            cok = boxMeets(h, cb, a.col[2 * c + 1]);
+            cok = boxMeets(h, cb, a.col[2 * c + 1], a.strayCol + 2 * c);
           }
         }
         unsigned cm = __ballot_sync(0xffffffffu, cok);
@@ -1049,23 +1065,25 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
 #ifdef WB_CLASSIFY_STATS
     bool farField = false;   // lane tests beyond the near field (instrumented builds)
 #endif
-    // envelope test of a box {x0, y0, x1, y1} (r1: lowest z and flags, as in boxMeets)
-    auto envMeets = [&](const int4 &b, const int4 &r1) -> bool {
+    // envelope test of a box {x0, y0, x1, y1} with lowest point zmin
+    auto envReached = [&](const int4 &b, int32_t zmin) -> bool {
       if (b.x == INT32_MAX)
         return false;
-      if (r1.w)
-        return true;
       const int4 cb0 = sm.cbox;
       const float apex = sm.apex, por2min = sm.por2min;
       float dx = (float)max(0, max(b.x - cb0.z, cb0.x - b.z)) * sx;
       float dy = (float)max(0, max(b.y - cb0.w, cb0.y - b.w)) * sy;
-      const float dz = (float)(r1.x - oz) * sz;
+      const float dz = (float)(zmin - oz) * sz;
       float zd = apex - dz + zdError(dz, 0.f);
       float r2 = s2 * (dx * dx + dy * dy);
       float mag = zd * zd + r2 + por2min;
       if (zd < -1e-4f * (fabsf(zd) + 1e-3f))
         return false;
       return zd * zd - r2 - por2min >= -(1e-4f * mag + 1e-9f);
+    };
+    // and of a column or super-cell, as boxMeets
+    auto envMeets = [&](const int4 &b, const int4 &r1, const int4 *sr) -> bool {
+      return envReached(b, r1.x) || (r1.w && envReached(sr[0], sr[1].x));
     };
     // height (record units above oz) above which no point of a column can be
     // inside any lane's hyperboloid; columns holding points beside or above
@@ -1140,6 +1158,31 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
       const uint32_t e = (uint32_t)r1.z;
       const int32_t zl = envZlim(box, r1);
       bool got = false;
+      // whether the lane's hyperboloid may reach the blocks of the column's outside
+      // points and may hold them as a whole, and, where they have one block, whether
+      // it does for certain (the record's bounds are a unit or two wider)
+      bool blockMeets = true, blockHolds = false, surelyMeets = false, surelyHolds = false;
+      if (r1.w)
+      {
+        const int4 s0 = a.strayCol[2 * cc], s1 = a.strayCol[2 * cc + 1];
+        // +1: inside for certain, -1: outside for certain
+        auto inside = [&](int dx, int dy, int z) -> int {
+          const float x = (float)max(0, dx) * sx, y = (float)max(0, dy) * sy, dz = (float)(me.z - z) * sz;
+          const float zd = dz + czp, ez = zdError(dz, czp), r2 = s2 * (x * x + y * y), f = zd * zd - r2 - por2;
+          const float tol = 1e-4f * (zd * zd + r2 + por2) + ez * (2 * fabsf(zd) + ez) + 1e-9f;
+          return zd > ez && f > tol ? 1 : (zd < -ez || f < -tol ? -1 : 0);
+        };
+        const int nx = max(s0.x - me.x, me.x - s0.z), ny = max(s0.y - me.y, me.y - s0.w);
+        const int fx = max(me.x - s0.x, s0.z - me.x), fy = max(me.y - s0.y, s0.w - me.y);
+        blockMeets = inside(nx, ny, s1.y) >= 0;
+        blockHolds = inside(nx, ny, s1.x) >= 0;
+        if (s1.z)
+        {
+          surelyMeets = inside(nx + 4, ny + 4, s1.y + 4) > 0;
+          surelyHolds = surelyMeets && inside(fx, fy, s1.x + 4) > 0;
+          blockHolds = blockHolds && inside(fx - 4, fy - 4, s1.x) >= 0;
+        }
+      }
       // whether candidate c is inside the lane's hyperboloid, in FP32: 1
       // inside, 0 outside (or no direction), 2 when the exact test decides
       // (points outside the root cube, and the band where FP32 cannot tell);
@@ -1162,6 +1205,9 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
         int m = sureIn ? 1 : 0;
         if ((gp & kStray) || (!sureIn && !sureOut))
           m = (!(gp & kStray) && a.fp32Only) ? (zd > 0 && f > 0 ? 1 : 0) : 2;
+        // a point outside the root cube: by its block
+        if (gp & kStray)
+          m = !(blockMeets && (blockHolds || !sureOut)) ? 0 : (surelyHolds || (surelyMeets && sureIn) ? 1 : 2);
         // dist(p,q) == 0 gives no direction (classify.cpp:142,153)
         return (dxi != 0 || dyi != 0) ? m : 0;
       };
@@ -1339,7 +1385,7 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
         {
           c = (uint64_t)jj * a.nx + i;
           cb = a.col[2 * c];
-          ok = envMeets(cb, a.col[2 * c + 1]);
+          ok = envMeets(cb, a.col[2 * c + 1], a.strayCol + 2 * c);
         }
       }
       unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -1383,7 +1429,7 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
           {
             const uint64_t sc = (uint64_t)SJ * a.snx + SI;
             sb = a.super[2 * sc];
-            ok = envMeets(sb, a.super[2 * sc + 1]);
+            ok = envMeets(sb, a.super[2 * sc + 1], a.straySuper + 2 * sc);
           }
         }
         unsigned mask = __ballot_sync(0xffffffffu, ok);
@@ -1409,7 +1455,7 @@ __device__ __forceinline__ void classifyGroup(const ClsArgs &a, uint2 grp, int l
             {
               c = (uint64_t)jj * a.nx + i;
               cb = a.col[2 * c];
-              cok = envMeets(cb, a.col[2 * c + 1]);
+              cok = envMeets(cb, a.col[2 * c + 1], a.strayCol + 2 * c);
             }
           }
           unsigned cm = __ballot_sync(0xffffffffu, cok);
@@ -1532,6 +1578,8 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
     a.off[k] = g.off[k];
     a.scale[k] = g.scale[k];
     a.rootLo[k] = g.root_lo[k];
+    a.unitOff[k] = g.off[k] * g.unit;
+    a.perStep[k] = 1.0 / (g.scale[k] * g.unit);
     mn[k] = g.root_lo[k];
     mx[k] = g.root_lo[k] + g.root_side;
   }
@@ -1577,6 +1625,9 @@ static int classifyPrepare(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDe
   a.snx = c->grid.snx;
   a.sny = c->grid.sny;
   a.super = (const int4 *)c->superRec.p;
+  a.strayCol = (const int4 *)c->strayCol.p;
+  a.straySuper = (const int4 *)c->straySuper.p;
+  a.strayGrp = (const int4 *)c->strayGrp.p;
   // the lowest height a member can have, for the reach: the lowest point's (the
   // highest record integer's where the z scale is negative), or that of the root
   // cube's top where a block there decides for points above it
@@ -1684,8 +1735,9 @@ __global__ void batchSetup(const BatchHdr *__restrict__ h)
 }
 
 /* MODE 0: every point of every job; 1: the points the groups deferred.  ARCS: by
- * open arcs, else by bins, which form every largest gap. */
-template <int MODE, bool ARCS, int W, int MINB>
+ * open arcs, else by bins, which form every largest gap.  STRAYS: some job has
+ * points outside the root cube. */
+template <int MODE, bool ARCS, bool STRAYS, int W, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const BatchOut *o)
 {
   __shared__ uint32_t bmin[W][ARCS ? 1 : kBins], bmax[W][ARCS ? 1 : kBins];
@@ -1724,7 +1776,7 @@ __global__ void __launch_bounds__(32 * W, MINB) batchRings(BatchHdr *h, const Ba
       uint64_t item = g - lo;
       const uint64_t j = MODE == 1 ? a.deferList[item] : item;
       if constexpr (ARCS)
-        classifyPointArcs(a, j, lane, psm[w]);
+        classifyPointArcs<STRAYS>(a, j, lane, psm[w]);
       else
         classifyPoint<false>(a, j, lane, bmin[w], bmax[w]);
     }
@@ -1812,7 +1864,7 @@ __global__ void __launch_bounds__(32 * W) batchExact(BatchHdr *h, const BatchOut
 /* The fast pass by point groups (ARCS) or, when decision margins are wanted,
  * by column groups, which form every largest gap: warps take chunks of groups
  * (of all jobs) from a global counter. */
-template <bool ARCS, int W, int MINB>
+template <bool ARCS, bool STRAYS, int W, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB) batchGroups(BatchHdr *h, const BatchOut *o)
 {
   __shared__ typename std::conditional<ARCS, GroupShared, GroupSmem>::type gsm[W];
@@ -1851,7 +1903,7 @@ __global__ void __launch_bounds__(32 * W, MINB) batchGroups(BatchHdr *h, const B
         {
         const uint64_t i = g - lo, high = (uint32_t)sa[w].groupsTaken[1];
         const uint32_t *order = (const uint32_t *)(sa[w].groups + 2 * sa[w].maxGroups);
-        classifyGroupArcs(sa[w], order[i < high ? i : sa[w].maxGroups - 1 - (i - high)], lane, gsm[w]);
+        classifyGroupArcs<STRAYS>(sa[w], order[i < high ? i : sa[w].maxGroups - 1 - (i - high)], lane, gsm[w]);
       }
       else
         classifyGroup(sa[w], sa[w].colGroups[g - lo], lane, gsm[w]);
@@ -1983,14 +2035,15 @@ __global__ void batchScatter(const BatchHdr *__restrict__ h)
 
 static_assert(sizeof(ClsArgs) <= sizeof(((wb_ctx *)nullptr)->clsArgs), "wb_ctx::clsArgs too small");
 
+#define WB_N_KERNELS (WB_N_SHAPES + 7)
 struct WbBatch
 {
   int device = 0, sm = 0;
   cudaStream_t capture = nullptr;
   BatchHdr *dIn = nullptr, *hIn = nullptr;
   BatchOut *dOut = nullptr, *hOut = nullptr;
-  int per[WB_N_SHAPES + 4] = {0};   /* resident blocks per SM of each classify kernel */
-  cudaGraphExec_t graphs[WB_N_SHAPES] = {nullptr};
+  int per[WB_N_KERNELS] = {0};   /* resident blocks per SM of each classify kernel */
+  cudaGraphExec_t graphs[WB_N_KERNELS] = {nullptr};   /* by fast pass */
 };
 
 const WbShape kWbShapes[WB_N_SHAPES] = {{4, 6}, {4, 5}, {4, 4}, {8, 3}, {4, 6}, {4, 8}, {8, 4}, {2, 12}};
@@ -2003,7 +2056,9 @@ typedef void (*RingsFn)(BatchHdr *, const BatchOut *);
  * shape (one point per warp, or point groups), kDeferred the one-point pass
  * over the points groups handed over, kExactPass the exact pass. */
 constexpr int kDeferred = WB_N_SHAPES, kExactPass = WB_N_SHAPES + 1, kMarginGroups = WB_N_SHAPES + 2,
-              kMarginDeferred = WB_N_SHAPES + 3;
+              kMarginDeferred = WB_N_SHAPES + 3, kStrayGroups = WB_N_SHAPES + 4, kStrayPoints = WB_N_SHAPES + 5,
+              kStrayDeferred = WB_N_SHAPES + 6;
+static_assert(kStrayDeferred + 1 == WB_N_KERNELS, "WbBatch has room for every kernel");
 
 RingsFn ringsFn(int idx)
 {
@@ -2011,30 +2066,45 @@ RingsFn ringsFn(int idx)
   // thread); 3-7: one point per warp (about 85, 85, 64, 64 and 85)
   switch (idx)
   {
-  case 1: return batchGroups<true, 4, 5>;
-  case 2: return batchGroups<true, 4, 4>;
-  case 3: return batchRings<0, true, 8, 3>;
-  case 4: return batchRings<0, true, 4, 6>;
-  case 5: return batchRings<0, true, 4, 8>;
-  case 6: return batchRings<0, true, 8, 4>;
-  case 7: return batchRings<0, true, 2, 12>;
-  case kDeferred: return batchRings<1, true, 4, 8>;
+  case 1: return batchGroups<true, false, 4, 5>;
+  case 2: return batchGroups<true, false, 4, 4>;
+  case 3: return batchRings<0, true, false, 8, 3>;
+  case 4: return batchRings<0, true, false, 4, 6>;
+  case 5: return batchRings<0, true, false, 4, 8>;
+  case 6: return batchRings<0, true, false, 8, 4>;
+  case 7: return batchRings<0, true, false, 2, 12>;
+  case kDeferred: return batchRings<1, true, false, 4, 8>;
   case kExactPass: return batchExact<8>;
-  case kMarginDeferred: return batchRings<1, false, 8, 3>;
-  case kMarginGroups: return batchGroups<false, 8, 3>;
-  default: return batchGroups<true, 4, 6>;
+  case kMarginDeferred: return batchRings<1, false, true, 8, 3>;
+  case kMarginGroups: return batchGroups<false, true, 8, 3>;
+  case kStrayGroups: return batchGroups<true, true, 4, 5>;
+  case kStrayPoints: return batchRings<0, true, true, 4, 6>;
+  case kStrayDeferred: return batchRings<1, true, true, 4, 6>;
+  default: return batchGroups<true, false, 4, 6>;
   }
 }
 
 int ringsWarps(int idx)
 {
-  return idx == kDeferred ? 4 : (idx == kExactPass || idx == kMarginDeferred || idx == kMarginGroups ? 8 : kWbShapes[idx].warps);
+  return idx < WB_N_SHAPES ? kWbShapes[idx].warps : (idx == kExactPass || idx == kMarginDeferred || idx == kMarginGroups ? 8 : 4);
 }
 
 /* The one-point pass that goes with a fast pass. */
 int deferredOf(int shape)
 {
-  return shape == kMarginGroups ? kMarginDeferred : kDeferred;
+  return shape == kMarginGroups ? kMarginDeferred : (shape == kStrayGroups || shape == kStrayPoints ? kStrayDeferred : kDeferred);
+}
+
+/* The fast pass of a shape for these jobs.  Points outside the root cube (a
+ * header's box just below a power of two leaves some at the lower faces, one in
+ * three placements of a 1000 m tile) have kernels of their own: their tests cost
+ * other clouds 2% where one kernel held both. */
+int fastPass(int shape, wb_ctx *const *jobs, int k)
+{
+  for (int q = 0; q < k; q++)
+    if (jobs[q]->grid.nStray)
+      return shape < 3 ? kStrayGroups : kStrayPoints;
+  return shape;
 }
 
 __global__ void batchAmbReset(const BatchHdr *__restrict__ h)
@@ -2222,7 +2292,7 @@ int wb_classify_stage(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDevice)
 int wb_batch_time(WbBatch *b, wb_ctx *const *jobs, int k, int shape, int chunk, cudaStream_t s,
                   float *ms, std::string &err)
 {
-  shape = clampShape(shape);
+  shape = fastPass(clampShape(shape), jobs, k);
   int rc = fillTable(b, jobs, k, chunk, err);
   if (rc)
     return rc;
@@ -2267,7 +2337,7 @@ int wb_batch_time(WbBatch *b, wb_ctx *const *jobs, int k, int shape, int chunk, 
 int wb_batch_launch(WbBatch *b, wb_ctx *const *jobs, int k, cudaStream_t s, int shape, int chunk,
                     uint64_t *launches, std::string &err)
 {
-  shape = clampShape(shape);
+  shape = fastPass(clampShape(shape), jobs, k);
   int rc = fillTable(b, jobs, k, chunk, err);
   if (rc)
     return rc;
@@ -2328,7 +2398,7 @@ int wb_classify_impl(wb_ctx *c, const wb_params *p, uint8_t *cls, int onDevice)
   if (!c->batch && (rc = wb_batch_create(c->device, &c->batch, err)))
     return wb_fail(c, rc, err);
   WbBatch *b = c->batch;
-  int shape = clampShape(c->shape);
+  int shape = fastPass(clampShape(c->shape), &c, 1);
   if (c->marginDst)
     shape = kMarginGroups;
   if ((rc = fillTable(b, &c, 1, c->chunk, err)))

@@ -256,6 +256,30 @@ __device__ __forceinline__ int splitArc(float ux, float uy, float &ax, float &ay
   return (int)o0 + (int)o1;
 }
 
+/* The block of a point outside the root cube, from the origin (X, Y, Z) in record
+ * units: x and y range, top and bottom of its cube. */
+struct BlockBounds
+{
+  float x0, x1, y0, y1, top, bottom;
+};
+__device__ __noinline__ BlockBounds blockBounds(const ClsArgs &a, uint32_t j, int X, int Y, int Z)
+{
+  const uint32_t l = a.leafId[j];
+  double cx, cy, cz, side;
+  wb_leaf_cube(a.leafKey[l], a.leafLev[l], a.rootLo, a.rootSide, cx, cy, cz, side);
+  const double h = side / 2;
+  BlockBounds b;
+  b.x0 = (float)((cx - h - a.unitOff[0]) * a.perStep[0] - X);
+  b.x1 = (float)((cx + h - a.unitOff[0]) * a.perStep[0] - X);
+  b.y0 = (float)((cy - h - a.unitOff[1]) * a.perStep[1] - Y);
+  b.y1 = (float)((cy + h - a.unitOff[1]) * a.perStep[1] - Y);
+  b.top = (float)((cz + h - a.unitOff[2]) * a.perStep[2] - Z);
+  b.bottom = (float)((cz - h - a.unitOff[2]) * a.perStep[2] - Z);
+  return b;
+}
+
+/* STRAYS: some cloud of the launch has points outside the root cube. */
+template <bool STRAYS>
 __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t group, int lane, GroupShared &sm)
 {
   constexpr unsigned kAll = 0xffffffffu;
@@ -340,16 +364,19 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
   };
   envelope();
   // can a box {x0, y0, x1, y1} with lowest point zmin hold a member of any lane?
-  // (always, when it holds a point beside or above the root cube: flags)
-  auto envMeets = [&](const int4 &b, int32_t zmin, int flags) -> bool {
+  auto envReached = [&](const int4 &b, int32_t zmin) -> bool {
     if (b.x == INT32_MAX)
       return false;
-    if (flags)
-      return true;
     const float dx = (float)max(0, max(b.x - gx1, gx0 - b.z)), dy = (float)max(0, max(b.y - gy1, gy0 - b.w)) * ky;
     const float zd = apex - (float)(zmin - gz0) * kz;
     const float r2 = __fmaf_rn(dx, dx, dy * dy);
     return __fmaf_rn(zd * fabsf(zd), 1.0004f, -pK) >= r2;
+  };
+  // the same of a super-cell or group (bounds, record), also by the blocks of its
+  // points beside or above the root cube (flags, sr): one whose block lies in a
+  // lane's hyperboloid as a whole is a member wherever it is itself
+  auto envMeets = [&](const int4 &b, const int4 &r, const int4 *sr) -> bool {
+    return envReached(b, r.x) || (STRAYS && r.w && envReached(sr[0], sr[1].x));
   };
 #ifdef WB_CLASSIFY_STATS
   unsigned long long gst[16] = {0};
@@ -518,8 +545,18 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
   // undecided lane in a direction of the lane's open arc: the nearest point of
   // the box against the hyperboloid, and the largest value of a cross product
   // over a box, its value at the centre plus the halves' shares.  Boxes holding
-  // points beside the root cube (flags) are judged by the arc only.
-  auto boxWanted = [&](const float4 &b, float zmin, int flags) -> bool {
+  // points beside or above the root cube (flags, their record's number plus one)
+  // are also reached by those points' blocks.
+  auto blocksReached = [&](const int4 &c, int z) -> bool {
+    const float4 b = boxOfInts(c);
+    const float dx = fmaxf(0.f, fabsf(b.x - mx) - b.z), dy = fmaxf(0.f, fabsf(b.y - mys) - b.w);
+    const float zd = __fmaf_rn(mz - (float)(z - gz0), kz, czp);
+    return __fmaf_rn(zd * fabsf(zd), kOut, -pOut) >= __fmaf_rn(dx, dx, dy * dy);
+  };
+  auto blockWanted = [&](int flags, const int4 *strays) -> bool {
+    return STRAYS && flags && blocksReached(strays[2 * (flags - 1)], strays[2 * (flags - 1) + 1].x);
+  };
+  auto boxWanted = [&](const float4 &b, float zmin, bool block) -> bool {
     const float ex = b.x - mx, ey = b.y - mys;
     const float dx = fmaxf(0.f, fabsf(ex) - b.z), dy = fmaxf(0.f, fabsf(ey) - b.w);
     const float zd = __fmaf_rn(mz - zmin, kz, czp);
@@ -527,7 +564,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
     const float A = __fmaf_rn(side, __fmaf_rn(ax, ey, -(ay * ex)), __fmaf_rn(fabsf(ay), b.z, fabsf(ax) * b.w));
     const float B = __fmaf_rn(side, __fmaf_rn(ex, by, -(ey * bx)), __fmaf_rn(fabsf(by), b.z, fabsf(bx) * b.w));
     const float v = side < 0.f ? fmaxf(A, B) : fminf(A, B);
-    return __any_sync(kAll, ((flags != 0) | reach) & !done & (v >= arcMin));
+    return __any_sync(kAll, (block | reach) & !done & (v >= arcMin));
   };
 
   // The walk, as one loop so that each part is there once: the next group of
@@ -548,7 +585,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       list &= list - 1;
       WB_STAT(gst[3], 1);
       const int4 r = sm.nrec[src];
-      if (!boxWanted(sm.nbox[src], __int_as_float(r.x), r.w))
+      if (!boxWanted(sm.nbox[src], __int_as_float(r.x), blockWanted(r.w, a.strayGrp)))
         continue;
       if (reads >= kGroupReads)
       {
@@ -566,15 +603,20 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       // stage the group, with its octets' boxes
       float x = 0.f, y = 0.f, z = INFINITY;
       bool stray = false;
+      BlockBounds block{};
       if (lane < r.z)
       {
         const int2 p = a.bxy[(uint32_t)r.y + lane], q = a.bzw[(uint32_t)r.y + lane];
         x = (float)(p.x - gx0);
         y = (float)(p.y - gy0);
         z = (float)(q.x - gz0);
-        stray = q.y < 0;
+        if (STRAYS && q.y < 0)
+        {
+          stray = true;
+          block = blockBounds(a, (uint32_t)q.y & 0x7fffffffu, gx0, gy0, gz0);
+        }
       }
-      const unsigned strays = __ballot_sync(kAll, stray);
+      const unsigned strays = STRAYS ? __ballot_sync(kAll, stray) : 0u;
       float x0 = z < INFINITY ? x : INFINITY, x1 = z < INFINITY ? x : -INFINITY;
       float y0 = z < INFINITY ? y : INFINITY, y1 = z < INFINITY ? y : -INFINITY, z0 = z;
 #pragma unroll
@@ -589,7 +631,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       __syncwarp();
       sm.cx[lane] = x;
       sm.cy[lane] = y;
-      sm.cz[lane] = stray ? -INFINITY : -z;   // left to the exact test
+      sm.cz[lane] = stray ? -INFINITY : -z;   // not in the octets' test
       if ((lane & 7) == 0)
       {
         sm.obox[lane >> 3] = boxOf(x0, x1, y0 * ky, y1 * ky);
@@ -597,12 +639,51 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       }
       __syncwarp();
       const bool wasDone = done;
-      pend = done ? 0u : strays;
+      pend = 0;
+      if (STRAYS && strays)
+      {
+        // The points outside the root cube, one after another: a member's block
+        // meets the lane's hyperboloid (its cube's nearest point at the bottom),
+        // and either the point is inside or the block as a whole is (its farthest
+        // corner at the top).  Decided in FP32 with the rounding of the bounds
+        // (half a record unit and 1e-6) and of the heights allowed for either way;
+        // what that leaves in doubt waits for the exact test.
+#pragma unroll 1
+        for (unsigned left = strays; left; left &= left - 1)
+        {
+          const int k = __ffs(left) - 1;
+          const float x0 = __shfl_sync(kAll, block.x0, k), x1 = __shfl_sync(kAll, block.x1, k);
+          const float y0 = __shfl_sync(kAll, block.y0, k) * ky, y1 = __shfl_sync(kAll, block.y1, k) * ky;
+          const float zt = __shfl_sync(kAll, block.top, k), zb = __shfl_sync(kAll, block.bottom, k);
+          const float ex = sm.cx[k] - mx, ey = (sm.cy[k] - my) * ky, rr = __fmaf_rn(ex, ex, ey * ey);
+          const float zd = __fmaf_rn(mz - __shfl_sync(kAll, z, k), kz, czp);
+          const float px = 0.5f + 1e-6f * (fabsf(x0) + fabsf(x1) + bw), py = 0.5f * ky + 1e-6f * (fabsf(y0) + fabsf(y1) + bh);
+          const float nx = fmaxf(x0 - mx, mx - x1), ny = fmaxf(y0 - mys, mys - y1);
+          const float fx = fmaxf(mx - x0, x1 - mx), fy = fmaxf(mys - y0, y1 - mys), pz = 0.5f * kz;
+          auto may = [&](float h, float dx, float dy) -> bool {
+            const float d = fmaxf(0.f, dx), e = fmaxf(0.f, dy);
+            return __fmaf_rn(h * fabsf(h), kOut, -pOut) >= __fmaf_rn(d, d, e * e);
+          };
+          auto sure = [&](float h, float dx, float dy) -> bool {
+            const float d = fmaxf(0.f, dx), e = fmaxf(0.f, dy);
+            return h > 0.f && h * h > kOut * (__fmaf_rn(d, d, e * e) + por2 + a.gTiny);
+          };
+          const float hb = __fmaf_rn(mz - zb, kz, czp), ht = __fmaf_rn(mz - zt, kz, czp);
+          const bool arc = side * fminf(__fmaf_rn(ax, ey, -(ay * ex)), __fmaf_rn(ex, by, -(ey * bx))) > arcMin;
+          const bool wanted = !done & arc & (rr > 0.f);
+          const bool out = !may(hb + pz, nx - px, ny - py) || !(may(zd, fabsf(ex), fabsf(ey)) || may(ht + pz, fx - px, fy - py));
+          const bool in = sure(hb - pz, nx + px, ny + py) && (sure(zd, fabsf(ex), fabsf(ey)) || sure(ht - pz, fx + px, fy + py));
+          if (wanted & !in & !out)
+            pend |= 1u << k;
+          if (__any_sync(kAll, wanted & in))
+            addAny(wanted & in, ex, ey, rr);
+        }
+      }
 #pragma unroll 1
       for (int o = 0; 8 * o < r.z; o++)
       {
         WB_STAT(gst[2], 1);
-        if (boxWanted(sm.obox[o], sm.oz[o], 0))
+        if (boxWanted(sm.obox[o], sm.oz[o], false))
         {
           WB_STAT(gst[6], 8);
           WB_STAT(gst[7], 8 * __popc(__ballot_sync(kAll, !done)));
@@ -632,10 +713,13 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
         r = a.groups[2 * (uint64_t)(gNext + lane) + 1];
       }
       gNext += 32;
-      list = __ballot_sync(kAll, envMeets(b, r.x, r.w));
+      if constexpr (STRAYS)
+        list = __ballot_sync(kAll, envMeets(b, r, a.strayGrp + 2 * (uint64_t)(gNext - 32 + lane)));
+      else
+        list = __ballot_sync(kAll, envReached(b, r.x));
       __syncwarp();
       sm.nbox[lane] = boxOfInts(b);
-      sm.nrec[lane] = make_int4(__float_as_int((float)(r.x - gz0)), r.y, r.z, r.w);
+      sm.nrec[lane] = make_int4(__float_as_int((float)(r.x - gz0)), r.y, r.z, STRAYS ? (r.w ? (int)(gNext - 32 + lane) + 1 : 0) : r.w);
       __syncwarp();
       continue;
     }
@@ -645,7 +729,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       supers &= supers - 1;
       WB_STAT(gst[4], 1);
       const int4 s1 = sm.srec[src];
-      if (sr < 2 || boxWanted(sm.sbox[src], __int_as_float(s1.x), s1.w))
+      if (sr < 2 || boxWanted(sm.sbox[src], __int_as_float(s1.x), blockWanted(s1.w, a.straySuper)))
       {
         gNext = (uint32_t)s1.y;
         gEnd = gNext + (uint32_t)s1.z;
@@ -663,6 +747,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       m0 = 0;
     }
     WB_STAT(gst[5], 1);
+    uint32_t cell = 0;
     if (m0 + lane < nsc)
     {
       int di, dj;
@@ -671,14 +756,18 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       if (SI >= 0 && SI < a.snx && SJ >= 0 && SJ < a.sny)
       {
         const uint64_t sc = (uint64_t)SJ * a.snx + SI;
+        cell = (uint32_t)sc;
         b = a.super[2 * sc];
         r = a.super[2 * sc + 1];
       }
     }
-    supers = __ballot_sync(kAll, envMeets(b, r.x, r.w));
+    if constexpr (STRAYS)
+      supers = __ballot_sync(kAll, envMeets(b, r, a.straySuper + 2 * (uint64_t)cell));
+    else
+      supers = __ballot_sync(kAll, envReached(b, r.x));
     __syncwarp();
     sm.sbox[lane] = boxOfInts(b);
-    sm.srec[lane] = make_int4(__float_as_int((float)(r.x - gz0)), r.y, r.z, r.w);
+    sm.srec[lane] = make_int4(__float_as_int((float)(r.x - gz0)), r.y, r.z, STRAYS ? (r.w ? (int)cell + 1 : 0) : r.w);
     __syncwarp();
   }
 #ifdef WB_CLASSIFY_STATS
@@ -726,6 +815,7 @@ struct PointShared
   float2 arc2a, arc2b;   /* the point's second open arc, while it has one */
 };
 
+template <bool STRAYS>
 __device__ __forceinline__ void classifyPointArcs(const ClsArgs &a, uint64_t j, int lane, PointShared &sm)
 {
   constexpr unsigned kAll = 0xffffffffu;
@@ -760,19 +850,30 @@ __device__ __forceinline__ void classifyPointArcs(const ClsArgs &a, uint64_t j, 
   bool slow = true, two = false, done = false;
   float side = 1.f, arcMin = -INFINITY, ax = 0.f, ay = 0.f, bx = 0.f, by = 0.f;
 
-  // whether the lane's box may hold a member in a direction that matters
-  auto meets = [&](const int4 &b, int32_t zmin, int flags) -> bool {
+  // whether the point's hyperboloid reaches a box (record integers) at height z
+  auto reached = [&](const int4 &b, int32_t z) -> bool {
+    const float x0 = (float)(b.x - mex), x1 = (float)(b.z - mex), y0 = (float)(b.y - mey) * ky, y1 = (float)(b.w - mey) * ky;
+    const float pad = 2e-6f * (fabsf(x0) + fabsf(x1) + fabsf(y0) + fabsf(y1));
+    const float dx = fmaxf(0.f, fmaxf(x0, -x1) - pad), dy = fmaxf(0.f, fmaxf(y0, -y1) - pad);
+    const float zd = __fmaf_rn((float)(mez - z), kz, czp);
+    return __fmaf_rn(zd * fabsf(zd), kOut, -pOut) >= __fmaf_rn(dx, dx, dy * dy);
+  };
+  // whether the lane's box may hold a member in a direction that matters (flags,
+  // strays: as in classifyGroupArcs)
+  auto meets = [&](const int4 &b, int32_t zmin, int flags, const int4 *strays) -> bool {
     const float x0 = (float)(b.x - mex), x1 = (float)(b.z - mex), y0 = (float)(b.y - mey) * ky, y1 = (float)(b.w - mey) * ky;
     const float ex = 0.5f * (x0 + x1), ey = 0.5f * (y0 + y1);
     const float pad = 2e-6f * (fabsf(x0) + fabsf(x1) + fabsf(y0) + fabsf(y1));
     const float hx = 0.5f * (x1 - x0) + pad, hy = 0.5f * (y1 - y0) + pad;
     const float dx = fmaxf(0.f, fabsf(ex) - hx), dy = fmaxf(0.f, fabsf(ey) - hy);
     const float zd = __fmaf_rn((float)(mez - zmin), kz, czp);
-    const bool reach = __fmaf_rn(zd * fabsf(zd), kOut, -pOut) >= __fmaf_rn(dx, dx, dy * dy);
+    bool reach = __fmaf_rn(zd * fabsf(zd), kOut, -pOut) >= __fmaf_rn(dx, dx, dy * dy);
+    if (STRAYS && flags && !reach)
+      reach = reached(strays[0], strays[1].x);
     const float A = __fmaf_rn(side, __fmaf_rn(ax, ey, -(ay * ex)), __fmaf_rn(fabsf(ay), hx, fabsf(ax) * hy));
     const float B = __fmaf_rn(side, __fmaf_rn(ex, by, -(ey * bx)), __fmaf_rn(fabsf(by), hx, fabsf(bx) * hy));
     const float v = side < 0.f ? fmaxf(A, B) : fminf(A, B);
-    return (b.x != INT32_MAX) & ((flags != 0) | reach) & (v >= arcMin);
+    return (b.x != INT32_MAX) & reach & (v >= arcMin);
   };
   // adds the directions (ex, ey) of the lanes in hits; after each, those the
   // open arc no longer holds drop out
@@ -826,6 +927,7 @@ __device__ __forceinline__ void classifyPointArcs(const ClsArgs &a, uint64_t j, 
     for (int m0 = 0; m0 < nsc && !done; m0 += 32)
     {
       int4 b = make_int4(INT32_MAX, 0, 0, 0), r = make_int4(0, 0, 0, 0);
+      uint64_t sc = 0;
       if (m0 + lane < nsc)
       {
         int di, dj;
@@ -833,12 +935,12 @@ __device__ __forceinline__ void classifyPointArcs(const ClsArgs &a, uint64_t j, 
         const int SI = si + di, SJ = sj + dj;
         if (SI >= 0 && SI < a.snx && SJ >= 0 && SJ < a.sny)
         {
-          const uint64_t sc = (uint64_t)SJ * a.snx + SI;
+          sc = (uint64_t)SJ * a.snx + SI;
           b = a.super[2 * sc];
           r = a.super[2 * sc + 1];
         }
       }
-      unsigned supers = __ballot_sync(kAll, meets(b, r.x, r.w));
+      unsigned supers = __ballot_sync(kAll, meets(b, r.x, r.w, a.straySuper + 2 * sc));
       while (supers && !done)
       {
         const int src = __ffs(supers) - 1;
@@ -852,7 +954,7 @@ __device__ __forceinline__ void classifyPointArcs(const ClsArgs &a, uint64_t j, 
             gb = a.groups[2 * (uint64_t)(g + lane)];
             gr = a.groups[2 * (uint64_t)(g + lane) + 1];
           }
-          unsigned list = __ballot_sync(kAll, meets(gb, gr.x, gr.w));
+          unsigned list = __ballot_sync(kAll, meets(gb, gr.x, gr.w, a.strayGrp + 2 * (uint64_t)(g + lane)));
           while (list && !done)
           {
             const int gs = __ffs(list) - 1;
@@ -870,10 +972,18 @@ __device__ __forceinline__ void classifyPointArcs(const ClsArgs &a, uint64_t j, 
             const float rr = __fmaf_rn(ex, ex, ey * ey), w = zd * fabsf(zd);
             const bool arc = side * fminf(__fmaf_rn(ax, ey, -(ay * ex)), __fmaf_rn(ex, by, -(ey * bx))) > arcMin;
             // dist(p,q) == 0 gives no direction (classify.cpp:142,153)
-            const bool cand = (lane < n) & ((dxi != 0) | (dyi != 0)), stray = q.y < 0;
+            const bool cand = (lane < n) & ((dxi != 0) | (dyi != 0)), stray = STRAYS && q.y < 0;
+            // points outside the root cube: in or not by their blocks too
+            bool blockMeets = true, blockHolds = false;
+            if (STRAYS && __shfl_sync(kAll, gr.w, gs))
+            {
+              const int4 *s = a.strayGrp + 2 * (uint64_t)(g + gs);
+              blockMeets = reached(s[0], s[1].y);
+              blockHolds = reached(s[0], s[1].x);
+            }
             const bool may = (__fmaf_rn(w, kOut, -pOut) >= rr) & arc, sure = w > kOut * (rr + por2 + a.gTiny);
             const unsigned hits = __ballot_sync(kAll, cand & !stray & may & sure);
-            const bool unsure = cand & (stray | (may & !sure));
+            const bool unsure = cand & (stray ? (may & blockMeets) | (arc & blockHolds) : may & !sure);
             if (hits)
               add(hits, ex, ey, rr);
             if (__any_sync(kAll, unsure) && !done)

@@ -633,12 +633,161 @@ __global__ void __launch_bounds__(kOrderThreads) groupOrderKernel(int nx, int ny
   });
 }
 
+/* What the blocks of points outside the root cube are found from. */
+struct StrayArgs
+{
+  const uint32_t *leafId;
+  const uint64_t *leafKey;
+  const uint8_t *leafLev;
+  const uint8_t *stray;
+  double off[3], scale[3], unit, rootLo[3], rootSide;
+  int imin[3], imax[3];   /* the cloud's record integers */
+};
+
+/* The box of the blocks of outside points in record integers, and the lowest of
+ * their cubes' tops and bottoms: a shape that takes such a point by its block,
+ * without holding the point, reaches the box at that top; one that takes it at
+ * all reaches it at that bottom. */
+struct StrayBox
+{
+  int x0, y0, x1, y1, top, bottom;
+  __device__ void clear()
+  {
+    x0 = y0 = top = bottom = INT32_MAX;
+    x1 = y1 = INT32_MIN;
+  }
+  __device__ void add(const StrayBox &b)
+  {
+    x0 = min(x0, b.x0);
+    y0 = min(y0, b.y0);
+    x1 = max(x1, b.x1);
+    y1 = max(y1, b.y1);
+    top = min(top, b.top);
+    bottom = min(bottom, b.bottom);
+  }
+  __device__ void warpAdd()
+  {
+    x0 = __reduce_min_sync(0xffffffffu, x0);
+    y0 = __reduce_min_sync(0xffffffffu, y0);
+    x1 = __reduce_max_sync(0xffffffffu, x1);
+    y1 = __reduce_max_sync(0xffffffffu, y1);
+    top = __reduce_min_sync(0xffffffffu, top);
+    bottom = __reduce_min_sync(0xffffffffu, bottom);
+  }
+  __device__ void store(int4 *r) const
+  {
+    r[0] = make_int4(x0, y0, x1, y1);
+    r[1] = make_int4(top, bottom, 0, 0);
+  }
+  __device__ void load(const int4 *r)
+  {
+    x0 = r[0].x;
+    y0 = r[0].y;
+    x1 = r[0].z;
+    y1 = r[0].w;
+    top = r[1].x;
+    bottom = r[1].y;
+  }
+};
+
+/* The block of stored point j, a record unit wider on every side and within the
+ * cloud's extent (which holds every query's own point, so that nothing is nearer
+ * to one than before), its heights at most 2^29 units below it. */
+__device__ __noinline__ StrayBox strayBlock(const StrayArgs &a, uint32_t j)
+{
+  const uint32_t l = a.leafId[j];
+  double c[3], side;
+  wb_leaf_cube(a.leafKey[l], a.leafLev[l], a.rootLo, a.rootSide, c[0], c[1], c[2], side);
+  int lo[3], hi[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+  {
+    const double p = ((c[k] - side / 2) / a.unit - a.off[k]) / a.scale[k], q = ((c[k] + side / 2) / a.unit - a.off[k]) / a.scale[k];
+    const double least = k < 2 ? (double)a.imin[k] : fmax((double)a.imin[k] - 536870912.0, -2147483648.0);
+    lo[k] = (int)fmin(fmax(floor(fmin(p, q)) - 1, least), (double)a.imax[k]);
+    hi[k] = (int)fmin(fmax(k < 2 ? ceil(fmax(p, q)) + 1 : floor(fmax(p, q)) - 1, least), (double)a.imax[k]);
+  }
+  StrayBox b;
+  b.x0 = lo[0];
+  b.y0 = lo[1];
+  b.x1 = hi[0];
+  b.y1 = hi[1];
+  b.top = hi[2];
+  b.bottom = lo[2];
+  return b;
+}
+
+/* The records of the columns that hold points beside or above the root cube, of all
+ * their points outside it; one warp each (run only for clouds with outside
+ * points). */
+__global__ void strayColumnKernel(uint64_t ncell, StrayArgs a, const int4 *__restrict__ rec, const int4 *__restrict__ gpt,
+                                  int4 *__restrict__ out)
+{
+  const int lane = threadIdx.x & 31;
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < ncell; c += warps)
+  {
+    const int4 r1 = rec[2 * c + 1];
+    if (!r1.w)
+      continue;
+    StrayBox b;
+    b.clear();
+    uint32_t l0 = 0xffffffffu, l1 = 0;   // the least and the greatest of their leaves
+    for (uint32_t i = (uint32_t)r1.y + lane; i < (uint32_t)r1.z; i += 32)
+    {
+      const int w = gpt[i].w;
+      if (w < 0)
+      {
+        const uint32_t j = (uint32_t)w & 0x7fffffffu;
+        b.add(strayBlock(a, j));
+        l0 = min(l0, a.leafId[j]);
+        l1 = max(l1, a.leafId[j]);
+      }
+    }
+    __syncwarp();
+    b.warpAdd();
+    l0 = __reduce_min_sync(0xffffffffu, l0);
+    l1 = __reduce_max_sync(0xffffffffu, l1);
+    if (lane == 0)
+    {
+      b.store(out + 2 * c);
+      out[2 * c + 1].z = l0 == l1;   // one block: its bounds also tell for certain
+    }
+  }
+}
+
+/* The same per super-cell. */
+__global__ void straySuperKernel(int nx, int ny, int snx, int sny, const int4 *__restrict__ rec,
+                                 const int4 *__restrict__ srec, const int4 *__restrict__ col, int4 *__restrict__ out)
+{
+  const uint64_t ns = (uint64_t)snx * sny;
+  for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += (uint64_t)gridDim.x * blockDim.x)
+  {
+    if (!srec[2 * s + 1].w)
+      continue;
+    StrayBox b;
+    b.clear();
+    for (int q = 0; q < WB_SUPER * WB_SUPER; q++)
+    {
+      const int i = (int)(s % snx) * WB_SUPER + q % WB_SUPER, j = (int)(s / snx) * WB_SUPER + q / WB_SUPER;
+      const uint64_t c = (uint64_t)j * nx + i;
+      if (i < nx && j < ny && rec[2 * c + 1].w)
+      {
+        StrayBox o;
+        o.load(col + 2 * c);
+        b.add(o);
+      }
+    }
+    b.store(out + 2 * s);
+  }
+}
+
 /* The groups' records: two int4 per group, {x0, y0, x1, y1} and {zmin, first,
  * points, flags} (flags: holds a point beside or above the root cube, which
  * the queries can take with its block without the hyperboloid holding the point
- * itself); one warp per group. */
-__global__ void groupBoxKernel(GridArgs g, const unsigned long long *__restrict__ taken, const int2 *__restrict__ bxy,
-                               const int2 *__restrict__ bzw, int4 *__restrict__ groups)
+ * itself: strayGrp then has the blocks' box); one warp per group. */
+__global__ void groupBoxKernel(StrayArgs a, const unsigned long long *__restrict__ taken, const int2 *__restrict__ bxy,
+                               const int2 *__restrict__ bzw, int4 *__restrict__ groups, int4 *__restrict__ strayGrp)
 {
   const int lane = threadIdx.x & 31;
   const uint64_t n = *taken >> 36, warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -655,14 +804,19 @@ __global__ void groupBoxKernel(GridArgs g, const unsigned long long *__restrict_
     const int x0 = __reduce_min_sync(0xffffffffu, ok ? p.x : INT32_MAX), x1 = __reduce_max_sync(0xffffffffu, ok ? p.x : INT32_MIN);
     const int y0 = __reduce_min_sync(0xffffffffu, ok ? p.y : INT32_MAX), y1 = __reduce_max_sync(0xffffffffu, ok ? p.y : INT32_MIN);
     const int z0 = __reduce_min_sync(0xffffffffu, ok ? q.x : INT32_MAX);
-    bool stray = ok && q.y < 0;
+    const bool mine = ok && q.y < 0;   // outside the root cube
+    const bool stray = __any_sync(0xffffffffu, mine && (a.stray[(uint32_t)q.y & 0x7fffffffu] & 2));
     if (stray)
     {
-      const double x = wb_decode(p.x, g.off[0], g.scale[0], g.unit), y = wb_decode(p.y, g.off[1], g.scale[1], g.unit),
-                   z = wb_decode(q.x, g.off[2], g.scale[2], g.unit);
-      stray = x < g.rootLo[0] || y < g.rootLo[1] || x >= g.rootHi[0] || y >= g.rootHi[1] || z >= g.rootHi[2];
+      StrayBox b;
+      b.clear();
+      if (mine)
+        b = strayBlock(a, (uint32_t)q.y & 0x7fffffffu);
+      __syncwarp();
+      b.warpAdd();
+      if (lane == 0)
+        b.store(strayGrp + 2 * k);
     }
-    stray = __any_sync(0xffffffffu, stray);
     if (lane == 0)
     {
       groups[2 * k] = make_int4(x0, y0, x1, y1);
@@ -717,6 +871,27 @@ static GridArgs gridArgs(const wb_ctx *c)
     a.rootHi[k] = g.root_lo[k] + g.root_side;
   }
   a.unit = g.unit;
+  return a;
+}
+
+static StrayArgs strayArgs(const wb_ctx *c)
+{
+  StrayArgs a{};
+  const WbGeom &g = c->g;
+  a.leafId = (const uint32_t *)c->leafId.p;
+  a.leafKey = (const uint64_t *)c->leafKey.p;
+  a.leafLev = (const uint8_t *)c->leafLevel.p;
+  a.stray = (const uint8_t *)c->stray.p;
+  for (int k = 0; k < 3; k++)
+  {
+    a.off[k] = g.off[k];
+    a.scale[k] = g.scale[k];
+    a.rootLo[k] = g.root_lo[k];
+    a.imin[k] = c->grid.imin[k];
+    a.imax[k] = c->grid.imax[k];
+  }
+  a.unit = g.unit;
+  a.rootSide = g.root_side;
   return a;
 }
 
@@ -841,6 +1016,16 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
     c->grid.imin[k] = ext[k];
     c->grid.imax[k] = ext[3 + k];
   }
+  if (ns)
+  {
+    if ((rc = wb_ensure(c, c->strayCol, ncell * 32 + 64)) || (rc = wb_ensure(c, c->straySuper, nsup * 32 + 64)))
+      return rc;
+    { strayColumnKernel<<<(unsigned)std::min<uint64_t>((ncell * 32 + 255) / 256, (uint64_t)c->sm_count * 32), 256, 0, c->stream>>>(
+          ncell, strayArgs(c), cellRec, gpt, (int4 *)c->strayCol.p); ++c->launches; }
+    { straySuperKernel<<<(unsigned)std::min<uint64_t>((nsup + 255) / 256, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
+          nx, ny, snx, sny, cellRec, (const int4 *)c->superRec.p, (const int4 *)c->strayCol.p, (int4 *)c->straySuper.p); ++c->launches; }
+    WB_CUDA(c, cudaGetLastError());
+  }
   return 0;
 }
 
@@ -896,7 +1081,7 @@ int wb_point_groups(wb_ctx *c, const unsigned long long **taken, uint64_t *maxGr
   if (c->grid.grouped)
     return 0;
   int rc;
-  if ((rc = wb_ensure(c, c->groups, most * 36 + 64)))
+  if ((rc = wb_ensure(c, c->groups, most * 36 + 64)) || (c->grid.nStray && (rc = wb_ensure(c, c->strayGrp, most * 32 + 64))))
     return rc;
   WB_CUDA(c, cudaMemsetAsync(gTot, 0, 16, c->stream));
   if (nd)
@@ -908,7 +1093,8 @@ int wb_point_groups(wb_ctx *c, const unsigned long long **taken, uint64_t *maxGr
           (const int4 *)c->cellRec.p, (int4 *)c->superRec.p, (const int4 *)c->gpt.p, (int2 *)c->gKey0.p,
           (int2 *)c->gKey1.p, (int4 *)c->groups.p, most, gTot); ++c->launches; }
     { groupBoxKernel<<<(unsigned)std::min<uint64_t>((nd / 32 + 8) / 8, (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-          gridArgs(c), gTot, (const int2 *)c->gKey0.p, (const int2 *)c->gKey1.p, (int4 *)c->groups.p); ++c->launches; }
+          strayArgs(c), gTot, (const int2 *)c->gKey0.p, (const int2 *)c->gKey1.p, (int4 *)c->groups.p,
+          (int4 *)c->strayGrp.p); ++c->launches; }
     WB_CUDA(c, cudaGetLastError());
   }
   c->grid.grouped = true;

@@ -88,6 +88,11 @@ struct wb_ctx
      {x0, y0, x1, y1} and {zmin, begin, end, flags}, x0 == INT32_MAX for an
      empty column; superRec the same two int4 per super-cell */
   DevBuf gKey0, gKey1, gVal0, gVal1, stray, cellStart, gpt, cellRec, superRec, ptSetup;
+  /* blocks of the points outside the root cube, per column, super-cell and point
+     group that holds one beside or above it (its flags say so): two int4 each,
+     the blocks' {x0, y0, x1, y1} and {lowest top, lowest bottom, a column's have
+     one block, 0} in record integers; made when the cloud has outside points */
+  DevBuf strayCol, straySuper, strayGrp;
   DevBuf groups;                    /* point groups: two int4 each; their points are in gKey0 and gKey1 */
   DevBuf colGroups, groupCnt;       /* column groups {column, first point}, formed when margins are wanted */
   GridInfo grid;

@@ -64,6 +64,7 @@ struct GridDev
   uint64_t ncell;
   const int4 *gpt;     /* int4 {X, Y, Z, position | stray bit} per point, column order */
   const uint32_t *leafId;
+  const int4 *strayCol;   /* two int4 per flagged column: its outside points' blocks */
 };
 
 /* Cylinder::in for one point, exactly as the reference evaluates it; points
@@ -164,15 +165,9 @@ __device__ __forceinline__ bool cellMeetsCyl(const TileArgs &a, const int4 &box,
 /* The same column test in the tile's FP32 frame, with the radius widened by
  * 2e-4 (relative) and 1e-4 (absolute, squared units): a superset of the FP64
  * test (the frame's rounding is about 1e-7 relative), so no column with a
- * member is skipped; an extra column only costs its points' tests.  A column
- * with a point outside the root cube (flags) is always read: the cylinder can
- * hold that point's block without reaching the point.  The bound and both fills
- * use this one test, so a tile never gathers more points than its bound
- * counted. */
-__device__ __forceinline__ bool cellMeets(const TileArgs &a, const TileFrame &f, const int4 &box, int flags)
+ * member is skipped; an extra column only costs its points' tests. */
+__device__ __forceinline__ bool boxMeetsTile(const TileArgs &a, const TileFrame &f, const int4 &box)
 {
-  if (flags)
-    return true;
   if (!a.fast)
     return cellMeetsCyl(a, box, f.cx, f.cy);
   const float ax = ((float)(box.x - f.qx0) - f.fx) * f.sx, bx = ((float)(box.z - f.qx0) - f.fx) * f.sx;
@@ -182,6 +177,17 @@ __device__ __forceinline__ bool cellMeets(const TileArgs &a, const TileFrame &f,
   const float dx = x0 > 0 ? x0 : (x1 < 0 ? -x1 : 0.f);
   const float dy = y0 > 0 ? y0 : (y1 < 0 ? -y1 : 0.f);
   return dx * dx + dy * dy <= f.r2hi * 1.0002f + 1e-8f;
+}
+
+/* Whether column c (its box and flags) may hold a member of the tile.  The
+ * cylinder can hold the block of a point outside the root cube without reaching
+ * the point, so a column with such points is read for their blocks too.  The
+ * bound and both fills use this one test, so a tile never gathers more points
+ * than its bound counted. */
+__device__ __forceinline__ bool cellMeets(const TileArgs &a, const GridDev &gd, const TileFrame &f, uint64_t c,
+                                          const int4 &box, int flags)
+{
+  return boxMeetsTile(a, f, box) || (flags && boxMeetsTile(a, f, gd.strayCol[2 * c]));
 }
 
 /* Entries of the huge tiles as sort keys: (huge tile rank << 32) | store
@@ -238,7 +244,7 @@ __global__ void gridBound(TileArgs a, GridDev gd, uint32_t *__restrict__ bound, 
       {
         uint64_t c = (uint64_t)j * gd.nx + i;
         int4 box = gd.cell2[2 * c], r1 = gd.cell2[2 * c + 1];
-        if (r1.y != r1.z && cellMeets(a, f, box, r1.w))
+        if (r1.y != r1.z && cellMeets(a, gd, f, c, box, r1.w))
           room += (uint32_t)(r1.z - r1.y);
       }
     bound[k] = room;
@@ -296,7 +302,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) gridFillWarp(TileArgs a, Grid
       const int4 box = gd.cell2[2 * c], r1 = gd.cell2[2 * c + 1];
       cb = (uint32_t)r1.y;
       ce = (uint32_t)r1.z;
-      meets = cb != ce && cellMeets(a, f, box, r1.w);
+      meets = cb != ce && cellMeets(a, gd, f, c, box, r1.w);
     }
     unsigned left = __ballot_sync(0xffffffffu, meets);
     const unsigned apart = __ballot_sync(0xffffffffu, cb != ce && !meets);
@@ -381,7 +387,7 @@ __global__ void __launch_bounds__(kFillThreads) gridFill(TileArgs a, GridDev gd,
       uint64_t c = (uint64_t)(f.j0 + q / nc) * gd.nx + f.i0 + q % nc;
       int4 box = gd.cell2[2 * c], r1 = gd.cell2[2 * c + 1];
       uint32_t b = (uint32_t)r1.y, e = (uint32_t)r1.z;
-      if (b == e || !cellMeets(a, f, box, r1.w))
+      if (b == e || !cellMeets(a, gd, f, c, box, r1.w))
         continue;
       for (uint32_t t = b + (threadIdx.x & 31); t < e; t += 32)
       {
@@ -1554,6 +1560,7 @@ int wb_scan_impl(wb_ctx *c, const wb_params *p)
   gd.cell2 = (const int4 *)c->cellRec.p;
   gd.gpt = (const int4 *)c->gpt.p;
   gd.leafId = (const uint32_t *)c->leafId.p;
+  gd.strayCol = (const int4 *)c->strayCol.p;
   uint32_t *tileN = (uint32_t *)c->tileN.p, *tileStart = (uint32_t *)c->tileStart.p;
   int32_t *owner = (int32_t *)c->owner.p;
   unsigned blocks = (unsigned)((T + kTileWarps - 1) / kTileWarps);
