@@ -278,7 +278,8 @@ __device__ __noinline__ BlockBounds blockBounds(const ClsArgs &a, uint32_t j, in
   return b;
 }
 
-/* STRAYS: some cloud of the launch has points outside the root cube. */
+/* STRAYS: some cloud of the launch has points beside or above the root cube (those
+ * below it are members by themselves, when their block meets the hyperboloid). */
 template <bool STRAYS>
 __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t group, int lane, GroupShared &sm)
 {
@@ -497,8 +498,8 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
     }
   };
   // the candidates of the staged group (first: its first point) that FP32
-  // could not decide, and those outside the root cube
-  auto testExact = [&](uint32_t first) {
+  // could not decide, and members outside the root cube
+  auto testExact = [&](uint32_t first, unsigned members) {
 #pragma unroll 1
     while (__any_sync(kAll, pend != 0))
     {
@@ -512,7 +513,9 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
         // dist(p,q) == 0 gives no direction (classify.cpp:142,153)
         if (dxi != 0 || dyi != 0)
         {
-          if (a.fp32Only && r.y >= 0)
+          if (STRAYS && (members & pend & (0u - pend)))
+            in = true;
+          else if (a.fp32Only && r.y >= 0)
           {
             const float dx = (float)dxi * a.fsx, dy = (float)dyi * a.fsy;
             const float zd = (float)(me.z - r.x) * a.fsz + a.setup[j].czp;
@@ -602,21 +605,16 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       reads++;
       // stage the group, with its octets' boxes
       float x = 0.f, y = 0.f, z = INFINITY;
-      bool stray = false;
-      BlockBounds block{};
+      int where = 0;   // store position and stray bit
       if (lane < r.z)
       {
         const int2 p = a.bxy[(uint32_t)r.y + lane], q = a.bzw[(uint32_t)r.y + lane];
         x = (float)(p.x - gx0);
         y = (float)(p.y - gy0);
         z = (float)(q.x - gz0);
-        if (STRAYS && q.y < 0)
-        {
-          stray = true;
-          block = blockBounds(a, (uint32_t)q.y & 0x7fffffffu, gx0, gy0, gz0);
-        }
+        where = q.y;
       }
-      const unsigned strays = STRAYS ? __ballot_sync(kAll, stray) : 0u;
+      const unsigned strays = __ballot_sync(kAll, where < 0);
       float x0 = z < INFINITY ? x : INFINITY, x1 = z < INFINITY ? x : -INFINITY;
       float y0 = z < INFINITY ? y : INFINITY, y1 = z < INFINITY ? y : -INFINITY, z0 = z;
 #pragma unroll
@@ -631,7 +629,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       __syncwarp();
       sm.cx[lane] = x;
       sm.cy[lane] = y;
-      sm.cz[lane] = stray ? -INFINITY : -z;   // not in the octets' test
+      sm.cz[lane] = where < 0 ? -INFINITY : -z;   // not in the octets' test
       if ((lane & 7) == 0)
       {
         sm.obox[lane >> 3] = boxOf(x0, x1, y0 * ky, y1 * ky);
@@ -639,9 +637,14 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
       }
       __syncwarp();
       const bool wasDone = done;
-      pend = 0;
+      pend = STRAYS || done ? 0u : strays;   // for the exact test
+      unsigned members = 0;   // of pend: members for certain
       if (STRAYS && strays)
       {
+        BlockBounds block{};
+        if (where < 0)
+          block = blockBounds(a, (uint32_t)where & 0x7fffffffu, gx0, gy0, gz0);
+        __syncwarp();
         // The points outside the root cube, one after another: a member's block
         // meets the lane's hyperboloid (its cube's nearest point at the bottom),
         // and either the point is inside or the block as a whole is (its farthest
@@ -673,10 +676,10 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
           const bool wanted = !done & arc & (rr > 0.f);
           const bool out = !may(hb + pz, nx - px, ny - py) || !(may(zd, fabsf(ex), fabsf(ey)) || may(ht + pz, fx - px, fy - py));
           const bool in = sure(hb - pz, nx + px, ny + py) && (sure(zd, fabsf(ex), fabsf(ey)) || sure(ht - pz, fx + px, fy + py));
-          if (wanted & !in & !out)
+          if (wanted & (in | !out))
             pend |= 1u << k;
-          if (__any_sync(kAll, wanted & in))
-            addAny(wanted & in, ex, ey, rr);
+          if (wanted & in)
+            members |= 1u << k;
         }
       }
 #pragma unroll 1
@@ -694,7 +697,7 @@ __device__ __forceinline__ void classifyGroupArcs(const ClsArgs &a, uint64_t gro
           WB_STAT(gst[8], clock64() - tB);
         }
       }
-      testExact((uint32_t)r.y);
+      testExact((uint32_t)r.y, members);
       if (__any_sync(kAll, done != wasDone))
       {
         if (__all_sync(kAll, done))
@@ -972,7 +975,7 @@ __device__ __forceinline__ void classifyPointArcs(const ClsArgs &a, uint64_t j, 
             const float rr = __fmaf_rn(ex, ex, ey * ey), w = zd * fabsf(zd);
             const bool arc = side * fminf(__fmaf_rn(ax, ey, -(ay * ex)), __fmaf_rn(ex, by, -(ey * bx))) > arcMin;
             // dist(p,q) == 0 gives no direction (classify.cpp:142,153)
-            const bool cand = (lane < n) & ((dxi != 0) | (dyi != 0)), stray = STRAYS && q.y < 0;
+            const bool cand = (lane < n) & ((dxi != 0) | (dyi != 0)), stray = q.y < 0;
             // points outside the root cube: in or not by their blocks too
             bool blockMeets = true, blockHolds = false;
             if (STRAYS && __shfl_sync(kAll, gr.w, gs))

@@ -175,7 +175,7 @@ __global__ void cellKernel(GridArgs g, const int32_t *__restrict__ sx, const int
       cell = (uint32_t)cy * (uint32_t)g.nx + cx;
       stray[j] = (uint8_t)((s ? 1 : 0) | (beside ? 2 : 0));
       if (s)
-        atomicAdd(nStray, 1ull);
+        atomicAdd(nStray, beside ? (1ull << 32) + 1 : 1ull);   // those beside or above in the upper half
     }
     // the point's place among its column's points: the store order is local,
     // so neighbouring lanes share columns and each run of them takes its
@@ -640,7 +640,7 @@ struct StrayArgs
   const uint64_t *leafKey;
   const uint8_t *leafLev;
   const uint8_t *stray;
-  double off[3], scale[3], unit, rootLo[3], rootSide;
+  double unitOff[3], perStep[3], rootLo[3], rootSide;   /* off * unit, 1 / (scale * unit) */
   int imin[3], imax[3];   /* the cloud's record integers */
 };
 
@@ -702,7 +702,7 @@ __device__ __noinline__ StrayBox strayBlock(const StrayArgs &a, uint32_t j)
 #pragma unroll
   for (int k = 0; k < 3; k++)
   {
-    const double p = ((c[k] - side / 2) / a.unit - a.off[k]) / a.scale[k], q = ((c[k] + side / 2) / a.unit - a.off[k]) / a.scale[k];
+    const double p = (c[k] - side / 2 - a.unitOff[k]) * a.perStep[k], q = (c[k] + side / 2 - a.unitOff[k]) * a.perStep[k];
     const double least = k < 2 ? (double)a.imin[k] : fmax((double)a.imin[k] - 536870912.0, -2147483648.0);
     lo[k] = (int)fmin(fmax(floor(fmin(p, q)) - 1, least), (double)a.imax[k]);
     hi[k] = (int)fmin(fmax(k < 2 ? ceil(fmax(p, q)) + 1 : floor(fmax(p, q)) - 1, least), (double)a.imax[k]);
@@ -718,7 +718,7 @@ __device__ __noinline__ StrayBox strayBlock(const StrayArgs &a, uint32_t j)
 }
 
 /* The records of the columns that hold points beside or above the root cube, of all
- * their points outside it; one warp each (run only for clouds with outside
+ * their points outside it; one warp each (run only for clouds with such
  * points). */
 __global__ void strayColumnKernel(uint64_t ncell, StrayArgs a, const int4 *__restrict__ rec, const int4 *__restrict__ gpt,
                                   int4 *__restrict__ out)
@@ -884,13 +884,12 @@ static StrayArgs strayArgs(const wb_ctx *c)
   a.stray = (const uint8_t *)c->stray.p;
   for (int k = 0; k < 3; k++)
   {
-    a.off[k] = g.off[k];
-    a.scale[k] = g.scale[k];
+    a.unitOff[k] = g.off[k] * g.unit;
+    a.perStep[k] = 1.0 / (g.scale[k] * g.unit);
     a.rootLo[k] = g.root_lo[k];
     a.imin[k] = c->grid.imin[k];
     a.imax[k] = c->grid.imax[k];
   }
-  a.unit = g.unit;
   a.rootSide = g.root_side;
   return a;
 }
@@ -1010,13 +1009,14 @@ int wb_grid_impl(wb_ctx *c, double x0, double y0, double x1, double y1)
   WB_CUDA(c, cudaGetLastError());
   c->grid.grouped = c->grid.colGrouped = false;
   c->grid.nColGroups = 0;
-  c->grid.nStray = ns;
+  c->grid.nStray = (uint32_t)ns;
+  c->grid.nBeside = ns >> 32;
   for (int k = 0; k < 3; k++)
   {
     c->grid.imin[k] = ext[k];
     c->grid.imax[k] = ext[3 + k];
   }
-  if (ns)
+  if (c->grid.nBeside)
   {
     if ((rc = wb_ensure(c, c->strayCol, ncell * 32 + 64)) || (rc = wb_ensure(c, c->straySuper, nsup * 32 + 64)))
       return rc;
@@ -1081,7 +1081,7 @@ int wb_point_groups(wb_ctx *c, const unsigned long long **taken, uint64_t *maxGr
   if (c->grid.grouped)
     return 0;
   int rc;
-  if ((rc = wb_ensure(c, c->groups, most * 36 + 64)) || (c->grid.nStray && (rc = wb_ensure(c, c->strayGrp, most * 32 + 64))))
+  if ((rc = wb_ensure(c, c->groups, most * 36 + 64)) || (c->grid.nBeside && (rc = wb_ensure(c, c->strayGrp, most * 32 + 64))))
     return rc;
   WB_CUDA(c, cudaMemsetAsync(gTot, 0, 16, c->stream));
   if (nd)

@@ -34,7 +34,7 @@ struct GridInfo
 {
   double x0 = 0, y0 = 0, cell = 1;
   int nx = 0, ny = 0;
-  uint64_t ncell = 0, nStray = 0;
+  uint64_t ncell = 0, nStray = 0, nBeside = 0;   /* points outside the root cube; of them beside or above it */
   int32_t imin[3] = {0, 0, 0}, imax[3] = {0, 0, 0};   /* record-integer extent of the cloud */
   /* super-cells: blocks of WB_SUPER x WB_SUPER columns with their own bounds */
   int snx = 0, sny = 0;
