@@ -719,7 +719,8 @@ __device__ __noinline__ StrayBox strayBlock(const StrayArgs &a, uint32_t j)
 
 /* The records of the columns that hold points beside or above the root cube, of all
  * their points outside it; one warp each (run only for clouds with such
- * points). */
+ * points).  Bound by the FP64 pipe: with straySuperKernel 0.08 ms for 52,000 such
+ * points of 1.56M (0.16 with divisions by the step). */
 __global__ void strayColumnKernel(uint64_t ncell, StrayArgs a, const int4 *__restrict__ rec, const int4 *__restrict__ gpt,
                                   int4 *__restrict__ out)
 {
